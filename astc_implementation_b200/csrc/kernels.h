@@ -178,14 +178,22 @@ __device__ __forceinline__ uchar4 src_rgba8(const BlockSrc& s, int bx, int t) {
     return s.img[(size_t)y * s.width + x];
 }
 
-// Texel t of the block, edge-clamped, as (v / 255) * 65536 (compression_pipeline.cpp:32-46).
-__device__ __forceinline__ float4 src_texel(const BlockSrc& s, int bx, int t) {
-    const int x = min(s.x0 + t % bx, s.width - 1);
-    const int y = min(s.y0 + t / bx, s.height - 1);
-    const uchar4 p = s.img[(size_t)y * s.width + x];
-    return make_float4(((float)p.x / 255.0f) * 65536.0f, ((float)p.y / 255.0f) * 65536.0f,
-                       ((float)p.z / 255.0f) * 65536.0f, ((float)p.w / 255.0f) * 65536.0f);
+// An RGBA8 texel as (v / 255) * 65536 (compression_pipeline.cpp:32-46), rounded as the
+// division and the product round: v times 65536 / 255 split in two (Brisebarre, Muller and
+// Raina, "Accelerating correctly rounded floating-point division when the divisor is known in
+// advance", 2004; equal for all 256 values).  2^23 + v has v as its low bits.
+__device__ __forceinline__ float texel_channel(uint32_t bits) {
+    const float v = __uint_as_float(bits) - 8388608.0f;
+    return __fmaf_rn(v, 0x1.010102p+8f, v * -0x1.fdfdfep-17f);
 }
+__device__ __forceinline__ float4 texel_float(uchar4 c) {
+    const uint32_t p = *reinterpret_cast<const uint32_t*>(&c);
+    return make_float4(texel_channel(__byte_perm(p, 0x4B000000u, 0x7650)), texel_channel(__byte_perm(p, 0x4B000000u, 0x7651)),
+                       texel_channel(__byte_perm(p, 0x4B000000u, 0x7652)), texel_channel(__byte_perm(p, 0x4B000000u, 0x7653)));
+}
+
+// Texel t of the block, edge-clamped, as (v / 255) * 65536.
+__device__ __forceinline__ float4 src_texel(const BlockSrc& s, int bx, int t) { return texel_float(src_rgba8(s, bx, t)); }
 
 // Destination of block blk's 16 bytes.
 __device__ __forceinline__ uint4* block_dst(const KernelArgs& a, int blk) {

@@ -11,6 +11,8 @@
 //                  counts (compression_pipeline.cpp:500-519), then the ASTC
 //                  physical block layout (code/physical_compression.cpp:843)
 //                  written straight to the 16-byte output block.
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -38,6 +40,18 @@ __device__ __forceinline__ int32_t ic(const I4& v, int c) { return c == 0 ? v.x 
 __device__ __forceinline__ I4 ivec(float4 v) { return {f2i(v.x), f2i(v.y), f2i(v.z), f2i(v.w)}; }
 __device__ __forceinline__ float4 rnev(float4 v) { return make_float4(rintf(v.x), rintf(v.y), rintf(v.z), rintf(v.w)); }
 __device__ __forceinline__ int32_t shl1(int32_t v) { return (int32_t)((uint32_t)v << 1); }
+
+// x / 257 for an endpoint clamped to [0, 65535], rounded to nearest: the product with the
+// reciprocal split in two (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", 2004), equal to the division
+// for every float of the range at or above 1e-33 (checked exhaustively).
+__device__ __forceinline__ float over257(float color) {
+    const float x = fminf(fmaxf(color, 0.0f), 65535.0f);
+    float r = __fmaf_rn(x, 0x1.fe01fep-9f, x * 0x1.fe01fep-41f);
+    if (x > 0.0f && x < 1e-30f) r = x / 257.0f;
+    return r;
+}
+__device__ __forceinline__ float4 over257(float4 c) { return make_float4(over257(c.x), over257(c.y), over257(c.z), over257(c.w)); }
 
 // ------------------------------------------------------------ pass14 colour endpoint packing
 struct Packer {
@@ -219,11 +233,12 @@ struct Packer {
         out[0] = l0be; out[1] = l1de; out[2] = a0be; out[3] = a1de;
         return true;
     }
-    // pack_color_endpoints_helper (pass14:917-1224)
-    __device__ __noinline__ uint32_t pack(float4 color0, float4 color1, float4 rgbs, uint32_t fmt, uint32_t q, uint32_t* out) const {
-        const float4 c0 = vmin(vmax(color0, mk(0.0f)), mk(65535.0f)) / mk(257.0f);
-        const float4 c1 = vmin(vmax(color1, mk(0.0f)), mk(65535.0f)) / mk(257.0f);
+    // pack_color_endpoints_helper (pass14:917-1224).  Returns the format (x) and the up to
+    // eight packed values, one byte each (y, then z).
+    __device__ __noinline__ uint4 pack(float4 color0, float4 color1, float4 rgbs, uint32_t fmt, uint32_t q) const {
+        const float4 c0 = over257(color0), c1 = over257(color1);
         float best = ERR_DEFAULT;
+        uint32_t out[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) out[i] = 0;
         uint32_t bf = FMT_LUMINANCE;
@@ -279,14 +294,13 @@ struct Packer {
             out[0] = qflt(q, f2i(rintf(l0)), l0); out[1] = qflt(q, f2i(rintf(l1)), l1);
             bf = FMT_LUMINANCE;
         }
-        return bf;
+        return make_uint4(bf, out[0] | out[1] << 8 | out[2] << 16 | out[3] << 24, out[4] | out[5] << 8 | out[6] << 16 | out[7] << 24, 0u);
     }
 };
 
-// pass15: decode packed endpoints of one partition, scaled by 257.
-__device__ __noinline__ void unpack_endpoints(uint32_t fmt, const uint8_t* v, uint16_t* e0, uint16_t* e1) {
-    I4 o0, o1;
-    auto I = [&](int k) { return (int32_t)v[k]; };
+// pass15: decode the packed endpoints (bytes of lo, then hi) of one partition to 0..255.
+__device__ __forceinline__ void unpack_endpoints(uint32_t fmt, uint32_t lo, uint32_t hi, I4& o0, I4& o1) {
+    auto I = [&](int k) { return (int32_t)(((k < 4 ? lo : hi) >> (8 * (k & 3))) & 0xFF); };
     switch (fmt) {
         case FMT_LUMINANCE_DELTA: {
             const int32_t l0 = (I(0) >> 2) | (I(1) & 0xC0), l1 = min(l0 + (I(1) & 0x3F), 255);
@@ -319,12 +333,11 @@ __device__ __noinline__ void unpack_endpoints(uint32_t fmt, const uint8_t* v, ui
         case FMT_RGBA_DELTA: Packer::delta_unpack({I(0), I(2), I(4), I(6)}, {I(1), I(3), I(5), I(7)}, o0, o1); break;
         default: o0 = {I(0), I(0), I(0), 255}; o1 = {I(1), I(1), I(1), 255}; break;
     }
-    e0[0] = (uint16_t)(o0.x * 257); e0[1] = (uint16_t)(o0.y * 257); e0[2] = (uint16_t)(o0.z * 257); e0[3] = (uint16_t)(o0.w * 257);
-    e1[0] = (uint16_t)(o1.x * 257); e1[1] = (uint16_t)(o1.y * 257); e1[2] = (uint16_t)(o1.z * 257); e1[3] = (uint16_t)(o1.w * 257);
 }
 
 // ------------------------------------------------------------ k_refine
 constexpr int kRefineThreads = 128;
+constexpr int kRefineCtas = 5;
 
 // Candidate threads per partitioned block (the refinement top-N rounded up to a power of
 // two) and partitioned blocks per CTA: 16 x 8 for the full search; more, narrower ones when
@@ -336,24 +349,68 @@ __host__ __device__ inline int refine_pbs(int T, int topn) {
     return by_threads < by_smem ? by_threads : (by_smem > 16 ? by_smem : 16);
 }
 
-// A candidate's state in shared memory, kept at the candidate's staging position for all
-// iterations whichever thread runs it (73 words: an odd stride, so distinct candidates of a
-// warp mostly hit distinct banks).
-struct CandSmem {
-    uint16_t u0[4][4], u1[4][4];  // unpacked endpoints x257 (0..65535)
-    uint8_t qw[64];
-    uint8_t packed[32];
-    float ep[4][8];               // per partition: the least-squares endpoints ep0 (xyzw), ep1 (xyzw)
-    uint32_t item;                // partitioned block of this staging position (lb + 1 | slot << 27), 0 if none
+// Candidate state in shared memory, one slot per candidate a CTA runs, arrays of [row][slot]:
+// lanes on consecutive slots hit consecutive banks whatever rows they read.  A slot is the
+// candidate's rank in its group's initial order, so the first iteration's lanes are on
+// consecutive slots and the gathered ones of later iterations on increasing ones.
+//   ep   [8]      least-squares endpoints (float4): ep0 and ep1 of partition q in rows 2q, 2q + 1
+//   u    [4]      unpacked endpoints of partition q, 0..255 x 257, eight u16: ep0 xyzw, ep1 xyzw
+//   s    [T]      infilled weight of each texel times 16, 0..1024, exact in half precision
+//   qw   [max_w]  grid weights 0..64
+//   err           best error so far
+// The infilled weights are kept as sums of grid weight x (contribution x 16), small integers
+// that pass16 updates when it moves a weight; every use of one (pass13's weight s / 1024,
+// pass16's s / 16, pass17's rounded s / 16) is the exact value the passes' own sums of
+// products give, since those sums are exact too.  Before, each texel's four table entries
+// and weights were read again at every use (about 45 instructions, two to three uses per
+// texel and iteration in pass13 and pass17 and one per texel of each weight in pass16).
+// Measured with pass13's walk in partition order (B200): full search of 1024x1024 at 4x4 50.2 -> 47.5 ms,
+// of 64x64 1.08 -> 0.90 ms; proposal search of 2047x2050 at 6x6 8.98 -> 8.13 ms.
+constexpr int kSlotRow16 = kRefineThreads * 16;  // bytes of a row of 16-byte elements
+constexpr int kSlotRow4 = kRefineThreads * 4;    // of two s or four qw
+struct RefineLayout {
+    int ep, u, s, qw, err, item, pos, px, part, sdir, keys, aux, total;
 };
-static_assert(sizeof(CandSmem) == 292, "odd word stride");
-__device__ __forceinline__ float4 ld_ep(const float* e) { return make_float4(e[0], e[1], e[2], e[3]); }
-__device__ __forceinline__ void st_ep(float* e, float4 v) { e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w; }
-__device__ __forceinline__ uint4 ld_u4(const uint8_t* p) {  // 4-byte aligned shared memory
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
-    return make_uint4(w[0], w[1], w[2], w[3]);
+// Texel rows of the staged partitioned blocks, an odd number of banks (or 16-byte bank groups)
+// apart: a warp's candidates, sorted by path, belong to different partitioned blocks.
+__host__ __device__ inline int px_row_bytes(int T, bool u8) { return u8 ? (T | 1) * 4 : (T + 1) * 16; }
+__host__ __device__ inline int part_row_bytes(int T, int width) { return ((T * width + 3) / 4 | 1) * 4; }
+// rows: staged partitioned blocks (the tail stages one per slot, with partition bytes).
+__host__ __device__ inline RefineLayout refine_layout(int T, int max_w, int rows, bool u8, bool tail) {
+    RefineLayout f;
+    int o = 0;
+    auto take = [&](int bytes) { const int r = o; o += (bytes + 15) & ~15; return r; };
+    f.ep = take(8 * kSlotRow16);
+    f.u = take(4 * kSlotRow16);
+    f.s = take((T + 1) / 2 * kSlotRow4);
+    f.qw = take((max_w + 3) / 4 * kSlotRow4);
+    f.err = take(kRefineThreads * 4);
+    f.item = take(kRefineThreads * 4);
+    f.pos = take(kRefineThreads);
+    f.px = take(rows * px_row_bytes(T, u8));
+    f.part = take(rows * part_row_bytes(T, u8 && !tail ? 2 : 1));
+    f.sdir = take(tail ? 0 : rows * 64);
+    f.keys = take(kRefineThreads * 4);
+    f.aux = take(tail ? kRefineThreads * 4 : rows * 4);
+    f.total = o;
+    return f;
 }
-
+struct Cand {  // one slot of the arrays above
+    uint8_t *epb, *ub, *sb, *qb;
+    float* err;
+    __device__ Cand(uint8_t* sm, const RefineLayout& f, int slot)
+        : epb(sm + f.ep + slot * 16), ub(sm + f.u + slot * 16), sb(sm + f.s + slot * 4), qb(sm + f.qw + slot * 4),
+          err(reinterpret_cast<float*>(sm + f.err) + slot) {}
+    __device__ __forceinline__ float4& ep(int i) const { return *reinterpret_cast<float4*>(epb + i * kSlotRow16); }
+    __device__ __forceinline__ uint4& u(int q) const { return *reinterpret_cast<uint4*>(ub + q * kSlotRow16); }
+    __device__ __forceinline__ __half& s(int t) const { return *reinterpret_cast<__half*>(sb + (t >> 1) * kSlotRow4 + (t & 1) * 2); }
+    __device__ __forceinline__ uint8_t& qw(int w) const { return qb[(w >> 2) * kSlotRow4 + (w & 3)]; }
+    __device__ __forceinline__ uint32_t& qw4(int i) const { return *reinterpret_cast<uint32_t*>(qb + i * kSlotRow4); }
+};
+// The u16 in the low (hi = false) or high half of v as a float: 2^23 + v has v as its low bits.
+__device__ __forceinline__ float u16f(uint32_t v, bool hi) { return __uint_as_float(__byte_perm(v, 0x4B000000u, hi ? 0x7632 : 0x7610)) - 8388608.0f; }
+// Round to the nearest integer, ties to even, for 0 <= v < 2^22 (rintf on the FP32 adders).
+__device__ __forceinline__ float rn_small(float v) { return (v + 8388608.0f) - 8388608.0f; }
 
 struct RTabs {
     const uint8_t* b;
@@ -371,38 +428,64 @@ struct RTabs {
     __device__ uint32_t prev_next(int q, int v) const { return reinterpret_cast<const uint16_t*>(b + L->off_prev_next)[q * 65 + v]; }
 };
 
-// Infilled weight of texel t from the 0..64 weights (pass13:165-184, pass17:127-146).
-// Padding entries of the dense list add qw[0]/64 * 0 = +0, which never changes v.
-__device__ __forceinline__ float undec_weight(const RTabs& tb, int dm, const uint8_t* qw, int t, bool direct) {
-    if (direct) return (float)qw[t] / 64.0f;
-    const uint64_t e4 = tb.tw4(dm, t);
-    float v = 0.0f;
+// Sets the candidate's infilled weights from its grid weights (pass13:165-184, pass17:127-146).
+// Padding entries of the dense list contribute 0.
+__device__ __forceinline__ void infill(const RTabs& tb, const Cand& c, int dm, int T, bool direct) {
+    for (int t = 0; t < T; t++) {
+        uint32_t v;
+        if (direct) {
+            v = (uint32_t)c.qw(t) * 16u;
+        } else {
+            const uint64_t e4 = tb.tw4(dm, t);
+            v = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const uint32_t e = (uint32_t)(e4 >> (16 * j)) & 0xFFFF;
-        v = v + ((float)qw[e & 0xFF] / 64.0f) * ((float)(e >> 8) * (1.0f / 16.0f));
+            for (int j = 0; j < 4; j++) { const uint32_t e = (uint32_t)(e4 >> (16 * j)) & 0xFFFF; v += (e >> 8) * (uint32_t)c.qw(e & 0xFF); }
+        }
+        c.s(t) = __ushort2half_rn((unsigned short)v);
     }
-    return v;
 }
 
-
 // A partitioned block's staged texels.  Up to 16 texels they are floats; larger blocks
-// stage RGBA8 (4 bytes a texel, so more CTAs fit on an SM) read back through the CTA's
-// table of (v / 255) * 65536, the value src_texel computes.
+// stage RGBA8 (4 bytes a texel, so more CTAs fit on an SM), converted where read.
 __host__ __device__ inline bool refine_u8(int T) { return T > 16; }
 template <bool U8> struct TexelRow;
 template <> struct TexelRow<true> {
     const uchar4* c;
-    const float* lut;
-    __device__ __forceinline__ float4 operator[](int t) const {
-        const uchar4 v = c[t];
-        return make_float4(lut[v.x], lut[v.y], lut[v.z], lut[v.w]);
-    }
+    __device__ __forceinline__ float4 operator[](int t) const { return texel_float(c[t]); }
 };
 template <> struct TexelRow<false> {
     const float4* c;
     __device__ __forceinline__ float4 operator[](int t) const { return c[t]; }
 };
+// Its partitioning: entry i holds texel i's partition and, in the low bits, the i-th texel in
+// (partition, texel) order, which pass13 walks one partition after another.
+template <class E> struct PartRow {
+    static constexpr int kShift = sizeof(E) == 1 ? 6 : 8;  // bytes for blocks of up to 64 texels
+    E* v;
+    __device__ __forceinline__ int part(int t) const { return v[t] >> kShift; }
+    __device__ __forceinline__ int order(int i) const { return v[i] & ((1 << kShift) - 1); }
+    // prow: the partitioning's row of texel partitions (null: one partition); one thread
+    __device__ __forceinline__ void set(const uint8_t* prow, const uint8_t* counts, int T) const {
+        uint32_t next = 0;  // next position of each partition, a byte each
+        if (prow) next = (uint32_t)counts[0] << 8 | ((uint32_t)counts[0] + counts[1]) << 16 | ((uint32_t)counts[0] + counts[1] + counts[2]) << 24;
+        for (int t = 0; t < T; t++) v[t] = prow ? (E)((int)prow[t] << kShift) : (E)0;
+        for (int t = 0; t < T; t++) {
+            const int sh = prow ? 8 * (int)prow[t] : 0;
+            const int i = (next >> sh) & 0xFF;
+            v[i] = (E)(v[i] | t);
+            next += 1u << sh;
+        }
+    }
+};
+// Direction of the partition's average colour (pass13's scale direction), the same for every
+// candidate and iteration of a partitioned block.
+__device__ __forceinline__ float4 scale_dir(float4 avg, float ps) {
+    const float4 cw = chan_w();
+    const float4 rsum = (avg * ps) * cw;
+    const float4 rws = vmax(cw * ps, mk(1e-17f));
+    float4 sv = rsum / rws; sv.w = 0.0f;
+    return normalize4(sv);
+}
 
 // One refinement iteration (passes 13-17) of candidate k of a partitioned block, its
 // state in cs; iteration 0 first loads the front's initial state.  Returns whether pass16
@@ -411,151 +494,179 @@ template <> struct TexelRow<false> {
 // degenerate keep the previous values, which are these), so packing, unpacking, realignment
 // and the final error repeat exactly and can never lower the error: stopping there gives
 // the result of running the remaining iterations.
-template <class Row>
-__device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, int k, const Row px, const uint8_t* tp,
-                            CandSmem& cs, Snap* snap, const int it) {
+template <class Row, class Part, class SDir>
+__device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, int k, const Row px, const Part pt, const SDir sdir_of,
+                            const Cand cs, Snap* snap, const int it) {
     const RTabs tb{a.tables, &a.L};
     const int T = a.L.T;
     const CandInit& ci = rec.c[k];
     const DevBm bm = tb.bm(ci.bm);
     const DevDm dmi = tb.dm(bm.dm);
-    const bool direct = dmi.W == T;
+    const int W = dmi.W;
+    const bool direct = W == T;
     const float4 cw = chan_w();
     const float lsw = (cw.x + cw.y) + cw.z;
     const Packer pk{a.tables + a.L.off_cu2u};
     float4 rgbs[4];
-    uint8_t packed_mod[32];
+    uint2 packed[4], packed_mod[4];
     if (it == 0) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) { st_ep(cs.ep[q], rec.ep0[q]); st_ep(cs.ep[q] + 4, rec.ep1[q]); }
+        for (int q = 0; q < 4; q++) { cs.ep(2 * q) = rec.ep0[q]; cs.ep(2 * q + 1) = rec.ep1[q]; }
         const uint32_t* src = reinterpret_cast<const uint32_t*>(ci.qw);  // 8-byte aligned in PBRec
-        uint32_t* dst = reinterpret_cast<uint32_t*>(cs.qw);
-#pragma unroll
-        for (int w = 0; w < 16; w++) dst[w] = src[w];
+        for (int w = 0; w < (W + 3) / 4; w++) cs.qw4(w) = src[w];
+        *cs.err = ERR_DEFAULT;
+        infill(tb, cs, bm.dm, T, direct);
     }
     uint32_t ffmt[4] = {0, 0, 0, 0}, matched = 0, final_q = ci.ql;
-    // infilled weights are recomputed where read: caching them per thread in shared memory
-    // costs more resident CTAs than the recomputation
-    auto UW = [&](int t) { return undec_weight(tb, bm.dm, cs.qw, t, direct); };
 
+    // The texel's partition endpoints change only with the partition, so they are read again
+    // only when it does (never, for one partition).  A decoded channel is floor(v + 1/2) of
+    // v = u0 + (u1 - u0) w1 / 64, the integer (u0 w0 + u1 w1 + 32) >> 6: v is a multiple of 1/64
+    // below 2^16, so v + 1/128 is exact and rounds to that integer.
     auto final_error = [&]() {
         float total = 0.0f;
+        float4 base = mk(0.0f), offs = mk(0.0f);
+        int pc = -1;
         for (int t = 0; t < T; t++) {
-            const int p = tp[t];
-            const float w = UW(t);
-            const int32_t w1 = f2i(rintf(w * 64.0f)), w0 = 64 - w1;
+            const int p = pt.part(t);
+            if (p != pc) {
+                const uint4 u = cs.u(p);
+                base = make_float4(u16f(u.x, false), u16f(u.x, true), u16f(u.y, false), u16f(u.y, true));
+                offs = (make_float4(u16f(u.z, false), u16f(u.z, true), u16f(u.w, false), u16f(u.w, true)) - base) * (1.0f / 64.0f);
+                base = base + mk(1.0f / 128.0f);
+                pc = p;
+            }
+            const float w1 = rn_small(__half2float(cs.s(t)) * (1.0f / 16.0f));
             const float4 x = px[t];
             float4 d;
-            d.x = x.x - (float)((((int32_t)cs.u0[p][0] * w0) + ((int32_t)cs.u1[p][0] * w1) + 32) >> 6);
-            d.y = x.y - (float)((((int32_t)cs.u0[p][1] * w0) + ((int32_t)cs.u1[p][1] * w1) + 32) >> 6);
-            d.z = x.z - (float)((((int32_t)cs.u0[p][2] * w0) + ((int32_t)cs.u1[p][2] * w1) + 32) >> 6);
-            d.w = x.w - (float)((((int32_t)cs.u0[p][3] * w0) + ((int32_t)cs.u1[p][3] * w1) + 32) >> 6);
-            d = vmin(make_float4(fabsf(d.x), fabsf(d.y), fabsf(d.z), fabsf(d.w)), mk(1e15f));
-            total = total + fminf(dot4(d * d, cw), ERR_DEFAULT);
+            d.x = x.x - rn_small(base.x + offs.x * w1);
+            d.y = x.y - rn_small(base.y + offs.y * w1);
+            d.z = x.z - rn_small(base.z + offs.z * w1);
+            d.w = x.w - rn_small(base.w + offs.w * w1);
+            total = total + dot4(d * d, cw);
         }
-        if (total < snap->err) {  // the snapshot's error is the best so far (ERR_DEFAULT at first)
+        if (total < *cs.err) {  // the best so far (ERR_DEFAULT at first)
+            *cs.err = total;
             uint4* d = reinterpret_cast<uint4*>(snap);  // 16-byte aligned: 112-byte records
             d[0] = make_uint4(__float_as_uint(total), (uint32_t)ci.bm | final_q << 16 | matched << 24,
                               ffmt[0] | ffmt[1] << 8 | ffmt[2] << 16 | ffmt[3] << 24, 0u);
-            d[1] = ld_u4(cs.packed); d[2] = ld_u4(cs.packed + 16);
-#pragma unroll
-            for (int i = 0; i < 4; i++) d[3 + i] = ld_u4(cs.qw + 16 * i);
+            d[1] = make_uint4(packed[0].x, packed[0].y, packed[1].x, packed[1].y);
+            d[2] = make_uint4(packed[2].x, packed[2].y, packed[3].x, packed[3].y);
+            const int nw = (W + 3) / 4;
+            for (int i = 0; i < 4; i++) {
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (4 * i < nw) v.x = cs.qw4(4 * i);
+                if (4 * i + 1 < nw) v.y = cs.qw4(4 * i + 1);
+                if (4 * i + 2 < nw) v.z = cs.qw4(4 * i + 2);
+                if (4 * i + 3 < nw) v.w = cs.qw4(4 * i + 3);
+                d[3 + i] = v;
+            }
         }
     };
 
     // ---------------- pass13: least-squares endpoints from the current weights
+    int i0 = 0;  // the partition's first texel in partition order
 #pragma unroll 1
     for (int q = 0; q < P; q++) {
-        const float ps = P == 1 ? (float)T : (float)tb.part_count(P, rec.entry, q);
-        const float4 rsum = (rec.avg[q] * ps) * cw;
-        const float4 rws = vmax(cw * ps, mk(1e-17f));
-        float4 sv = rsum / rws; sv.w = 0.0f;
-        const float4 sdir = normalize4(sv);
+        const int n = P == 1 ? T : tb.part_count(P, rec.entry, q);
+        const float ps = (float)n;
+        // the scale direction and its sums are only read by the formats with a scale
+        const bool scale = ci.fmt[q] == FMT_RGB_SCALE || ci.fmt[q] == FMT_RGB_SCALE_ALPHA;
+        const float4 sdir = scale ? sdir_of(q, ps) : mk(0.0f);
         float wmin = 1.0f, wmax = 0.0f, ls = 0.0f, ms = 0.0f, rs = 0.0f, smin = 1e10f, smax = 0.0f, sv0 = 0.0f, sv1 = 0.0f;
         float4 cx = mk(0.0f), cy = mk(0.0f);
-        for (int t = 0; t < T; t++) {
-            if (tp[t] != q) continue;
+        for (int i = i0; i < i0 + n; i++) {
+            const int t = pt.order(i);
             const float4 rgba = px[t];
-            const float w = UW(t);
-            if (w < wmin) wmin = w;
-            if (w > wmax) wmax = w;
-            const float sc = dot3(rgba, sdir);
-            if (sc < smin) smin = sc;
-            if (sc > smax) smax = sc;
+            const float w = __half2float(cs.s(t)) * (1.0f / 1024.0f);
+            wmin = fminf(wmin, w);
+            wmax = fmaxf(wmax, w);
             const float om = 1.0f - w;
             ls = ls + om * om; ms = ms + om * w; rs = rs + w * w;
             const float4 cyc = rgba * w;
             cy = cy + cyc;
             cx = cx + (rgba - cyc);
-            sv0 = sv0 + (om * sc) * lsw;
-            sv1 = sv1 + (w * sc) * lsw;
+            if (scale) {
+                const float sc = dot3(rgba, sdir);
+                if (sc < smin) smin = sc;
+                if (sc > smax) smax = sc;
+                sv0 = sv0 + (om * sc) * lsw;
+                sv1 = sv1 + (w * sc) * lsw;
+            }
         }
+        i0 += n;
         const float4 colx = cx * cw, coly = cy * cw;
         const float4 lv = mk(ls) * cw, mv = mk(ms) * cw, rv = mk(rs) * cw;
-        const float lx = ls * lsw, my = ms * lsw, rz = rs * lsw;
-        const float scalediv = clampf(smin / fmaxf(smax, 1e-10f), 0.0f, 1.0f);
-        const float4 sds = sdir * smax;
-        rgbs[q] = make_float4(sds.x, sds.y, sds.z, scalediv);
-        float4 e0 = ld_ep(cs.ep[q]), e1 = ld_ep(cs.ep[q] + 4);
+        float4 rg = mk(0.0f);
+        if (scale) {
+            const float scalediv = clampf(smin / fmaxf(smax, 1e-10f), 0.0f, 1.0f);
+            const float4 sds = sdir * smax;
+            rg = make_float4(sds.x, sds.y, sds.z, scalediv);
+        }
+        float4 e0 = cs.ep(2 * q), e1 = cs.ep(2 * q + 1);
         if (wmin >= wmax * 0.999f) {
             const float4 ac = (colx + coly) / vmax(cw * ps, mk(1e-17f));
             if (ac.x == ac.x) { e0.x = ac.x; e1.x = ac.x; }
             if (ac.y == ac.y) { e0.y = ac.y; e1.y = ac.y; }
             if (ac.z == ac.z) { e0.z = ac.z; e1.z = ac.z; }
             if (ac.w == ac.w) { e0.w = ac.w; e1.w = ac.w; }
-            rgbs[q] = make_float4(sds.x, sds.y, sds.z, 1.0f);
+            rg.w = 1.0f;
         } else {
             const float4 det = (lv * rv) - (mv * mv);
             const float4 rdet = mk(1.0f) / det;
-            const float lsdet = (lx * rz) - (my * my), lsrdet = 1.0f / lsdet;
             const float4 mss = ((lv * lv) + mk(2.0f) * (mv * mv)) + (rv * rv);
-            const float lsmss = ((lx * lx) + 2.0f * (my * my)) + (rz * rz);
             const float4 ne0 = ((rv * colx) - (mv * coly)) * rdet;
             const float4 ne1 = ((lv * coly) - (mv * colx)) * rdet;
             if (fabsf(det.x) > (mss.x * 1e-4f) && ne0.x == ne0.x && ne1.x == ne1.x) { e0.x = ne0.x; e1.x = ne1.x; }
             if (fabsf(det.y) > (mss.y * 1e-4f) && ne0.y == ne0.y && ne1.y == ne1.y) { e0.y = ne0.y; e1.y = ne1.y; }
             if (fabsf(det.z) > (mss.z * 1e-4f) && ne0.z == ne0.z && ne1.z == ne1.z) { e0.z = ne0.z; e1.z = ne1.z; }
             if (fabsf(det.w) > (mss.w * 1e-4f) && ne0.w == ne0.w && ne1.w == ne1.w) { e0.w = ne0.w; e1.w = ne1.w; }
-            const float se0 = ((rz * sv0) - (my * sv1)) * lsrdet;
-            const float se1 = ((lx * sv1) - (my * sv0)) * lsrdet;
-            if ((fabsf(lsdet) > (lsmss * 1e-4f)) && se0 == se0 && se1 == se1 && se0 < se1) {
-                const float4 sdsm = sdir * se1;
-                rgbs[q] = make_float4(sdsm.x, sdsm.y, sdsm.z, se0 / se1);
+            if (scale) {
+                const float lx = ls * lsw, my = ms * lsw, rz = rs * lsw;
+                const float lsdet = (lx * rz) - (my * my), lsrdet = 1.0f / lsdet;
+                const float lsmss = ((lx * lx) + 2.0f * (my * my)) + (rz * rz);
+                const float se0 = ((rz * sv0) - (my * sv1)) * lsrdet;
+                const float se1 = ((lx * sv1) - (my * sv0)) * lsrdet;
+                if ((fabsf(lsdet) > (lsmss * 1e-4f)) && se0 == se0 && se1 == se1 && se0 < se1) {
+                    const float4 sdsm = sdir * se1;
+                    rg = make_float4(sdsm.x, sdsm.y, sdsm.z, se0 / se1);
+                }
             }
         }
-        st_ep(cs.ep[q], e0); st_ep(cs.ep[q] + 4, e1);
+        rgbs[q] = rg;
+        cs.ep(2 * q) = e0; cs.ep(2 * q + 1) = e1;
     }
     // ---------------- pass14: pack at the trial quant level, then the "mod" level
     {
         bool all_same = ci.ql != ci.qlm;
-        uint32_t fn[4] = {0, 0, 0, 0}, vals[8];
-        for (int i = 0; i < 32; i++) cs.packed[i] = 0;
+        uint32_t fn[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int q = 0; q < 4; q++) packed[q] = make_uint2(0u, 0u);
 #pragma unroll 1
         for (int q = 0; q < P; q++) {
-            const uint32_t f = pk.pack(ld_ep(cs.ep[q]), ld_ep(cs.ep[q] + 4), rgbs[q], ci.fmt[q], ci.ql, vals);
+            const uint4 v = pk.pack(cs.ep(2 * q), cs.ep(2 * q + 1), rgbs[q], ci.fmt[q], ci.ql);
+            const uint32_t f = v.x;
             fn[0] = q == 0 ? f : fn[0]; fn[1] = q == 1 ? f : fn[1]; fn[2] = q == 2 ? f : fn[2]; fn[3] = q == 3 ? f : fn[3];
-#pragma unroll
-            for (int i = 0; i < 8; i++) cs.packed[q * 8 + i] = (uint8_t)vals[i];
+            packed[q] = make_uint2(v.y, v.z);
             if (q > 0) all_same = all_same && f == fn[0];
         }
         bool m = false;
         if (P >= 2 && all_same) {
             uint32_t fm[4] = {0, 0, 0, 0};
-            uint8_t* vm = packed_mod;
             bool same_mod = true;
 #pragma unroll 1
             for (int q = 0; q < P; q++) {
-                const uint32_t f = pk.pack(ld_ep(cs.ep[q]), ld_ep(cs.ep[q] + 4), rgbs[q], ci.fmt[q], ci.qlm, vals);
+                const uint4 v = pk.pack(cs.ep(2 * q), cs.ep(2 * q + 1), rgbs[q], ci.fmt[q], ci.qlm);
+                const uint32_t f = v.x;
                 fm[0] = q == 0 ? f : fm[0]; fm[1] = q == 1 ? f : fm[1]; fm[2] = q == 2 ? f : fm[2]; fm[3] = q == 3 ? f : fm[3];
-#pragma unroll
-                for (int i = 0; i < 8; i++) vm[q * 8 + i] = (uint8_t)vals[i];
+                packed_mod[q] = make_uint2(v.y, v.z);
                 if (q > 0 && f != fm[0]) { same_mod = false; break; }
             }
             if (same_mod) {
                 m = true;
 #pragma unroll
                 for (int q = 0; q < 4; q++) fn[q] = fm[q];
-                for (int i = 0; i < 32; i++) cs.packed[i] = i < P * 8 ? vm[i] : 0;
+                for (int q = 0; q < P; q++) packed[q] = packed_mod[q];
             }
         }
         matched = m ? 1 : 0;
@@ -565,28 +676,45 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     }
     // ---------------- pass15
 #pragma unroll 1
-    for (int q = 0; q < P; q++) unpack_endpoints(ffmt[q], cs.packed + q * 8, cs.u0[q], cs.u1[q]);
+    for (int q = 0; q < P; q++) {
+        I4 o0, o1;
+        unpack_endpoints(q == 0 ? ffmt[0] : q == 1 ? ffmt[1] : q == 2 ? ffmt[2] : ffmt[3], packed[q].x, packed[q].y, o0, o1);
+        cs.u(q) = make_uint4((uint32_t)(o0.x * 257) | (uint32_t)(o0.y * 257) << 16, (uint32_t)(o0.z * 257) | (uint32_t)(o0.w * 257) << 16,
+                             (uint32_t)(o1.x * 257) | (uint32_t)(o1.y * 257) << 16, (uint32_t)(o1.z * 257) | (uint32_t)(o1.w * 257) << 16);
+    }
     if (it == 0) final_error();
     // ---------------- pass16: move each weight one quant step if that lowers the error
     bool moved = false;
+    float4 base = mk(0.0f), offs = mk(0.0f);
+    int pc = -1;
+    auto endpoints = [&](int p) {  // of texel partition p, read again when it changes
+        if (p == pc) return;
+        const uint4 u = cs.u(p);
+        base = make_float4(u16f(u.x, false), u16f(u.x, true), u16f(u.y, false), u16f(u.y, true));
+        offs = (make_float4(u16f(u.z, false), u16f(u.z, true), u16f(u.w, false), u16f(u.w, true)) - base) * (1.0f / 64.0f);
+        pc = p;
+    };
     if (direct) {
         for (int t = 0; t < T; t++) {
-            const int p = tp[t];
-            const int32_t uqw = cs.qw[t];
+            const int32_t uqw = cs.qw(t);
             const uint32_t pn = tb.prev_next(bm.quant, uqw);
             const int32_t dn = pn & 0xFF, up = (pn >> 8) & 0xFF;
-            const float4 base = make_float4((float)cs.u0[p][0], (float)cs.u0[p][1], (float)cs.u0[p][2], (float)cs.u0[p][3]);
-            const float4 offs = make_float4((float)((int32_t)cs.u1[p][0] - (int32_t)cs.u0[p][0]), (float)((int32_t)cs.u1[p][1] - (int32_t)cs.u0[p][1]),
-                                            (float)((int32_t)cs.u1[p][2] - (int32_t)cs.u0[p][2]), (float)((int32_t)cs.u1[p][3] - (int32_t)cs.u0[p][3])) * (1.0f / 64.0f);
+            endpoints(pt.part(t));
             const float4 cd = (base + offs * (float)uqw) - px[t];
             const float4 cdd = cd + offs * (float)(dn - uqw), cdu = cd + offs * (float)(up - uqw);
             const float eb = dot4(cd * cd, cw), ed = dot4(cdd * cdd, cw), eu = dot4(cdu * cdu, cw);
-            if ((eu < eb) && (eu < ed) && (uqw < 64)) { cs.qw[t] = (uint8_t)up; moved |= up != uqw; }
-            else if ((ed < eb) && (uqw > 0)) { cs.qw[t] = (uint8_t)dn; moved |= dn != uqw; }
+            int32_t nw = uqw;
+            if ((eu < eb) && (eu < ed) && (uqw < 64)) nw = up;
+            else if ((ed < eb) && (uqw > 0)) nw = dn;
+            if (nw != uqw) {
+                moved = true;
+                cs.qw(t) = (uint8_t)nw;
+                cs.s(t) = __ushort2half_rn((unsigned short)(nw * 16));
+            }
         }
     } else {
-        for (int we = 0; we < dmi.W; we++) {
-            const int32_t uqw = cs.qw[we];
+        for (int we = 0; we < W; we++) {
+            const int32_t uqw = cs.qw(we);
             const uint32_t pn = tb.prev_next(bm.quant, uqw);
             const float dn = (float)(pn & 0xFF), up = (float)((pn >> 8) & 0xFF), ub = (float)uqw;
             const float ddn = dn - ub, dup = up - ub;
@@ -598,24 +726,25 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
                 const uint32_t we2 = tb.w2t(wbase + te);
                 const int t = we2 & 0xFF;
                 const float twb = (float)(we2 >> 8) * (1.0f / 16.0f);
-                const uint64_t e4 = tb.tw4(bm.dm, t);
-                float wb = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const uint32_t e = (uint32_t)(e4 >> (16 * j)) & 0xFFFF;
-                    wb = wb + (float)cs.qw[e & 0xFF] * ((float)(e >> 8) * (1.0f / 16.0f));
-                }
-                const int p = tp[t];
-                const float4 base = make_float4((float)cs.u0[p][0], (float)cs.u0[p][1], (float)cs.u0[p][2], (float)cs.u0[p][3]);
-                const float4 offs = make_float4((float)((int32_t)cs.u1[p][0] - (int32_t)cs.u0[p][0]), (float)((int32_t)cs.u1[p][1] - (int32_t)cs.u0[p][1]),
-                                                (float)((int32_t)cs.u1[p][2] - (int32_t)cs.u0[p][2]), (float)((int32_t)cs.u1[p][3] - (int32_t)cs.u0[p][3])) * (1.0f / 64.0f);
+                const float wb = __half2float(cs.s(t)) * (1.0f / 16.0f);
+                endpoints(pt.part(t));
                 const float4 cd = (base + offs * wb) - px[t];
                 const float4 cdd = cd + offs * (ddn * twb), cdu = cd + offs * (dup * twb);
                 ebv = ebv + cd * cd; edv = edv + cdd * cdd; euv = euv + cdu * cdu;
             }
             const float eb = dot4(ebv, cw), ed = dot4(edv, cw), eu = dot4(euv, cw);
-            if ((eu < eb) && (eu < ed) && (uqw < 64)) { cs.qw[we] = (uint8_t)up; moved |= (int32_t)up != uqw; }
-            else if ((ed < eb) && (uqw > 0)) { cs.qw[we] = (uint8_t)dn; moved |= (int32_t)dn != uqw; }
+            float dw = 0.0f;
+            if ((eu < eb) && (eu < ed) && (uqw < 64)) dw = dup;
+            else if ((ed < eb) && (uqw > 0)) dw = ddn;
+            if (dw != 0.0f) {
+                moved = true;
+                cs.qw(we) = (uint8_t)(uqw + (int)dw);
+                for (int te = 0; te < nt; te++) {
+                    const uint32_t we2 = tb.w2t(wbase + te);
+                    __half& sv = cs.s(we2 & 0xFF);
+                    sv = __float2half_rn(__half2float(sv) + dw * (float)(we2 >> 8));
+                }
+            }
         }
     }
     // In iteration 0 a pass16 that moved no weight leaves the weights and endpoints of the
@@ -624,39 +753,38 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     return moved;
 }
 
-// A refinement-tail entry: the partitioned block (lb * slots + slot), the candidate, the
-// next iteration, then the state an iteration carries over (endpoints, weights; the best
-// result so far is in the candidate's snapshot already).
-__device__ __forceinline__ void write_tail(const KernelArgs& a, const CandSmem& c, uint32_t pbi, int k, int it, int pos) {
+// A refinement-tail entry: the partitioned block (lb * slots + slot), the candidate and the
+// next iteration, the best error so far, then the state an iteration carries over (endpoints,
+// weights; the best result so far is in the candidate's snapshot already).
+__device__ __forceinline__ void write_tail(const KernelArgs& a, const Cand& c, uint32_t pbi, int k, int it, int pos) {
     uint4* e = a.tail + (size_t)pos * kTailWords;
-    e[0] = make_uint4(pbi, (uint32_t)k | (uint32_t)it << 8, 0u, 0u);
-    const uint8_t* ep = reinterpret_cast<const uint8_t*>(c.ep);
+    e[0] = make_uint4(pbi, (uint32_t)k | (uint32_t)it << 8, __float_as_uint(*c.err), 0u);
+    float4* ep = reinterpret_cast<float4*>(e + 1);
 #pragma unroll
-    for (int i = 0; i < 8; i++) e[1 + i] = ld_u4(ep + 16 * i);
-#pragma unroll
-    for (int i = 0; i < 4; i++) e[9 + i] = ld_u4(c.qw + 16 * i);
-}
-__device__ __forceinline__ void st_u4(uint8_t* p, uint4 v) {  // 4-byte aligned shared memory
-    uint32_t* w = reinterpret_cast<uint32_t*>(p);
-    w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    for (int i = 0; i < 8; i++) ep[i] = c.ep(i);
+    const int n4 = (a.L.max_w + 3) / 4;
+    uint32_t* w = reinterpret_cast<uint32_t*>(e + 9);
+    for (int i = 0; i < n4; i++) w[i] = c.qw4(i);
 }
 
 // CPB: candidate threads per partitioned block (refine_cpb of the launch's top-N), a
 // template parameter so that the full search's instance (8) keeps constant indexing.
-// U8: texels staged as RGBA8 (refine_u8).  Registers are capped for five resident CTAs
-// (the packer's call would otherwise raise the whole kernel's allocation).
+// U8: texels staged as RGBA8 (refine_u8).
 template <int CPB, bool U8>
-__global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_constant__ KernelArgs a) {
+__global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __grid_constant__ KernelArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int T = a.L.T;
     constexpr int cpb = CPB;
     const int pbs = CPB == 8 ? kRefineThreads / 8 : refine_pbs(T, CPB);
-    CandSmem* cs = reinterpret_cast<CandSmem*>(smem);
-    float* lut = reinterpret_cast<float*>(smem + sizeof(CandSmem) * kRefineThreads);
+    const RefineLayout fl = refine_layout(T, a.L.max_w, pbs, U8, false);
     using Px = typename std::conditional<U8, uchar4, float4>::type;
-    Px* pxs = reinterpret_cast<Px*>(U8 ? smem + sizeof(CandSmem) * kRefineThreads + 256 * 4 : smem + sizeof(CandSmem) * kRefineThreads);
-    uint8_t* tps = reinterpret_cast<uint8_t*>(pxs + pbs * T);
-    int* keys = reinterpret_cast<int*>(tps + ((pbs * T + 15) & ~15));
+    using Pe = typename std::conditional<U8, uint16_t, uint8_t>::type;
+    const int px_row = px_row_bytes(T, U8), part_row = part_row_bytes(T, sizeof(Pe));
+    uint32_t* item_of = reinterpret_cast<uint32_t*>(smem + fl.item);  // by slot: lb * slots + slot
+    uint8_t* pos_of = smem + fl.pos;                                  // by slot: staging position
+    uint32_t* staged = reinterpret_cast<uint32_t*>(smem + fl.aux);    // by staged partitioned block: lb + 1 | slot << 27, 0 if none
+    float4* sdirs = reinterpret_cast<float4*>(smem + fl.sdir);
+    int* keys = reinterpret_cast<int*>(smem + fl.keys);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // Items: every slot of every block in slot-major order (consecutive CTAs hold
     // partitioned blocks of the same slot, hence the same partition count, so
@@ -670,8 +798,6 @@ __global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_const
     __shared__ int spill_base;
     if (tid < 4) refined[tid] = 0;
     bool spill = a.tail != nullptr && T <= kTailMaxTexels;  // until the tail is found full
-    if (U8)
-        for (int v = tid; v < 256; v += kRefineThreads) lut[v] = ((float)v / 255.0f) * 65536.0f;  // as src_texel
     // (the first group's barrier below orders these writes before any read)
     for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
         {
@@ -684,7 +810,7 @@ __global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_const
                 if (a.pb_list) pb_item(a, li, lb, slot);
                 else { slot = li / nb; lb = li % nb; }
                 item = (uint32_t)(lb + 1) | ((uint32_t)slot << 27);
-                const PBRec& r = a.pbrec[lb * a.slots + slot];
+                const PBRec& r = a.pbrec[(size_t)lb * a.slots + slot];
                 if (k < (int)r.ncand) {
                     const int dm = reinterpret_cast<const DevBm*>(a.tables + a.L.off_bm)[r.c[k].bm].dm;
                     int fk = 0;
@@ -694,22 +820,25 @@ __global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_const
                 if (r.ncand > 0) {
                     const int P = r.P;
                     const uint8_t* prow = P > 1 ? a.tables + a.L.off_part_texel + ((size_t)(P - 2) * 1024 + r.entry) * T : nullptr;
+                    const uint8_t* counts = P > 1 ? a.tables + a.L.off_part_counts + ((size_t)(P - 2) * 1024 + r.entry) * 4 : nullptr;
                     const BlockSrc src = block_src(a, chunk_block(a, lb));
+                    Px* row = reinterpret_cast<Px*>(smem + fl.px + pbl * px_row);
                     for (int t = k; t < T; t += cpb) {
-                        if constexpr (U8) pxs[pbl * T + t] = src_rgba8(src, a.L.bx, t);
-                        else pxs[pbl * T + t] = src_texel(src, a.L.bx, t);
-                        tps[pbl * T + t] = P > 1 ? prow[t] : 0;
+                        if constexpr (U8) row[t] = src_rgba8(src, a.L.bx, t);
+                        else row[t] = src_texel(src, a.L.bx, t);
                     }
+                    if (k == 0) PartRow<Pe>{reinterpret_cast<Pe*>(smem + fl.part + pbl * part_row)}.set(prow, counts, T);
+                    for (int q = k; q < P; q += cpb) sdirs[pbl * 4 + q] = scale_dir(r.avg[q], (float)(P == 1 ? T : (int)counts[q]));
                 }
             }
             keys[tid] = key * kRefineThreads + tid;  // unique keys: P, formats, decimation mode, then position
-            cs[tid].item = item;  // of staging position tid
+            if (k == 0 && pbl < pbs) staged[pbl] = item;
         }
         __syncthreads();
         // Thread tid takes the candidate of rank tid in (partition count, endpoint formats,
         // decimation mode) order, so a warp's candidates mostly take the same packing path
-        // and share loop bounds and table rows.
-        int cand = -1;  // staging position of the candidate this thread runs
+        // and share loop bounds and table rows; the rank is also its slot.
+        int cand = -1;  // slot of the candidate this thread runs
         {
             const int kk = keys[tid];
             int rank = 0;
@@ -719,13 +848,15 @@ __global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_const
             __syncthreads();
             const int mine = keys[tid];
             const int pbl = mine / cpb, k = mine % cpb;
-            const uint32_t item = cs[pbl * cpb].item;
+            const uint32_t item = pbl < pbs ? staged[pbl] : 0u;
             if (item != 0) {
                 const int lb = (int)(item & 0x07FFFFFFu) - 1, slot = (int)(item >> 27);
                 const size_t pbi = (size_t)lb * a.slots + slot;
                 a.snaps[pbi * kNumCand + k].err = ERR_DEFAULT;  // inert slot unless refined below
                 if (k < (int)a.pbrec[pbi].ncand) {
-                    cand = mine;
+                    cand = tid;
+                    item_of[tid] = (uint32_t)pbi;
+                    pos_of[tid] = (uint8_t)mine;
                     if (a.work) atomicAdd(&refined[a.pbrec[pbi].P - 1], 1u);
                 }
             }
@@ -751,13 +882,7 @@ __global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_const
             const int rank = before + __popc(bal & ((1u << lane) - 1u));
             if (spill && it > 0 && nlive <= a.spill_live) {
                 // Few candidates left: hand them to the tail pass, which runs them densely, and
-                // take the next group instead of holding the CTA for them.  The item words are
-                // read before the barrier: after it, threads that are done stage the next group.
-                uint32_t pbi = 0;
-                if (live) {
-                    const uint32_t item = cs[(cand / cpb) * cpb].item;
-                    pbi = (uint32_t)((int)(item & 0x07FFFFFFu) - 1) * (uint32_t)a.slots + (item >> 27);
-                }
+                // take the next group instead of holding the CTA for them.
                 if (tid == 0) {
                     spill_base = atomicAdd(a.tail_count, nlive);
                     if (a.work) atomicAdd(a.work + 13, (unsigned long long)nlive);
@@ -765,9 +890,9 @@ __global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_const
                 __syncthreads();
                 const int sb = spill_base, pos = sb + rank;
                 if (sb + nlive <= a.tail_cap) {
-                    // (the next group's staging writes no candidate state: ep and qw are first
-                    // written by its iteration 0, after its barriers)
-                    if (live) write_tail(a, cs[cand], pbi, cand % cpb, it, pos);
+                    // (the next group's staging writes no slot state: it is first written after
+                    // its staging barriers)
+                    if (live) write_tail(a, Cand(smem, fl, cand), item_of[cand], pos_of[cand] % cpb, it, pos);
                     break;
                 }
                 if (live && pos < a.tail_cap) a.tail[(size_t)pos * kTailWords].x = 0xFFFFFFFFu;  // reserved, left empty
@@ -777,15 +902,14 @@ __global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_const
             __syncthreads();
             cand = tid < nlive ? keys[tid] : -1;
             if (cand >= 0) {
-                const int pbl = cand / cpb, k = cand % cpb;
-                const uint32_t item = cs[pbl * cpb].item;
-                const int lb = (int)(item & 0x07FFFFFFu) - 1, slot = (int)(item >> 27);
-                const size_t pbi = (size_t)lb * a.slots + slot;
+                const int pbl = pos_of[cand] / cpb, k = pos_of[cand] % cpb;
+                const size_t pbi = item_of[cand];
                 const PBRec& rec = a.pbrec[pbi];
                 Snap* snap = &a.snaps[pbi * kNumCand + k];
-                bool moved;
-                if constexpr (U8) moved = refine_step(a, rec, (int)rec.P, k, TexelRow<true>{pxs + pbl * T, lut}, tps + pbl * T, cs[cand], snap, it);
-                else moved = refine_step(a, rec, (int)rec.P, k, TexelRow<false>{pxs + pbl * T}, tps + pbl * T, cs[cand], snap, it);
+                const TexelRow<U8> row{reinterpret_cast<const Px*>(smem + fl.px + pbl * px_row)};
+                const PartRow<Pe> part{reinterpret_cast<Pe*>(smem + fl.part + pbl * part_row)};
+                const float4* sd = sdirs + pbl * 4;
+                const bool moved = refine_step(a, rec, (int)rec.P, k, row, part, [&](int q, float) { return sd[q]; }, Cand(smem, fl, cand), snap, it);
                 if (!moved || it + 1 >= iters) cand = -1;
             }
             // (the next pass's first barrier orders this iteration's state writes before
@@ -795,9 +919,8 @@ __global__ void __launch_bounds__(kRefineThreads, 5) k_refine(const __grid_const
     if (a.work && tid < 4 && refined[tid]) atomicAdd(a.work + 6 + tid, (unsigned long long)refined[tid]);
 }
 
-// The candidates k_refine handed over, one per thread with its own staged texels (RGBA8
-// through the table of src_texel's values, so every texel value is the same), iterated
-// with the same gathering of live candidates onto the lowest threads.  The CTAs stay
+// The candidates k_refine handed over, one per thread with its own staged texels (RGBA8),
+// iterated with the same gathering of live candidates onto the lowest threads.  The CTAs stay
 // resident: a CTA's 128 slots are refilled whenever at most kTailRefillAt of them hold a
 // live candidate, each warp claiming list entries for its own free slots from
 // tail_count[1], and the new candidates join the live list behind the running ones.  (Fixed
@@ -807,19 +930,17 @@ constexpr int kTailRefillAt = 64;
 __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const __grid_constant__ KernelArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int T = a.L.T;
-    CandSmem* cs = reinterpret_cast<CandSmem*>(smem);
-    float* lut = reinterpret_cast<float*>(smem + sizeof(CandSmem) * kRefineThreads);
-    uchar4* pxs = reinterpret_cast<uchar4*>(smem + sizeof(CandSmem) * kRefineThreads + 256 * 4);
-    uint8_t* tps = reinterpret_cast<uint8_t*>(pxs + kRefineThreads * T);
-    int* keys = reinterpret_cast<int*>(tps + ((kRefineThreads * T + 15) & ~15));
-    int* next_it = keys + kRefineThreads;                                  // by slot
-    uint32_t* pbi_of = reinterpret_cast<uint32_t*>(next_it + kRefineThreads);  // by slot
+    const RefineLayout fl = refine_layout(T, a.L.max_w, kRefineThreads, true, true);
+    const int px_row = px_row_bytes(T, true), part_row = part_row_bytes(T, 1);
+    int* keys = reinterpret_cast<int*>(smem + fl.keys);
+    int* next_it = reinterpret_cast<int*>(smem + fl.aux);             // by slot
+    uint32_t* pbi_of = reinterpret_cast<uint32_t*>(smem + fl.item);   // by slot
+    uint8_t* k_of = smem + fl.pos;                                    // by slot: the candidate
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned below = (1u << lane) - 1u;
     __shared__ int live_in_warp[kRefineThreads / 32], new_in_warp[kRefineThreads / 32];
     __shared__ uint8_t busy[kRefineThreads];  // slot holds a candidate that has not ended
     __shared__ int dry_flag;                  // the list has no unclaimed entry left
-    for (int v = tid; v < 256; v += kRefineThreads) lut[v] = ((float)v / 255.0f) * 65536.0f;  // as src_texel
     busy[tid] = 0;
     if (tid == 0) dry_flag = 0;
     const int total = min(*a.tail_count, a.tail_cap);
@@ -839,7 +960,7 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
             nlive += n;
             before += w < warp ? n : 0;
         }
-        int nnew = 0, new_before = 0, staged = -1;
+        int nnew = 0, new_before = 0, filled = -1;
         unsigned bnew = 0;
         if (!dry && nlive <= kTailRefillAt) {
             // Thread tid stages into slot tid when that slot is free and its warp's claim
@@ -858,24 +979,30 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
                 if (h.x != 0xFFFFFFFFu) {
                     const int lb = (int)(h.x / (uint32_t)a.slots);
                     const PBRec& r = a.pbrec[h.x];
-                    const int P = (int)r.P;
+                    const int P = (int)r.P, k = (int)(h.y & 0xFF);
                     const uint8_t* prow = P > 1 ? a.tables + a.L.off_part_texel + ((size_t)(P - 2) * 1024 + r.entry) * T : nullptr;
+                    const uint8_t* counts = P > 1 ? a.tables + a.L.off_part_counts + ((size_t)(P - 2) * 1024 + r.entry) * 4 : nullptr;
                     const BlockSrc src = block_src(a, chunk_block(a, lb));
-                    for (int t = 0; t < T; t++) {
-                        pxs[tid * T + t] = src_rgba8(src, a.L.bx, t);
-                        tps[tid * T + t] = P > 1 ? prow[t] : 0;
-                    }
-                    uint8_t* ep = reinterpret_cast<uint8_t*>(cs[tid].ep);
-                    for (int i = 0; i < 8; i++) st_u4(ep + 16 * i, e[1 + i]);
-                    for (int i = 0; i < 4; i++) st_u4(cs[tid].qw + 16 * i, e[9 + i]);
-                    cs[tid].item = h.y & 0xFF;  // the candidate
+                    uchar4* row = reinterpret_cast<uchar4*>(smem + fl.px + tid * px_row);
+                    for (int t = 0; t < T; t++) row[t] = src_rgba8(src, a.L.bx, t);
+                    PartRow<uint8_t>{smem + fl.part + tid * part_row}.set(prow, counts, T);
+                    const Cand c(smem, fl, tid);
+                    for (int i = 0; i < 8; i++) c.ep(i) = reinterpret_cast<const float4*>(e + 1)[i];
+                    const int n4 = (a.L.max_w + 3) / 4;
+                    const uint32_t* w = reinterpret_cast<const uint32_t*>(e + 9);
+                    for (int i = 0; i < n4; i++) c.qw4(i) = w[i];
+                    *c.err = __uint_as_float(h.z);
+                    const RTabs tb{a.tables, &a.L};
+                    const int dm = tb.bm(r.c[k].bm).dm;
+                    infill(tb, c, dm, T, tb.dm(dm).W == T);
+                    k_of[tid] = (uint8_t)k;
                     next_it[tid] = (int)((h.y >> 8) & 0xFF);
                     pbi_of[tid] = h.x;
                     busy[tid] = 1;
-                    staged = tid;
+                    filled = tid;
                 }
             }
-            bnew = __ballot_sync(0xFFFFFFFFu, staged >= 0);
+            bnew = __ballot_sync(0xFFFFFFFFu, filled >= 0);
             if (lane == 0) new_in_warp[warp] = __popc(bnew);
             __syncthreads();  // the staged slots, the new counts and the flag
 #pragma unroll
@@ -892,15 +1019,18 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
             continue;  // every claimed entry was a reservation left empty: claim again
         }
         if (live) keys[before + __popc(bal & below)] = cand;
-        if (staged >= 0) keys[nlive + new_before + __popc(bnew & below)] = staged;
+        if (filled >= 0) keys[nlive + new_before + __popc(bnew & below)] = filled;
         __syncthreads();
         cand = tid < n ? keys[tid] : -1;
         if (cand >= 0) {
             const uint32_t pbi = pbi_of[cand];
-            const int k = (int)cs[cand].item, it = next_it[cand];
+            const int k = (int)k_of[cand], it = next_it[cand];
             const PBRec& rec = a.pbrec[pbi];
             Snap* snap = &a.snaps[(size_t)pbi * kNumCand + k];
-            const bool moved = refine_step(a, rec, (int)rec.P, k, TexelRow<true>{pxs + cand * T, lut}, tps + cand * T, cs[cand], snap, it);
+            const TexelRow<true> row{reinterpret_cast<const uchar4*>(smem + fl.px + cand * px_row)};
+            const PartRow<uint8_t> part{smem + fl.part + cand * part_row};
+            const bool moved = refine_step(a, rec, (int)rec.P, k, row, part, [&](int q, float ps) { return scale_dir(rec.avg[q], ps); },
+                                           Cand(smem, fl, cand), snap, it);
             next_it[cand] = it + 1;
             if (!moved || it + 1 >= iters) {
                 busy[cand] = 0;  // released: read by the next refill, after the next barrier
@@ -910,10 +1040,7 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
     }
 }
 
-size_t refine_tail_smem_bytes(int T) {
-    return sizeof(CandSmem) * kRefineThreads + 256 * 4 + (size_t)kRefineThreads * T * 4 +
-           (((size_t)kRefineThreads * T + 15) & ~(size_t)15) + kRefineThreads * 4 * 3;
-}
+size_t refine_tail_smem_bytes(int T, int max_w) { return (size_t)refine_layout(T, max_w, kRefineThreads, true, true).total; }
 
 // ------------------------------------------------------------ k_select_pack
 __device__ __forceinline__ void write_bits(uint32_t value, uint32_t count, uint32_t off, uint8_t* p) {
@@ -1436,10 +1563,7 @@ cudaError_t launch_extend(const KernelArgs& a, int flags, cudaStream_t s) {
 }
 
 size_t refine_smem_bytes(const TableLayout& L, int topn) {
-    const size_t pbs = (size_t)refine_pbs(L.T, topn);
-    const bool u8 = refine_u8(L.T);
-    return sizeof(CandSmem) * kRefineThreads + (u8 ? 256 * 4 : 0) + pbs * L.T * (u8 ? 4 : 16) + ((pbs * L.T + 15) & ~(size_t)15) +
-           kRefineThreads * 4;
+    return (size_t)refine_layout(L.T, L.max_w, refine_pbs(L.T, topn), refine_u8(L.T), false).total;
 }
 
 size_t refine_smem_bytes(const TableLayout& L) {  // the largest over the refinement top-N
@@ -1471,7 +1595,7 @@ cudaError_t configure_kernels(const TableLayout& L) {
     for (auto f : {k_refine<1, false>, k_refine<2, false>, k_refine<4, false>, k_refine<8, false>, k_refine<1, true>,
                    k_refine<2, true>, k_refine<4, true>, k_refine<8, true>})
         if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m[2])) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_refine_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)refine_tail_smem_bytes(kTailMaxTexels));
+    return cudaFuncSetAttribute(k_refine_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)refine_tail_smem_bytes(kTailMaxTexels, kTailMaxTexels));
 }
 
 cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s) {
@@ -1497,7 +1621,7 @@ cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s) {
 cudaError_t launch_refine_tail(const KernelArgs& a, cudaStream_t s) {
     if (!a.tail || a.L.T > kTailMaxTexels) return cudaSuccess;
     const int grid = std::min((a.tail_cap + kRefineThreads - 1) / kRefineThreads, 148 * kTailCtas);
-    k_refine_tail<<<std::max(grid, 1), kRefineThreads, refine_tail_smem_bytes(a.L.T), s>>>(a);
+    k_refine_tail<<<std::max(grid, 1), kRefineThreads, refine_tail_smem_bytes(a.L.T, a.L.max_w), s>>>(a);
     return cudaGetLastError();
 }
 
