@@ -45,16 +45,9 @@ __device__ __forceinline__ float4 normalize4(float4 v) {
     return make_float4(v.x / l, v.y / l, v.z / l, v.w / l);
 }
 __device__ __forceinline__ float comp(const float4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
-__device__ __forceinline__ uint32_t f2u(float v) {
-    if (!(v <= 4294967040.0f)) return 4294967295u;
-    if (v < 0.0f) return 0u;
-    return __float2uint_rz(v);
-}
-__device__ __forceinline__ int32_t f2i(float v) {
-    if (!(v <= 2147483520.0f)) return 2147483647;
-    if (v < -2147483648.0f) return (int32_t)0x80000000u;
-    return __float2int_rz(v);
-}
+// (the conversion instructions saturate; only NaN needs its own value)
+__device__ __forceinline__ uint32_t f2u(float v) { return v == v ? __float2uint_rz(v) : 4294967295u; }
+__device__ __forceinline__ int32_t f2i(float v) { return v == v ? __float2int_rz(v) : 2147483647; }
 __device__ __forceinline__ uint32_t fbits(float f) { return __float_as_uint(f); }
 
 __device__ __forceinline__ float atan_pos(float x) {

@@ -54,33 +54,35 @@ __device__ __forceinline__ float over257(float color) {
 __device__ __forceinline__ float4 over257(float4 c) { return make_float4(over257(c.x), over257(c.y), over257(c.z), over257(c.w)); }
 
 // ------------------------------------------------------------ pass14 colour endpoint packing
+// The endpoints it packs are clamped to 0..255, so every value converted to an integer here is
+// finite and small.  The refinement kernels stalled on instruction fetch first (4.7 of 13 warps
+// per issue at 7,500 instructions), so this code and the iteration are written for size: one
+// copy of each encoding's body and of the final error, loops left rolled; 4,200 instructions.
+// Measured with f2i / f2u as one conversion: full search of 1024x1024 at 4x4 47.5 -> 39.3 ms, of
+// 1021x765 at 10x8 72.5 -> 69.6 ms; proposal search of 2048x2048 at 4x4 10.2 -> 8.8 ms.
+__device__ __forceinline__ int32_t rni(float v) { return __float2int_rn(v); }
 struct Packer {
-    const uint8_t* cu2u;  // [17][512]
-    __device__ int32_t tab(uint32_t q, int32_t idx) const { return cu2u[(q - 4) * 512 + idx]; }
-    __device__ float enc_err(float4 u0, float4 u1, I4 q0, I4 q1) const {
+    const uint8_t* t;  // quantise-unquantise row of the quant level (cu2u, [512])
+    __device__ __forceinline__ int32_t tab(int32_t idx) const { return t[idx]; }
+    __device__ __forceinline__ int32_t qf1(int32_t v, float vf) const { return tab(v * 2 + ((vf - (float)v) >= -0.1f ? 1 : 0)); }
+    __device__ __forceinline__ int32_t qint(int32_t v) const { return tab(v * 2 + 1); }
+    __device__ __forceinline__ int32_t qrn(float v) const { return qf1(rni(v), v); }
+    __device__ static float enc_err(float4 u0, float4 u1, I4 q0, I4 q1) {
         const float4 e0 = u0 - make_float4((float)q0.x, (float)q0.y, (float)q0.z, (float)q0.w);
         const float4 e1 = u1 - make_float4((float)q1.x, (float)q1.y, (float)q1.z, (float)q1.w);
         const float4 e = e0 * e0 + e1 * e1;
         return ((e.x + e.y) + e.z) + e.w;
     }
-    __device__ I4 q3int(uint32_t q, I4 v) const { return {tab(q, v.x * 2 + 1), tab(q, v.y * 2 + 1), tab(q, v.z * 2 + 1), 0}; }
-    __device__ int32_t qf1(uint32_t q, int32_t v, float vf) const { return tab(q, v * 2 + ((vf - (float)v) >= -0.1f ? 1 : 0)); }
-    __device__ I4 q3flt(uint32_t q, I4 v, float4 vf) const { return {qf1(q, v.x, vf.x), qf1(q, v.y, vf.y), qf1(q, v.z, vf.z), 0}; }
-    __device__ uint32_t qint(uint32_t q, int32_t v) const { return (uint32_t)tab(q, v * 2 + 1); }
-    __device__ uint32_t qflt(uint32_t q, int32_t v, float vf) const { return (uint32_t)qf1(q, v, vf); }
 
     // bit_transfer_signed(&a, &b) (pass14:355-369)
-    __device__ static void bts(I4& a, I4& b) {
-        int32_t* pa = &a.x; int32_t* pb = &b.x;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const uint32_t a0 = (uint32_t)pa[c], b0 = (uint32_t)pb[c];
-            int32_t na = (int32_t)((a0 >> 1) & 0x3F);
-            if (na & 0x20) na -= 0x40;
-            pb[c] = (int32_t)((b0 >> 1) | (a0 & 0x80));
-            pa[c] = na;
-        }
+    __device__ static void bts1(int32_t& a, int32_t& b) {
+        const uint32_t a0 = (uint32_t)a, b0 = (uint32_t)b;
+        int32_t na = (int32_t)((a0 >> 1) & 0x3F);
+        if (na & 0x20) na -= 0x40;
+        b = (int32_t)((b0 >> 1) | (a0 & 0x80));
+        a = na;
     }
+    __device__ static void bts(I4& a, I4& b) { bts1(a.x, b.x); bts1(a.y, b.y); bts1(a.z, b.z); bts1(a.w, b.w); }
     __device__ static I4 uncontract(I4 v) { return {(v.x + v.z) >> 1, (v.y + v.z) >> 1, v.z, v.w}; }
     __device__ static int32_t clamp255(int32_t v) { return min(max(v, 0), 255); }
     __device__ static void delta_unpack(I4 i0, I4 i1, I4& o0, I4& o1) {
@@ -100,47 +102,46 @@ struct Packer {
     }
     __device__ static float4 inv_bc(float4 c) { return make_float4((c.x + c.x) - c.z, (c.y + c.y) - c.z, (c.z + c.z) - c.z, (c.w + c.w) - c.w); }
 
-    // try_quantize_rgb_delta(_blue_contract) body after the optional inverse contraction
-    __device__ bool rgb_delta(float4 c0, float4 c1, I4& o0, I4& o1, uint32_t q, bool want_bc) const {
-        I4 c0a = ivec(rnev(c0));
-        c0a = {shl1(c0a.x), shl1(c0a.y), shl1(c0a.z), shl1(c0a.w)};
-        I4 c0b = {c0a.x & 0xFF, c0a.y & 0xFF, c0a.z & 0xFF, c0a.w & 0xFF};
-        const I4 c0be = q3int(q, c0b);
-        c0b = {c0be.x | (c0a.x & 0x100), c0be.y | (c0a.y & 0x100), c0be.z | (c0a.z & 0x100), c0be.w | (c0a.w & 0x100)};
-        I4 c1d = ivec(rnev(c1));
-        c1d = {shl1(c1d.x) - c0b.x, shl1(c1d.y) - c0b.y, shl1(c1d.z) - c0b.z, 0};
-        if (c1d.x > 63 || c1d.x < -64 || c1d.y > 63 || c1d.y < -64 || c1d.z > 63 || c1d.z < -64) return false;
-        c1d = {(c1d.x & 0x7F) | ((c0b.x & 0x100) >> 1), (c1d.y & 0x7F) | ((c0b.y & 0x100) >> 1),
-               (c1d.z & 0x7F) | ((c0b.z & 0x100) >> 1), (c1d.w & 0x7F) | ((c0b.w & 0x100) >> 1)};
-        const I4 c1de = q3int(q, c1d);
-        if (((c1d.x ^ c1de.x) & 0xC0) || ((c1d.y ^ c1de.y) & 0xC0) || ((c1d.z ^ c1de.z) & 0xC0)) return false;
-        I4 e0 = c0be, e1 = c1de;
+    // One channel of a delta encoding: the low endpoint v0 and the difference to the high one
+    // v1 (8-bit units), quantised to q0 and q1; false when the difference does not fit.
+    __device__ __forceinline__ bool delta1(float v0, float v1, int32_t& q0, int32_t& q1, int32_t& base9) const {
+        const int32_t a = shl1(rni(v0));
+        q0 = qint(a & 0xFF);
+        base9 = q0 | (a & 0x100);
+        const int32_t d = shl1(rni(v1)) - base9;
+        const bool fits = d <= 63 && d >= -64;
+        const int32_t d8 = (d & 0x7F) | ((base9 & 0x100) >> 1);
+        q1 = qint(d8);
+        return fits && ((d8 ^ q1) & 0xC0) == 0;
+    }
+    // try_quantize_rgb_delta(_blue_contract) body after the optional inverse contraction (w is
+    // left to the alpha)
+    __device__ __forceinline__ bool rgb_delta(float4 c0, float4 c1, I4& o0, I4& o1, bool want_bc) const {
+        int32_t b9;
+        bool ok = delta1(c0.x, c1.x, o0.x, o1.x, b9);
+        ok = delta1(c0.y, c1.y, o0.y, o1.y, b9) && ok;
+        ok = delta1(c0.z, c1.z, o0.z, o1.z, b9) && ok;
+        I4 e0 = {o0.x, o0.y, o0.z, 0}, e1 = {o1.x, o1.y, o1.z, 0};
         bts(e1, e0);
         const int32_t s = e1.x + e1.y + e1.z;
-        if (want_bc ? (s >= 0) : (s < 0)) return false;
-        e0 = {e0.x + e1.x, e0.y + e1.y, e0.z + e1.z, e0.w + e1.w};
-        if (e0.x < 0 || e0.x > 0xFF || e0.y < 0 || e0.y > 0xFF || e0.z < 0 || e0.z > 0xFF || e0.w < 0 || e0.w > 0xFF) return false;
-        o0 = c0be; o1 = c1de;
-        return true;
+        ok = ok && (want_bc ? (s < 0) : (s >= 0));
+        e0 = {e0.x + e1.x, e0.y + e1.y, e0.z + e1.z, 0};
+        return ok && (uint32_t)e0.x <= 0xFFu && (uint32_t)e0.y <= 0xFFu && (uint32_t)e0.z <= 0xFFu;
     }
-    __device__ bool try_rgb_delta_bc(float4 a0, float4 a1, I4& o0, I4& o1, uint32_t q) const {
-        const float4 c0 = inv_bc(a1), c1 = inv_bc(a0);
-        if (out_of_range(c0) || out_of_range(c1)) return false;
-        return rgb_delta(c0, c1, o0, o1, q, true);
+    __device__ __forceinline__ bool alpha_delta(float v0, float v1, int32_t& q0, int32_t& q1) const {
+        int32_t b9;
+        if (!delta1(v0, v1, q0, q1, b9)) return false;
+        int32_t du = q1 & 0x7F;
+        if (du & 0x40) du -= 0x80;
+        du += b9;
+        return du >= 0 && du <= 0x1FF;
     }
-    __device__ bool try_rgb_bc(float4 a0, float4 a1, I4& o0, I4& o1, uint32_t q) const {
-        const float4 c0 = inv_bc(a0), c1 = inv_bc(a1);
-        if (out_of_range(c0) || out_of_range(c1)) return false;
-        const I4 c0i = q3flt(q, ivec(rnev(c0)), c0), c1i = q3flt(q, ivec(rnev(c1)), c1);
-        if ((c1i.x + c1i.y + c1i.z) <= (c0i.x + c0i.y + c0i.z)) return false;
-        o0 = c1i; o1 = c0i;
-        return true;
-    }
+    __device__ __forceinline__ I4 q3flt(float4 c) const { return {qrn(c.x), qrn(c.y), qrn(c.z), 0}; }
     // Quantised channel sums of the endpoints at one step of the loop below: true when the
     // step ends it (the low endpoint's sum no longer above the high one's).
-    __device__ bool qrgb_probe(uint32_t q, float x0, float y0, float z0, float x1, float y1, float z1, I4& c0i, I4& c1i) const {
-        c0i = q3flt(q, I4{max(f2i(rintf(x0)), 0), max(f2i(rintf(y0)), 0), max(f2i(rintf(z0)), 0), 0}, make_float4(x0, y0, z0, 0.0f));
-        c1i = q3flt(q, I4{min(f2i(rintf(x1)), 255), min(f2i(rintf(y1)), 255), min(f2i(rintf(z1)), 255), 0}, make_float4(x1, y1, z1, 0.0f));
+    __device__ __forceinline__ bool qrgb_probe(float x0, float y0, float z0, float x1, float y1, float z1, I4& c0i, I4& c1i) const {
+        c0i = {qf1(max(rni(x0), 0), x0), qf1(max(rni(y0), 0), y0), qf1(max(rni(z0), 0), z0), 0};
+        c1i = {qf1(min(rni(x1), 255), x1), qf1(min(rni(y1), 255), y1), qf1(min(rni(z1), 255), z1), 0};
         return (c0i.x + c0i.y + c0i.z) <= (c1i.x + c1i.y + c1i.z);
     }
     // The reference's loop nudges the endpoints 0.2 apart per step (at most 4096 steps) and
@@ -151,148 +152,103 @@ struct Packer {
     // 3, 7, ... and bisecting the last bracket; the endpoints are always brought to a probed
     // step by the loop's own float subtractions and additions from an earlier probed step,
     // so each probe sees the values the loop would.
-    __device__ void quant_rgb(float4 c0, float4 c1, I4& o0, I4& o1, uint32_t q) const {
-        float x0 = c0.x, y0 = c0.y, z0 = c0.z, x1 = c1.x, y1 = c1.y, z1 = c1.z;  // step lo
-        I4 c0i, c1i;
-        if (!qrgb_probe(q, x0, y0, z0, x1, y1, z1, c0i, c1i)) {
-            auto advance = [](float& a, float& b, float& c, float& d, float& e, float& f, int n) {
-#pragma unroll 4
-                for (int i = 0; i < n; i++) { a = a - 0.2f; b = b - 0.2f; c = c - 0.2f; d = d + 0.2f; e = e + 0.2f; f = f + 0.2f; }
-            };
-            int lo = 0, hi = 0, step = 1;
-            for (;;) {  // the test fails at lo; at most 13 trips
-                hi = min(lo + step, 4095);
-                float a = x0, b = y0, c = z0, d = x1, e = y1, f = z1;
-                advance(a, b, c, d, e, f, hi - lo);
-                if (qrgb_probe(q, a, b, c, d, e, f, c0i, c1i) || hi == 4095) break;
+    __device__ __forceinline__ void quant_rgb(float4 c0, float4 c1, I4& o0, I4& o1) const {
+        float x0 = c0.x, y0 = c0.y, z0 = c0.z, x1 = c1.x, y1 = c1.y, z1 = c1.z;  // at step lo
+        int lo = 0, hi = 0, at = 0, step = 1;  // at: the step to probe
+        bool bracketed = false;                // the stop is in (lo, hi] (hi = 4095: the last step)
+        for (;;) {
+            float a = x0, b = y0, c = z0, d = x1, e = y1, f = z1;
+#pragma unroll 1
+            for (int i = lo; i < at; i++) { a = a - 0.2f; b = b - 0.2f; c = c - 0.2f; d = d + 0.2f; e = e + 0.2f; f = f + 0.2f; }
+            const bool stop = qrgb_probe(a, b, c, d, e, f, o0, o1);
+            if (bracketed ? at == hi : (stop && at <= 1)) return;
+            if (stop || at == 4095) {
+                hi = at;
+                bracketed = true;
+            } else {
                 x0 = a; y0 = b; z0 = c; x1 = d; y1 = e; z1 = f;
-                lo = hi;
+                lo = at;
+            }
+            if (bracketed) {
+                at = hi - lo > 1 ? lo + (hi - lo) / 2 : hi;
+            } else {
+                at = min(lo + step, 4095);
                 step *= 2;
             }
-            while (hi - lo > 1) {  // the stop is in (lo, hi] (hi = 4095: the last step)
-                const int mid = lo + (hi - lo) / 2;
-                float a = x0, b = y0, c = z0, d = x1, e = y1, f = z1;
-                advance(a, b, c, d, e, f, mid - lo);
-                if (qrgb_probe(q, a, b, c, d, e, f, c0i, c1i)) {
-                    hi = mid;
-                } else {
-                    lo = mid;
-                    x0 = a; y0 = b; z0 = c; x1 = d; y1 = e; z1 = f;
-                }
-            }
-            advance(x0, y0, z0, x1, y1, z1, 1);
-            qrgb_probe(q, x0, y0, z0, x1, y1, z1, c0i, c1i);
         }
-        o0 = c0i; o1 = c1i;
     }
-    __device__ bool try_alpha_delta(float4 color0, float4 color1, I4& o0, I4& o1, uint32_t q) const {
-        const int32_t a0a = shl1(f2i(rintf(color0.w)));
-        int32_t a0b = a0a & 0xFF;
-        const int32_t a0be = (int32_t)qint(q, a0b);
-        a0b = a0be | (a0a & 0x100);
-        int32_t a1d = shl1(f2i(rintf(color1.w))) - a0b;
-        if (a1d > 63 || a1d < -64) return false;
-        a1d = (a1d & 0x7F) | ((a0b & 0x100) >> 1);
-        const int32_t a1de = (int32_t)qint(q, a1d);
-        if (((a1d ^ a1de) & 0xC0) != 0) return false;
-        int32_t a1du = a1de & 0x7F;
-        if (a1du & 0x40) a1du -= 0x80;
-        a1du += a0b;
-        if (a1du < 0 || a1du > 0x1FF) return false;
-        o0.w = a0be; o1.w = a1de;
-        return true;
-    }
-    __device__ void quant_rgbs(float4 color, uint32_t* out, uint32_t q) const {
+    __device__ __forceinline__ void quant_rgbs(float4 color, uint32_t* out) const {
         const float scale = 1.0f / 257.0f;
         const float r = clampf(color.x * scale, 0.0f, 255.0f), g = clampf(color.y * scale, 0.0f, 255.0f), b = clampf(color.z * scale, 0.0f, 255.0f);
-        const uint32_t ri = qflt(q, f2i(rintf(r)), r), gi = qflt(q, f2i(rintf(g)), g), bi = qflt(q, f2i(rintf(b)), b);
+        const uint32_t ri = (uint32_t)qrn(r), gi = (uint32_t)qrn(g), bi = (uint32_t)qrn(b);
         const float oldsum = ((color.x + color.y) + color.z) * scale;
         const float newsum = (float)(ri + gi + bi);
         const float sa = clampf((color.w * (oldsum + 1e-10f)) / (newsum + 1e-10f), 0.0f, 1.0f);
-        const int32_t si = min(max(f2i(rintf(sa * 256.0f)), 0), 255);
-        out[0] = ri; out[1] = gi; out[2] = bi; out[3] = qint(q, si);
+        const int32_t si = min(max(rni(sa * 256.0f), 0), 255);
+        out[0] = ri; out[1] = gi; out[2] = bi; out[3] = (uint32_t)qint(si);
     }
-    __device__ bool try_la_delta(float4 c0, float4 c1, uint32_t* out, uint32_t q) const {
-        const float l0 = ((c0.x + c0.y) + c0.z) / 3.0f, l1 = ((c1.x + c1.y) + c1.z) / 3.0f;
-        const int32_t l0a = shl1(f2i(rintf(l0))), a0a = shl1(f2i(rintf(c0.w)));
-        const uint32_t l0be = qint(q, l0a & 0xFF), a0be = qint(q, a0a & 0xFF);
-        const int32_t l0b = (int32_t)l0be | (l0a & 0x100), a0b = (int32_t)a0be | (a0a & 0x100);
-        int32_t l1d = shl1(f2i(rintf(l1))) - l0b, a1d = shl1(f2i(rintf(c1.w))) - a0b;
-        if (l1d > 63 || l1d < -64 || a1d > 63 || a1d < -64) return false;
-        l1d = (l1d & 0x7F) | ((l0b & 0x100) >> 1);
-        a1d = (a1d & 0x7F) | ((a0b & 0x100) >> 1);
-        const uint32_t l1de = qint(q, l1d), a1de = qint(q, a1d);
-        int32_t l1du = (int32_t)l1de, a1du = (int32_t)a1de;
-        if (((l1d ^ l1du) & 0xC0) != 0) return false;
-        if (((a1d ^ a1du) & 0xC0) != 0) return false;
-        l1du &= 0x7F; a1du &= 0x7F;
-        if (l1du & 0x40) l1du -= 0x80;
-        if (a1du & 0x40) a1du -= 0x80;
-        l1du += l0b; a1du += a0b;
-        if (l1du < 0 || l1du > 0x1FF || a1du < 0 || a1du > 0x1FF) return false;
-        out[0] = l0be; out[1] = l1de; out[2] = a0be; out[3] = a1de;
-        return true;
-    }
-    // pack_color_endpoints_helper (pass14:917-1224).  Returns the format (x) and the up to
-    // eight packed values, one byte each (y, then z).
-    __device__ __noinline__ uint4 pack(float4 color0, float4 color1, float4 rgbs, uint32_t fmt, uint32_t q) const {
+    // pack_color_endpoints_helper (pass14:917-1224) at quant level q.  Returns the format (x)
+    // and the up to eight packed values, one byte each (y, then z).
+    __device__ static __noinline__ uint4 pack(const uint8_t* cu2u, float4 color0, float4 color1, float4 rgbs, uint32_t fmt, uint32_t q) {
+        const Packer k{cu2u + (q - 4) * 512};
         const float4 c0 = over257(color0), c1 = over257(color1);
-        float best = ERR_DEFAULT;
         uint32_t out[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) out[i] = 0;
         uint32_t bf = FMT_LUMINANCE;
         if (fmt == FMT_RGB || fmt == FMT_RGBA) {
             const bool rgba = fmt == FMT_RGBA;
-            const uint32_t dfmt = rgba ? FMT_RGBA_DELTA : FMT_RGB_DELTA;
-            I4 o0 = {0, 0, 0, 0}, o1 = {0, 0, 0, 0}, p0 = {0, 0, 0, 0}, p1 = {0, 0, 0, 0}, u0, u1;
-            if (q <= 18) {
-                bool ok = try_rgb_delta_bc(c0, c1, o0, o1, q);
-                if (rgba && ok) ok = try_alpha_delta(c1, c0, o0, o1, q);
-                if (ok) { delta_unpack(o0, o1, u0, u1); bf = dfmt; best = enc_err(c0, c1, u0, u1); }
-                ok = rgb_delta(c0, c1, p0, p1, q, false);
-                if (rgba && ok) ok = try_alpha_delta(c0, c1, p0, p1, q);
-                if (ok) {
-                    delta_unpack(p0, p1, u0, u1);
-                    const float e = enc_err(c0, c1, u0, u1);
-                    if (e < best) { best = e; bf = dfmt; o0 = p0; o1 = p1; }
+            float best = ERR_DEFAULT;
+            I4 o0 = {0, 0, 0, 0}, o1 = {0, 0, 0, 0};
+            // the four encodings in the order the reference tries them: delta with blue
+            // contraction, delta, blue contraction, plain; the first of the smallest error wins
+#pragma unroll 1
+            for (int v = q <= 18 ? 0 : q < 20 ? 2 : 3; v < 4; v++) {
+                const bool contract = v == 0 || v == 2;
+                float4 a0 = c0, a1 = c1;
+                if (contract) {
+                    a0 = inv_bc(c1); a1 = inv_bc(c0);
+                    if (out_of_range(a0) || out_of_range(a1)) continue;
                 }
-            }
-            if (q < 20 && try_rgb_bc(c0, c1, p0, p1, q)) {
-                if (rgba) { p0.w = (int32_t)qflt(q, f2i(rintf(c1.w)), c1.w); p1.w = (int32_t)qflt(q, f2i(rintf(c0.w)), c0.w); }
-                rgba_unpack(p0, p1, u0, u1);
+                I4 p0, p1, u0, u1;
+                p0.w = p1.w = 0;
+                if (v < 2) {
+                    if (!k.rgb_delta(a0, a1, p0, p1, contract)) continue;
+                    if (rgba && !k.alpha_delta(contract ? c1.w : c0.w, contract ? c0.w : c1.w, p0.w, p1.w)) continue;
+                    delta_unpack(p0, p1, u0, u1);
+                } else {
+                    if (contract) {
+                        p0 = k.q3flt(a0); p1 = k.q3flt(a1);
+                        if ((p0.x + p0.y + p0.z) <= (p1.x + p1.y + p1.z)) continue;
+                    } else {
+                        k.quant_rgb(c0, c1, p0, p1);
+                    }
+                    if (rgba) { p0.w = k.qrn(contract ? c1.w : c0.w); p1.w = k.qrn(contract ? c0.w : c1.w); }
+                    rgba_unpack(p0, p1, u0, u1);
+                }
                 const float e = enc_err(c0, c1, u0, u1);
-                if (e < best) { best = e; bf = fmt; o0 = p0; o1 = p1; }
-            }
-            {
-                quant_rgb(c0, c1, p0, p1, q);
-                if (rgba) { p0.w = (int32_t)qflt(q, f2i(rintf(c0.w)), c0.w); p1.w = (int32_t)qflt(q, f2i(rintf(c1.w)), c1.w); }
-                rgba_unpack(p0, p1, u0, u1);
-                const float e = enc_err(c0, c1, u0, u1);
-                if (e < best) { best = e; bf = fmt; o0 = p0; o1 = p1; }
+                if (e < best) { best = e; bf = v < 2 ? fmt + 1 : fmt; o0 = p0; o1 = p1; }
             }
             out[0] = (uint32_t)o0.x; out[1] = (uint32_t)o1.x; out[2] = (uint32_t)o0.y;
             out[3] = (uint32_t)o1.y; out[4] = (uint32_t)o0.z; out[5] = (uint32_t)o1.z;
             if (rgba) { out[6] = (uint32_t)o0.w; out[7] = (uint32_t)o1.w; }
-        } else if (fmt == FMT_RGB_SCALE) {
-            quant_rgbs(rgbs, out, q); bf = FMT_RGB_SCALE;
-        } else if (fmt == FMT_RGB_SCALE_ALPHA) {
-            out[4] = qflt(q, f2i(rintf(c0.w)), c0.w); out[5] = qflt(q, f2i(rintf(c1.w)), c1.w);
-            quant_rgbs(rgbs, out, q); bf = FMT_RGB_SCALE_ALPHA;
-        } else if (fmt == FMT_LUMINANCE_ALPHA) {
-            if (q <= 18 && try_la_delta(c0, c1, out, q)) {
+        } else if (fmt == FMT_RGB_SCALE || fmt == FMT_RGB_SCALE_ALPHA) {
+            if (fmt == FMT_RGB_SCALE_ALPHA) { out[4] = (uint32_t)k.qrn(c0.w); out[5] = (uint32_t)k.qrn(c1.w); }
+            k.quant_rgbs(rgbs, out);
+            bf = fmt;
+        } else {  // FMT_LUMINANCE_ALPHA, FMT_LUMINANCE and any other format
+            const bool la = fmt == FMT_LUMINANCE_ALPHA;
+            float l0 = ((c0.x + c0.y) + c0.z) / 3.0f, l1 = ((c1.x + c1.y) + c1.z) / 3.0f;
+            int32_t q0, q1, a0, a1;
+            if (la && q <= 18 && k.alpha_delta(l0, l1, q0, q1) && k.alpha_delta(c0.w, c1.w, a0, a1)) {
                 bf = FMT_LUMINANCE_ALPHA_DELTA;
             } else {
-                const float l0 = ((c0.x + c0.y) + c0.z) / 3.0f, l1 = ((c1.x + c1.y) + c1.z) / 3.0f;
-                out[0] = qflt(q, f2i(rintf(l0)), l0); out[1] = qflt(q, f2i(rintf(l1)), l1);
-                out[2] = qflt(q, f2i(rintf(c0.w)), c0.w); out[3] = qflt(q, f2i(rintf(c1.w)), c1.w);
-                bf = FMT_LUMINANCE_ALPHA;
+                if (!la && l0 > l1) { const float av = (l0 + l1) * 0.5f; l0 = av; l1 = av; }
+                q0 = k.qrn(l0); q1 = k.qrn(l1);
+                a0 = la ? k.qrn(c0.w) : 0; a1 = la ? k.qrn(c1.w) : 0;
+                bf = la ? FMT_LUMINANCE_ALPHA : FMT_LUMINANCE;
             }
-        } else {  // FMT_LUMINANCE and any other format
-            float l0 = ((c0.x + c0.y) + c0.z) / 3.0f, l1 = ((c1.x + c1.y) + c1.z) / 3.0f;
-            if (l0 > l1) { const float av = (l0 + l1) * 0.5f; l0 = av; l1 = av; }
-            out[0] = qflt(q, f2i(rintf(l0)), l0); out[1] = qflt(q, f2i(rintf(l1)), l1);
-            bf = FMT_LUMINANCE;
+            out[0] = (uint32_t)q0; out[1] = (uint32_t)q1; out[2] = (uint32_t)a0; out[3] = (uint32_t)a1;
         }
         return make_uint4(bf, out[0] | out[1] << 8 | out[2] << 16 | out[3] << 24, out[4] | out[5] << 8 | out[6] << 16 | out[7] << 24, 0u);
     }
@@ -431,6 +387,7 @@ struct RTabs {
 // Sets the candidate's infilled weights from its grid weights (pass13:165-184, pass17:127-146).
 // Padding entries of the dense list contribute 0.
 __device__ __forceinline__ void infill(const RTabs& tb, const Cand& c, int dm, int T, bool direct) {
+#pragma unroll 1
     for (int t = 0; t < T; t++) {
         uint32_t v;
         if (direct) {
@@ -468,7 +425,9 @@ template <class E> struct PartRow {
     __device__ __forceinline__ void set(const uint8_t* prow, const uint8_t* counts, int T) const {
         uint32_t next = 0;  // next position of each partition, a byte each
         if (prow) next = (uint32_t)counts[0] << 8 | ((uint32_t)counts[0] + counts[1]) << 16 | ((uint32_t)counts[0] + counts[1] + counts[2]) << 24;
+#pragma unroll 1
         for (int t = 0; t < T; t++) v[t] = prow ? (E)((int)prow[t] << kShift) : (E)0;
+#pragma unroll 1
         for (int t = 0; t < T; t++) {
             const int sh = prow ? 8 * (int)prow[t] : 0;
             const int i = (next >> sh) & 0xFF;
@@ -506,13 +465,14 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     const bool direct = W == T;
     const float4 cw = chan_w();
     const float lsw = (cw.x + cw.y) + cw.z;
-    const Packer pk{a.tables + a.L.off_cu2u};
+    const uint8_t* cu2u = a.tables + a.L.off_cu2u;
     float4 rgbs[4];
     uint2 packed[4], packed_mod[4];
     if (it == 0) {
 #pragma unroll
         for (int q = 0; q < 4; q++) { cs.ep(2 * q) = rec.ep0[q]; cs.ep(2 * q + 1) = rec.ep1[q]; }
         const uint32_t* src = reinterpret_cast<const uint32_t*>(ci.qw);  // 8-byte aligned in PBRec
+#pragma unroll 1
         for (int w = 0; w < (W + 3) / 4; w++) cs.qw4(w) = src[w];
         *cs.err = ERR_DEFAULT;
         infill(tb, cs, bm.dm, T, direct);
@@ -527,6 +487,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         float total = 0.0f;
         float4 base = mk(0.0f), offs = mk(0.0f);
         int pc = -1;
+#pragma unroll 1
         for (int t = 0; t < T; t++) {
             const int p = pt.part(t);
             if (p != pc) {
@@ -553,6 +514,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
             d[1] = make_uint4(packed[0].x, packed[0].y, packed[1].x, packed[1].y);
             d[2] = make_uint4(packed[2].x, packed[2].y, packed[3].x, packed[3].y);
             const int nw = (W + 3) / 4;
+#pragma unroll 1
             for (int i = 0; i < 4; i++) {
                 uint4 v = make_uint4(0u, 0u, 0u, 0u);
                 if (4 * i < nw) v.x = cs.qw4(4 * i);
@@ -575,6 +537,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         const float4 sdir = scale ? sdir_of(q, ps) : mk(0.0f);
         float wmin = 1.0f, wmax = 0.0f, ls = 0.0f, ms = 0.0f, rs = 0.0f, smin = 1e10f, smax = 0.0f, sv0 = 0.0f, sv1 = 0.0f;
         float4 cx = mk(0.0f), cy = mk(0.0f);
+#pragma unroll 1
         for (int i = i0; i < i0 + n; i++) {
             const int t = pt.order(i);
             const float4 rgba = px[t];
@@ -644,7 +607,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         for (int q = 0; q < 4; q++) packed[q] = make_uint2(0u, 0u);
 #pragma unroll 1
         for (int q = 0; q < P; q++) {
-            const uint4 v = pk.pack(cs.ep(2 * q), cs.ep(2 * q + 1), rgbs[q], ci.fmt[q], ci.ql);
+            const uint4 v = Packer::pack(cu2u, cs.ep(2 * q), cs.ep(2 * q + 1), rgbs[q], ci.fmt[q], ci.ql);
             const uint32_t f = v.x;
             fn[0] = q == 0 ? f : fn[0]; fn[1] = q == 1 ? f : fn[1]; fn[2] = q == 2 ? f : fn[2]; fn[3] = q == 3 ? f : fn[3];
             packed[q] = make_uint2(v.y, v.z);
@@ -656,7 +619,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
             bool same_mod = true;
 #pragma unroll 1
             for (int q = 0; q < P; q++) {
-                const uint4 v = pk.pack(cs.ep(2 * q), cs.ep(2 * q + 1), rgbs[q], ci.fmt[q], ci.qlm);
+                const uint4 v = Packer::pack(cu2u, cs.ep(2 * q), cs.ep(2 * q + 1), rgbs[q], ci.fmt[q], ci.qlm);
                 const uint32_t f = v.x;
                 fm[0] = q == 0 ? f : fm[0]; fm[1] = q == 1 ? f : fm[1]; fm[2] = q == 2 ? f : fm[2]; fm[3] = q == 3 ? f : fm[3];
                 packed_mod[q] = make_uint2(v.y, v.z);
@@ -666,6 +629,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
                 m = true;
 #pragma unroll
                 for (int q = 0; q < 4; q++) fn[q] = fm[q];
+#pragma unroll 1
                 for (int q = 0; q < P; q++) packed[q] = packed_mod[q];
             }
         }
@@ -682,9 +646,11 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         cs.u(q) = make_uint4((uint32_t)(o0.x * 257) | (uint32_t)(o0.y * 257) << 16, (uint32_t)(o0.z * 257) | (uint32_t)(o0.w * 257) << 16,
                              (uint32_t)(o1.x * 257) | (uint32_t)(o1.y * 257) << 16, (uint32_t)(o1.z * 257) | (uint32_t)(o1.w * 257) << 16);
     }
-    if (it == 0) final_error();
     // ---------------- pass16: move each weight one quant step if that lowers the error
     bool moved = false;
+#pragma unroll 1
+    for (int turn = it == 0 ? 0 : 1; turn < 2; turn++) {
+    if (turn == 1) {
     float4 base = mk(0.0f), offs = mk(0.0f);
     int pc = -1;
     auto endpoints = [&](int p) {  // of texel partition p, read again when it changes
@@ -695,6 +661,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         pc = p;
     };
     if (direct) {
+#pragma unroll 1
         for (int t = 0; t < T; t++) {
             const int32_t uqw = cs.qw(t);
             const uint32_t pn = tb.prev_next(bm.quant, uqw);
@@ -713,6 +680,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
             }
         }
     } else {
+#pragma unroll 1
         for (int we = 0; we < W; we++) {
             const int32_t uqw = cs.qw(we);
             const uint32_t pn = tb.prev_next(bm.quant, uqw);
@@ -720,6 +688,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
             const float ddn = dn - ub, dup = up - ub;
             float4 ebv = mk(0.0f), edv = mk(0.0f), euv = mk(0.0f);
             const int nt = tb.wt_count(bm.dm, we), wbase = dmi.wt_base + tb.wt_start(bm.dm, we);
+#pragma unroll 1
             for (int te = 0; te < nt; te++) {
                 // the weight's own contribution to texel t is the w2t entry's
                 // (each (texel, weight) pair appears once in both maps)
@@ -739,6 +708,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
             if (dw != 0.0f) {
                 moved = true;
                 cs.qw(we) = (uint8_t)(uqw + (int)dw);
+#pragma unroll 1
                 for (int te = 0; te < nt; te++) {
                     const uint32_t we2 = tb.w2t(wbase + te);
                     __half& sv = cs.s(we2 & 0xFF);
@@ -749,7 +719,10 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     }
     // In iteration 0 a pass16 that moved no weight leaves the weights and endpoints of the
     // error taken before it: the same total, which cannot improve the snapshot.
-    if (it > 0 || moved) final_error();
+    if (it == 0 && !moved) break;
+    }
+    final_error();
+    }
     return moved;
 }
 
@@ -764,6 +737,7 @@ __device__ __forceinline__ void write_tail(const KernelArgs& a, const Cand& c, u
     for (int i = 0; i < 8; i++) ep[i] = c.ep(i);
     const int n4 = (a.L.max_w + 3) / 4;
     uint32_t* w = reinterpret_cast<uint32_t*>(e + 9);
+#pragma unroll 1
     for (int i = 0; i < n4; i++) w[i] = c.qw4(i);
 }
 
@@ -814,6 +788,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                 if (k < (int)r.ncand) {
                     const int dm = reinterpret_cast<const DevBm*>(a.tables + a.L.off_bm)[r.c[k].bm].dm;
                     int fk = 0;
+#pragma unroll 1
                     for (int q = 0; q < 4; q++) { const int f = r.c[k].fmt[q]; fk = fk * 8 + (f == 0 ? 0 : f == 4 ? 1 : f == 6 ? 2 : f == 8 ? 3 : f == 10 ? 4 : f == 12 ? 5 : 6); }
                     key = ((((int)r.P - 1) << 12 | fk) << 7) | dm;  // partition count, formats, decimation mode
                 }
@@ -823,11 +798,13 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                     const uint8_t* counts = P > 1 ? a.tables + a.L.off_part_counts + ((size_t)(P - 2) * 1024 + r.entry) * 4 : nullptr;
                     const BlockSrc src = block_src(a, chunk_block(a, lb));
                     Px* row = reinterpret_cast<Px*>(smem + fl.px + pbl * px_row);
+#pragma unroll 1
                     for (int t = k; t < T; t += cpb) {
                         if constexpr (U8) row[t] = src_rgba8(src, a.L.bx, t);
                         else row[t] = src_texel(src, a.L.bx, t);
                     }
                     if (k == 0) PartRow<Pe>{reinterpret_cast<Pe*>(smem + fl.part + pbl * part_row)}.set(prow, counts, T);
+#pragma unroll 1
                     for (int q = k; q < P; q += cpb) sdirs[pbl * 4 + q] = scale_dir(r.avg[q], (float)(P == 1 ? T : (int)counts[q]));
                 }
             }
@@ -842,7 +819,12 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
         {
             const int kk = keys[tid];
             int rank = 0;
-            for (int j = 0; j < kRefineThreads; j++) rank += keys[j] < kk;
+            const int4* k4 = reinterpret_cast<const int4*>(keys);
+#pragma unroll 2
+            for (int j = 0; j < kRefineThreads / 4; j++) {
+                const int4 o = k4[j];
+                rank += (o.x < kk) + (o.y < kk) + (o.z < kk) + (o.w < kk);
+            }
             __syncthreads();
             keys[rank] = tid;
             __syncthreads();
@@ -984,12 +966,15 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
                     const uint8_t* counts = P > 1 ? a.tables + a.L.off_part_counts + ((size_t)(P - 2) * 1024 + r.entry) * 4 : nullptr;
                     const BlockSrc src = block_src(a, chunk_block(a, lb));
                     uchar4* row = reinterpret_cast<uchar4*>(smem + fl.px + tid * px_row);
+#pragma unroll 1
                     for (int t = 0; t < T; t++) row[t] = src_rgba8(src, a.L.bx, t);
                     PartRow<uint8_t>{smem + fl.part + tid * part_row}.set(prow, counts, T);
                     const Cand c(smem, fl, tid);
+#pragma unroll 1
                     for (int i = 0; i < 8; i++) c.ep(i) = reinterpret_cast<const float4*>(e + 1)[i];
                     const int n4 = (a.L.max_w + 3) / 4;
                     const uint32_t* w = reinterpret_cast<const uint32_t*>(e + 9);
+#pragma unroll 1
                     for (int i = 0; i < n4; i++) c.qw4(i) = w[i];
                     *c.err = __uint_as_float(h.z);
                     const RTabs tb{a.tables, &a.L};
