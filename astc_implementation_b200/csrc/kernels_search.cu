@@ -60,6 +60,7 @@ struct Tabs {
     __device__ uint64_t tw4(int m, int t) const { return reinterpret_cast<const uint64_t*>(b + L->off_tw4)[m * L->T + t]; }
     __device__ int bm_order(int j) const { return reinterpret_cast<const uint16_t*>(b + L->off_bm_order)[j]; }
     __device__ const uint8_t* part_texels(int P, int e) const { return b + L->off_part_texel + ((size_t)(P - 2) * 1024 + e) * L->T; }
+    __device__ const uint32_t* part2(int P, int e) const { return reinterpret_cast<const uint32_t*>(b + L->off_part2) + ((size_t)(P - 2) * 1024 + e) * ((L->T + 15) >> 4); }
     __device__ int part_count(int P, int e, int q) const { return b[L->off_part_counts + ((P - 2) * 1024 + e) * 4 + q]; }
     __device__ uint32_t part_seed(int P, int e) const { return reinterpret_cast<const uint32_t*>(b + L->off_part_info)[(P - 2) * 1024 + e]; }
     __device__ uint64_t cov(int P, int e, int q) const { return reinterpret_cast<const uint64_t*>(b + L->off_cov)[((size_t)(P - 2) * 1024 + e) * 4 + q]; }
@@ -77,19 +78,53 @@ __device__ __forceinline__ float dist_sq(float4 a, float4 b) {
 }
 
 // ============================================================ passes 001-007
+// A warp searches one partition count of a block (small launches: a CTA of four warps, each
+// taking one of the four rounds of 32 candidates).  The kernel issues about a thousand
+// instructions per candidate and waits on instruction fetch, branches and the conversion pipe,
+// not on memory, so: loops are left rolled (18,400 -> 13,400 instructions for the three counts),
+// sort keys are 32 bits with the reference's partial network on registers and shuffles, the
+// mismatch is one matching over popcounts of the overlaps, texel partitions come two bits a
+// texel, and sums of truncated texels reuse the truncations.  Measured (B200): 11.6 -> 5.4 ms for
+// 65,536 4x4 blocks with FIXED semantics, 6.2 -> 1.1 ms for 9,888 10x8 blocks with the reference's.
 constexpr int kSearchWarps = 4;
-// Per warp: texels, 1024 sort keys, 128 + 128 candidate errors, k-means assignments, then
-// (FIXED semantics) the 128 first keys of the full order and a 132-bin histogram.
-constexpr int kSearchWarpBytes = 144 * 16 + 1024 * 8 + 128 * 4 * 2 + 160 + 128 * 8 + 132 * 4;
+constexpr int kSearchCtas = 5;
+// A launch of few items is as long as one item, so each gets a CTA's four warps then (the
+// clustering and the order are made four times, the errors once): up to two waves of CTAs.
+constexpr int kSearchWideItems = 148 * kSearchCtas * 2;
+constexpr int kSearchKeys = 1024;
+// Per warp: texels and their truncations, then the sort keys (dead once the order is known:
+// the same bytes hold each lane's partition averages and directions), the first 128 table
+// entries of the order, the counting sort's histogram, errors, k-means assignments.
+constexpr int kSearchLaneVecs = 4 * 3;  // per lane: average, direction, scale direction of P <= 4 partitions
+struct SearchLayout { int px, xi, key, ord, hist, eu, es, asg, zero, total; };
+__host__ __device__ inline SearchLayout search_layout(int T) {
+    SearchLayout f;
+    int o = 0;
+    auto take = [&](int bytes) { const int r = o; o += (bytes + 15) & ~15; return r; };
+    f.px = take(T * 16);
+    f.xi = take(T * 16);
+    f.key = take(kSearchLaneVecs * 32 * 16);
+    f.ord = take(kPartCandLimit * 2);
+    f.hist = take(132 * 4);
+    f.eu = take(kPartCandLimit * 4);
+    f.es = take(kPartCandLimit * 4);
+    f.asg = take(T);
+    f.zero = take(T);
+    f.total = o;
+    return f;
+}
+static_assert(kSearchLaneVecs * 32 * 16 >= kSearchKeys * 4, "the keys fit the lanes' vectors");
+constexpr uint32_t kNoEntry = 0x3FFFu;  // mismatch of an entry that is not selected: after all others
 
-// FIXED semantics of pass005 (full sort): the first 128 of all 1024 keys m << 32 | i in
-// ascending order, into ord.  The mismatch counts m of the sel selected entries are at most
-// 128 (the sum of P popcounts of 64-bit words, halved), so a stable counting sort by m in
-// index order gives the full order; entries i >= sel (m = 0xFFFFFFFF) keep rank i.
-__device__ void full_order(const unsigned long long* key, unsigned long long* ord, uint32_t* hist, uint32_t sel, int lane) {
+// FIXED semantics of pass005 (full sort): the table entries of the first 128 of all keys
+// m << 10 | i in ascending order, into ord.  The mismatch counts m of the sel selected entries
+// are at most 64, so a stable counting sort by m in index order gives the full order (sel is
+// above 128 for every footprint and partition count).
+__device__ __forceinline__ void full_order(const uint32_t* key, uint16_t* ord, uint32_t* hist, uint32_t sel, int lane) {
     for (int b = lane; b < 132; b += 32) hist[b] = 0;
     __syncwarp();
-    for (uint32_t i = lane; i < sel; i += 32) atomicAdd(&hist[(uint32_t)(key[i] >> 32)], 1u);
+#pragma unroll 1
+    for (uint32_t i = lane; i < sel; i += 32) atomicAdd(&hist[key[i] >> 10], 1u);
     __syncwarp();
     uint32_t v[5], s = 0;  // exclusive scan of bins 0..128, five per lane
 #pragma unroll
@@ -103,338 +138,489 @@ __device__ void full_order(const unsigned long long* key, unsigned long long* or
     for (int j = 0; j < 5; j++) { const int b = lane * 5 + j; if (b < 129) hist[b] = run; run += v[j]; }
     __syncwarp();
     const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t end = sel > 128u ? sel : 128u;
-    for (uint32_t base = 0; base < end; base += 32) {
+#pragma unroll 1
+    for (uint32_t base = 0; base < sel; base += 32) {
         const uint32_t i = base + lane;
-        const unsigned long long k = key[i];
-        const uint32_t m = (uint32_t)(k >> 32);
         const bool selected = i < sel;
-        const uint32_t grp = __match_any_sync(FULL, selected ? m : 0xFFFFFFFFu);
-        const uint32_t rank = selected ? hist[m] + __popc(grp & lt) : i;
-        if (rank < 128u) ord[rank] = k;
+        const uint32_t m = selected ? key[i] >> 10 : kNoEntry;
+        const uint32_t grp = __match_any_sync(FULL, m);
+        if (selected) {
+            const uint32_t rank = hist[m] + __popc(grp & lt);
+            if (rank < (uint32_t)kPartCandLimit) ord[rank] = (uint16_t)i;
+        }
         __syncwarp();
         if (selected && 31 - __clz(grp) == lane) hist[m] += __popc(grp);
         __syncwarp();
     }
-    __syncwarp();
 }
 
+// The reference's pass005: its bitonic network run by 256 invocations, which only compares
+// pairs whose lower index is below 256.  Keys 0..255 stay in registers (key lane + 32 r in
+// x[r]); only the two steps of distance 256 and 512 reach the others, in shared memory.
+__device__ __forceinline__ void partial_order(uint32_t* key, uint16_t* ord, int lane) {
+    uint32_t x[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) x[r] = key[lane + 32 * r];
+    auto within = [&](unsigned k, unsigned j) {  // one step of distance j < 256
+        if (j >= 32) {
+            const int jr = (int)(j >> 5);
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+#pragma unroll
+                for (int d = 1; d < 8; d <<= 1) {
+                    if ((r & d) || jr != d) continue;
+                    const bool asc = ((32u * r) & k) == 0;  // k > j >= 32: the lane does not enter
+                    const uint32_t lo = min(x[r], x[r | d]), hi = max(x[r], x[r | d]);
+                    x[r] = asc ? lo : hi;
+                    x[r | d] = asc ? hi : lo;
+                }
+            }
+        } else {
+            const bool lower = (lane & j) == 0;
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const uint32_t o = __shfl_xor_sync(FULL, x[r], j);
+                const bool asc = ((lane + 32 * r) & k) == 0;
+                x[r] = lower == asc ? min(x[r], o) : max(x[r], o);
+            }
+        }
+    };
+    auto across = [&](int d) {  // distance d >= 256, ascending (indices below 256)
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            uint32_t& o = key[lane + 32 * r + d];
+            const uint32_t lo = min(x[r], o), hi = max(x[r], o);
+            x[r] = lo;
+            o = hi;
+        }
+    };
+#pragma unroll 1
+    for (unsigned k = 2; k <= (unsigned)kSearchKeys; k <<= 1) {
+        if (k == 1024) across(512);
+        if (k >= 512) across(256);
+#pragma unroll 1
+        for (unsigned j = min(k >> 1, 128u); j > 0; j >>= 1) within(k, j);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++) ord[lane + 32 * r] = (uint16_t)(x[r] & 1023u);
+}
+
+// wide: this warp is one of four that search the same partition count of a block and only
+// takes round `round` of the candidates; the errors go to warp 0's arrays (eu0, es0), and the
+// CTA's barrier before pass007 is the caller's.
 template <int P>
-__device__ void search_one(const KernelArgs& a, int blk, int lb, uint8_t* ws, int lane) {
+__device__ __forceinline__ void search_errors(const KernelArgs& a, int blk, uint8_t* ws, int lane, bool wide, int round, float* eu0, float* es0) {
     const Tabs tb{a.tables, &a.L};
     const int T = a.L.T;
-    float4* px = reinterpret_cast<float4*>(ws);
-    unsigned long long* key = reinterpret_cast<unsigned long long*>(ws + 144 * 16);
-    float* eu = reinterpret_cast<float*>(ws + 144 * 16 + 1024 * 8);
-    float* es = eu + 128;
-    uint8_t* asg = reinterpret_cast<uint8_t*>(es + 128);
-    unsigned long long* ord_buf = reinterpret_cast<unsigned long long*>(ws + 144 * 16 + 1024 * 8 + 128 * 4 * 2 + 160);
-    uint32_t* hist = reinterpret_cast<uint32_t*>(ord_buf + 128);
+    const SearchLayout fl = search_layout(T);
+    float4* px = reinterpret_cast<float4*>(ws + fl.px);
+    uint4* xi = reinterpret_cast<uint4*>(ws + fl.xi);
+    uint32_t* key = reinterpret_cast<uint32_t*>(ws + fl.key);
+    uint16_t* ord = reinterpret_cast<uint16_t*>(ws + fl.ord);
+    uint8_t* asg = ws + fl.asg;
+    uint8_t* zero = ws + fl.zero;  // per texel: bit c set when channel c is 0
+    const float4 cw = chan_w();
     const BlockSrc src = block_src(a, blk);
-    for (int t = lane; t < T; t += 32) px[t] = src_texel(src, a.L.bx, t);
+    uint32_t u_all = 0;  // sum over all texels of f2u(|x|^2 weighted), the line error of a zero direction
+    bool any_zero = false;
+#pragma unroll 1
+    for (int t = lane; t < T; t += 32) {
+        const float4 x = src_texel(src, a.L.bx, t);
+        px[t] = x;
+        xi[t] = make_uint4(__float2uint_rz(x.x), __float2uint_rz(x.y), __float2uint_rz(x.z), __float2uint_rz(x.w));
+        const int z = (x.x > 0.0f ? 0 : 1) | (x.y > 0.0f ? 0 : 2) | (x.z > 0.0f ? 0 : 4) | (x.w > 0.0f ? 0 : 8);
+        zero[t] = (uint8_t)z;
+        any_zero |= z != 0;
+        u_all += f2u(dot4(x * x, cw));
+    }
+    any_zero = __any_sync(FULL, any_zero);
+    u_all = __reduce_add_sync(FULL, u_all);
     __syncwarp();
 
     // pass001: farthest-point initial centres; ties pick the highest texel index
     float4 c[P];
     c[0] = px[145897 % T];
-    float dist[5];
+    {
+        auto dist = [&](int t, int n) {  // to the nearest of the first n centres
+            float d = dist_sq(c[0], px[t]);
 #pragma unroll
-    for (int j = 0; j < 5; j++) { const int t = lane + 32 * j; dist[j] = t < T ? dist_sq(c[0], px[t]) : 0.0f; }
+            for (int q = 1; q < P; q++) if (q < n) d = fminf(d, dist_sq(c[q], px[t]));
+            return d;
+        };
 #pragma unroll
-    for (int pp = 1; pp < P; pp++) {
-        uint32_t mx = 0;
-#pragma unroll
-        for (int j = 0; j < 5; j++) if (lane + 32 * j < T) mx = max(mx, fbits(dist[j]));
-        mx = __reduce_max_sync(FULL, mx);
-        int idx = -1;
-#pragma unroll
-        for (int j = 0; j < 5; j++) if (lane + 32 * j < T && fbits(dist[j]) == mx) idx = lane + 32 * j;
-        idx = __reduce_max_sync(FULL, idx);
-        c[pp] = px[idx];
-        if (pp < P - 1) {
-#pragma unroll
-            for (int j = 0; j < 5; j++) { const int t = lane + 32 * j; if (t < T) dist[j] = fminf(dist[j], dist_sq(c[pp], px[t])); }
+        for (int pp = 1; pp < P; pp++) {
+            uint32_t mx = 0;
+            int idx = -1;
+#pragma unroll 1
+            for (int t = lane; t < T; t += 32) { const uint32_t d = fbits(dist(t, pp)); if (d >= mx) { mx = d; idx = t; } }
+            const uint32_t best = __reduce_max_sync(FULL, mx);
+            idx = __reduce_max_sync(FULL, mx == best ? idx : -1);
+            c[pp] = px[idx];
         }
     }
     // passes 002/003, four iterations
-    uint32_t as[5];
+#pragma unroll 1
     for (int it = 0; it < 4; it++) {
+        uint32_t have = 0;
+#pragma unroll 1
+        for (int t = lane; t < T; t += 32) {
+            float best = 1e30f;
+            uint32_t as = 0;
+            const float4 x = px[t];
 #pragma unroll
-        for (int j = 0; j < 5; j++) {
-            const int t = lane + 32 * j;
-            as[j] = 0;
-            if (t < T) {
-                float best = 1e30f;
-#pragma unroll
-                for (int q = 0; q < P; q++) { const float d = dist_sq(px[t], c[q]); if (d < best) { best = d; as[j] = q; } }
-            }
+            for (int q = 0; q < P; q++) { const float d = dist_sq(x, c[q]); if (d < best) { best = d; as = q; } }
+            asg[t] = (uint8_t)as;
+            have |= 1u << as;
         }
-        bool problem = false;
-#pragma unroll
-        for (int q = 0; q < P; q++) {
-            int n = 0;
-#pragma unroll
-            for (int j = 0; j < 5; j++) n += __popc(__ballot_sync(FULL, lane + 32 * j < T && as[j] == (uint32_t)q));
-            if (n == 0) problem = true;
-        }
-        if (problem && lane < P) as[0] = lane;
+        have = __reduce_or_sync(FULL, have);
+        if (have != (1u << P) - 1u && lane < P) asg[lane] = (uint8_t)lane;  // an empty cluster
 #pragma unroll
         for (int q = 0; q < P; q++) {
             uint32_t n = 0, s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-#pragma unroll
-            for (int j = 0; j < 5; j++) {
-                const int t = lane + 32 * j;
-                if (t < T && as[j] == (uint32_t)q) {
-                    n++; s0 += f2u(px[t].x); s1 += f2u(px[t].y); s2 += f2u(px[t].z); s3 += f2u(px[t].w);
-                }
-            }
+#pragma unroll 1
+            for (int t = lane; t < T; t += 32)
+                if (asg[t] == q) { const uint4 x = xi[t]; n++; s0 += x.x; s1 += x.y; s2 += x.z; s3 += x.w; }
             n = __reduce_add_sync(FULL, n);
             s0 = __reduce_add_sync(FULL, s0); s1 = __reduce_add_sync(FULL, s1);
             s2 = __reduce_add_sync(FULL, s2); s3 = __reduce_add_sync(FULL, s3);
-            if (n > 0) {
-                const float fc = (float)n;
-                c[q] = make_float4((float)s0 / fc, (float)s1 / fc, (float)s2 / fc, (float)s3 / fc);
-            } else {
-                c[q] = mk(0.0f);
-            }
+            c[q] = mk(0.0f);
+            if (n > 0) { const float fc = (float)n; c[q] = make_float4((float)s0 / fc, (float)s1 / fc, (float)s2 / fc, (float)s3 / fc); }
         }
     }
-#pragma unroll
-    for (int j = 0; j < 5; j++) { const int t = lane + 32 * j; if (t < T) asg[t] = (uint8_t)as[j]; }
     __syncwarp();
-    // pass004: k-means bitmaps over the 64 k-means texels, mismatch per partitioning
+    // pass004: k-means bitmaps over the 64 k-means texels, mismatch per partitioning.  The
+    // mismatch is half the smallest sum over assignments x -> y of popc(km_x ^ cov_y); the xor
+    // counts popc(km_x) + popc(cov_y) - 2 popc(km_x & cov_y), whose first two terms sum to the
+    // same total for every assignment, so it is half that total less the largest matching over
+    // the overlaps n.  The cov of an entry split the first min(T, 64) bits between them, and so
+    // do the km, so the overlaps of the last row and column follow from the others.
+    const int nbits = min(T, 64);
     uint64_t km[P];
+    int kn[P];  // of the first nbits
     {
         const int k0 = asg[a.L.kmeans[lane]], k1 = asg[a.L.kmeans[lane + 32]];
+        const uint64_t valid = nbits == 64 ? ~0ull : (1ull << nbits) - 1;
 #pragma unroll
         for (int q = 0; q < P; q++) {
             const uint32_t lo = __ballot_sync(FULL, k0 == q), hi = __ballot_sync(FULL, k1 == q);
-            km[q] = (uint64_t)lo | ((uint64_t)hi << 32);
+            km[q] = ((uint64_t)lo | ((uint64_t)hi << 32)) & valid;
+            kn[q] = __popcll(km[q]);
         }
     }
+    const uint32_t half_total = (uint32_t)(64 + nbits) / 2;
     const uint32_t sel = a.L.count_selected[P - 1];
-    for (int i = lane; i < 1024; i += 32) {
-        uint32_t m = 0xFFFFFFFFu;
-        if ((uint32_t)i < sel) {
-            uint32_t p[P][P];
+    const uint32_t nkeys = a.fixed ? (sel + 31u) & ~31u : (uint32_t)kSearchKeys;
+#pragma unroll 1
+    for (uint32_t i = lane; i < nkeys; i += 32) {
+        uint32_t m = kNoEntry;
+        if (i < sel) {
+            int n[P][P], rest = nbits;
 #pragma unroll
-            for (int x = 0; x < P; x++)
+            for (int y = 0; y < P - 1; y++) {
+                const uint64_t cv = tb.cov(P, i, y);
+                int col = T <= 32 ? __popc((uint32_t)cv) : __popcll(cv);
+                rest -= col;
 #pragma unroll
-                for (int y = 0; y < P; y++) p[x][y] = __popcll(km[x] ^ tb.cov(P, i, y));
-            if (P == 2) {
-                m = min(p[0][0] + p[1][1], p[0][1] + p[1][0]) / 2;
-            } else if (P == 3) {
-                const uint32_t v0 = min(p[1][1] + p[2][2], p[1][2] + p[2][1]) + p[0][0];
-                const uint32_t v1 = min(p[1][0] + p[2][2], p[1][2] + p[2][0]) + p[0][1];
-                const uint32_t v2 = min(p[1][0] + p[2][1], p[1][1] + p[2][0]) + p[0][2];
-                m = min(v0, min(v1, v2)) / 2;
-            } else {
-                const uint32_t mx23 = min(p[2][2] + p[3][3], p[2][3] + p[3][2]);
-                const uint32_t mx13 = min(p[2][1] + p[3][3], p[2][3] + p[3][1]);
-                const uint32_t mx12 = min(p[2][1] + p[3][2], p[2][2] + p[3][1]);
-                const uint32_t mx03 = min(p[2][0] + p[3][3], p[2][3] + p[3][0]);
-                const uint32_t mx02 = min(p[2][0] + p[3][2], p[2][2] + p[3][0]);
-                const uint32_t mx01 = min(p[2][1] + p[3][0], p[2][0] + p[3][1]);
-                const uint32_t v0 = p[0][0] + min(p[1][1] + mx23, min(p[1][2] + mx13, p[1][3] + mx12));
-                const uint32_t v1 = p[0][1] + min(p[1][0] + mx23, min(p[1][2] + mx03, p[1][3] + mx02));
-                const uint32_t v2 = p[0][2] + min(p[1][1] + mx03, min(p[1][0] + mx13, p[1][3] + mx01));
-                const uint32_t v3 = p[0][3] + min(p[1][1] + mx02, min(p[1][2] + mx01, p[1][0] + mx12));
-                m = min(v0, min(v1, min(v2, v3))) / 2;
+                for (int x = 0; x < P - 1; x++) {
+                    n[x][y] = T <= 32 ? __popc((uint32_t)km[x] & (uint32_t)cv) : __popcll(km[x] & cv);
+                    col -= n[x][y];
+                }
+                n[P - 1][y] = col;
             }
+#pragma unroll
+            for (int x = 0; x < P - 1; x++) {
+                int r = kn[x];
+#pragma unroll
+                for (int y = 0; y < P - 1; y++) r -= n[x][y];
+                n[x][P - 1] = r;
+                rest -= r;
+            }
+            n[P - 1][P - 1] = rest;
+            int best;
+            if (P == 2) {
+                best = max(n[0][0] + n[P - 1][P - 1], n[0][P - 1] + n[P - 1][0]);
+            } else if (P == 3) {
+                best = max(n[0][0] + max(n[1][1] + n[P - 1][P - 1], n[1][P - 1] + n[P - 1][1]),
+                           max(n[0][1] + max(n[1][0] + n[P - 1][P - 1], n[1][P - 1] + n[P - 1][0]),
+                               n[0][P - 1] + max(n[1][0] + n[P - 1][1], n[1][1] + n[P - 1][0])));
+            } else {
+                best = 0;
+#pragma unroll
+                for (int x = 0; x < 4; x++)
+#pragma unroll
+                    for (int y = x + 1; y < 4; y++) {  // rows 0, 1 on columns x, y, rows 2, 3 on the others
+                        const int u = x == 0 ? (y == 1 ? 2 : 1) : 0, v = 6 - x - y - u;
+                        const int top = max(n[0][x] + n[1][y], n[0][y] + n[1][x]);
+                        const int bot = max(n[P - 2][u] + n[P - 1][v], n[P - 2][v] + n[P - 1][u]);
+                        best = max(best, top + bot);
+                    }
+            }
+            m = half_total - (uint32_t)best;
         }
-        key[i] = ((unsigned long long)m << 32) | (uint32_t)i;
+        key[i] = m << 10 | i;
     }
     __syncwarp();
-    // pass005: the reference's bitonic network run by 256 invocations (a partial sort); FIXED
-    // semantics: the full order
-    const unsigned long long* ord = key;
-    if (a.fixed) {
-        full_order(key, ord_buf, hist, sel, lane);
-        ord = ord_buf;
-    }
-    for (unsigned k = 2; k <= 1024 && !a.fixed; k <<= 1)
-        for (unsigned j = k >> 1; j > 0; j >>= 1) {
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const unsigned l = lane + 32 * r, partner = l ^ j;
-                if (partner > l) {
-                    const bool asc = (l & k) == 0;
-                    const unsigned long long x = key[l], y = key[partner];
-                    if ((x > y) == asc) { key[l] = y; key[partner] = x; }
-                }
-            }
-            __syncwarp();
-        }
+    if (a.fixed) full_order(key, ord, reinterpret_cast<uint32_t*>(ws + fl.hist), sel, lane);
+    else partial_order(key, ord, lane);
+    __syncwarp();
     // pass006: error estimate of the first 128 ordered partitionings.  The
     // shader keeps avg/dir in per-invocation arrays, so texel t only sees its
     // own partition's average/direction when t < P and its partition is t.
     float wie = T <= 20 ? 0.03f : T <= 31 ? 0.04f : T <= 41 ? 0.05f : 0.055f;
     wie = wie * wie;
-    const float4 cw = chan_w();
-    uint32_t u_all = 0;  // sum over all texels of f2u(|x|^2 weighted), the line error of a zero direction
-    for (int t = lane; t < T; t += 32) { const float4 x = px[t]; u_all += f2u(dot4(x * x, cw)); }
-    for (int o = 16; o > 0; o >>= 1) u_all += __shfl_xor_sync(FULL, u_all, o);
-    for (int r = 0; r < 4; r++) {
+    float4* lv = reinterpret_cast<float4*>(key) + lane;  // lane's vectors: (3 q + kind) * 32
+#pragma unroll 1
+    for (int r = wide ? round : 0; r < (wide ? round + 1 : 4); r++) {
         const int cand = lane + 32 * r;
-        const int e = (int)(uint32_t)ord[cand];
-        const uint8_t* row = tb.part_texels(P, e);
+        const int e = ord[cand];
+        const uint32_t* row = tb.part2(P, e);
+        // counts and sums of the truncated texels; partition 0's are what the others leave
         uint32_t cnt[P], sm[P][4];
 #pragma unroll
         for (int q = 0; q < P; q++) { cnt[q] = 0; sm[q][0] = sm[q][1] = sm[q][2] = sm[q][3] = 0; }
-        for (int t = 0; t < T; t++) {
-            const int p = row[t];
-            const float4 x = px[t];
-            const uint32_t u0 = f2u(x.x), u1 = f2u(x.y), u2 = f2u(x.z), u3 = f2u(x.w);
+#pragma unroll 1
+        for (int w0 = 0; w0 < T; w0 += 16) {
+            uint32_t w = row[w0 >> 4];
+            const int tn = min(T - w0, 16);
+#pragma unroll 1
+            for (int t = 0; t < tn; t++, w >>= 2) {
+                const uint32_t p = w & 3u;
+                const uint4 x = xi[w0 + t];
+                sm[0][0] += x.x; sm[0][1] += x.y; sm[0][2] += x.z; sm[0][3] += x.w;
 #pragma unroll
-            for (int q = 0; q < P; q++) if (p == q) { cnt[q]++; sm[q][0] += u0; sm[q][1] += u1; sm[q][2] += u2; sm[q][3] += u3; }
+                for (int q = 1; q < P; q++) if (p == (uint32_t)q) { cnt[q]++; sm[q][0] += x.x; sm[q][1] += x.y; sm[q][2] += x.z; sm[q][3] += x.w; }
+            }
         }
-        float4 tavg[P], tdir[P];
+        cnt[0] = (uint32_t)T;
+#pragma unroll
+        for (int q = 1; q < P; q++) {
+            cnt[0] -= cnt[q];
+#pragma unroll
+            for (int ch = 0; ch < 4; ch++) sm[0][ch] -= sm[q][ch];
+        }
+        uint32_t usum = u_all, ssum = 0u - (uint32_t)T;
+        const uint32_t w_first = row[0];
 #pragma unroll
         for (int q = 0; q < P; q++) {
             const float fc = (float)cnt[q];
-            tavg[q] = fc > 0.0f ? make_float4((float)sm[q][0] / fc, (float)sm[q][1] / fc, (float)sm[q][2] / fc, (float)sm[q][3] / fc) : mk(0.0f);
-        }
-#pragma unroll
-        for (int q = 0; q < P; q++) {
+            const float4 tavg = fc > 0.0f ? make_float4((float)sm[q][0] / fc, (float)sm[q][1] / fc, (float)sm[q][2] / fc, (float)sm[q][3] / fc) : mk(0.0f);
             uint32_t ax[4][4];
+            const bool own = ((w_first >> (2 * q)) & 3u) == (uint32_t)q;  // texel q is in partition q
+            if (a.fixed) {
+                // sums of the deviations along each positive half axis, over the partition's texels
 #pragma unroll
-            for (int u = 0; u < 4; u++) ax[u][0] = ax[u][1] = ax[u][2] = ax[u][3] = 0;
-            for (int t = 0; t < T; t++) {
-                if (row[t] != q) continue;
-                const float4 av = (a.fixed || t == q) ? tavg[q] : mk(0.0f);
-                const float4 d = px[t] - av;
-                const uint32_t d0 = (uint32_t)f2i(d.x), d1 = (uint32_t)f2i(d.y), d2 = (uint32_t)f2i(d.z), d3 = (uint32_t)f2i(d.w);
-                if (d.x > 0.0f) { ax[0][0] += d0; ax[0][1] += d1; ax[0][2] += d2; ax[0][3] += d3; }
-                if (d.y > 0.0f) { ax[1][0] += d0; ax[1][1] += d1; ax[1][2] += d2; ax[1][3] += d3; }
-                if (d.z > 0.0f) { ax[2][0] += d0; ax[2][1] += d1; ax[2][2] += d2; ax[2][3] += d3; }
-                if (d.w > 0.0f) { ax[3][0] += d0; ax[3][1] += d1; ax[3][2] += d2; ax[3][3] += d3; }
+                for (int u = 0; u < 4; u++) ax[u][0] = ax[u][1] = ax[u][2] = ax[u][3] = 0;
+#pragma unroll 1
+                for (int w0 = 0; w0 < T; w0 += 16) {
+                    uint32_t w = row[w0 >> 4] ^ (0x55555555u * (uint32_t)q);
+                    w = ~(w | w >> 1) & 0x55555555u;
+                    if (T - w0 < 16) w &= (1u << (2 * (T - w0))) - 1u;
+                    while (w) {
+                        const int t = w0 + ((__ffs(w) - 1) >> 1);
+                        w &= w - 1;
+                        const float4 d = px[t] - tavg;
+                        const uint32_t d0 = (uint32_t)__float2int_rz(d.x), d1 = (uint32_t)__float2int_rz(d.y);
+                        const uint32_t d2 = (uint32_t)__float2int_rz(d.z), d3 = (uint32_t)__float2int_rz(d.w);
+                        if (d.x > 0.0f) { ax[0][0] += d0; ax[0][1] += d1; ax[0][2] += d2; ax[0][3] += d3; }
+                        if (d.y > 0.0f) { ax[1][0] += d0; ax[1][1] += d1; ax[1][2] += d2; ax[1][3] += d3; }
+                        if (d.z > 0.0f) { ax[2][0] += d0; ax[2][1] += d1; ax[2][2] += d2; ax[2][3] += d3; }
+                        if (d.w > 0.0f) { ax[3][0] += d0; ax[3][1] += d1; ax[3][2] += d2; ax[3][3] += d3; }
+                    }
+                }
+            } else {
+                // Every texel but texel q sees a zero average: its deviation is itself, so the
+                // sums along axis u are the partition's less the texels whose channel u is 0;
+                // texel q, when it is of partition q, sees the average.
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+#pragma unroll
+                    for (int ch = 0; ch < 4; ch++) ax[u][ch] = sm[q][ch];
+                if (any_zero) {
+#pragma unroll 1
+                    for (int t = 0; t < T; t++) {
+                        const int z = zero[t];
+                        if (z == 0) continue;  // the same for every lane
+                        if (((row[t >> 4] >> (2 * (t & 15))) & 3u) != (uint32_t)q) continue;
+                        const uint4 x = xi[t];
+#pragma unroll
+                        for (int u = 0; u < 4; u++)
+                            if ((z >> u) & 1) { ax[u][0] -= x.x; ax[u][1] -= x.y; ax[u][2] -= x.z; ax[u][3] -= x.w; }
+                    }
+                }
+                if (own) {
+                    const uint4 x = xi[q];
+                    const int z = zero[q];
+                    const float4 d = px[q] - tavg;
+                    const uint32_t d0 = (uint32_t)__float2int_rz(d.x), d1 = (uint32_t)__float2int_rz(d.y);
+                    const uint32_t d2 = (uint32_t)__float2int_rz(d.z), d3 = (uint32_t)__float2int_rz(d.w);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        if (!((z >> u) & 1)) { ax[u][0] -= x.x; ax[u][1] -= x.y; ax[u][2] -= x.z; ax[u][3] -= x.w; }
+                        if (comp(d, u) > 0.0f) { ax[u][0] += d0; ax[u][1] += d1; ax[u][2] += d2; ax[u][3] += d3; }
+                    }
+                }
             }
-            float4 s[4];
+            float4 best = mk(0.0f);
+            float mp = 0.0f;
 #pragma unroll
-            for (int u = 0; u < 4; u++) s[u] = make_float4((float)(int32_t)ax[u][0], (float)(int32_t)ax[u][1], (float)(int32_t)ax[u][2], (float)(int32_t)ax[u][3]);
-            float4 best = s[0];
-            float mp = dot4(s[0], s[0]);
-#pragma unroll
-            for (int u = 1; u < 4; u++) { const float pr = dot4(s[u], s[u]); if (pr > mp) { mp = pr; best = s[u]; } }
-            tdir[q] = normalize4(best);
+            for (int u = 0; u < 4; u++) {
+                const float4 s = make_float4((float)(int32_t)ax[u][0], (float)(int32_t)ax[u][1], (float)(int32_t)ax[u][2], (float)(int32_t)ax[u][3]);
+                const float pr = dot4(s, s);
+                if (u == 0 || pr > mp) { mp = pr; best = s; }
+            }
+            const float4 tdir = normalize4(best);
+            if (a.fixed) {
+                lv[(3 * q) * 32] = tavg;
+                lv[(3 * q + 1) * 32] = tdir;
+                lv[(3 * q + 2) * 32] = normalize4(tavg);
+            } else {
+                // Every texel but those t < P of partition t sees a zero average and direction: its
+                // projection is 0, its line error |x|^2 (weighted) and its scale error NaN (the zero
+                // direction's normalisation), so f2u gives 0xFFFFFFFF.  The integer sums take those
+                // terms for every texel at once (u_all, -T) and the few texels that see their
+                // partition's own average and direction are corrected; integer sums do not depend
+                // on their order.
+                int32_t lmin = 2147483647, lmax = -2147483647;
+                if (own) {
+                    const float4 x = px[q];
+                    usum -= f2u(dot4(x * x, cw));
+                    ssum += 1u;
+                    const float up = dot4(x, tdir);
+                    const float4 uproj = tavg + tdir * dot4(x - tavg, tdir);
+                    const float4 udiff = x - uproj;
+                    const float4 sd = normalize4(tavg);
+                    const float4 sproj = sd * dot4(x, sd);
+                    const float4 sdiff = x - sproj;
+                    usum += f2u(dot4(udiff * udiff, cw));
+                    ssum += f2u(dot4(sdiff * sdiff, cw));
+                    const int32_t upi = f2i(up * 4096.0f);
+                    lmin = min(lmin, upi); lmax = max(lmax, upi);
+                }
+                if ((int)cnt[q] > (own ? 1 : 0)) { lmin = min(lmin, 0); lmax = max(lmax, 0); }  // a texel of projection 0
+                lv[(3 * q) * 32] = make_float4(__int_as_float(lmin), __int_as_float(lmax), q == 0 ? dot4(tavg, tavg) : 0.0f, 0.0f);
+            }
         }
-        // Every texel but those t < P of partition t sees a zero average and direction: its
-        // projection is 0, its line error |x|^2 (weighted) and its scale error NaN (the zero
-        // direction's normalisation), so f2u gives 0xFFFFFFFF.  The integer sums take those
-        // terms for every texel at once (u_all, -T) and the loop corrects the few texels
-        // that see their partition's own average and direction; integer sums do not depend
-        // on their order.
-        uint32_t usum = u_all, ssum = 0u - (uint32_t)T;
         int32_t lmin[P], lmax[P];
-#pragma unroll
-        for (int q = 0; q < P; q++) { lmin[q] = 2147483647; lmax[q] = -2147483647; }
         if (a.fixed) {  // every texel sees its partition's average and direction
-            float4 sdir[P];
-#pragma unroll
-            for (int q = 0; q < P; q++) sdir[q] = normalize4(tavg[q]);
             usum = 0u; ssum = 0u;
-            for (int t = 0; t < T; t++) {
-                const int p = row[t];
-                float4 av = tavg[0], ud = tdir[0], sd = sdir[0];
 #pragma unroll
-                for (int q = 1; q < P; q++) if (p == q) { av = tavg[q]; ud = tdir[q]; sd = sdir[q]; }
-                const float4 x = px[t];
-                const float up = dot4(x, ud);
-                const float4 uproj = av + ud * dot4(x - av, ud);
-                const float4 udiff = x - uproj;
-                usum += f2u(dot4(udiff * udiff, cw));
-                const float4 sproj = sd * dot4(x, sd);
-                const float4 sdiff = x - sproj;
-                ssum += f2u(dot4(sdiff * sdiff, cw));
-                const int32_t upi = f2i(up * 4096.0f);
+            for (int q = 0; q < P; q++) { lmin[q] = 2147483647; lmax[q] = -2147483647; }
+#pragma unroll 1
+            for (int w0 = 0; w0 < T; w0 += 16) {
+                uint32_t w = row[w0 >> 4];
+                const int tn = min(T - w0, 16);
+#pragma unroll 1
+                for (int t = 0; t < tn; t++, w >>= 2) {
+                    const int p = (int)(w & 3u);
+                    const float4 av = lv[(3 * p) * 32], ud = lv[(3 * p + 1) * 32], sd = lv[(3 * p + 2) * 32];
+                    const float4 x = px[w0 + t];
+                    const float up = dot4(x, ud);
+                    const float4 uproj = av + ud * dot4(x - av, ud);
+                    const float4 udiff = x - uproj;
+                    usum += f2u(dot4(udiff * udiff, cw));
+                    const float4 sproj = sd * dot4(x, sd);
+                    const float4 sdiff = x - sproj;
+                    ssum += f2u(dot4(sdiff * sdiff, cw));
+                    const int32_t upi = f2i(up * 4096.0f);
 #pragma unroll
-                for (int q = 0; q < P; q++) if (p == q) { lmin[q] = min(lmin[q], upi); lmax[q] = max(lmax[q], upi); }
+                    for (int q = 0; q < P; q++) if (p == q) { lmin[q] = min(lmin[q], upi); lmax[q] = max(lmax[q], upi); }
+                }
             }
         }
-#pragma unroll
-        for (int t = 0; t < P && !a.fixed; t++) {
-            if (row[t] != t) continue;
-            const float4 av = tavg[t], ud = tdir[t];
-            const float4 x = px[t];
-            usum -= f2u(dot4(x * x, cw));
-            ssum += 1u;
-            const float up = dot4(x, ud);
-            const float4 uproj = av + ud * dot4(x - av, ud);
-            const float4 udiff = x - uproj;
-            const float ud2 = dot4(udiff * udiff, cw);
-            const float4 sd = normalize4(av);
-            const float4 sproj = sd * dot4(x, sd);
-            const float4 sdiff = x - sproj;
-            const float sd2 = dot4(sdiff * sdiff, cw);
-            usum += f2u(ud2);
-            ssum += f2u(sd2);
-            const int32_t upi = f2i(up * 4096.0f);
-            lmin[t] = min(lmin[t], upi); lmax[t] = max(lmax[t], upi);
-        }
-#pragma unroll
-        for (int q = 0; q < P; q++)  // the partition has a texel of projection 0
-            if (!a.fixed && tb.part_count(P, e, q) > (row[q] == q ? 1 : 0)) { lmin[q] = min(lmin[q], 0); lmax[q] = max(lmax[q], 0); }
         float tu = (float)usum, ts = (float)ssum;
 #pragma unroll
         for (int q = 0; q < P; q++) {
+            float sq;  // |average|^2 the scale term sees
+            if (a.fixed) {
+                const float4 a0 = lv[(3 * q) * 32];
+                sq = dot4(a0, a0);
+            } else {
+                const float4 v = lv[(3 * q) * 32];
+                lmin[q] = __float_as_int(v.x); lmax[q] = __float_as_int(v.y);
+                sq = v.z;
+            }
             const float mn = (float)lmin[q] / 4096.0f, mxv = (float)lmax[q] / 4096.0f;
             const float ll = fmaxf(mxv - mn, 1e-7f);
-            const float ew = (float)tb.part_count(P, e, q) * wie;
+            const float ew = (float)cnt[q] * wie;
             tu = tu + ew * (ll * ll);
-            const float4 a0 = (q == 0 || a.fixed) ? tavg[q] : mk(0.0f);
-            ts = ts + ew * dot4(a0, a0);
+            ts = ts + ew * sq;
         }
-        eu[cand] = tu;
-        es[cand] = ts;
-    }
-    __syncwarp();
-    // pass007: best 4 by each error, interleaved and deduplicated; the rank is
-    // used as the table entry (REF-BUG-4, pass007:93,156)
-    if (lane == 0) {
-        uint32_t bui[4] = {0, 0, 0, 0}, bsi[4] = {0, 0, 0, 0};
-        float bue[4] = {1e30f, 1e30f, 1e30f, 1e30f}, bse[4] = {1e30f, 1e30f, 1e30f, 1e30f};
-        for (int i = 0; i < 128; i++) {
-            const float u = eu[i], s = es[i];
-            if (u < bue[3]) {
-                bue[3] = u; bui[3] = i;
-                for (int j = 3; j > 0; j--)
-                    if (bue[j] < bue[j - 1]) { float te = bue[j]; bue[j] = bue[j - 1]; bue[j - 1] = te; uint32_t ti = bui[j]; bui[j] = bui[j - 1]; bui[j - 1] = ti; }
-            }
-            if (s < bse[3]) {
-                bse[3] = s; bsi[3] = i;
-                for (int j = 3; j > 0; j--)
-                    if (bse[j] < bse[j - 1]) { float te = bse[j]; bse[j] = bse[j - 1]; bse[j - 1] = te; uint32_t ti = bsi[j]; bsi[j] = bsi[j - 1]; bsi[j - 1] = ti; }
-            }
-        }
-        uint32_t fin[4] = {0, 0, 0, 0};
-        int emitted = 0;
-        for (int i = 0; i < 8 && emitted < 4; i++) {
-            const uint32_t idx = (i & 1) ? bsi[i >> 1] : bui[i >> 1];
-            bool seen = false;
-            for (int j = 0; j < emitted; j++) seen |= fin[j] == idx;
-            if (!seen) fin[emitted++] = idx;
-        }
-        uint16_t* out = a.picks[lb].v + (P - 2) * 5;
-        // FIXED semantics: the table entry the candidate was evaluated for
-        for (int i = 0; i < 4; i++) out[i] = (uint16_t)(a.fixed && i < emitted ? (uint32_t)ord[fin[i]] : fin[i]);
-        out[4] = (uint16_t)emitted;
+        eu0[cand] = tu;
+        es0[cand] = ts;
     }
 }
 
-__global__ void __launch_bounds__(kSearchWarps * 32) k_partition_search(const __grid_constant__ KernelArgs a) {
+// pass007 by one warp: the best 4 by each error (value, then rank), interleaved and
+// deduplicated; the rank is used as the table entry (REF-BUG-4, pass007:93,156), in FIXED
+// semantics the entry of that rank.
+__device__ __forceinline__ void search_picks(const KernelArgs& a, int P, int lb, const float* eu, const float* es, const uint16_t* ord, int lane) {
+    uint32_t best[2][4];
+#pragma unroll 1
+    for (int kind = 0; kind < 2; kind++) {
+        const float* v = kind ? es : eu;
+        uint32_t taken = 0;  // rounds of this lane already picked
+        uint32_t got[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            float mv = 1e30f;
+            int mr = -1;
+#pragma unroll
+            for (int r = 0; r < 4; r++) { const float x = v[lane + 32 * r]; if (!((taken >> r) & 1) && x < mv) { mv = x; mr = r; } }
+            const uint32_t bits = mr >= 0 ? fbits(mv) : 0xFFFFFFFFu;  // the errors are never negative
+            const uint32_t mn = __reduce_min_sync(FULL, bits);
+            const uint32_t idx = mr >= 0 ? (uint32_t)(lane + 32 * mr) : 0xFFFFFFFFu;
+            const uint32_t win = mn == 0xFFFFFFFFu ? 0xFFFFFFFFu : __reduce_min_sync(FULL, bits == mn ? idx : 0xFFFFFFFFu);
+            if (win == idx && mr >= 0) taken |= 1u << mr;
+            got[j] = win == 0xFFFFFFFFu ? 0u : win;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) { if (kind) best[1][j] = got[j]; else best[0][j] = got[j]; }
+    }
+    uint32_t fin[4] = {0, 0, 0, 0};
+    int emitted = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t idx = best[i & 1][i >> 1];
+        bool seen = emitted >= 4;
+#pragma unroll
+        for (int j = 0; j < 4; j++) seen |= j < emitted && fin[j] == idx;
+#pragma unroll
+        for (int j = 0; j < 4; j++) if (!seen && j == emitted) fin[j] = idx;
+        emitted += seen ? 0 : 1;
+    }
+    uint16_t* out = a.picks[lb].v + (P - 2) * 5;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (lane == i) out[i] = (uint16_t)(a.fixed && i < emitted ? (uint32_t)ord[fin[i]] : fin[i]);
+    if (lane == 4) out[4] = (uint16_t)emitted;
+}
+
+__host__ __device__ inline bool search_wide(int items) { return items <= kSearchWideItems; }
+
+__global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtas) k_partition_search(const __grid_constant__ KernelArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t* ws = smem + warp * kSearchWarpBytes;
+    const SearchLayout fl = search_layout(a.L.T);
     const int nb = list_blocks(a);
+    const bool wide = search_wide(nb * 3);
+    uint8_t* ws = smem + warp * fl.total;
+    uint8_t* w0 = wide ? smem : ws;  // where the errors and the order are read for pass007
+    float* eu = reinterpret_cast<float*>(w0 + fl.eu);
+    float* es = reinterpret_cast<float*>(w0 + fl.es);
     // P-major items: a CTA's warps share P; one pass for a chunk, a grid-stride loop over a block list
-    for (int item = blockIdx.x * kSearchWarps + warp; item < nb * 3; item += gridDim.x * kSearchWarps) {
+    const int first = wide ? blockIdx.x : blockIdx.x * kSearchWarps + warp, step = wide ? gridDim.x : gridDim.x * kSearchWarps;
+    for (int item = first; item < nb * 3; item += step) {
         const int lb = item % nb, P = item / nb + 2;
         const int blk = chunk_block(a, lb);
-        if (P == 2) search_one<2>(a, blk, lb, ws, lane);
-        else if (P == 3) search_one<3>(a, blk, lb, ws, lane);
-        else search_one<4>(a, blk, lb, ws, lane);
-        if (a.work && lane == 0) atomicAdd(a.work + 10 + (P - 2), 1ull);
-        __syncwarp();
+        if (P == 2) search_errors<2>(a, blk, ws, lane, wide, warp, eu, es);
+        else if (P == 3) search_errors<3>(a, blk, ws, lane, wide, warp, eu, es);
+        else search_errors<4>(a, blk, ws, lane, wide, warp, eu, es);
+        if (wide) __syncthreads(); else __syncwarp();
+        if (!wide || warp == 0) {
+            search_picks(a, P, lb, eu, es, reinterpret_cast<const uint16_t*>(w0 + fl.ord), lane);
+            if (a.work && lane == 0) atomicAdd(a.work + 10 + (P - 2), 1ull);
+        }
+        if (wide) __syncthreads(); else __syncwarp();
     }
 }
 
@@ -1313,7 +1499,7 @@ __global__ void __launch_bounds__(NT, kFrontMinBlocks128 * 128 / NT > 32 ? 32 : 
 
 }  // namespace
 
-size_t search_smem_bytes(const TableLayout&) { return (size_t)kSearchWarps * kSearchWarpBytes; }
+size_t search_smem_bytes(const TableLayout& L) { return (size_t)kSearchWarps * search_layout(L.T).total; }
 size_t front_smem_bytes(const TableLayout& L, int nt, bool list) { return (size_t)front_layout(L.T, L.ndm, L.nbm, L.max_w, nt, list).total; }
 
 // front_bytes: the 128-thread layout, the largest of the three.
@@ -1330,8 +1516,8 @@ cudaError_t configure_search_kernels(size_t search_bytes, size_t front_bytes) {
 
 cudaError_t launch_partition_search(const KernelArgs& a, cudaStream_t s) {
     const int items = a.nblocks * 3;
-    int grid = (items + kSearchWarps - 1) / kSearchWarps;
-    if (a.block_list) grid = std::min(grid, kListGridSearch);
+    int grid = search_wide(items) ? items : (items + kSearchWarps - 1) / kSearchWarps;
+    if (a.block_list) grid = std::min(items, kListGridSearch);
     k_partition_search<<<grid, kSearchWarps * 32, search_smem_bytes(a.L), s>>>(a);
     return cudaGetLastError();
 }

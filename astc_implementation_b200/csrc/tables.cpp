@@ -532,13 +532,15 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
         bms[i] = DevBm{(uint16_t)b.mode, (uint8_t)h.valid_bms[i].second, (uint8_t)b.quant, (uint8_t)b.bits, {0, 0, 0}};
     }
     std::vector<uint8_t> ptex((size_t)3 * 1024 * T), pcnt((size_t)3 * 1024 * 4);
-    std::vector<uint32_t> pinfo(3 * 1024);
+    const int part2_words = (T + 15) / 16;
+    std::vector<uint32_t> pinfo(3 * 1024), part2((size_t)3 * 1024 * part2_words, 0);
     std::vector<uint64_t> cov((size_t)3 * 1024 * 4, 0);
     for (int pc = 2; pc <= 4; pc++)
         for (int e = 0; e < 1024; e++) {
             const HostTables::Part& p = h.parts[(pc - 2) * 1024 + e];
             const size_t k = (size_t)(pc - 2) * 1024 + e;
             std::memcpy(&ptex[k * T], p.of, T);
+            for (int t = 0; t < T; t++) part2[k * part2_words + t / 16] |= (uint32_t)p.of[t] << (2 * (t & 15));
             for (int q = 0; q < 4; q++) pcnt[k * 4 + q] = (uint8_t)p.tcount[q];
             pinfo[k] = p.seed;
             for (int q = 0; q < pc; q++) cov[k * 4 + q] = h.cov[pc][(size_t)e * pc + q];
@@ -567,6 +569,7 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     L.off_bm_order = put(blob, order.data(), order.size());
     L.off_dual = put(blob, dual.data(), dual.size());
     L.off_part_texel = put(blob, ptex.data(), ptex.size());
+    L.off_part2 = put(blob, part2.data(), part2.size());
     L.off_part_info = put(blob, pinfo.data(), pinfo.size());
     L.off_part_counts = put(blob, pcnt.data(), pcnt.size());
     L.off_cov = put(blob, cov.data(), cov.size());

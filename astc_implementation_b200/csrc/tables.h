@@ -60,6 +60,7 @@ struct TableLayout {
     int32_t ndual;
     uint32_t off_w2t;         // u16 entries: texel index  | (contribution*16) << 8
     uint32_t off_part_texel;  // u8 [3][1024][T]  partition of texel (P = 2..4)
+    uint32_t off_part2;       // u32[3][1024][(T + 15) / 16]  the same, two bits a texel, texel t at bit 2 (t & 15)
     uint32_t off_part_info;   // u32[3][1024]     seed | count0<<10 | ... (see kernels)
     uint32_t off_part_counts; // u8 [3][1024][4]  texels per partition
     uint32_t off_cov;         // u64[3][1024][4]  coverage bitmaps over k-means texels
