@@ -62,7 +62,7 @@ struct Pruning {
     float coverage = 0.8f, threshold = 0.5f;
     float reroute_error = 8.0f;  // per-texel weighted squared error (8-bit units) above which
                                  // a proposal-search block also takes the full search; 0: off
-    int front_threads = 0;  // 0: by footprint (64 up to 16 texels, else 128)
+    int front_threads = 0;  // 0: by footprint and launch size
     int refine_iters = 0;
     int fallback_iters = 0;  // refinement iterations of the full-search pass over the fallback list
     float p1_floor = 0.0f;

@@ -96,7 +96,7 @@ struct KernelArgs {
     // refined, by P; [10..12] partition searches, P = 2..4; [13] candidates the refinement
     // handed to its tail pass.
     unsigned long long* work;
-    int front_threads;        // threads per front CTA: 128 (0 selects it), 64 or 32
+    int front_threads;        // threads per front CTA: 128, 64 or 32; 0: by footprint and launch size
     int refine_iters;         // refinement iterations (0 selects the reference's 6)
     int fixed;                // 1: FIXED semantics (ASTCB200_FLAG_FIXED_SEMANTICS), 0: the reference's
     // Refinement tail (null: off): once a refinement CTA has at most spill_live candidates
@@ -205,7 +205,7 @@ __device__ __forceinline__ uint4* block_dst(const KernelArgs& a, int blk) {
 #endif
 
 // Shared-memory sizes the launches need for one footprint.
-size_t front_smem_bytes(const TableLayout& L, int threads = 128, bool list = false);
+size_t front_smem_bytes(const TableLayout& L);
 size_t refine_smem_bytes(const TableLayout& L);
 size_t search_smem_bytes(const TableLayout& L);
 

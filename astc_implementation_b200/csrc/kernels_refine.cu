@@ -373,11 +373,8 @@ struct RTabs {
     const TableLayout* L;
     __device__ const DevDm& dm(int m) const { return reinterpret_cast<const DevDm*>(b + L->off_dm)[m]; }
     __device__ const DevBm& bm(int i) const { return reinterpret_cast<const DevBm*>(b + L->off_bm)[i]; }
-    __device__ int tw_count(int m, int t) const { return b[L->off_tw_count + m * L->T + t]; }
-    __device__ int tw_start(int m, int t) const { return reinterpret_cast<const uint16_t*>(b + L->off_tw_start)[m * L->T + t]; }
     __device__ int wt_count(int m, int w) const { return b[L->off_wt_count + m * 64 + w]; }
     __device__ int wt_start(int m, int w) const { return reinterpret_cast<const uint16_t*>(b + L->off_wt_start)[m * 64 + w]; }
-    __device__ uint32_t t2w(int i) const { return reinterpret_cast<const uint16_t*>(b + L->off_t2w)[i]; }
     __device__ uint32_t w2t(int i) const { return reinterpret_cast<const uint16_t*>(b + L->off_w2t)[i]; }
     __device__ uint64_t tw4(int m, int t) const { return reinterpret_cast<const uint64_t*>(b + L->off_tw4)[m * L->T + t]; }
     __device__ int part_count(int P, int e, int q) const { return b[L->off_part_counts + ((P - 2) * 1024 + e) * 4 + q]; }
@@ -422,20 +419,24 @@ template <class E> struct PartRow {
     __device__ __forceinline__ int part(int t) const { return v[t] >> kShift; }
     __device__ __forceinline__ int order(int i) const { return v[i] & ((1 << kShift) - 1); }
     // prow: the partitioning's row of texel partitions (null: one partition); one thread
-    __device__ __forceinline__ void set(const uint8_t* prow, const uint8_t* counts, int T) const {
+    __device__ __forceinline__ void set(const uint32_t* prow, const uint8_t* counts, int T) const {
         uint32_t next = 0;  // next position of each partition, a byte each
         if (prow) next = (uint32_t)counts[0] << 8 | ((uint32_t)counts[0] + counts[1]) << 16 | ((uint32_t)counts[0] + counts[1] + counts[2]) << 24;
 #pragma unroll 1
-        for (int t = 0; t < T; t++) v[t] = prow ? (E)((int)prow[t] << kShift) : (E)0;
+        for (int t = 0; t < T; t++) v[t] = prow ? (E)(((prow[t >> 4] >> (2 * (t & 15))) & 3u) << kShift) : (E)0;
 #pragma unroll 1
         for (int t = 0; t < T; t++) {
-            const int sh = prow ? 8 * (int)prow[t] : 0;
+            const int sh = 8 * part(t);
             const int i = (next >> sh) & 0xFF;
             v[i] = (E)(v[i] | t);
             next += 1u << sh;
         }
     }
 };
+// Row of a partitioning's texel partitions, two bits a texel.
+__device__ __forceinline__ const uint32_t* part2_row(const KernelArgs& a, int P, int entry) {
+    return reinterpret_cast<const uint32_t*>(a.tables + a.L.off_part2) + ((size_t)(P - 2) * 1024 + entry) * ((a.L.T + 15) >> 4);
+}
 // Direction of the partition's average colour (pass13's scale direction), the same for every
 // candidate and iteration of a partitioned block.
 __device__ __forceinline__ float4 scale_dir(float4 avg, float ps) {
@@ -794,7 +795,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                 }
                 if (r.ncand > 0) {
                     const int P = r.P;
-                    const uint8_t* prow = P > 1 ? a.tables + a.L.off_part_texel + ((size_t)(P - 2) * 1024 + r.entry) * T : nullptr;
+                    const uint32_t* prow = P > 1 ? part2_row(a, P, (int)r.entry) : nullptr;
                     const uint8_t* counts = P > 1 ? a.tables + a.L.off_part_counts + ((size_t)(P - 2) * 1024 + r.entry) * 4 : nullptr;
                     const BlockSrc src = block_src(a, chunk_block(a, lb));
                     Px* row = reinterpret_cast<Px*>(smem + fl.px + pbl * px_row);
@@ -962,7 +963,7 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
                     const int lb = (int)(h.x / (uint32_t)a.slots);
                     const PBRec& r = a.pbrec[h.x];
                     const int P = (int)r.P, k = (int)(h.y & 0xFF);
-                    const uint8_t* prow = P > 1 ? a.tables + a.L.off_part_texel + ((size_t)(P - 2) * 1024 + r.entry) * T : nullptr;
+                    const uint32_t* prow = P > 1 ? part2_row(a, P, (int)r.entry) : nullptr;
                     const uint8_t* counts = P > 1 ? a.tables + a.L.off_part_counts + ((size_t)(P - 2) * 1024 + r.entry) * 4 : nullptr;
                     const BlockSrc src = block_src(a, chunk_block(a, lb));
                     uchar4* row = reinterpret_cast<uchar4*>(smem + fl.px + tid * px_row);

@@ -51,26 +51,35 @@ struct Tabs {
     const TableLayout* L;
     __device__ const DevDm& dm(int m) const { return reinterpret_cast<const DevDm*>(b + L->off_dm)[m]; }
     __device__ const DevBm& bm(int i) const { return reinterpret_cast<const DevBm*>(b + L->off_bm)[i]; }
-    __device__ int tw_count(int m, int t) const { return b[L->off_tw_count + m * L->T + t]; }
-    __device__ int tw_start(int m, int t) const { return reinterpret_cast<const uint16_t*>(b + L->off_tw_start)[m * L->T + t]; }
-    __device__ int wt_count(int m, int w) const { return b[L->off_wt_count + m * 64 + w]; }
-    __device__ int wt_start(int m, int w) const { return reinterpret_cast<const uint16_t*>(b + L->off_wt_start)[m * 64 + w]; }
-    __device__ uint32_t t2w(int i) const { return reinterpret_cast<const uint16_t*>(b + L->off_t2w)[i]; }
-    __device__ uint32_t w2t(int i) const { return reinterpret_cast<const uint16_t*>(b + L->off_w2t)[i]; }
-    __device__ uint64_t tw4(int m, int t) const { return reinterpret_cast<const uint64_t*>(b + L->off_tw4)[m * L->T + t]; }
     __device__ int bm_order(int j) const { return reinterpret_cast<const uint16_t*>(b + L->off_bm_order)[j]; }
-    __device__ const uint8_t* part_texels(int P, int e) const { return b + L->off_part_texel + ((size_t)(P - 2) * 1024 + e) * L->T; }
     __device__ const uint32_t* part2(int P, int e) const { return reinterpret_cast<const uint32_t*>(b + L->off_part2) + ((size_t)(P - 2) * 1024 + e) * ((L->T + 15) >> 4); }
     __device__ int part_count(int P, int e, int q) const { return b[L->off_part_counts + ((P - 2) * 1024 + e) * 4 + q]; }
     __device__ uint32_t part_seed(int P, int e) const { return reinterpret_cast<const uint32_t*>(b + L->off_part_info)[(P - 2) * 1024 + e]; }
     __device__ uint64_t cov(int P, int e, int q) const { return reinterpret_cast<const uint64_t*>(b + L->off_cov)[((size_t)(P - 2) * 1024 + e) * 4 + q]; }
-    __device__ float sin_t(int i) const { return reinterpret_cast<const float*>(b + L->off_sin)[i]; }
-    __device__ float cos_t(int i) const { return reinterpret_cast<const float*>(b + L->off_cos)[i]; }
+    __device__ float2 trig(int i) const { return reinterpret_cast<const float2*>(b + L->off_trig)[i]; }
+    __device__ uint4 tw4f(int m, int t) const { return reinterpret_cast<const uint4*>(b + L->off_tw4f)[m * L->T + t]; }
+    __device__ uint32_t wt_info(int m, int w) const { return reinterpret_cast<const uint32_t*>(b + L->off_wt_info)[m * 64 + w]; }
+    __device__ int witem(int i) const { return reinterpret_cast<const uint16_t*>(b + L->off_witem)[i]; }
+    __device__ int sitem(int i) const { return reinterpret_cast<const uint16_t*>(b + L->off_sitem)[i]; }
+    __device__ const uint4* w2tf(int i) const { return reinterpret_cast<const uint4*>(b + L->off_w2tf) + i; }
+    __device__ uint32_t wgroup(int i) const { return reinterpret_cast<const uint32_t*>(b + L->off_wgroup)[i]; }
+    __device__ const uint4* wgent(int i) const { return reinterpret_cast<const uint4*>(b + L->off_wgent) + 32 * i; }
     __device__ int q2u(int i) const { return b[L->off_q2u + i]; }
     __device__ int q2u_start(int q) const { return b[L->off_q2u_start + q]; }
     __device__ int qmt(int row, int bits) const { return reinterpret_cast<const int8_t*>(b + L->off_qmt)[row * 128 + bits]; }
     __device__ float bqe(int i) const { return reinterpret_cast<const float*>(b + L->off_bqe)[i]; }
 };
+
+// Index and contribution of a tw4f or w2tf entry.
+__device__ __forceinline__ int entry_index(uint32_t e) { return (int)(e & 0xFFFFu); }
+__device__ __forceinline__ float entry_factor(uint32_t e) { return __uint_as_float(e & 0xFFFF0000u); }
+// Round to the nearest integer, ties to even, on the FP32 adders: as a float for |v| < 2^22, as
+// an integer for 0 <= v < 2^22.
+__device__ __forceinline__ float rn_small(float v) { return (v + 12582912.0f) - 12582912.0f; }
+__device__ __forceinline__ uint32_t rn_bits(float v) { return fbits(v + 8388608.0f) - 0x4B000000u; }
+// Small integers as floats and non-negative floats truncated, without the conversion pipe.
+__device__ __forceinline__ float small_float(uint32_t v) { return __uint_as_float(0x4B000000u | v) - 8388608.0f; }
+__device__ __forceinline__ uint32_t small_trunc(float v) { return fbits(__fadd_rz(v, 8388608.0f)) - 0x4B000000u; }
 
 __device__ __forceinline__ float dist_sq(float4 a, float4 b) {
     const float4 d = a - b;
@@ -625,20 +634,13 @@ __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtas) k_partition_se
 }
 
 // ============================================================ passes 01-12
-// One CTA of NT threads per partitioned block: 128 for the full search; the proposal
-// search, whose partitioned blocks evaluate few block modes, may use 64 or 32 so that more
-// of them are resident per SM.  Every value is computed by the same thread sequence
-// whatever NT is (loops only spread independent items), so results do not depend on it.
+// One CTA of NT threads per partitioned block (front_nt).  Every value is computed by the same
+// thread sequence whatever NT is (loops only spread independent items), so results do not
+// depend on it.
 
 struct FrontLayout {
-    int px, w, wes, tp, dec, lo, hi, scratch, bm_err, bm_bits, ccr_tot, ccr_q, ccr_fmt, qf, misc, dml, bml, total;
+    int px, w, wes, tp, dec, lo, hi, bm_err, ints, trig, qf, misc, dml, bml, total;
 };
-
-// Scratch of passes 02-05 per half-warp: the pass03 table indices [64], angular offsets
-// [16], pass05 keys [16] (u64) and minidx [16].  pass02's infilled weights (T floats per
-// half-warp) go to pass07's buffer, unused between pass08's sums and pass07.
-constexpr int kDmScratchHalf = 64 * 4 + 16 * 4 + 16 * 8 + 16 * 4;
-constexpr int kDmScratchPerWarp = 2 * kDmScratchHalf;
 
 struct FrontMisc {
     float4 avg[4], dir[4], ep0[4], ep1[4];
@@ -653,43 +655,46 @@ struct FrontMisc {
     float cerr[4][21][4];
     uint8_t cfmt[4][21][4];
     float combo_err[21][13];
-    uint8_t combo_fmt[21][13][4];
+    __align__(4) uint8_t combo_fmt[21][13][4];
     int top[kNumCand];
     int ncand;
     int nlive;  // block modes in the proposal search's list
 };
 
-// pass07's buffer in floats, before pass02 also the texel channels and projections,
-// then pass08's error terms (5 x Tp; Tp = T rounded up to 4).  The full search's
+// pass07's buffer in floats, before it in turn the texel channels and projections of pass01,
+// pass08's error terms (5 x Tp; Tp = T rounded up to 4), pass02's infilled weights (T per
+// decimation mode) and the angular steps of pass04 (kStepFloats each).  The full search's
 // pass07 takes one thread per mode (max_w x nt); the proposal search's (`list`) works on
 // groups of kListGroup modes (max_w + Tp each), so its launches need less shared memory
 // and more of its CTAs fit on an SM.
 constexpr int kListGroup = 16;
+constexpr int kStepFloats = 7;  // four errors, then span and lowest index, then the offset
 __host__ __device__ inline int front_layout_qf_floats(int T, int max_w, int nt, bool list) {
     const int Tp = (T + 3) & ~3;
     int f = list ? kListGroup * (max_w + Tp) : max_w * nt;
     if (f < 5 * Tp) f = 5 * Tp;
-    if (f < (nt / 32) * 2 * T) f = (nt / 32) * 2 * T;  // pass02's infill, two modes per warp
     return f;
 }
 __host__ __device__ inline int take16(int& o, int bytes) { const int r = o; o = (o + bytes + 15) & ~15; return r; }
-__host__ __device__ inline FrontLayout front_layout(int T, int ndm, int nbm, int max_w, int nt, bool list) {
+__host__ __device__ inline FrontLayout front_layout(const TableLayout& L, int nt, bool list) {
+    const int T = L.T, ndm = L.ndm, nbm = L.nbm, max_w = L.max_w;
     FrontLayout f;
     int o = 0;
     f.px = take16(o, T * 16);
     f.w = take16(o, T * 4);
     f.wes = take16(o, T * 4);
     f.tp = take16(o, T);
-    f.dec = take16(o, ndm * 64 * 4);
+    f.dec = take16(o, L.nw_total * 4);
     f.lo = take16(o, ndm * 8 * 4);
     f.hi = take16(o, ndm * 8 * 4);
-    f.scratch = take16(o, (nt / 32) * kDmScratchPerWarp);
     f.bm_err = take16(o, nbm * 4);
-    f.bm_bits = take16(o, nbm * 4);
-    f.ccr_tot = take16(o, nbm * 4);
-    f.ccr_q = take16(o, nbm * 2);
-    f.ccr_fmt = take16(o, nbm * 4);
-    f.qf = take16(o, front_layout_qf_floats(T, max_w, nt, list) * 4);
+    f.ints = take16(o, nbm);
+    // pass03's table rows are read before pass07's buffer is written: one region, the rows after
+    // the steps and pass02's infill
+    const int early = ((ndm * (T > kMaxAngularSteps * kStepFloats ? T : kMaxAngularSteps * kStepFloats) * 4) + 15) & ~15;
+    const int rows = early + L.nw_total * 2, qf = front_layout_qf_floats(T, max_w, nt, list) * 4;
+    f.qf = take16(o, rows > qf ? rows : qf);
+    f.trig = f.qf + early;
     f.misc = take16(o, (int)sizeof(FrontMisc));
     f.dml = take16(o, 16 + ndm * 2);
     f.bml = take16(o, nbm * 2);  // the proposal search's block modes, ascending
@@ -702,7 +707,7 @@ __host__ __device__ inline FrontLayout front_layout(int T, int ndm, int nbm, int
 // 0..64 scale and writes the rescaled float weight.
 struct BmQuant {
     float low, scale, slb, rscale, qlm1;
-    int q2u_start, quant;
+    uint32_t q2u_start, top;  // first entry and last level of the quantisation's values
 };
 __device__ __forceinline__ BmQuant bm_quant_setup(const Tabs& tb, const DevBm& bm, const float* lo, const float* hi, float min_cutoff) {
     float low = lo[bm.quant < 8 ? bm.quant : 0], high = hi[bm.quant < 8 ? bm.quant : 0];
@@ -710,185 +715,230 @@ __device__ __forceinline__ BmQuant bm_quant_setup(const Tabs& tb, const DevBm& b
     if (high > 1.02f * min_cutoff) high = 1.0f;
     if (high <= low) { low = 0.0f; high = 1.0f; }
     BmQuant r;
-    r.qlm1 = (float)(c_levels[bm.quant] - 1);
+    r.top = (uint32_t)(c_levels[bm.quant] - 1);
+    r.qlm1 = (float)r.top;
     float rscale = high - low;
     r.scale = 1.0f / rscale;
     r.slb = low * r.scale;
     r.rscale = rscale / 64.0f;
     r.low = low;
-    r.q2u_start = tb.q2u_start(bm.quant);
-    r.quant = bm.quant;
+    r.q2u_start = (uint32_t)tb.q2u_start(bm.quant);
     return r;
 }
-__device__ __forceinline__ int bm_quant_weight(const Tabs& tb, const BmQuant& s, float ideal, float* qf) {
+__device__ __forceinline__ uint32_t bm_quant_weight(const Tabs& tb, const BmQuant& s, float ideal, float* qf) {
     const float ix = clampf(ideal * s.scale - s.slb, 0.0f, 1.0f);
-    const float ix1 = ix * s.qlm1;
-    const uint32_t wl = f2u(ix1), wh = min(wl + 1, f2u(s.qlm1));
-    const int li = tb.q2u(s.q2u_start + wl), hi = tb.q2u(s.q2u_start + wh);
-    const bool uh = ((float)li + (float)hi) < (128.0f * ix);
-    const int v = uh ? hi : li;
-    *qf = (float)v * s.rscale + s.low;
+    const uint32_t wl = small_trunc(ix * s.qlm1), wh = min(wl + 1, s.top);
+    const uint32_t li = (uint32_t)tb.q2u((int)(s.q2u_start + wl)), hi = (uint32_t)tb.q2u((int)(s.q2u_start + wh));
+    const bool uh = small_float(li + hi) < (128.0f * ix);
+    const uint32_t v = uh ? hi : li;
+    *qf = small_float(v) * s.rscale + s.low;
     return v;
 }
 
-// pass02 of one decimation mode by a half-warp (lane gl of 16): the ideal decimated
-// weights dw, then for decimated modes the infill and the one-step correction.  Every lane
-// of the warp takes the syncs (both halves run this together, each on its own mode).
-__device__ __forceinline__ void pass02_mode(const Tabs& tb, int T, int m, const DevDm& dmi, int W, bool act, int gl, float* inf,
-                                            const float* iw, const float* wes, bool is_const, float* dw) {
-    if (W == T || !act) {
-        for (int w = gl; w < W; w += 16) dw[w] = iw[w];
-    } else {
-        for (int w = gl; w < W; w += 16) {
-            const int n = tb.wt_count(m, w);
-            float v = 0.0f;
-            if (n) {
-                const int base = dmi.wt_base + tb.wt_start(m, w);
-                float ws = 0.0f, tc = 1e-10f;
-                for (int j = 0; j < n; j++) {
-                    const uint32_t e = tb.w2t(base + j);
-                    const int t = e & 0xFF;
-                    const float cwt = ((float)(e >> 8) * (1.0f / 16.0f)) * wes[is_const ? 0 : t];
+// Passes 02-05 for the decimation modes of a partitioned block: each step over items of all
+// modes at once, a barrier between steps.  Items are (mode, weight) for pass02's sums, (mode,
+// texel) for its infill, (mode, weight) for its correction, (mode, angular step) for passes 03
+// and 04, (mode, quant level) for pass05.  The full search takes the first and the step items
+// from the tables, sorted by their inner loop's length, so that a warp's lanes end together; a
+// half-warp per mode, which this replaces, kept 16 of 32 lanes busy (a mode has 4 to 64 weights,
+// 1 to 36 texels a weight and 2 to 12 steps) and spent three instructions in four on the loops
+// around the sums.  The proposal search's few modes are numbered by shifts instead.  The sums'
+// entries are stored four to a load and, for the sorted items, 32 items side by side; the
+// weights of all modes are packed, which with the steps kept in pass07's buffer takes a 10x8
+// block from 70 to 51 KB of shared memory and from three to four CTAs.  Measured (B200, 128
+// threads): passes 02-05 of 13,312 partitioned blocks at 10x8 3.04 -> 1.43 ms, at 8x8 3.18 ->
+// 1.61 ms; with 32 threads 83,200 at 4x4 0.44 -> 0.41 ms.
+template <int NT>
+__device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int ndm_run, const int16_t* dm_run, const float* iw,
+                                          const float* wes, bool is_const, float* dec, uint16_t* trig, float* lov, float* hiv,
+                                          float* buf) {
+    const int tid = threadIdx.x;
+    const int tmask = is_const ? 0 : -1;
+    const int wsh = max_w <= 16 ? 4 : max_w <= 32 ? 5 : 6;  // weights per listed mode, rounded up
+    const int nw = dm_run ? ndm_run << wsh : tb.L->nwi;
+    // item it's mode and weight, and its texel entries, `stride` fours apart
+    const int stride = dm_run ? 1 : 32;
+    auto weight_item = [&](int it, int& m, int& w, const uint4*& ent, int& n4) {
+        uint32_t info;
+        if (dm_run) {
+            m = dm_run[it >> wsh]; w = it & ((1 << wsh) - 1);
+            info = tb.wt_info(m, w);
+            ent = tb.w2tf(info & 0xFFFF);
+        } else {
+            const int e = tb.witem(it);
+            m = e >> 6; w = e & 63;
+            info = tb.wgroup(it >> 5);
+            ent = tb.wgent(info & 0xFFFF) + (it & 31);
+        }
+        n4 = info >> 16;
+    };
+    // pass02: the ideal decimated weights (padding entries add 0 to sums that are never -0)
+#pragma unroll 1
+    for (int it = tid; it < nw; it += NT) {
+        int m, w, n4;
+        const uint4* ent;
+        weight_item(it, m, w, ent, n4);
+        const DevDm dmi = tb.dm(m);
+        if (w >= (int)dmi.W) continue;
+        float v = iw[w];
+        if (dmi.W != T) {
+            float ws = 0.0f, tc = 1e-10f;
+#pragma unroll 1
+            for (; n4 > 0; n4--, ent += stride) {
+                const uint4 e4 = *ent;
+                const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int t = entry_index(e[k]);
+                    const float cwt = entry_factor(e[k]) * wes[t & tmask];
                     ws = ws + iw[t] * cwt;
                     tc = tc + cwt;
                 }
-                v = ws / tc;
             }
-            dw[w] = v;
+            v = ws / tc;
         }
+        dec[dmi.w_off + w] = v;
     }
-    const bool decim = act && W != T;
-    __syncwarp();
-    if (decim) {
-        for (int t = gl; t < T; t += 16) {
-            // the texel's entries in list order; padding entries add dw[0] * 0, which never changes v
-            const uint64_t e4 = tb.tw4(m, t);
-            float v = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 4; j++) { const uint32_t e = (uint32_t)(e4 >> (16 * j)) & 0xFFFF; v = v + dw[e & 0xFF] * ((float)(e >> 8) * (1.0f / 16.0f)); }
-            inf[t] = v;
-        }
-    }
-    __syncwarp();
-    if (decim) {
-        for (int w = gl; w < W; w += 16) {
-            const int n = tb.wt_count(m, w), base = dmi.wt_base + tb.wt_start(m, w);
-            float e0 = 1e-10f, e1 = 0.0f;
-            for (int j = 0; j < n; j++) {
-                const uint32_t e = tb.w2t(base + j);
-                const int t = e & 0xFF;
-                const float c = (float)(e >> 8) * (1.0f / 16.0f);
-                const float sc = wes[is_const ? 0 : t] * c;
-                e0 = e0 + c * sc;
-                e1 = e1 + (inf[t] - iw[t]) * sc;
-            }
-            dw[w] = dw[w] + clampf((e1 * -16.0f) / e0, -0.25f, 0.25f);
-        }
-    }
-}
-
-// Passes 02-05 for the decimation modes of a partitioned block, a half-warp per mode, two
-// modes per warp at a time (passes 03-05 need at most 16 lanes: 16 angular steps at most,
-// 12 for every valid mode).  Every lane of a warp runs the same number of loop trips (a
-// half without a mode idles), so the warp-wide __syncwarp()s are reached by all of its
-// lanes.
-template <int kFrontWarps>
-__device__ __forceinline__ void dm_passes(const Tabs& tb, int T, const FrontLayout& fl, uint8_t* sm, int ndm_run,
-                                          const int16_t* dm_run, const float* iw, const float* wes, bool is_const,
-                                          float* dec, float* lov, float* hiv, float* infbuf) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int half = lane >> 4, hl = lane & 15;
-    float* inf = infbuf + (warp * 2 + half) * T;
-    uint8_t* hs = sm + fl.scratch + warp * kDmScratchPerWarp + half * kDmScratchHalf;
-    uint32_t* smp = reinterpret_cast<uint32_t*>(hs);
-    float* ang = reinterpret_cast<float*>(hs + 64 * 4);
-    float* lh = reinterpret_cast<float*>(hs + 64 * 4 + 16 * 4);  // pass05 keys [16] (u64), minidx [16]
-    for (int mb = warp * 2; mb < ndm_run; mb += kFrontWarps * 2) {
-        const int mi = mb + half;
-        const bool act = mi < ndm_run;
-        const int m = act ? (dm_run ? dm_run[mi] : mi) : 0;
+    __syncthreads();
+    // the infilled weights less the ideal ones
+    float* inf = buf;
+    const uint32_t per_t = 0xFFFFFFFFu / (uint32_t)T + 1u;  // n / T is umulhi(n, per_t) for n < 2^16
+#pragma unroll 1
+    for (int it = tid; it < ndm_run * T; it += NT) {
+        const int mi = (int)__umulhi((uint32_t)it, per_t), t = it - mi * T;
+        const int m = dm_run ? dm_run[mi] : mi;
         const DevDm dmi = tb.dm(m);
-        const int W = act ? (int)dmi.W : 0;
-        float* dw = dec + m * 64;
-        pass02_mode(tb, T, m, dmi, W, act, hl, inf, iw, wes, is_const, dw);
-        __syncwarp();
-        for (int w = hl; w < W; w += 16) smp[w] = f2u(rintf(clampf(dw[w], 0.0f, 1.0f) * (1024.0f - 1.0f)));
-        __syncwarp();
-        // pass03: angular offsets
-        if (act) {
-            // table values fetched four at a time, then summed in weight order
-            float ax = 0.0f, ay = 0.0f;
-            int j = 0;
-            for (; j + 4 <= W; j += 4) {
-                float c[4], sn[4];
+        if (dmi.W == T) continue;
+        // the texel's entries in list order; padding entries add dw[0] * 0, which never changes v
+        const uint4 e = tb.tw4f(m, t);
+        const float* dw = dec + dmi.w_off;
+        float v = dw[entry_index(e.x)] * entry_factor(e.x);
+        v = v + dw[entry_index(e.y)] * entry_factor(e.y);
+        v = v + dw[entry_index(e.z)] * entry_factor(e.z);
+        v = v + dw[entry_index(e.w)] * entry_factor(e.w);
+        inf[m * T + t] = v - iw[t];
+    }
+    __syncthreads();
+    // the one-step correction, and pass03's table rows (padded to a multiple of four weights with
+    // the row of zeros, which changes no sum)
+#pragma unroll 1
+    for (int it = tid; it < nw; it += NT) {
+        int m, w, n4;
+        const uint4* ent;
+        weight_item(it, m, w, ent, n4);
+        const DevDm dmi = tb.dm(m);
+        const int W = dmi.W;
+        if (w >= W) continue;
+        float v = dec[dmi.w_off + w];
+        if (W != T) {
+            const float* im = inf + m * T;
+            float e0 = 1e-10f, e1 = 0.0f;
+#pragma unroll 1
+            for (; n4 > 0; n4--, ent += stride) {
+                const uint4 e4 = *ent;
+                const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
-                for (int u = 0; u < 4; u++) { const int k = smp[j + u] * 16 + hl; c[u] = tb.cos_t(k); sn[u] = tb.sin_t(k); }
-#pragma unroll
-                for (int u = 0; u < 4; u++) { ax = ax + c[u]; ay = ay + sn[u]; }
+                for (int k = 0; k < 4; k++) {
+                    const int t = entry_index(e[k]);
+                    const float c = entry_factor(e[k]), sc = wes[t & tmask] * c;
+                    e0 = e0 + c * sc;
+                    e1 = e1 + im[t] * sc;
+                }
             }
-            for (; j < W; j++) { const int k = smp[j] * 16 + hl; ax = ax + tb.cos_t(k); ay = ay + tb.sin_t(k); }
-            ang[hl] = atan2_search(ay, ax) * (1.0f / (2.0f * 3.14159265358979323846f));
+            v = v + clampf((e1 * -16.0f) / e0, -0.25f, 0.25f);
+            dec[dmi.w_off + w] = v;
         }
-        __syncwarp();
-        // pass04 + pass05: lane i < S evaluates angular step i (rounding error and cut
-        // errors over the weights) and offers its candidates to the weight spans the
-        // sequential scan of pass05 would update with them: span sp takes e, sp - 1 takes
-        // e + cl and then e + ch, sp - 2 takes e + cl + ch, each only when strictly below the
-        // span's best so far (initially 1e37), steps in ascending order.  That scan keeps,
-        // per span, the first minimum in this order, which is the smallest key
-        //   error bits << 32 | step << 2 | order within the step << 1 | low-cut flag:
-        // errors are sums of non-negative products (never -0.0f, NaN or 1e37), so their
-        // bit patterns order like their values.  Only spans 0..15 are read (q <= 7 needs
-        // span c_steps_for_quant[q] <= 12; S <= 12 for every valid decimation mode).
-        const int S = act ? (int)dmi.max_angular_steps : 0;
-        unsigned long long* best = reinterpret_cast<unsigned long long*>(lh);  // [16]
-        float* lmin = lh + 32;                                                 // [16] minidx per step
-        best[hl] = ~0ull;
-        __syncwarp();
-        if (hl < S) {
-            float mnw = 3.4e38f, mxw = -3.4e38f;
-            for (int j = 0; j < W; j++) { const float v = dw[j]; if (v < mnw) mnw = v; if (v > mxw) mxw = v; }
-            const float rcp = (float)(hl + 1), off = ang[hl];
-            const float minidx = rintf(mnw * rcp - off), maxidx = rintf(mxw * rcp - off);
-            float ev = 0.0f, cl = 0.0f, ch = 0.0f;
-            for (int j = 0; j < W; j++) {
-                const float sv = dw[j] * rcp - off, r = rintf(sv), d = sv - r;
-                ev = ev + d * d;
-                cl = cl + (r == minidx ? 1.0f - (2.0f * d) : 0.0f);
-                ch = ch + (r == maxidx ? 1.0f + (2.0f * d) : 0.0f);
+        trig[dmi.w_off + w] = (uint16_t)(rn_bits(clampf(v, 0.0f, 1.0f) * (1024.0f - 1.0f)) * 16);
+        if (w == W - 1)
+            for (int p = W; p & 3; p++) trig[dmi.w_off + p] = 1024 * 16;
+    }
+    __syncthreads();
+    // passes 03 and 04: the angular offset of a step, its rounding error and cut errors over
+    // the weights, and its span
+    float4* step_err = reinterpret_cast<float4*>(buf);  // e, e + low cut, e + high cut, e + both
+    const int nstep = tb.L->ndm * kMaxAngularSteps;
+    int2* step_span = reinterpret_cast<int2*>(buf + 4 * nstep);  // span, lowest index (float bits)
+    float* ang = buf + 6 * nstep;
+    const int ns = dm_run ? ndm_run << 4 : tb.L->nsi;
+#pragma unroll 1
+    for (int it = tid; it < ns; it += NT) {
+        int m, i;
+        if (dm_run) { m = dm_run[it >> 4]; i = it & 15; }
+        else { const int e = tb.sitem(it); m = e >> 4; i = e & 15; }
+        const DevDm dmi = tb.dm(m);
+        const int W = dmi.W;
+        if (i >= (int)dmi.max_angular_steps) continue;
+        const float* dw = dec + dmi.w_off;
+        const uint2* rows = reinterpret_cast<const uint2*>(trig + dmi.w_off);
+        float ax = 0.0f, ay = 0.0f;
+#pragma unroll 2
+        for (int j = 0; j < W; j += 4) {  // four table values in flight, summed in weight order
+            const uint2 k = rows[j >> 2];
+            const float2 c0 = tb.trig((int)(k.x & 0xFFFF) + i), c1 = tb.trig((int)(k.x >> 16) + i);
+            const float2 c2 = tb.trig((int)(k.y & 0xFFFF) + i), c3 = tb.trig((int)(k.y >> 16) + i);
+            ax = ax + c0.x; ay = ay + c0.y;
+            ax = ax + c1.x; ay = ay + c1.y;
+            ax = ax + c2.x; ay = ay + c2.y;
+            ax = ax + c3.x; ay = ay + c3.y;
+        }
+        const float off = atan2_search(ay, ax) * (1.0f / (2.0f * 3.14159265358979323846f));
+        float mnw = 3.4e38f, mxw = -3.4e38f;
+#pragma unroll 4
+        for (int j = 0; j < W; j++) { const float v = dw[j]; mnw = fminf(mnw, v); mxw = fmaxf(mxw, v); }
+        const float rcp = (float)(i + 1);
+        const float minidx = rn_small(mnw * rcp - off), maxidx = rn_small(mxw * rcp - off);
+        float ev = 0.0f, cl = 0.0f, ch = 0.0f;
+#pragma unroll 2
+        for (int j = 0; j < W; j++) {
+            const float sv = dw[j] * rcp - off, r = rn_small(sv), d = sv - r, d2 = d + d;
+            ev = ev + d * d;
+            cl = cl + (r == minidx ? 1.0f - d2 : 0.0f);
+            ch = ch + (r == maxidx ? 1.0f + d2 : 0.0f);
+        }
+        const int sp = min(max((int)rn_small((maxidx - minidx) + 1.0f), 2), (int)dmi.max_quant_steps + 3);
+        const float ss = 1.0f / rcp, esc = ss * ss;
+        const float e = ev * esc, ecl0 = cl * esc, ech0 = ch * esc;
+        const int at = m * kMaxAngularSteps + i;
+        step_err[at] = make_float4(e, e + ecl0, e + ech0, (e + ecl0) + ech0);
+        step_span[at] = make_int2(sp, __float_as_int(minidx));
+        ang[at] = off;
+    }
+    __syncthreads();
+    // pass05: low/high value per quant level from the best step of its span.  The scan over
+    // the steps updates span sp with e, sp - 1 with the low cut's error and then the high
+    // cut's, sp - 2 with both cuts', each only when strictly below the span's best so far
+    // (initially 1e37: step 0 and no low cut when nothing got below); an item runs it for
+    // its own span.
+#pragma unroll 1
+    for (int it = tid; it < ndm_run * 8; it += NT) {
+        const int m = dm_run ? dm_run[it >> 3] : it >> 3, q = it & 7;
+        const DevDm dmi = tb.dm(m);
+        float lo_v = 0.0f, hi_v = 0.0f;
+        if (q <= (int)dmi.max_quant_level) {
+            const int qs = c_steps_for_quant[q], S = dmi.max_angular_steps, at = m * kMaxAngularSteps;
+            float best = 1e37f, lwi = __int_as_float(step_span[at].y);
+            int bsi = 0;
+#pragma unroll 1
+            for (int i = 0; i < S; i++) {
+                const float4 e = step_err[at + i];
+                const int2 si = step_span[at + i];
+                const int d = si.x - qs;
+                const bool high = e.z < e.y;
+                const float c = d == 0 ? e.x : d == 1 ? (high ? e.z : e.y) : d == 2 ? e.w : 3.4e38f;
+                if (c < best) {
+                    best = c;
+                    bsi = i;
+                    lwi = __int_as_float(si.y) + ((d == 2 || (d == 1 && !high)) ? 1.0f : 0.0f);
+                }
             }
-            const int sp = min(max(f2i((maxidx - minidx) + 1.0f), 2), (int)dmi.max_quant_steps + 3);
-            const float ss = 1.0f / rcp, esc = ss * ss;
-            const float e = ev * esc, ecl0 = cl * esc, ech0 = ch * esc;
-            const float ecl = e + ecl0, ech = e + ech0, eclh = (e + ecl0) + ech0;
-            lmin[hl] = minidx;
-            const unsigned long long ik = (unsigned long long)hl << 2;
-            if (sp < 16 && e < 1e37f) atomicMin(&best[sp], ((unsigned long long)__float_as_uint(e) << 32) | ik);
-            if (sp - 1 < 16 && ecl < 1e37f) atomicMin(&best[sp - 1], ((unsigned long long)__float_as_uint(ecl) << 32) | ik | 1ull);
-            if (sp - 1 < 16 && ech < 1e37f) atomicMin(&best[sp - 1], ((unsigned long long)__float_as_uint(ech) << 32) | ik | 2ull);
-            if (sp - 2 < 16 && eclh < 1e37f) atomicMin(&best[sp - 2], ((unsigned long long)__float_as_uint(eclh) << 32) | ik | 1ull);
+            const float hwi = (lwi + (float)qs) - 1.0f;
+            const float step = 1.0f / (1.0f + (float)bsi);
+            const float o = ang[at + bsi];
+            lo_v = (o + lwi) * step;
+            hi_v = (o + hwi) * step;
         }
-        __syncwarp();
-        // pass05: low/high value per quant level from the best step of its span (step 0
-        // and no low cut when no candidate got below 1e37)
-        if (act && hl < 8) {
-            const int q = hl;
-            float lo_v = 0.0f, hi_v = 0.0f;
-            if (q <= (int)dmi.max_quant_level) {
-                const int qs = c_steps_for_quant[q];
-                const unsigned long long k = best[qs];
-                const int bsi = k == ~0ull ? 0 : (int)(((uint32_t)k) >> 2);
-                const float lwi = lmin[bsi] + ((k != ~0ull && (k & 1ull)) ? 1.0f : 0.0f);
-                const float hwi = (lwi + (float)qs) - 1.0f;
-                const float step = 1.0f / (1.0f + (float)bsi);
-                const float off = ang[bsi];
-                lo_v = (off + lwi) * step;
-                hi_v = (off + hwi) * step;
-            }
-            lov[m * 8 + q] = lo_v;
-            hiv[m * 8 + q] = hi_v;
-        }
-        __syncwarp();
+        lov[m * 8 + q] = lo_v;
+        hiv[m * 8 + q] = hi_v;
     }
 }
 
@@ -899,29 +949,43 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, const FrontLayo
 template <int kFrontThreads>
 __device__ __noinline__ void pass07_all_modes(const Tabs& tb, int T, int P, int nbm, const float* lov, const float* hiv,
                                               float min_cutoff, const float* dec, float* qfs, const float* iw,
-                                              const float* wes, bool is_const, float* bm_err, int* bm_bits) {
+                                              const float* wes, bool is_const, float* bm_err) {
     const int tid = threadIdx.x;
+    const int tmask = is_const ? 0 : -1;
+    float* qw = qfs + tid;  // this thread's weights, kFrontThreads apart
     // one thread per mode; neighbouring threads get modes of the same decimation
+#pragma unroll 1
     for (int j = tid; j < nbm; j += kFrontThreads) {
         const int i = tb.bm_order(j);
         const DevBm bm = tb.bm(i);
         const int bc = c_free_bits[P - 1] - (int)bm.weight_bits;
-        if (bm.quant > 11 || bc <= 0) { bm_err[i] = 1e38f; bm_bits[i] = 0; continue; }
+        if (bm.quant > 11 || bc <= 0) { bm_err[i] = 1e38f; continue; }
         const DevDm dmi = tb.dm(bm.dm);
+        const int W = dmi.W;
         const BmQuant s = bm_quant_setup(tb, bm, lov + bm.dm * 8, hiv + bm.dm * 8, min_cutoff);
-        const float* dw = dec + bm.dm * 64;
-        for (int w = 0; w < dmi.W; w++) { float qf; bm_quant_weight(tb, s, dw[w], &qf); qfs[w * kFrontThreads + tid] = qf; }
+        const float* dw = dec + dmi.w_off;
+#pragma unroll 2
+        for (int w = 0; w < W; w++) { float qf; bm_quant_weight(tb, s, dw[w], &qf); qw[w * kFrontThreads] = qf; }
         float err = 0.0f;
-        for (int t = 0; t < T; t++) {
-            const uint64_t e4 = tb.tw4(bm.dm, t);
-            float v = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 4; j++) { const uint32_t e = (uint32_t)(e4 >> (16 * j)) & 0xFFFF; v = v + qfs[(e & 0xFF) * kFrontThreads + tid] * ((float)(e >> 8) * (1.0f / 16.0f)); }
-            const float d = v - iw[t];
-            err = err + (d * d) * wes[is_const ? 0 : t];
+        if (W == T) {  // one weight a texel, contribution 1
+#pragma unroll 2
+            for (int t = 0; t < T; t++) {
+                const float d = qw[t * kFrontThreads] - iw[t];
+                err = err + (d * d) * wes[t & tmask];
+            }
+        } else {
+#pragma unroll 2
+            for (int t = 0; t < T; t++) {
+                const uint4 e = tb.tw4f(bm.dm, t);
+                float v = qw[entry_index(e.x) * kFrontThreads] * entry_factor(e.x);
+                v = v + qw[entry_index(e.y) * kFrontThreads] * entry_factor(e.y);
+                v = v + qw[entry_index(e.z) * kFrontThreads] * entry_factor(e.z);
+                v = v + qw[entry_index(e.w) * kFrontThreads] * entry_factor(e.w);
+                const float d = v - iw[t];
+                err = err + (d * d) * wes[t & tmask];
+            }
         }
         bm_err[i] = err;
-        bm_bits[i] = bc;
     }
 }
 
@@ -934,7 +998,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     const Tabs tb{a.tables, &a.L};
     const int T = a.L.T, ndm = a.L.ndm, nbm = a.L.nbm;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const FrontLayout fl = front_layout(T, ndm, nbm, a.L.max_w, NT, a.bm_mask != nullptr);
+    const FrontLayout fl = front_layout(a.L, NT, a.bm_mask != nullptr);
     float4* px = reinterpret_cast<float4*>(sm + fl.px);
     float* iw = reinterpret_cast<float*>(sm + fl.w);
     float* wes = reinterpret_cast<float*>(sm + fl.wes);
@@ -943,10 +1007,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     float* lov = reinterpret_cast<float*>(sm + fl.lo);
     float* hiv = reinterpret_cast<float*>(sm + fl.hi);
     float* bm_err = reinterpret_cast<float*>(sm + fl.bm_err);
-    int* bm_bits = reinterpret_cast<int*>(sm + fl.bm_bits);
-    float* ccr_tot = reinterpret_cast<float*>(sm + fl.ccr_tot);
-    uint8_t* ccr_q = sm + fl.ccr_q;
-    uint8_t* ccr_fmt = sm + fl.ccr_fmt;
+    uint8_t* mode_ints = sm + fl.ints;  // pass11's integer count per block mode
     float* qfs = reinterpret_cast<float*>(sm + fl.qf);
     FrontMisc& M = *reinterpret_cast<FrontMisc*>(sm + fl.misc);
     const float4 cw = chan_w();
@@ -982,12 +1043,13 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     // pass01's chain.  With one warp, roles are its lanes.
     const int role = (tid + kFrontThreads - 32) % kFrontThreads;
 
-    const uint8_t* prow = P > 1 ? tb.part_texels(P, entry) : nullptr;
+    const uint32_t* prow = P > 1 ? tb.part2(P, entry) : nullptr;
     const BlockSrc src = block_src(a, blk);
+#pragma unroll 1
     for (int t = tid; t < Tp; t += kFrontThreads) {
         float4 v = mk(0.0f);
         uint8_t q = 0xFF;
-        if (t < T) { v = src_texel(src, a.L.bx, t); q = P > 1 ? prow[t] : 0; px[t] = v; }
+        if (t < T) { v = src_texel(src, a.L.bx, t); q = P > 1 ? (prow[t >> 4] >> (2 * (t & 15))) & 3u : 0; px[t] = v; }
         pxc[t] = v.x; pxc[Tp + t] = v.y; pxc[2 * Tp + t] = v.z; pxc[3 * Tp + t] = v.w;
         tp[t] = q;
     }
@@ -1001,6 +1063,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         const float* v = pxc + gc * Tp;
         float s = 0.0f;
         int n = 0;
+#pragma unroll 1
         for (int t = 0; t < Tp; t += 4) {
             const float4 x = *reinterpret_cast<const float4*>(v + t);
             const uint32_t q = tp4(t);
@@ -1018,6 +1081,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     if (warp == 0) {
         const float* v = pxc + gc * Tp;
         float dd = 0.0f;
+#pragma unroll 1
         for (int t = 0; t < Tp; t += 4) {
             const float4 x = *reinterpret_cast<const float4*>(v + t);
             const uint32_t q = tp4(t);
@@ -1035,6 +1099,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
                                                 __shfl_sync(FULL, dd, g0 + 2), __shfl_sync(FULL, dd, g0 + 3)));
         if (lane < 16 && gc == 0) M.dir[gp] = d;
         __syncwarp();
+#pragma unroll 1
         for (int t = lane; t < Tp; t += 32) {
             float pr = 0.0f;
             if (t < T) { const int p = tp1(t); pr = dot4(px[t] - M.avg[p], M.dir[p]); }
@@ -1043,6 +1108,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         __syncwarp();
         // range of the projections, taken in texel order as the oracle does
         float mn = 1e10f, mx = -1e10f;
+#pragma unroll 1
         for (int t = 0; t < Tp; t += 4) {
             const float4 x = *reinterpret_cast<const float4*>(prj + t);
             const uint32_t q = tp4(t);
@@ -1069,12 +1135,14 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     }
     // pass08, first part (needs only the averages): role 9p + 3s + c sums channel c of the
     // deviations from the average over the texels of partition p whose channel s is above it
+#pragma unroll 1
     for (int v = role; v < 9 * P; v += kFrontThreads) {
         const int p = v / 9, s = (v / 3) % 3, c = v % 3;
         const float as = comp(M.avg[p], s), ac = comp(M.avg[p], c);
         const float* xs = pxc + s * Tp;
         const float* xc = pxc + c * Tp;
         float sum = 0.0f;
+#pragma unroll 1
         for (int t = 0; t < Tp; t += 4) {
             const float4 vs = *reinterpret_cast<const float4*>(xs + t), vc = *reinterpret_cast<const float4*>(xc + t);
             const uint32_t q = tp4(t);
@@ -1087,6 +1155,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     }
     if (warp == kFrontWarps - 1) {
         bool gray = true, same_a = true;
+#pragma unroll 1
         for (int t = lane; t < T; t += 32) {
             gray = gray && px[t].x == px[t].y && px[t].x == px[t].z;
             same_a = same_a && px[t].w == px[0].w;
@@ -1098,6 +1167,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     __syncthreads();
     const bool is_const = M.is_const != 0;
     const float ew = (((cw.x + cw.y) + cw.z) + cw.w) / 4.0f;
+#pragma unroll 1
     for (int t = tid; t < T; t += kFrontThreads) {
         const int p = tp1(t);
         const float span = fmaxf(M.mx[p] - M.mn[p], 1e-6f);
@@ -1105,6 +1175,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         wes[t] = M.lsq[p] * ew;
     }
     // pass08, second part: the encoding-choice axes of partition p (role p)
+#pragma unroll 1
     for (int p = role; p < P; p += kFrontThreads) {
         const float4 sx = make_float4(M.sxyz[p][0][0], M.sxyz[p][0][1], M.sxyz[p][0][2], 0.0f);
         const float4 sy = make_float4(M.sxyz[p][1][0], M.sxyz[p][1][1], M.sxyz[p][1][2], 0.0f);
@@ -1144,10 +1215,12 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     __syncthreads();
     int16_t* blist = reinterpret_cast<int16_t*>(sm + fl.bml);
     if (bmm) {
+#pragma unroll 1
         for (int i = tid; i < nbm; i += kFrontThreads)
             if ((bmm[i >> 6] >> (i & 63)) & 1) { const int d = tb.bm(i).dm; atomicOr(&flags[d >> 5], 1u << (d & 31)); }
         if (warp == 0) {  // the masked block modes in ascending order: each 32-bit half word is its own ballot
             int n = 0;
+#pragma unroll 1
             for (int i0 = 0; i0 < nbm; i0 += 32) {
                 uint32_t b = (uint32_t)(bmm[i0 >> 6] >> (i0 & 63));
                 if (nbm - i0 < 32) b &= (1u << (nbm - i0)) - 1u;
@@ -1158,6 +1231,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         }
     }
     // pass08 error terms of every texel against its partition's axes
+#pragma unroll 1
     for (int t = tid; t < Tp; t += kFrontThreads) {
         float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f, t3 = 0.0f, t4 = 0.0f;
         if (t < T) {
@@ -1184,7 +1258,9 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     // sums (role 5p + k)
     if (bmm && warp == 0) {
         int n = 0;
+#pragma unroll 1
         for (int pass = 0; pass < 2; pass++)
+#pragma unroll 1
             for (int d0 = 0; d0 < ndm; d0 += 32) {
                 const int d = d0 + lane;
                 const bool f = d < ndm && ((flags[d >> 5] >> (d & 31)) & 1) && ((tb.dm(d).W == T) == (pass == 1));
@@ -1195,10 +1271,12 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         __syncwarp();
         if (lane == 0) flags[0] = n;  // the flags are no longer needed
     }
+#pragma unroll 1
     for (int v = role; v < 5 * P; v += kFrontThreads) {
         const int p = v / 5, k = v % 5;
         const float* x = terms + k * Tp;
         float s = 0.0f;
+#pragma unroll 1
         for (int t = 0; t < Tp; t += 4) {
             const float4 y = *reinterpret_cast<const float4*>(x + t);
             const uint32_t q = tp4(t);
@@ -1212,6 +1290,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     const int16_t* dm_run = bmm ? list : nullptr;
     // ---------------- pass09: colour error per partition, quant level and integer count
     // (role 21p + q; runs beside passes 02-05, which do not read it)
+#pragma unroll 1
     for (int c = role; c < P * 21; c += kFrontThreads) {
         const int p = c / 21, q = c % 21;
         if (q < 4) {
@@ -1241,22 +1320,24 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     }
 
     // ---------------- passes 02-05
-    dm_passes<kFrontWarps>(tb, T, fl, sm, ndm_run, dm_run, iw, wes, is_const, dec, lov, hiv, qfs);
+    dm_passes<NT>(tb, T, a.L.max_w, ndm_run, dm_run, iw, wes, is_const, dec, reinterpret_cast<uint16_t*>(sm + fl.trig), lov, hiv, qfs);
     __syncthreads();
 
     // ---------------- pass07: weight quantisation error per block mode
     const int nlist = bmm ? M.nlive : nbm;  // block modes evaluated: the list, or all of them
-    if (!bmm) pass07_all_modes<kFrontThreads>(tb, T, P, nbm, lov, hiv, M.min_cutoff, dec, qfs, iw, wes, is_const, bm_err, bm_bits);
+    if (!bmm) pass07_all_modes<kFrontThreads>(tb, T, P, nbm, lov, hiv, M.min_cutoff, dec, qfs, iw, wes, is_const, bm_err);
     // ---------------- pass10: best format combination per quant level and integer total
     // One item per (quant level, integer total), beside pass07 (role-indexed): the format
     // combinations with that total, in the order the one-thread loops visit them (i, j, k, l
     // ascending, each format class within one of the others), so the first minimum is the same.
     if (P > 1) {
         const int NC = P == 2 ? 7 : P == 3 ? 10 : 13;
+#pragma unroll 1
         for (int it = role; it < 17 * NC; it += kFrontThreads) {
             const int q = 4 + it / NC, c = it - (it / NC) * NC;
             float be = ERR_DEFAULT;
             uint32_t bf = 0;
+#pragma unroll 1
             for (int o = c_combo_off[P - 2][c]; o < c_combo_off[P - 2][c + 1]; o++) {
                 const uint32_t cb = c_combo[o];
                 const int i = cb & 3, j = (cb >> 2) & 3, k = (cb >> 4) & 3, l = cb >> 6;
@@ -1283,30 +1364,35 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         const int G = qf_floats / (mw + Tp);
         float* qw = qfs;           // [G][mw]
         float* et = qfs + G * mw;  // [G][Tp]
+#pragma unroll 1
         for (int g0 = 0; g0 < nlist; g0 += G) {
             const int g = min(G, nlist - g0);
+#pragma unroll 1
             for (int it = tid; it < g * mw; it += kFrontThreads) {
                 const int k = it / mw, w = it - k * mw;
                 const DevBm bm = tb.bm(blist[g0 + k]);
                 const int bc = c_free_bits[P - 1] - (int)bm.weight_bits;
-                if (bm.quant > 11 || bc <= 0 || w >= (int)tb.dm(bm.dm).W) continue;
+                const DevDm dmi = tb.dm(bm.dm);
+                if (bm.quant > 11 || bc <= 0 || w >= (int)dmi.W) continue;
                 const BmQuant s = bm_quant_setup(tb, bm, lov + bm.dm * 8, hiv + bm.dm * 8, M.min_cutoff);
                 float qf;
-                bm_quant_weight(tb, s, dec[bm.dm * 64 + w], &qf);
+                bm_quant_weight(tb, s, dec[dmi.w_off + w], &qf);
                 qw[k * mw + w] = qf;
             }
             __syncthreads();
+#pragma unroll 1
             for (int it = tid; it < g * Tp; it += kFrontThreads) {
                 const int k = it / Tp, t = it - k * Tp;
                 const DevBm bm = tb.bm(blist[g0 + k]);
                 const int bc = c_free_bits[P - 1] - (int)bm.weight_bits;
                 float term = 0.0f;
                 if (t < T && !(bm.quant > 11 || bc <= 0)) {
-                    const uint64_t e4 = tb.tw4(bm.dm, t);
+                    const uint4 e = tb.tw4f(bm.dm, t);
                     const float* qk = qw + k * mw;
-                    float v = 0.0f;
-#pragma unroll
-                    for (int j = 0; j < 4; j++) { const uint32_t e = (uint32_t)(e4 >> (16 * j)) & 0xFFFF; v = v + qk[e & 0xFF] * ((float)(e >> 8) * (1.0f / 16.0f)); }
+                    float v = qk[entry_index(e.x)] * entry_factor(e.x);
+                    v = v + qk[entry_index(e.y)] * entry_factor(e.y);
+                    v = v + qk[entry_index(e.z)] * entry_factor(e.z);
+                    v = v + qk[entry_index(e.w)] * entry_factor(e.w);
                     const float d = v - iw[t];
                     term = (d * d) * wes[is_const ? 0 : t];
                 }
@@ -1314,69 +1400,57 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
             }
             __syncthreads();
             // (the next group's first phase writes only qw, which this one does not read)
+#pragma unroll 1
             for (int k = tid; k < g; k += kFrontThreads) {
                 const int i = blist[g0 + k];
                 const DevBm bm = tb.bm(i);
                 const int bc = c_free_bits[P - 1] - (int)bm.weight_bits;
-                if (bm.quant > 11 || bc <= 0) { bm_err[i] = 1e38f; bm_bits[i] = 0; continue; }
+                if (bm.quant > 11 || bc <= 0) { bm_err[i] = 1e38f; continue; }
                 const float* x = et + k * Tp;
                 float err = 0.0f;
+#pragma unroll 1
                 for (int t = 0; t < Tp; t += 4) {
                     const float4 y = *reinterpret_cast<const float4*>(x + t);
                     err = err + y.x; err = err + y.y; err = err + y.z; err = err + y.w;
                 }
                 bm_err[i] = err;
-                bm_bits[i] = bc;
             }
         }
     }
     __syncthreads();
-    // ---------------- pass11: best colour combination per block mode
+    // ---------------- pass11: best colour combination per block mode, its error added to the
+    // weights'
+#pragma unroll 1
     for (int k = tid; k < nlist; k += kFrontThreads) {
         const int i = bmm ? blist[k] : k;
         const float werr = bm_err[i];
-        uint8_t* fm = ccr_fmt + i * 4;
-        if (werr >= ERR_DEFAULT) { ccr_tot[i] = ERR_DEFAULT; ccr_q[i * 2] = ccr_q[i * 2 + 1] = 0; fm[0] = fm[1] = fm[2] = fm[3] = 0; continue; }
-        const int bits = bm_bits[i];
-        int best_i = 0;
-        float best_e = ERR_DEFAULT;
-        if (P == 1) {
-            for (int ic = 1; ic <= 4; ic++) {
-                const int ql = tb.qmt(ic, bits);
-                if (ql < 4) continue;
-                const float e = M.cerr[0][ql][ic - 1];
-                if (e < best_e) { best_e = e; best_i = ic; }
-            }
-            const int fql = tb.qmt(best_i, bits);
-            fm[0] = fql >= 4 ? M.cfmt[0][fql][best_i - 1] : FMT_LUMINANCE;
-            fm[1] = fm[2] = fm[3] = 0;
-            ccr_q[i * 2] = ccr_q[i * 2 + 1] = (uint8_t)fql;
-        } else {
-            const int hi = P == 2 ? 8 : 9, modb = P == 2 ? 2 : P == 3 ? 5 : 8;
-            for (int ic = P; ic <= hi; ic++) {
-                const int ql = tb.qmt(ic, bits);
-                if (ql < 4) break;
-                const float e = M.combo_err[ql][ic - P];
-                if (e < best_e) { best_e = e; best_i = ic; }
-            }
-            const int fql = tb.qmt(best_i, bits), fqlm = tb.qmt(best_i, bits + modb);
-            for (int k = 0; k < 4; k++) fm[k] = fql >= 4 ? M.combo_fmt[fql][best_i - P][k] : 0;
-            ccr_q[i * 2] = (uint8_t)fql; ccr_q[i * 2 + 1] = (uint8_t)fqlm;
+        if (werr >= ERR_DEFAULT) { bm_err[i] = ERR_DEFAULT; continue; }
+        const int bits = c_free_bits[P - 1] - (int)tb.bm(i).weight_bits;
+        const int lo = P == 1 ? 1 : P, hi = P == 1 ? 4 : P == 2 ? 8 : 9;
+        float best = ERR_DEFAULT;
+        int ints = 0;
+#pragma unroll 1
+        for (int ic = lo; ic <= hi; ic++) {
+            const int ql = tb.qmt(ic, bits);
+            if (ql < 4) { if (P == 1) continue; break; }
+            const float e = P == 1 ? M.cerr[0][ql][ic - 1] : M.combo_err[ql][ic - P];
+            if (e < best) { best = e; ints = ic; }
         }
-        ccr_tot[i] = best_e + werr;
+        bm_err[i] = best + werr;
+        mode_ints[i] = (uint8_t)ints;
     }
     __syncthreads();
     // ---------------- pass12: the 8 best trials (first minimum wins ties)
     // warp 0 picks them in order: each round the (error, index)-smallest mode after the
-    // previous pick -- the order in which counting, for every mode, the modes ranked
-    // before it would place them
+    // previous pick
     if (warp == 0 && bmm && nlist <= 32) {
         // up to 32 listed modes, one per lane: a usable mode's pick position is the number
         // of usable modes before it in (error, index) order
         const int i = lane < nlist ? blist[lane] : 0x7FFFFFFF;
-        const float e = lane < nlist ? ccr_tot[i] : ERR_DEFAULT;
+        const float e = lane < nlist ? bm_err[i] : ERR_DEFAULT;
         const bool ok = e < ERR_DEFAULT;
         int rank = 0;
+#pragma unroll 1
         for (int j = 0; j < nlist; j++) {
             const float ej = __shfl_sync(FULL, e, j);
             const int ij = __shfl_sync(FULL, i, j);
@@ -1386,29 +1460,37 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         if (ok && rank < kNumCand) M.top[rank] = i;
         if (lane >= nok && lane < kNumCand) M.top[lane] = -1;
     } else if (warp == 0) {
-        float pv = 0.0f;
+        // each lane keeps the best of its own modes (in a key that orders like the error) and
+        // looks for its next one only when its best was picked
+        uint32_t mine = 0xFFFFFFFFu;
+        int mi = 0x7FFFFFFF;
+        float pv = -3.4e38f;  // the lane's last pick
         int pi = -1;
+        bool look = true;
+#pragma unroll 1
         for (int r = 0; r < kNumCand; r++) {
-            float be = 3.4e38f;
-            int bi = 0x7FFFFFFF;
-            for (int k = lane; k < nlist; k += 32) {
-                const int i = bmm ? blist[k] : k;
-                const float e = ccr_tot[i];
-                if (!(e < ERR_DEFAULT)) continue;
-                if (r > 0 && !(e > pv || (e == pv && i > pi))) continue;
-                if (e < be || (e == be && i < bi)) { be = e; bi = i; }
+            if (look) {
+                float be = ERR_DEFAULT;
+                mi = 0x7FFFFFFF;
+#pragma unroll 1
+                for (int k = lane; k < nlist; k += 32) {
+                    const int i = bmm ? blist[k] : k;
+                    const float e = bm_err[i];
+                    if (e < be && (e > pv || (e == pv && i > pi))) { be = e; mi = i; }  // a lane's modes ascend
+                }
+                const uint32_t u = fbits(be + 0.0f);
+                mine = mi == 0x7FFFFFFF ? 0xFFFFFFFFu : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
+                pv = be;
+                look = false;
             }
-            for (int o = 16; o > 0; o >>= 1) {
-                const float oe = __shfl_xor_sync(0xFFFFFFFFu, be, o);
-                const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-                if (oe < be || (oe == be && oi < bi)) { be = oe; bi = oi; }
-            }
-            if (bi == 0x7FFFFFFF) {  // fewer than kNumCand usable modes
+            const uint32_t best = __reduce_min_sync(FULL, mine);
+            if (best == 0xFFFFFFFFu) {  // fewer than kNumCand usable modes
                 if (lane >= r && lane < kNumCand) M.top[lane] = -1;
                 break;
             }
-            if (lane == 0) M.top[r] = bi;
-            pv = be; pi = bi;
+            const uint32_t bi = __reduce_min_sync(FULL, mine == best ? (uint32_t)mi : 0xFFFFFFFFu);
+            if (lane == 0) M.top[r] = (int)bi;
+            if ((uint32_t)mi == bi) { pi = mi; look = true; }
         }
     }
     __syncthreads();
@@ -1417,6 +1499,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         int nbm_run = nbm;
         if (bmm) {
             nbm_run = 0;
+#pragma unroll 1
             for (int w = 0; w < kMaskWords; w++) {
                 const int lo = w * 64;
                 if (lo >= nbm) break;
@@ -1440,27 +1523,38 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     // candidate initial state: the trial's quantised weights (REF-BUG-6: only
     // floor(W/4)*4 weights are packed by pass07, the rest read as 0; FIXED semantics: all W)
     const int ncand = M.ncand;
+#pragma unroll 1
     for (int k = tid >> 3; k < ncand; k += kFrontThreads / 8) {
         const int i = M.top[k];
         const DevBm bm = tb.bm(i);
         const DevDm dmi = tb.dm(bm.dm);
         CandInit& c = rec.c[k];
         if ((tid & 7) == 0) {
-            c.bm = (uint16_t)i; c.ql = ccr_q[i * 2]; c.qlm = ccr_q[i * 2 + 1];
-            for (int f = 0; f < 4; f++) c.fmt[f] = ccr_fmt[i * 4 + f];
+            const int bits = c_free_bits[P - 1] - (int)bm.weight_bits, ints = mode_ints[i];
+            const int ql = tb.qmt(ints, bits), qlm = P == 1 ? ql : tb.qmt(ints, bits + (P == 2 ? 2 : P == 3 ? 5 : 8));
+            uint32_t fmt = 0;
+            if (P == 1) fmt = ql >= 4 ? M.cfmt[0][ql][ints - 1] : (uint32_t)FMT_LUMINANCE;
+            else if (ql >= 4) fmt = *reinterpret_cast<const uint32_t*>(M.combo_fmt[ql][ints - P]);
+            // bm, ql, qlm and the four formats: 8-byte aligned in PBRec
+            *reinterpret_cast<uint2*>(&c) = make_uint2((uint32_t)i | (uint32_t)(ql & 0xFF) << 16 | (uint32_t)(qlm & 0xFF) << 24, fmt);
         }
         const BmQuant s = bm_quant_setup(tb, bm, lov + bm.dm * 8, hiv + bm.dm * 8, M.min_cutoff);
         const int packed_w = a.fixed ? dmi.W : (dmi.W / 4) * 4;
-        for (int w = tid & 7; w < 64; w += 8) {
-            int v = 0;
-            if (w < packed_w) { float qf; v = bm_quant_weight(tb, s, dec[bm.dm * 64 + w], &qf); }
-            c.qw[w] = (uint8_t)v;
+        const float* dw = dec + dmi.w_off;
+#pragma unroll 1
+        for (int j = tid & 7; j < 16; j += 8) {  // four weights a word
+            uint32_t word = 0;
+#pragma unroll 1
+            for (int w = 4 * j; w < min(4 * j + 4, packed_w); w++) {
+                float qf;
+                word |= bm_quant_weight(tb, s, dw[w], &qf) << (8 * (w & 3));
+            }
+            reinterpret_cast<uint32_t*>(c.qw)[j] = word;
         }
     }
 }
 
-// Resident CTAs of 128 threads the register budget is sized for (the proposal search's
-// compact layout lets that many fit in shared memory for the small footprints).
+// Resident CTAs of 128 threads the register budget is sized for.
 constexpr int kFrontMinBlocks128 = 8;
 template <int NT, bool P1>
 __global__ void __launch_bounds__(NT, kFrontMinBlocks128 * 128 / NT > 32 ? 32 : kFrontMinBlocks128 * 128 / NT) k_front(const __grid_constant__ KernelArgs a) {
@@ -1499,15 +1593,37 @@ __global__ void __launch_bounds__(NT, kFrontMinBlocks128 * 128 / NT > 32 ? 32 : 
 
 }  // namespace
 
-size_t search_smem_bytes(const TableLayout& L) { return (size_t)kSearchWarps * search_layout(L.T).total; }
-size_t front_smem_bytes(const TableLayout& L, int nt, bool list) { return (size_t)front_layout(L.T, L.ndm, L.nbm, L.max_w, nt, list).total; }
+// Threads per partitioned block.  Small blocks have few items per step (4x4: 6 decimation
+// modes, 53 block modes), so one warp, whose barriers are cheap and of which more are resident,
+// is fastest; large ones hold enough for more, and their shared memory, the same for any
+// number of threads but for pass07's weights, limits the resident CTAs to two or three.
+// Measured (B200, 2,048 blocks, all 13 partitioned blocks), 32 / 64 / 128 / 256 threads, in us: 4x4
+// 411 / 465 / 567 / 995, 5x4 584 / 651 / 680 / 1110, 5x5 928 / 895 / 893 / 1304, 6x6 2198 / 1616 /
+// 1542 / 1836, 10x8 15259 / 8785 / 6768 / 8017, 12x10 40427 / 21252 / 12438 / 11803, 12x12 74917 /
+// 40147 / 23795 / 15542.  Proposal search's lists of 1024x1024: 4x4 861 / 1060 / 1377, 6x6 712 / 669
+// / 720.  A launch that leaves SMs without a warp is as long as one item: 128 threads then.
+static int front_nt(int T, bool list, int items) {
+    if (items < 148 * 4) return 128;
+    if (T <= 20) return 32;
+    if (list) return 64;
+    return T >= 120 ? 256 : 128;
+}
+static int front_nt(const KernelArgs& a) {
+    if (a.front_threads == 32 || a.front_threads == 64 || a.front_threads == 128) return a.front_threads;
+    return front_nt(a.L.T, a.bm_mask != nullptr, a.nblocks * a.slots);
+}
 
-// front_bytes: the 128-thread layout, the largest of the three.
+size_t search_smem_bytes(const TableLayout& L) { return (size_t)kSearchWarps * search_layout(L.T).total; }
+size_t front_smem_bytes(const TableLayout& L, int nt, bool list) { return (size_t)front_layout(L, nt, list).total; }
+size_t front_smem_bytes(const TableLayout& L) {  // the largest over the launches of this footprint
+    return std::max(front_smem_bytes(L, 128, false), front_smem_bytes(L, front_nt(L.T, false, 1 << 30), false));
+}
+
 cudaError_t configure_search_kernels(size_t search_bytes, size_t front_bytes) {
     cudaError_t e = cudaFuncSetAttribute(k_partition_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)search_bytes);
     // the largest shared-memory carveout: occupancy of the front is bounded by shared memory
-    for (auto f : {k_front<128, false>, k_front<64, false>, k_front<32, false>, k_front<128, true>, k_front<64, true>,
-                   k_front<32, true>}) {
+    for (auto f : {k_front<256, false>, k_front<128, false>, k_front<64, false>, k_front<32, false>, k_front<128, true>,
+                   k_front<64, true>, k_front<32, true>}) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)front_bytes);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
@@ -1523,13 +1639,14 @@ cudaError_t launch_partition_search(const KernelArgs& a, cudaStream_t s) {
 }
 
 cudaError_t launch_front(const KernelArgs& a, cudaStream_t s) {
-    const int nt = a.front_threads == 32 || a.front_threads == 64 ? a.front_threads : 128;
+    const int nt = front_nt(a);
     int grid = a.nblocks * a.slots;
-    if (a.block_list) grid = std::min(grid, kListGridFront * (128 / nt));
+    if (a.block_list) grid = std::min(grid, kListGridFront * 128 / nt);
     const size_t smem = front_smem_bytes(a.L, nt, a.bm_mask != nullptr);
     auto go = [&](const KernelArgs& k, bool p1) {
         if (nt == 32) { if (p1) k_front<32, true><<<grid, 32, smem, s>>>(k); else k_front<32, false><<<grid, 32, smem, s>>>(k); }
         else if (nt == 64) { if (p1) k_front<64, true><<<grid, 64, smem, s>>>(k); else k_front<64, false><<<grid, 64, smem, s>>>(k); }
+        else if (nt == 256) k_front<256, false><<<grid, 256, smem, s>>>(k);
         else { if (p1) k_front<128, true><<<grid, 128, smem, s>>>(k); else k_front<128, false><<<grid, 128, smem, s>>>(k); }
     };
     if (a.pb_list && a.pb_from == 0 && a.pb_to == 0) {

@@ -38,7 +38,7 @@ namespace astcb200 {
 namespace {
 
 constexpr size_t kNoallocBytes = size_t(52) << 20;
-constexpr size_t kNoallocTableBytes = size_t(8) << 20;  // every footprint's tables: 7.80 MiB
+constexpr size_t kNoallocTableBytes = size_t(8) << 20;  // every footprint's tables: 6.95 MiB
 constexpr uint32_t kNoallocMaxBlocks = 2048;
 
 __device__ __align__(256) uint8_t g_noalloc_scratch[kNoallocBytes];

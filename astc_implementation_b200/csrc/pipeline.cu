@@ -151,8 +151,7 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
     ap.block_list = r.pruned; ap.block_count = counts;
     ap.prop = r.prop; ap.bm_mask = r.masks;
     ap.slots = 1 + pr.kmax; ap.topn = pr.topn;
-    // small blocks: two warps per partitioned block keep twice as many of them resident
-    ap.front_threads = pr.front_threads ? pr.front_threads : (ft->L.T <= 16 ? 64 : 128);
+    ap.front_threads = pr.front_threads;
     ap.refine_iters = pr.refine_iters;
     ap.reroute_list = r.full; ap.reroute_count = counts + 1;  // blocks left without a candidate
     ap.pb_list = r.pb_list; ap.pb_count = counts + 2; ap.pb_stride = r.pb_stride;

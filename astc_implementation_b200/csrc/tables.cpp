@@ -492,16 +492,18 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     const int T = h.T, ndm = L.ndm;
     std::vector<DevDm> dms(ndm);
     std::vector<uint8_t> twc((size_t)ndm * T, 0), wtc((size_t)ndm * 64, 0);
+    std::vector<int> tw_base(ndm);
     std::vector<uint16_t> tws((size_t)ndm * T, 0), wts((size_t)ndm * 64, 0), t2w, w2t;
     for (int m = 0; m < ndm; m++) {
         const HostTables::Dm& d = h.dms[h.valid_dms[m]];
         DevDm& o = dms[m];
         o.W = (uint8_t)d.W; o.wx = (uint8_t)d.wx; o.wy = (uint8_t)d.wy; o.max_quant_level = (uint8_t)d.maxq;
-        o.max_angular_steps = (uint8_t)d.steps; o.max_quant_steps = (uint8_t)d.qsteps; o.pad0 = o.pad1 = 0;
-        o.tw_base = (uint16_t)t2w.size(); o.wt_base = (uint16_t)w2t.size();
+        o.max_angular_steps = (uint8_t)d.steps; o.max_quant_steps = (uint8_t)d.qsteps; o.w_off = (uint16_t)L.nw_total;
+        L.nw_total += (int)((d.W + 3) & ~3u);
+        tw_base[m] = (int)t2w.size(); o.pad = 0; o.wt_base = (uint16_t)w2t.size();
         for (int t = 0; t < T; t++) {
             twc[(size_t)m * T + t] = (uint8_t)d.tw_count[t];
-            tws[(size_t)m * T + t] = (uint16_t)(t2w.size() - o.tw_base);
+            tws[(size_t)m * T + t] = (uint16_t)(t2w.size() - tw_base[m]);
             for (uint32_t j = 0; j < d.tw_count[t]; j++) {
                 const uint32_t e = d.tw_off[t] + j;
                 t2w.push_back((uint16_t)(h.t2w_w[e] | (h.t2w_k[e] << 8)));
@@ -520,7 +522,7 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     for (int m = 0; m < ndm; m++)
         for (int t = 0; t < T; t++) {
             uint64_t v = 0;
-            const int n = twc[(size_t)m * T + t], base = dms[m].tw_base + tws[(size_t)m * T + t];
+            const int n = twc[(size_t)m * T + t], base = tw_base[m] + tws[(size_t)m * T + t];
             for (int j = 0; j < n; j++) v |= (uint64_t)t2w[base + j] << (16 * j);
             tw4[(size_t)m * T + t] = v;
         }
@@ -531,7 +533,7 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
         const HostTables::Bm& b = h.bms[h.valid_bms[i].first];
         bms[i] = DevBm{(uint16_t)b.mode, (uint8_t)h.valid_bms[i].second, (uint8_t)b.quant, (uint8_t)b.bits, {0, 0, 0}};
     }
-    std::vector<uint8_t> ptex((size_t)3 * 1024 * T), pcnt((size_t)3 * 1024 * 4);
+    std::vector<uint8_t> pcnt((size_t)3 * 1024 * 4);
     const int part2_words = (T + 15) / 16;
     std::vector<uint32_t> pinfo(3 * 1024), part2((size_t)3 * 1024 * part2_words, 0);
     std::vector<uint64_t> cov((size_t)3 * 1024 * 4, 0);
@@ -539,7 +541,6 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
         for (int e = 0; e < 1024; e++) {
             const HostTables::Part& p = h.parts[(pc - 2) * 1024 + e];
             const size_t k = (size_t)(pc - 2) * 1024 + e;
-            std::memcpy(&ptex[k * T], p.of, T);
             for (int t = 0; t < T; t++) part2[k * part2_words + t / 16] |= (uint32_t)p.of[t] << (2 * (t & 15));
             for (int q = 0; q < 4; q++) pcnt[k * 4 + q] = (uint8_t)p.tcount[q];
             pinfo[k] = p.seed;
@@ -559,22 +560,65 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     std::stable_sort(order.begin(), order.end(), [&](uint16_t x, uint16_t y) { return bms[x].dm < bms[y].dm; });
     L.off_dm = put(blob, dms.data(), dms.size());
     L.off_bm = put(blob, bms.data(), bms.size());
-    L.off_tw_count = put(blob, twc.data(), twc.size());
-    L.off_tw_start = put(blob, tws.data(), tws.size());
     L.off_wt_count = put(blob, wtc.data(), wtc.size());
     L.off_wt_start = put(blob, wts.data(), wts.size());
-    L.off_t2w = put(blob, t2w.data(), t2w.size());
     L.off_w2t = put(blob, w2t.data(), w2t.size());
     L.off_tw4 = put(blob, tw4.data(), tw4.size());
     L.off_bm_order = put(blob, order.data(), order.size());
     L.off_dual = put(blob, dual.data(), dual.size());
-    L.off_part_texel = put(blob, ptex.data(), ptex.size());
     L.off_part2 = put(blob, part2.data(), part2.size());
     L.off_part_info = put(blob, pinfo.data(), pinfo.size());
     L.off_part_counts = put(blob, pcnt.data(), pcnt.size());
     L.off_cov = put(blob, cov.data(), cov.size());
-    L.off_sin = put(blob, h.sin_t.data(), h.sin_t.size());
-    L.off_cos = put(blob, h.cos_t.data(), h.cos_t.size());
+    std::vector<float> trig(2 * (h.cos_t.size() + 16), 0.0f);
+    for (size_t i = 0; i < h.cos_t.size(); i++) { trig[2 * i] = h.cos_t[i]; trig[2 * i + 1] = h.sin_t[i]; }
+    L.off_trig = put(blob, trig.data(), trig.size());
+    // entries with the contribution k / 16 (k <= 16, exact in bf16) ready to use as the high half of a float
+    auto ready = [](uint32_t e) {
+        const float c = (float)(e >> 8) * (1.0f / 16.0f);
+        uint32_t u;
+        std::memcpy(&u, &c, 4);
+        return (u & 0xFFFF0000u) | (e & 0xFF);
+    };
+    std::vector<uint32_t> tw4f((size_t)ndm * T * 4), w2tf;
+    for (size_t i = 0; i < tw4.size(); i++)
+        for (int j = 0; j < 4; j++) tw4f[4 * i + j] = ready((uint32_t)(tw4[i] >> (16 * j)) & 0xFFFF);
+    std::vector<uint32_t> wt_info((size_t)ndm * 64, 0);
+    std::vector<uint16_t> witem, sitem;
+    for (int m = 0; m < ndm; m++) {
+        if (dms[m].max_angular_steps > kMaxAngularSteps) return false;
+        for (int w = 0; w < dms[m].W; w++) {
+            const int first = dms[m].wt_base + wts[(size_t)m * 64 + w], n = wtc[(size_t)m * 64 + w];
+            wt_info[(size_t)m * 64 + w] = (uint32_t)(w2tf.size() / 4) | (uint32_t)((n + 3) / 4) << 16;
+            for (int j = 0; j < ((n + 3) & ~3); j++) w2tf.push_back(j < n ? ready(w2t[first + j]) : 0u);
+            witem.push_back((uint16_t)(m << 6 | w));
+        }
+        for (int i = 0; i < dms[m].max_angular_steps; i++) sitem.push_back((uint16_t)(m << 4 | i));
+    }
+    auto texels_of = [&](uint16_t e) -> uint32_t { return dms[e >> 6].W == T ? 0 : wt_info[e] >> 16; };  // in fours
+    std::stable_sort(witem.begin(), witem.end(), [&](uint16_t x, uint16_t y) { return texels_of(x) > texels_of(y); });
+    std::stable_sort(sitem.begin(), sitem.end(), [&](uint16_t x, uint16_t y) { return dms[x >> 4].W > dms[y >> 4].W; });
+    L.nwi = (int)witem.size(); L.nsi = (int)sitem.size();
+    std::vector<uint32_t> wgroup, wgent;  // items of a mode of one weight a texel have no entries
+    for (size_t g = 0; g < witem.size(); g += 32) {
+        uint32_t n4 = 0;
+        for (size_t i = g; i < std::min(g + 32, witem.size()); i++) n4 = std::max(n4, (texels_of(witem[i]) + 0u));
+        wgroup.push_back((uint32_t)(wgent.size() / 128) | n4 << 16);
+        for (uint32_t j = 0; j < n4; j++)
+            for (size_t i = g; i < g + 32; i++)
+                for (int k = 0; k < 4; k++) {
+                    const bool has = i < witem.size() && j < texels_of(witem[i]);
+                    wgent.push_back(has ? w2tf[((wt_info[witem[i]] & 0xFFFF) + j) * 4 + k] : 0u);
+                }
+    }
+    if (w2tf.size() / 4 > 0xFFFF || wgent.size() / 128 > 0xFFFF) return false;
+    L.off_wgroup = put(blob, wgroup.data(), wgroup.size());
+    L.off_wgent = put(blob, wgent.data(), wgent.size());
+    L.off_wt_info = put(blob, wt_info.data(), wt_info.size());
+    L.off_witem = put(blob, witem.data(), witem.size());
+    L.off_sitem = put(blob, sitem.data(), sitem.size());
+    L.off_tw4f = put(blob, tw4f.data(), tw4f.size());
+    L.off_w2tf = put(blob, w2tf.data(), w2tf.size());
     L.off_q2u = put(blob, c.q2u, 142);
     L.off_q2u_start = put(blob, c.q2u_start, 12);
     L.off_qmt = put(blob, &c.qmt[0][0], 1280);

@@ -234,7 +234,7 @@ typedef struct astcb200_pruning {
                                    B 0.2475, A 1) also takes the full search, and the better of
                                    the two results is kept; 0 disables */
     uint32_t front_threads;     /* threads per CTA of the proposal pass's front kernel: 32, 64 or
-                                   128 (0 = 64 for blocks of up to 16 texels, else 128); results
+                                   128 (0 = chosen by footprint and launch size); results
                                    do not depend on it */
     uint32_t refine_iterations; /* refinement iterations of the proposal pass, 1..6 (0 = tuned: 6,
                                    as the reference and the full search) */

@@ -47,3 +47,15 @@ def test_partition_search_around_the_wide_limit(w, h, bx, by, fixed):
     hole = rng.random((h, w, 4)) < 0.02
     img[hole] = 0
     check_full_search(img, bx, by, fixed)
+
+
+@pytest.mark.parametrize("fixed", [False, True])
+@pytest.mark.parametrize("bx,by,blocks_x,blocks_y", [(4, 4, 9, 5),    # 585 partitioned blocks: 128 threads each
+                                                     (4, 4, 23, 2),   # 598: 32
+                                                     (5, 4, 23, 2),   # 32
+                                                     (5, 5, 23, 2),   # 128
+                                                     (12, 10, 23, 2),  # 256
+                                                     (12, 12, 12, 4)])  # 256
+def test_front_threads_by_footprint_and_launch_size(bx, by, blocks_x, blocks_y, fixed):
+    img = synth.make_texture(bx * blocks_x - 1, by * blocks_y, 57 + bx)
+    check_full_search(img, bx, by, fixed)
