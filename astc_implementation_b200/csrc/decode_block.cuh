@@ -10,15 +10,15 @@
 #include <stdint.h>
 
 #ifdef __CUDACC__
-#define ASTC_HD __host__ __device__ __forceinline__
+#define ASTC_HD __host__ __device__ __forceinline__ constexpr
 // The unquantisation functions stay out of line in device code: inlined into
 // parse_block, the optimised device build decoded some weights wrongly (found by the
 // device-against-host decoder tests; the debug build and the out-of-line build agree
 // with the host on every block).
-#define ASTC_HD_CALL static __host__ __device__ __noinline__
+#define ASTC_HD_CALL static __host__ __device__ __noinline__ constexpr
 #else
-#define ASTC_HD inline
-#define ASTC_HD_CALL inline
+#define ASTC_HD inline constexpr
+#define ASTC_HD_CALL inline constexpr
 #endif
 
 namespace astcb200 {
@@ -46,7 +46,7 @@ ASTC_HD void btq(int q, int& bits, int& trits, int& quints) {
     while ((1 << bits) < L) bits++;
 }
 ASTC_HD int ise_bits(int n, int q) {
-    int b, t, qu;
+    int b = 0, t = 0, qu = 0;
     btq(q, b, t, qu);
     if (t) return (n * (8 + 5 * b) + 4) / 5;
     if (qu) return (n * (7 + 3 * b) + 2) / 3;
@@ -55,7 +55,7 @@ ASTC_HD int ise_bits(int n, int q) {
 ASTC_HD int bit_of(int x, int i) { return (x >> i) & 1; }
 // the five trits packed in the 8-bit value T
 ASTC_HD void trit_digits(int T, int t[5]) {
-    int C;
+    int C = 0;
     if (((T >> 2) & 7) == 7) { C = (((T >> 5) & 7) << 2) | (T & 3); t[4] = 2; t[3] = 2; }
     else {
         C = T & 31;
@@ -73,14 +73,14 @@ ASTC_HD void quint_digits(int Q, int q[3]) {
         q[1] = 4; q[0] = 4;
         return;
     }
-    int C;
+    int C = 0;
     if (((Q >> 1) & 3) == 3) { q[2] = 4; C = (((Q >> 3) & 3) << 3) | (((~Q >> 5) & 3) << 1) | (Q & 1); }
     else { q[2] = (Q >> 5) & 3; C = Q & 31; }
     if ((C & 7) == 5) { q[1] = 4; q[0] = (C >> 3) & 3; } else { q[1] = (C >> 3) & 3; q[0] = C & 7; }
 }
 // Integer-sequence decode of n values of method q starting at bit `off`.
 ASTC_HD void decode_ise(const Bits& b, int off, int n, int q, int* out) {
-    int bits, trits, quints;
+    int bits = 0, trits = 0, quints = 0;
     btq(q, bits, trits, quints);
     if (trits) {
         for (int i = 0; i < n; i += 5) {
@@ -90,7 +90,7 @@ ASTC_HD void decode_ise(const Bits& b, int off, int n, int q, int* out) {
                 m[e] = (int)b.get(off, bits); off += bits;
                 T |= (int)b.get(off, tb) << sh; off += tb; sh += tb;
             }
-            int d[5];
+            int d[5] = {0, 0, 0, 0, 0};
             trit_digits(T, d);
             for (int e = 0; e < 5 && i + e < n; e++) out[i + e] = (d[e] << bits) | m[e];
         }
@@ -102,7 +102,7 @@ ASTC_HD void decode_ise(const Bits& b, int off, int n, int q, int* out) {
                 m[e] = (int)b.get(off, bits); off += bits;
                 Q |= (int)b.get(off, qb) << sh; off += qb; sh += qb;
             }
-            int d[3];
+            int d[3] = {0, 0, 0};
             quint_digits(Q, d);
             for (int e = 0; e < 3 && i + e < n; e++) out[i + e] = (d[e] << bits) | m[e];
         }
@@ -120,7 +120,7 @@ ASTC_HD int replicate(int v, int bits, int width) {
     return out >> (have - width);
 }
 ASTC_HD_CALL int unq_color(int q, int v) {
-    int bits, trits, quints;
+    int bits = 0, trits = 0, quints = 0;
     btq(q, bits, trits, quints);
     if (!trits && !quints) return replicate(v, bits, 8);
     const int D = v >> bits, m = v & ((1 << bits) - 1), A = (m & 1) ? 0x1FF : 0;
@@ -143,9 +143,9 @@ ASTC_HD_CALL int unq_color(int q, int v) {
     return (A & 0x80) | (((D * C + B) ^ A) >> 2);
 }
 ASTC_HD_CALL int unq_weight(int q, int v) {
-    int bits, trits, quints;
+    int bits = 0, trits = 0, quints = 0;
     btq(q, bits, trits, quints);
-    int r;
+    int r = 0;
     if (!trits && !quints) r = replicate(v, bits, 6);
     else {
         const int D = v >> bits, m = v & ((1 << bits) - 1), A = (m & 1) ? 0x7F : 0, b1 = (m >> 1) & 1, b2 = (m >> 2) & 1;
@@ -156,7 +156,7 @@ ASTC_HD_CALL int unq_weight(int q, int v) {
             const int tq[8] = {0, 32, 63, 0, 16, 32, 47, 63};
             r = tq[trits ? D : 3 + D];
         } else {
-            int B, C;
+            int B = 0, C = 0;
             if (trits) { C = bits == 1 ? 50 : bits == 2 ? 23 : 11; B = bits == 1 ? 0 : bits == 2 ? b1 * 0x45 : b2 * 0x42 + b1 * 0x21; }
             else { C = bits == 1 ? 28 : 13; B = bits == 1 ? 0 : b1 * 0x42; }
             r = (A & 0x20) | (((D * C + B) ^ A) >> 2);
@@ -165,9 +165,9 @@ ASTC_HD_CALL int unq_weight(int q, int v) {
     return r > 32 ? r + 1 : r;
 }
 struct Mode { int xw, yw, q; bool dual; };
-// Weight grid, weight quantisation and dual-plane flag of the 11-bit block mode m;
-// false for reserved modes and grids whose weights do not fit the spec's limits.
-ASTC_HD bool decode_mode(int m, Mode& o) {
+// Weight grid, weight quantisation and dual-plane flag of the 11-bit block mode m; false for
+// reserved modes.
+ASTC_HD bool decode_grid(int m, Mode& o) {
     int q = (m >> 4) & 1, H = (m >> 9) & 1, D = (m >> 10) & 1;
     const int A = (m >> 5) & 3;
     if (m & 3) {
@@ -195,7 +195,12 @@ ASTC_HD bool decode_mode(int m, Mode& o) {
     }
     o.q = (q - 2) + 6 * H;
     o.dual = D != 0;
-    const int n = o.xw * o.yw * (D + 1);
+    return true;
+}
+// The same, false also for grids whose weights do not fit the spec's limits.
+ASTC_HD bool decode_mode(int m, Mode& o) {
+    if (!decode_grid(m, o)) return false;
+    const int n = o.xw * o.yw * (o.dual ? 2 : 1);
     return n <= 64 && ise_bits(n, o.q) >= 24 && ise_bits(n, o.q) <= 96;
 }
 ASTC_HD uint32_t hash52(uint32_t v) {
@@ -208,9 +213,9 @@ ASTC_HD int select_partition(int seed, int x, int y, int pc, bool small) {
     if (small) { x <<= 1; y <<= 1; }
     seed += (pc - 1) * 1024;
     const uint32_t r = hash52((uint32_t)seed);
-    uint32_t s[8];
+    uint32_t s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int i = 0; i < 8; i++) { const uint32_t v = (r >> (4 * i)) & 0xF; s[i] = v * v; }
-    int sh1, sh2;
+    int sh1 = 0, sh2 = 0;
     if (seed & 1) { sh1 = (seed & 2) ? 4 : 5; sh2 = pc == 3 ? 6 : 5; } else { sh1 = pc == 3 ? 6 : 5; sh2 = (seed & 2) ? 4 : 5; }
     for (int i = 0; i < 8; i++) s[i] >>= (i & 1) ? sh2 : sh1;
     int a = (int)((s[0] * x + s[1] * y + (r >> 14)) & 0x3F), b = (int)((s[2] * x + s[3] * y + (r >> 10)) & 0x3F);
@@ -254,7 +259,7 @@ ASTC_HD bool decode_endpoints(int cem, const int* v, int* e0, int* e1) {
             return true;
         }
         case 9: case 13: {
-            int x[8];
+            int x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             for (int i = 0; i < 8; i++) x[i] = v[i];
             bts(x[1], x[0]); bts(x[3], x[2]); bts(x[5], x[4]);
             if (cem == 13) bts(x[7], x[6]);
@@ -289,12 +294,12 @@ ASTC_HD void parse_block(const uint8_t* blk, int bx, int by, Block& o) {
         o.kind = 1;
         return;
     }
-    Mode m;
+    Mode m{};
     if (!decode_mode(mode, m) || m.xw > bx || m.yw > by) return;
     const int pc = (int)b.get(11, 2) + 1;
     if (pc == 4 && m.dual) return;
     const int W = m.xw * m.yw, nw = W * (m.dual ? 2 : 1), wbits = ise_bits(nw, m.q);
-    int cem[4] = {0, 0, 0, 0}, seed = 0, below = 128 - wbits, cstart;
+    int cem[4] = {0, 0, 0, 0}, seed = 0, below = 128 - wbits, cstart = 0;
     if (pc == 1) { cem[0] = (int)b.get(13, 4); cstart = 17; }
     else {
         seed = (int)b.get(13, 10);
@@ -318,10 +323,10 @@ ASTC_HD void parse_block(const uint8_t* blk, int bx, int by, Block& o) {
     int cq = -1;
     for (int q = 20; q >= 0; q--) if (ise_bits(nv, q) <= avail) { cq = q; break; }
     if (cq < 4) return;
-    int cv[20], wv[64];
+    int cv[20] = {}, wv[64] = {};
     decode_ise(b, cstart, nv, cq, cv);
     for (int i = 0; i < nv; i++) cv[i] = unq_color(cq, cv[i]);
-    uint8_t rev[16];
+    uint8_t rev[16] = {};
     for (int i = 0; i < 16; i++) {
         int p = blk[15 - i];
         p = ((p & 0x0F) << 4) | ((p >> 4) & 0x0F); p = ((p & 0x33) << 2) | ((p >> 2) & 0x33); p = ((p & 0x55) << 1) | ((p >> 1) & 0x55);
@@ -331,7 +336,7 @@ ASTC_HD void parse_block(const uint8_t* blk, int bx, int by, Block& o) {
     for (int i = 0; i < nw; i++) o.w[i] = (uint8_t)unq_weight(m.q, wv[i]);
     int vo = 0;
     for (int i = 0; i < pc; i++) {
-        int e0[4], e1[4];
+        int e0[4] = {}, e1[4] = {};
         if (!decode_endpoints(cem[i], cv + vo, e0, e1)) return;
         for (int c = 0; c < 4; c++) { o.e0[i][c] = (uint8_t)e0[c]; o.e1[i][c] = (uint8_t)e1[c]; }
         vo += 2 * (cem[i] >> 2) + 2;

@@ -59,3 +59,37 @@ def test_partition_search_around_the_wide_limit(w, h, bx, by, fixed):
 def test_front_threads_by_footprint_and_launch_size(bx, by, blocks_x, blocks_y, fixed):
     img = synth.make_texture(bx * blocks_x - 1, by * blocks_y, 57 + bx)
     check_full_search(img, bx, by, fixed)
+
+
+def gpu_decode(bx, by, w, h, blocks, shift=0):
+    import torch
+    d_blk = torch.zeros(blocks.size + 16, dtype=torch.uint8, device="cuda")
+    d_blk[shift:shift + blocks.size] = torch.from_numpy(blocks.reshape(-1)).cuda()
+    d_out = torch.zeros(w * h * 4, dtype=torch.uint8, device="cuda")
+    d_sse = torch.zeros(4, dtype=torch.int64, device="cuda")
+    ref = torch.full((w * h * 4,), 100, dtype=torch.uint8, device="cuda")
+    s = torch.cuda.current_stream()
+    ab.decode_device(bx, by, w, h, d_blk.data_ptr() + shift, d_out.data_ptr(), s.cuda_stream)
+    ab.decode_error_device(bx, by, w, h, d_blk.data_ptr() + shift, ref.data_ptr(), d_sse.data_ptr(), s.cuda_stream)
+    torch.cuda.synchronize()
+    return d_out.cpu().numpy().reshape(h, w, 4), d_sse.cpu().numpy()
+
+
+@pytest.mark.parametrize("bx,by", [(4, 4), (6, 5), (8, 8), (12, 12)])
+@pytest.mark.parametrize("blocks_x,blocks_y", [(1, 70), (3, 43), (63, 2), (64, 2), (65, 3), (130, 1)])
+def test_decode_groups_of_blocks(bx, by, blocks_x, blocks_y):
+    """Images narrower than a CTA's 64 blocks, exactly as wide and wider, ragged, of random bits
+    (a third with a valid void-extent or common block mode), aligned and not."""
+    rng = np.random.default_rng(blocks_x * 100 + blocks_y + bx)
+    n = blocks_x * blocks_y
+    blocks = rng.integers(0, 256, (n, 16)).astype(np.uint8)
+    blocks[::3, 0] = 0x42 + 16 * rng.integers(0, 4, len(blocks[::3]))  # 4x4-grid modes and their neighbours
+    blocks[::3, 1] = (blocks[::3, 1] & 0xF8) | rng.integers(0, 2, len(blocks[::3]))
+    blocks[::17, :2] = (0xFC, 0xFD)  # LDR void extent
+    w, h = bx * blocks_x - 1, by * blocks_y - 2
+    host = ab.decode(bx, by, w, h, blocks)
+    for shift in (0, 1):
+        img, sse = gpu_decode(bx, by, w, h, blocks, shift)
+        assert np.array_equal(img, host)
+        d = host.astype(np.int64) - 100
+        assert np.array_equal(sse, (d * d).reshape(-1, 4).sum(axis=0))
