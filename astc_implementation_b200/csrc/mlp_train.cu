@@ -1,15 +1,15 @@
 // Training kernels of the proposal network (FP32 throughout, deterministic:
-// every output element is summed by one thread in a fixed order).
+// every output element is summed in a fixed order).
 //
 //   k_gemm      C = A . B (+ bias) (ReLU), A and B addressed by arbitrary row and
 //               column strides, so forward (X W^T), input gradient (dY W) and
-//               weight gradient (dY^T X) are the same kernel; 64x64 tiles,
-//               16-deep K slices staged in shared memory, 4x4 outputs a thread.
+//               weight gradient (dY^T X) are the same kernel.
 //   k_xent      softmax cross-entropy of the partition head (all valid
 //               partitionings and the single-partition class) plus that of the
 //               block-mode head of the label's partition count; writes dZ
 //               (already divided by the batch) and the two losses per row.
 //   k_relu_bwd, k_colsum (bias gradients), k_adam.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -19,57 +19,151 @@
 namespace astcb200 {
 namespace {
 
-constexpr int kBM = 64, kBN = 64, kBK = 16;
+namespace cg = cooperative_groups;
 
-__global__ void __launch_bounds__(256) k_gemm(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
-                                              int M, int N, int K, long long sa_i, long long sa_l, long long sb_l, long long sb_j,
-                                              const float* __restrict__ bias, int relu, int accumulate) {
-    __shared__ float As[kBK][kBM + 4];
-    __shared__ float Bs[kBK][kBN + 4];
-    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    const int i0 = blockIdx.y * kBM, j0 = blockIdx.x * kBN;
-    float acc[4][4] = {};
-    for (int l0 = 0; l0 < K; l0 += kBK) {
-        for (int e = tid; e < kBK * kBM; e += 256) {
-            const int l = e / kBM, i = e % kBM;
-            const int gi = i0 + i, gl = l0 + l;
-            As[l][i] = (gi < M && gl < K) ? A[gi * sa_i + gl * sa_l] : 0.0f;
+// 128x64 tiles, 16-deep K slices double-buffered in shared memory, 8x8 outputs a thread of 128:
+// four 16-byte shared loads for 64 multiply-adds, so the FP32 pipe is the bound.  The network's
+// products have few tiles (a 256x256 gradient eight) and long sums (2,048 rows), so K is split
+// over the CTAs of a thread-block cluster (at most 8, as many as fill the GPU), whose partial
+// tiles are added in rank order through distributed shared memory: no workspace, and the order
+// depends on the shape only.  Measured (B200, one step at 4x4, 2,048 rows): one 64x64 tile a CTA
+// without a split and 4x4 outputs a thread 743 us, this with k_colsum below 189 us.
+constexpr int kBM = 128, kBN = 64, kBK = 16, kGemmThreads = 128;
+constexpr int kMaxSplit = 8;
+constexpr int kRowA = kBM + 4, kRowB = kBN + 4;  // floats of a K row in shared memory
+constexpr int kStageFloats = kBK * (kRowA + kRowB);
+
+// Loads a `rows` x kBK slice (rows along the stride s_r, K along s_k) of a matrix of n_r x n_k, zeros
+// outside, into registers: kind 0 four floats along K, 1 four along the rows, 2 single floats.
+template <int ROWS>
+struct Slice {
+    static constexpr int kVec = ROWS * kBK / 4 / kGemmThreads;
+    float4 v[kVec];
+    __device__ __forceinline__ void load(const float* __restrict__ p, int kind, int r0, int k0, int n_r, int n_k, long long s_r, long long s_k) {
+#pragma unroll
+        for (int j = 0; j < kVec; j++) {
+            const int e = threadIdx.x + j * kGemmThreads;
+            // along K: consecutive threads on consecutive fours of a row; else on consecutive rows
+            const int r = r0 + (kind == 1 ? (e % (ROWS / 4)) * 4 : kind == 0 ? e / (kBK / 4) : e % ROWS);
+            const int k = k0 + (kind == 1 ? e / (ROWS / 4) : kind == 0 ? (e % (kBK / 4)) * 4 : (e / ROWS) * 4);
+            float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (kind == 2) {
+                if (r < n_r) {
+                    if (k < n_k) x.x = p[r * s_r + k * s_k];
+                    if (k + 1 < n_k) x.y = p[r * s_r + (k + 1) * s_k];
+                    if (k + 2 < n_k) x.z = p[r * s_r + (k + 2) * s_k];
+                    if (k + 3 < n_k) x.w = p[r * s_r + (k + 3) * s_k];
+                }
+            } else if (r < n_r && k < n_k) {  // the extent along the four is a multiple of 4
+                x = *reinterpret_cast<const float4*>(p + r * s_r + k * s_k);
+            }
+            v[j] = x;
         }
-        for (int e = tid; e < kBK * kBN; e += 256) {
-            const int l = e / kBN, j = e % kBN;
-            const int gj = j0 + j, gl = l0 + l;
-            Bs[l][j] = (gj < N && gl < K) ? B[gl * sb_l + gj * sb_j] : 0.0f;
+    }
+    __device__ __forceinline__ void store(float* sm, int row_floats, int kind) const {  // [kBK][row_floats]
+#pragma unroll
+        for (int j = 0; j < kVec; j++) {
+            const int e = threadIdx.x + j * kGemmThreads;
+            if (kind == 1) {
+                *reinterpret_cast<float4*>(sm + (e / (ROWS / 4)) * row_floats + (e % (ROWS / 4)) * 4) = v[j];
+            } else {
+                const int r = kind == 0 ? e / (kBK / 4) : e % ROWS, k = kind == 0 ? (e % (kBK / 4)) * 4 : (e / ROWS) * 4;
+                sm[k * row_floats + r] = v[j].x;
+                sm[(k + 1) * row_floats + r] = v[j].y;
+                sm[(k + 2) * row_floats + r] = v[j].z;
+                sm[(k + 3) * row_floats + r] = v[j].w;
+            }
         }
-        __syncthreads();
+    }
+};
+
+__global__ void __launch_bounds__(kGemmThreads, 3) k_gemm(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
+                                                          int M, int N, int K, long long sa_i, long long sa_l, long long sb_l,
+                                                          long long sb_j, int kind_a, int kind_b, const float* __restrict__ bias,
+                                                          int relu, int accumulate) {
+    // two stages, afterwards the partial tile [kBM][kRowB]
+    __shared__ __align__(16) float sm[2 * kStageFloats > kBM * kRowB ? 2 * kStageFloats : kBM * kRowB];
+    float* part = sm;
+    cg::cluster_group cl = cg::this_cluster();
+    const int split = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;  // 8 x 16 threads of 8 x 8 outputs
+    const int tiles_n = (N + kBN - 1) / kBN, tile = (int)(blockIdx.x / (unsigned)split);
+    const int i0 = tile / tiles_n * kBM, j0 = tile % tiles_n * kBN;
+    // this CTA's K range: whole slices, in rank order
+    const int slices = (K + kBK - 1) / kBK, per = (slices + split - 1) / split;
+    const int s0 = min(rank * per, slices), s1 = min(s0 + per, slices);
+    float acc[8][8] = {};
+    Slice<kBM> sa;
+    Slice<kBN> sb;
+    if (s0 < s1) {
+        sa.load(A, kind_a, i0, s0 * kBK, M, K, sa_i, sa_l);
+        sb.load(B, kind_b, j0, s0 * kBK, N, K, sb_j, sb_l);
+        sa.store(sm, kRowA, kind_a);
+        sb.store(sm + kBK * kRowA, kRowB, kind_b);
+    }
+    __syncthreads();
+    for (int sl = s0; sl < s1; sl++) {
+        const float* as = sm + ((sl - s0) & 1) * kStageFloats;
+        const float* bs = as + kBK * kRowA;
+        const bool more = sl + 1 < s1;
+        if (more) {
+            sa.load(A, kind_a, i0, (sl + 1) * kBK, M, K, sa_i, sa_l);
+            sb.load(B, kind_b, j0, (sl + 1) * kBK, N, K, sb_j, sb_l);
+        }
 #pragma unroll
         for (int l = 0; l < kBK; l++) {
-            float a[4], b[4];
+            // rows 4 ty and 64 + 4 ty on, columns 4 tx and 32 + 4 tx on: neighbouring threads on neighbouring banks
+            const float4 a0 = *reinterpret_cast<const float4*>(as + l * kRowA + 4 * ty), a1 = *reinterpret_cast<const float4*>(as + l * kRowA + 64 + 4 * ty);
+            const float4 b0 = *reinterpret_cast<const float4*>(bs + l * kRowB + 4 * tx), b1 = *reinterpret_cast<const float4*>(bs + l * kRowB + 32 + 4 * tx);
+            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-            for (int r = 0; r < 4; r++) a[r] = As[l][ty * 4 + r];
+            for (int r = 0; r < 8; r++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) b[c] = Bs[l][tx * 4 + c];
-#pragma unroll
-            for (int r = 0; r < 4; r++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
+                for (int c = 0; c < 8; c++) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
+        }
+        if (more) {
+            float* nx = sm + ((sl - s0 + 1) & 1) * kStageFloats;
+            sa.store(nx, kRowA, kind_a);
+            sb.store(nx + kBK * kRowA, kRowB, kind_b);
         }
         __syncthreads();
     }
+    auto write = [&](int gi, int gj, float v) {
+        if (gi >= M || gj >= N) return;
+        if (accumulate) v += C[(size_t)gi * N + gj];
+        if (bias) v += bias[gj];
+        if (relu) v = fmaxf(v, 0.0f);
+        C[(size_t)gi * N + gj] = v;
+    };
+    if (split == 1) {
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const int gi = i0 + ty * 4 + r;
-        if (gi >= M) continue;
+        for (int r = 0; r < 8; r++)
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int gj = j0 + tx * 4 + c;
-            if (gj >= N) continue;
-            float v = acc[r][c];
-            if (accumulate) v += C[(size_t)gi * N + gj];
-            if (bias) v += bias[gj];
-            if (relu) v = fmaxf(v, 0.0f);
-            C[(size_t)gi * N + gj] = v;
-        }
+            for (int c = 0; c < 8; c++) write(i0 + (r >> 2) * 64 + 4 * ty + (r & 3), j0 + (c >> 2) * 32 + 4 * tx + (c & 3), acc[r][c]);
+        return;
     }
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+            *reinterpret_cast<float4*>(part + ((r >> 2) * 64 + 4 * ty + (r & 3)) * kRowB + c * 32 + 4 * tx) =
+                make_float4(acc[r][4 * c], acc[r][4 * c + 1], acc[r][4 * c + 2], acc[r][4 * c + 3]);
+    cl.sync();
+    // each CTA adds up its share of the tile's rows from all of them, in rank order
+    const int rows = kBM / split;
+    for (int e = tid; e < rows * (kBN / 4); e += kGemmThreads) {
+        const int r = rank * rows + e / (kBN / 4), c = (e % (kBN / 4)) * 4;
+        float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int q = 0; q < split; q++) {
+            const float4 x = *reinterpret_cast<const float4*>(cl.map_shared_rank(part, q) + r * kRowB + c);
+            t.x += x.x; t.y += x.y; t.z += x.z; t.w += x.w;
+        }
+        write(i0 + r, j0 + c, t.x);
+        write(i0 + r, j0 + c + 1, t.y);
+        write(i0 + r, j0 + c + 2, t.z);
+        write(i0 + r, j0 + c + 3, t.w);
+    }
+    cl.sync();  // the others may still be reading this CTA's tile
 }
 
 struct XentShape {
@@ -134,12 +228,25 @@ __global__ void k_relu_bwd(float* __restrict__ dh, const float* __restrict__ h, 
         if (!(h[i] > 0.0f)) dh[i] = 0.0f;
 }
 
-__global__ void k_colsum(const float* __restrict__ dy, float* __restrict__ db, int rows, int cols) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= cols) return;
+// 32 columns a CTA, each summed by 32 threads over every 32nd row (consecutive threads on
+// consecutive columns), their sums added in order: one thread a column, which this replaces,
+// waited for 2,048 loads one after another.
+constexpr int kColsumGroups = 32;
+__global__ void __launch_bounds__(32 * kColsumGroups) k_colsum(const float* __restrict__ dy, float* __restrict__ db, int rows, int cols) {
+    __shared__ float part[kColsumGroups][32];
+    const int c = threadIdx.x & 31, g = threadIdx.x >> 5, j = blockIdx.x * 32 + c;
     float s = 0.0f;
-    for (int r = 0; r < rows; r++) s += dy[(size_t)r * cols + j];
-    db[j] = s;
+    if (j < cols) {
+#pragma unroll 8
+        for (int r = g; r < rows; r += kColsumGroups) s += dy[(size_t)r * cols + j];
+    }
+    part[g][c] = s;
+    __syncthreads();
+    if (g == 0 && j < cols) {
+        float t = 0.0f;
+        for (int q = 0; q < kColsumGroups; q++) t += part[q][c];
+        db[j] = t;
+    }
 }
 
 __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, size_t n,
@@ -166,8 +273,33 @@ extern "C" {
 int astcb200_train_gemm(const float* A, const float* B, float* C, int M, int N, int K, int64_t sa_i, int64_t sa_l, int64_t sb_l,
                         int64_t sb_j, const float* bias, int relu, int accumulate, void* stream) {
     if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return ASTCB200_BAD_ARG;
-    const dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM);
-    k_gemm<<<grid, 256, 0, (cudaStream_t)stream>>>(A, B, C, M, N, K, sa_i, sa_l, sb_l, sb_j, bias, relu, accumulate);
+    // four floats at a time along a stride of 1, when every row starts on 16 bytes and the extent is a multiple of four
+    auto kind = [](const float* p, int n_r, int n_k, int64_t s_r, int64_t s_k) {
+        if ((uintptr_t)p & 15) return 2;
+        if (s_k == 1 && s_r % 4 == 0 && n_k % 4 == 0) return 0;
+        if (s_r == 1 && s_k % 4 == 0 && n_r % 4 == 0) return 1;
+        return 2;
+    };
+    const int kind_a = kind(A, M, K, sa_i, sa_l), kind_b = kind(B, N, K, sb_j, sb_l);
+    const long long tiles = (long long)((N + kBN - 1) / kBN) * ((M + kBM - 1) / kBM);
+    // CTAs for two on every SM where K allows at least four slices each
+    int split = 1;
+    while (split < kMaxSplit && tiles * split < 296 && K / (2 * split) >= 4 * kBK) split *= 2;
+    cudaLaunchConfig_t cfg = {};
+    if (tiles * split > 0x7FFFFFFFll) return ASTCB200_CUDA_ERROR;
+    cfg.gridDim = dim3((unsigned)(tiles * split));
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)split; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_gemm, A, B, C, M, N, K, (long long)sa_i, (long long)sa_l, (long long)sb_l, (long long)sb_j, kind_a, kind_b,
+                           bias, relu, accumulate) != cudaSuccess) {
+        cudaGetLastError();
+        return ASTCB200_CUDA_ERROR;
+    }
     return launch_status();
 }
 
@@ -190,7 +322,7 @@ int astcb200_train_relu_backward(float* dH, const float* H, size_t n, void* stre
 
 int astcb200_train_colsum(const float* dY, float* db, uint32_t rows, uint32_t cols, void* stream) {
     if (!dY || !db) return ASTCB200_BAD_ARG;
-    k_colsum<<<(cols + 127) / 128, 128, 0, (cudaStream_t)stream>>>(dY, db, (int)rows, (int)cols);
+    k_colsum<<<(cols + 31) / 32, 32 * kColsumGroups, 0, (cudaStream_t)stream>>>(dY, db, (int)rows, (int)cols);
     return launch_status();
 }
 

@@ -93,3 +93,59 @@ def test_decode_groups_of_blocks(bx, by, blocks_x, blocks_y):
         assert np.array_equal(img, host)
         d = host.astype(np.int64) - 100
         assert np.array_equal(sse, (d * d).reshape(-1, 4).sum(axis=0))
+
+
+def _gemm(A, B, M, N, K, sa, sb, bias=None, relu=0, C=None):
+    import ctypes
+    import torch
+    out = torch.zeros(M, N, dtype=torch.float32, device="cuda") if C is None else C.clone()
+    p = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    ab._check(ab.load_library().astcb200_train_gemm(p(A), p(B), p(out), M, N, K, sa[0], sa[1], sb[0], sb[1], p(bias), relu,
+                                                    0 if C is None else 1, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    return out.cpu().numpy().astype(np.float64)
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn", "odd stride", "unaligned"])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (127, 63, 17), (129, 65, 128), (64, 256, 2048), (256, 256, 2047), (700, 1408, 256)])
+def test_training_gemm_tiles_splits_and_layouts(M, N, K, layout):
+    """Against float64 with the bound of K + 8 roundings per sum (split sums add a few)."""
+    import torch
+    g = torch.Generator().manual_seed(M + N + K)
+    a, b = torch.randn(M, K, generator=g), torch.randn(K, N, generator=g)
+    bias, c0 = torch.randn(N, generator=g), torch.randn(M, N, generator=g)
+    ref = a.double() @ b.double()
+    bound = (K + 8) * 2.0 ** -24 * (a.abs().double() @ b.abs().double()) + 2.0 ** -22 * (ref.abs() + bias.abs() + c0.abs())
+    if layout == "nt":
+        A, sa, B, sb = a.cuda(), (K, 1), b.T.contiguous().cuda(), (1, K)
+    elif layout == "nn":
+        A, sa, B, sb = a.cuda(), (K, 1), b.cuda(), (N, 1)
+    elif layout == "tn":
+        A, sa, B, sb = a.T.contiguous().cuda(), (1, M), b.cuda(), (N, 1)
+    else:
+        pad = 3 if layout == "odd stride" else 0
+        sh = 1 if layout == "unaligned" else 0
+        fa, fb = torch.zeros(M * (K + pad) + 4).cuda(), torch.zeros(K * (N + pad) + 4).cuda()
+        A, B = fa[sh:], fb[sh:]
+        A.as_strided((M, K), (K + pad, 1)).copy_(a)
+        B.as_strided((K, N), (N + pad, 1)).copy_(b)
+        sa, sb = (K + pad, 1), (N + pad, 1)
+    ref, bound = ref.numpy(), bound.numpy()
+    assert np.all(np.abs(_gemm(A, B, M, N, K, sa, sb) - ref) <= bound)
+    got = _gemm(A, B, M, N, K, sa, sb, bias=bias.cuda(), relu=1)
+    assert np.all(np.abs(got - np.maximum(ref + bias.double().numpy(), 0.0)) <= bound)
+    got = _gemm(A, B, M, N, K, sa, sb, C=c0.cuda())
+    assert np.all(np.abs(got - (ref + c0.double().numpy())) <= bound)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (31, 33), (33, 32), (2048, 1408)])
+def test_training_column_sums(rows, cols):
+    import ctypes
+    import torch
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(rows))
+    d, out = x.cuda(), torch.zeros(cols, device="cuda")
+    ab._check(ab.load_library().astcb200_train_colsum(ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(out.data_ptr()), rows, cols,
+                                                      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    bound = rows * 2.0 ** -24 * x.abs().double().sum(0) + 1e-30
+    assert bool(((out.cpu().double() - x.double().sum(0)).abs() <= bound).all())
