@@ -116,7 +116,7 @@ constexpr int kWorkCounters = 16;
 constexpr int kListGridFront = 148 * 8 * 4;
 constexpr int kListGridRefine = 148 * 6 * 4;
 constexpr int kListGridSearch = 148 * 4 * 4;
-constexpr int kListGridPack = 148 * 8;
+constexpr int kListGridPack = 148 * 16;
 
 // Global index of the chunk's lb-th block, or -1 past the end of a block list.
 __host__ __device__ inline int chunk_block(const KernelArgs& a, int lb) {

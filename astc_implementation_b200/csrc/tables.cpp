@@ -1,6 +1,8 @@
 // Host construction of the search tables (see tables.h for the reference map).
 #include "tables.h"
 
+#include "decode_block.cuh"
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -531,7 +533,7 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     std::vector<DevBm> bms(L.nbm);
     for (int i = 0; i < L.nbm; i++) {
         const HostTables::Bm& b = h.bms[h.valid_bms[i].first];
-        bms[i] = DevBm{(uint16_t)b.mode, (uint8_t)h.valid_bms[i].second, (uint8_t)b.quant, (uint8_t)b.bits, {0, 0, 0}};
+        bms[i] = DevBm{(uint16_t)b.mode, (uint8_t)h.valid_bms[i].second, (uint8_t)b.quant, (uint8_t)b.bits, 0, 0, 0};
     }
     std::vector<uint8_t> pcnt((size_t)3 * 1024 * 4);
     const int part2_words = (T + 15) / 16;
@@ -552,9 +554,23 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
         for (uint32_t d = 0; d < h.valid_dms.size(); d++) lookup[h.valid_dms[d]] = d;
         for (const HostTables::Bm& b : h.bms)
             if (b.dual && lookup[b.dm] != 0xFFFF)
-                dual.push_back(DevBm{(uint16_t)b.mode, (uint8_t)lookup[b.dm], (uint8_t)b.quant, (uint8_t)b.bits, {0, 0, 0}});
+{
+                DevBm d{(uint16_t)b.mode, (uint8_t)lookup[b.dm], (uint8_t)b.quant, (uint8_t)b.bits, 0, 0, 0};
+                for (int q = 4; q <= 20; q++) {
+                    if (dec::ise_bits(6, q) <= 109 - (int)b.bits) d.colour6 = (uint8_t)q;
+                    if (dec::ise_bits(8, q) <= 109 - (int)b.bits) d.colour8 = (uint8_t)q;
+                }
+                dual.push_back(d);
+            }
     }
     L.ndual = (int)dual.size();
+    std::vector<uint16_t> dual_w, dual_first(ndm, 0xFFFF);
+    for (const DevBm& d : dual)
+        if (dual_first[d.dm] == 0xFFFF) {
+            dual_first[d.dm] = (uint16_t)dual_w.size();
+            for (int w = 0; w < dms[d.dm].W; w++) dual_w.push_back((uint16_t)(d.dm << 6 | w));
+        }
+    L.ndual_w = (int)dual_w.size();
     std::vector<uint16_t> order(L.nbm);
     for (int i = 0; i < L.nbm; i++) order[i] = (uint16_t)i;
     std::stable_sort(order.begin(), order.end(), [&](uint16_t x, uint16_t y) { return bms[x].dm < bms[y].dm; });
@@ -566,6 +582,8 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     L.off_tw4 = put(blob, tw4.data(), tw4.size());
     L.off_bm_order = put(blob, order.data(), order.size());
     L.off_dual = put(blob, dual.data(), dual.size());
+    L.off_dual_w = put(blob, dual_w.data(), dual_w.size());
+    L.off_dual_first = put(blob, dual_first.data(), dual_first.size());
     L.off_part2 = put(blob, part2.data(), part2.size());
     L.off_part_info = put(blob, pinfo.data(), pinfo.size());
     L.off_part_counts = put(blob, pcnt.data(), pcnt.size());

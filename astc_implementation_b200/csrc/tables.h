@@ -37,7 +37,8 @@ struct DevBm {
     uint8_t dm;            // decimation-mode trial lookup index
     uint8_t quant;         // weight quant method
     uint8_t weight_bits;
-    uint8_t pad[3];
+    uint8_t colour6, colour8;  // dual-plane modes: the finest colour method of 6 and of 8 values beside the weights (0: none)
+    uint8_t pad;
 };
 
 // Byte offsets of every table inside the device blob; passed to kernels by value.
@@ -57,6 +58,10 @@ struct TableLayout {
     uint32_t off_dual;        // DevBm[ndual]: dual-plane block modes on trial decimation modes, in
                               // block-mode order (the optional dual-plane search; no reference use)
     int32_t ndual;
+    uint32_t off_dual_w;      // u16[ndual_w]: decimation mode << 6 | weight of every weight of the dual-plane modes' grids,
+                              // a mode's weights consecutive
+    uint32_t off_dual_first;  // u16[ndm]: a mode's first position there (0xFFFF: not a dual-plane grid)
+    int32_t ndual_w;
     uint32_t off_w2t;         // u16 entries: texel index  | (contribution*16) << 8
     uint32_t off_part2;       // u32[3][1024][(T + 15) / 16]  partition of texel (P = 2..4), two bits a texel, texel t at
                               // bit 2 (t & 15)

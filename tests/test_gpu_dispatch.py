@@ -149,3 +149,27 @@ def test_training_column_sums(rows, cols):
     torch.cuda.synchronize()
     bound = rows * 2.0 ** -24 * x.abs().double().sum(0) + 1e-30
     assert bool(((out.cpu().double() - x.double().sum(0)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("bx,by", [(4, 4), (8, 8), (10, 8), (12, 12)])
+def test_extensions_with_and_without_kept_sums(bx, by):
+    """Blocks of up to 64 texels keep the infill sums of a dual-plane candidate, larger ones do not."""
+    w, h = bx * 7 - 2, by * 3
+    img = synth.make_texture(w, h, 77)
+    rng = np.random.default_rng(bx)
+    img[:, :, 3] = rng.integers(0, 256, (h, w))  # an independent alpha: dual-plane blocks win
+    img[:by, : 2 * bx] = (9, 200, 31, 40)        # two void-extent blocks
+    enc = ab.ASTCEncoder(device=0, fixed=True, void_extent=True, dual_plane=True)
+    enc.secondaryInit(w, h, bx, by)
+    sym = enc.encode_symbolic(img)
+    out = enc.encode(img).reshape(-1, 16)
+    enc.close()
+    orc = _libs.oracle()
+    prev = orc.orc_set_extensions(3)
+    try:
+        ref_out, ref_sym = oracle_encode(img, bx, by, True)
+    finally:
+        orc.orc_set_extensions(prev)
+    assert np.array_equal(sym, ref_sym)
+    assert np.array_equal(out, ref_out)
+    assert np.any(sym[:, 6] > 0) and np.any(sym[:, 7] > 0)
