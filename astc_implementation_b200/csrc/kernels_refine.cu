@@ -791,7 +791,13 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                     int fk = 0;
 #pragma unroll 1
                     for (int q = 0; q < 4; q++) { const int f = r.c[k].fmt[q]; fk = fk * 8 + (f == 0 ? 0 : f == 4 ? 1 : f == 6 ? 2 : f == 8 ? 3 : f == 10 ? 4 : f == 12 ? 5 : 6); }
-                    key = ((((int)r.P - 1) << 12 | fk) << 7) | dm;  // partition count, formats, decimation mode
+                    if constexpr (U8) {
+                        // weight count, decimation mode, partition count, first format: pass16's loops are most of an iteration
+                        const int W = reinterpret_cast<const DevDm*>(a.tables + a.L.off_dm)[dm].W;
+                        key = (((W - 1) << 7 | dm) << 2 | ((int)r.P - 1)) << 3 | fk >> 9;
+                    } else {
+                        key = ((((int)r.P - 1) << 12 | fk) << 7) | dm;  // partition count, formats, decimation mode
+                    }
                 }
                 if (r.ncand > 0) {
                     const int P = r.P;
