@@ -418,97 +418,198 @@ __device__ __forceinline__ float okey_value(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
 }
 
-// K: length of each lane's list of its best partition classes (>= kmax), so one pass over
-// the logits finds them; the warp then merges the lanes' lists with two redux steps per pick.
-template <int K>
-__global__ void __launch_bounds__(128) k_select(const __grid_constant__ KernelArgs a, const __grid_constant__ Shape S,
-                                                 const float* __restrict__ logits, const __grid_constant__ Select sel,
-                                                 const __grid_constant__ Routes r) {
+// The kbm best of nbm modes (at most 32 NW) by (logit descending, index ascending) as a bit mask, 64
+// modes per lane from lane 0; lane l holds modes l + 32 u.  One pick per round; when kbm is above
+// half the modes, the rounds pick the others instead, worst first (logit ascending, index
+// descending): the same set in fewer rounds.  A lane has its two best at hand and looks for more
+// only when both were picked.
+template <int NW>
+__device__ __forceinline__ uint64_t mode_mask(const float* h, int nbm, int kbm, int lane) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    const int lb = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (lb >= a.nblocks) return;
-    const int blk = chunk_block(a, lb);
-    if (blk < 0) return;
-    const float* z = logits + (size_t)lb * S.nout;
-    // First pass: the softmax maximum and each lane's best partitioning logit.  The kmax-th
-    // largest of the 32 lane maxima bounds the kmax-th largest logit from below (those lanes'
-    // maxima are kmax distinct logits at least that large), so only logits at or above it
-    // can be among the kmax best.
-    float mx = -3.0e38f, lm = -3.0e38f;
-    for (int c = lane; c <= S.p1; c += 32) {
-        const float v = z[c];
-        mx = fmaxf(mx, v);
-        if (c < S.p1) lm = fmaxf(lm, v);
-    }
-    mx = warp_max(mx);
-    float theta = 3.0e38f;
-    if (sel.kmax >= 1) {
-        int rank = 0;  // lanes ahead of this one in (maximum descending, lane ascending) order
-        for (int j = 0; j < 32; j++) {
-            const float o = __shfl_sync(kFull, lm, j);
-            rank += (o > lm || (o == lm && j < lane)) ? 1 : 0;
-        }
-        const uint32_t at = __ballot_sync(kFull, rank == sel.kmax - 1);
-        theta = __shfl_sync(kFull, lm, __ffs(at) - 1);
-    }
-    // Second pass: the softmax sum (in the same order as ever) and this lane's K best
-    // partitionings among those at or above the bound (value desc, index asc).
-    float lv[K];
-    int lc[K];
+    const int kk = kbm < nbm ? kbm : nbm;
+    const bool worst = 2 * kk > nbm;
+    const int rounds = worst ? nbm - kk : kk;
+    uint32_t key[NW];  // 0: absent or picked
 #pragma unroll
-    for (int k = 0; k < K; k++) { lv[k] = -3.0e38f; lc[k] = 0x7FFFFFFF; }
-    float se = 0.0f;
-    for (int c = lane; c <= S.p1; c += 32) {
-        const float v = z[c];
-        se += __expf(v - mx);
-        if (c < S.p1 && v >= theta && v > lv[K - 1]) {  // a lane sees its classes in increasing order
-            lv[K - 1] = v; lc[K - 1] = c;
-#pragma unroll
-            for (int k = K - 1; k > 0; k--)
-                if (lv[k] > lv[k - 1]) {
-                    const float tv = lv[k]; lv[k] = lv[k - 1]; lv[k - 1] = tv;
-                    const int tc = lc[k]; lc[k] = lc[k - 1]; lc[k - 1] = tc;
-                }
-        }
+    for (int u = 0; u < NW; u++) {
+        const int c = lane + 32 * u;
+        key[u] = 0;
+        if (c < nbm) { const uint32_t k = okey(h[c] + 0.0f); key[u] = worst ? ~k : k; }  // -0 as +0
     }
-    se = warp_sum(se);
-    const float p1 = __expf(z[S.p1] - mx) / se;
-    // the kmax best partitionings, merged from the lanes' lists
-    uint16_t picks[kMaxProposals];
-    float mass[kMaxProposals];
-    int n = 0;
-    float acc = p1;
-    for (int k = 0; k < sel.kmax; k++) {
-        const uint32_t key = lc[0] == 0x7FFFFFFF ? 0u : okey(lv[0]);
-        const uint32_t best = __reduce_max_sync(kFull, key);
+    uint32_t picked = 0, k1 = 0, k2 = 0;
+    int u1 = 0, u2 = 0;
+    bool look = true;
+#pragma unroll 1
+    for (int k = 0; k < rounds; k++) {
+        if (look) {
+            k1 = k2 = 0;
+#pragma unroll
+            for (int i = 0; i < NW; i++) {
+                const int u = worst ? NW - 1 - i : i;  // the first of equal keys: the lowest index, the highest when picking the worst
+                const uint32_t x = worst ? key[NW - 1 - i] : key[i];
+                if (((picked >> u) & 1) || x == 0) continue;
+                if (x > k1) { k2 = k1; u2 = u1; k1 = x; u1 = u; }
+                else if (x > k2) { k2 = x; u2 = u; }
+            }
+            look = false;
+        }
+        const uint32_t best = __reduce_max_sync(kFull, k1);
         if (best == 0u) break;
-        const uint32_t ci = __reduce_min_sync(kFull, key == best ? (uint32_t)lc[0] : 0xFFFFFFFFu);
-        if ((uint32_t)lc[0] == ci) {  // the winning lane drops it from its list
-#pragma unroll
-            for (int j = 0; j < K - 1; j++) { lv[j] = lv[j + 1]; lc[j] = lc[j + 1]; }
-            lv[K - 1] = -3.0e38f; lc[K - 1] = 0x7FFFFFFF;
+        const uint32_t idx = (uint32_t)(lane + 32 * u1);
+        const uint32_t ci = worst ? __reduce_max_sync(kFull, k1 == best ? idx : 0u) : __reduce_min_sync(kFull, k1 == best ? idx : 0xFFFFFFFFu);
+        if (k1 == best && idx == ci) {
+            picked |= 1u << u1;
+            look = k2 == 0;
+            k1 = k2; u1 = u2; k2 = 0;
         }
-        picks[n] = (uint16_t)pick_of_class(S, (int)ci);
-        acc += __expf(okey_value(best) - mx) / se;
-        mass[n] = acc;
-        n++;
     }
-    const bool confident = acc >= sel.threshold;
-    if (r.confidence && lane == 0) r.confidence[lb] = acc;
-    int pos = 0;
-    if (lane == 0) pos = atomicAdd(&r.counts[confident ? 0 : 1], 1);
-    pos = __shfl_sync(kFull, pos, 0);
+    uint64_t word = 0;
+#pragma unroll
+    for (int u = 0; u < NW; u++) {
+        const bool valid = lane + 32 * u < nbm;
+        const uint32_t chosen = __ballot_sync(kFull, valid && (((picked >> u) & 1) != 0) != worst);
+        if (lane == (u >> 1)) word |= (uint64_t)chosen << (32 * (u & 1));
+    }
+    return word;
+}
+
+// One warp per block, kSelectWarps a CTA, which take their places in the lists together: one
+// atomic per list and CTA.  (One per block put 262,144 additions on each of two addresses.)  Most
+// blocks' single-partition probability reaches the coverage on its own; they need the softmax
+// alone, not the ranking of the partitionings; the others collect the logits that can be among the
+// kmax best, a few more than kmax, one a lane, and pick with two redux steps each.
+// Measured (B200, 262,144 blocks of 1,408 logits): 875 -> 470 us, of which 225 is reading them.
+constexpr int kSelectWarps = 8;
+constexpr int kHeld = 36;  // partition logits a lane keeps in registers (of 35 at 4x4 and 6x6); more are read again
+__global__ void __launch_bounds__(kSelectWarps * 32, 3) k_select(const __grid_constant__ KernelArgs a, const __grid_constant__ Shape S,
+                                                              const float* __restrict__ logits, const __grid_constant__ Select sel,
+                                                              const __grid_constant__ Routes r) {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    // per warp: its place counts (0 proposal list, 1 full-search list, 2..5 partitioned blocks of
+    // P = 1..4), then the CTA's first places
+    __shared__ int places[6][kSelectWarps];
+    __shared__ int base[6];
+    __shared__ float cand_v[kSelectWarps][32];
+    __shared__ int cand_c[kSelectWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lb = blockIdx.x * kSelectWarps + warp;
+    const int blk = lb < a.nblocks ? chunk_block(a, lb) : -1;
+    const bool live = blk >= 0;
+    const float* z = logits + (size_t)(live ? lb : 0) * S.nout;
+    bool confident = false, skip_p1 = false;
+    int used = 0;
+    uint16_t picks[kMaxProposals];
+    if (live) {
+        // the softmax maximum and each lane's best partitioning logit
+        float v[kHeld], mx = -3.0e38f, lm = -3.0e38f;
+#pragma unroll
+        for (int i = 0; i < kHeld; i++) { const int c = lane + 32 * i; v[i] = c <= S.p1 ? z[c] : -3.0e38f; }
+#pragma unroll
+        for (int i = 0; i < kHeld; i++) { mx = fmaxf(mx, v[i]); if (lane + 32 * i != S.p1) lm = fmaxf(lm, v[i]); }
+        for (int c = lane + 32 * kHeld; c <= S.p1; c += 32) { const float x = z[c]; mx = fmaxf(mx, x); if (c < S.p1) lm = fmaxf(lm, x); }
+        mx = warp_max(mx);
+        float se = 0.0f;  // (absent classes add 0)
+#pragma unroll
+        for (int i = 0; i < kHeld; i++) se += __expf(v[i] - mx);
+        for (int c = lane + 32 * kHeld; c <= S.p1; c += 32) se += __expf(z[c] - mx);
+        se = warp_sum(se);
+        const float p1 = __expf(z[S.p1] - mx) / se;
+        // the masses only add to p1: at or above both limits the block is confident and proposes nothing
+        confident = p1 >= sel.threshold && p1 >= sel.coverage && !r.confidence;
+        if (!confident) {
+            // The kmax-th largest of the 32 lane maxima bounds the kmax-th largest logit from below
+            // (those lanes' maxima are kmax distinct logits at least that large), so only logits at
+            // or above it can be among the kmax best.
+            float theta = 3.0e38f;
+            if (sel.kmax >= 1) {
+                int rank = 0;  // lanes ahead of this one in (maximum descending, lane ascending) order
+                for (int j = 0; j < 32; j++) {
+                    const float o = __shfl_sync(kFull, lm, j);
+                    rank += (o > lm || (o == lm && j < lane)) ? 1 : 0;
+                }
+                const uint32_t at = __ballot_sync(kFull, rank == sel.kmax - 1);
+                theta = __shfl_sync(kFull, lm, __ffs(at) - 1);
+            }
+            // the partitionings at or above the bound, at most 32 of them kept
+            int ncand = 0;
+            auto collect = [&](float x, int c) {
+                const bool in = x >= theta && x > -3.0e38f && c < S.p1;
+                const uint32_t m = __ballot_sync(kFull, in);
+                if (m == 0u) return;
+                const int at = ncand + __popc(m & ((1u << lane) - 1u));
+                if (in && at < 32) { cand_v[warp][at] = x; cand_c[warp][at] = c; }
+                ncand += __popc(m);
+            };
+#pragma unroll
+            for (int i = 0; i < kHeld; i++) collect(v[i], lane + 32 * i);
+#pragma unroll 1
+            for (int c0 = 32 * kHeld; c0 < S.p1; c0 += 32) collect(c0 + lane < S.p1 ? z[c0 + lane] : -3.0e38f, c0 + lane);
+            __syncwarp();
+            // the kmax best, by value, the first class of equal ones
+            float mass[kMaxProposals];
+            int n = 0;
+            float acc = p1;
+            uint32_t key = 0;
+            int mine = 0x7FFFFFFF;
+            if (lane < ncand) { key = okey(cand_v[warp][lane]); mine = cand_c[warp][lane]; }
+            uint32_t last = 0xFFFFFFFFu;  // the last pick
+            int last_c = -1;
+#pragma unroll 1
+            for (int k = 0; k < sel.kmax; k++) {
+                if (ncand > 32) {  // (equal logits, or a large kmax) each lane's best after the last pick
+                    key = 0; mine = 0x7FFFFFFF;
+                    for (int c = lane; c < S.p1; c += 32) {
+                        const float x = z[c];
+                        if (!(x >= theta && x > -3.0e38f)) continue;
+                        const uint32_t u = okey(x);
+                        if ((u < last || (u == last && c > last_c)) && u > key) { key = u; mine = c; }
+                    }
+                }
+                const uint32_t best = __reduce_max_sync(kFull, key);
+                if (best == 0u) break;
+                const uint32_t ci = __reduce_min_sync(kFull, key == best ? (uint32_t)mine : 0xFFFFFFFFu);
+                if ((uint32_t)mine == ci) key = 0;
+                last = best; last_c = (int)ci;
+                picks[n] = (uint16_t)pick_of_class(S, (int)ci);
+                acc += __expf(okey_value(best) - mx) / se;
+                mass[n] = acc;
+                n++;
+            }
+            confident = acc >= sel.threshold;
+            if (r.confidence && lane == 0) r.confidence[lb] = acc;
+            // propose the shortest best-first prefix whose mass reaches the coverage
+            used = n;
+            for (int k = 0; k < n; k++)
+                if (mass[k] >= sel.coverage) { used = k + 1; break; }
+            if (p1 >= sel.coverage) used = 0;
+            skip_p1 = used > 0 && p1 < sel.p1_floor;
+        }
+    }
+    // places in the lists
+    if (lane < 6) {
+        int n = 0;
+        if (live && confident) {
+            if (lane == 0) n = 1;
+            else if (lane == 2) n = skip_p1 ? 0 : 1;
+            else if (lane > 2) for (int k = 0; k < used; k++) n += (picks[k] >> 10) == lane - 3 ? 1 : 0;
+        } else if (live && lane == 1) {
+            n = 1;
+        }
+        places[lane][warp] = n;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        int t = 0;
+        for (int w = 0; w < kSelectWarps; w++) { const int n = places[threadIdx.x][w]; places[threadIdx.x][w] = t; t += n; }
+        base[threadIdx.x] = t > 0 ? atomicAdd(&r.counts[threadIdx.x], t) : 0;
+    }
+    __syncthreads();
+    if (!live) return;
     if (!confident) {
-        if (lane == 0) { r.full[pos] = blk; r.full_err[pos] = 3e38f; }
+        if (lane == 0) { const int pos = base[1] + places[1][warp]; r.full[pos] = blk; r.full_err[pos] = 3e38f; }
         return;
     }
-    // propose the shortest best-first prefix whose mass reaches the coverage
-    int used = n;
-    for (int k = 0; k < n; k++)
-        if (mass[k] >= sel.coverage) { used = k + 1; break; }
-    if (p1 >= sel.coverage) used = 0;
-    const bool skip_p1 = used > 0 && p1 < sel.p1_floor;
+    const int pos = base[0] + places[0][warp];
     uint32_t heads = skip_p1 ? 0u : 1u;  // block-mode heads the front will read: P = 1 and the proposed counts
     for (int k = 0; k < used; k++) heads |= 2u << (picks[k] >> 10);
     if (lane == 0) {
@@ -518,10 +619,12 @@ __global__ void __launch_bounds__(128) k_select(const __grid_constant__ KernelAr
         pp.flags = skip_p1 ? 1 : 0;
         for (int k = 0; k < kMaxProposals; k++) pp.v[k] = k < used ? picks[k] : 0;
         // the work list: slot 0 (P = 1) and one slot per proposed partitioning, by P
-        if (!skip_p1) r.pb_list[atomicAdd(&r.counts[2], 1)] = (uint32_t)pos << 5;
+        if (!skip_p1) r.pb_list[base[2] + places[2][warp]] = (uint32_t)pos << 5;
+        int at[3] = {base[3] + places[3][warp], base[4] + places[4][warp], base[5] + places[5][warp]};
         for (int k = 0; k < used; k++) {
-            const int p = 1 + (picks[k] >> 10);  // list of P = 2 + (v >> 10)
-            r.pb_list[(size_t)p * r.pb_stride + atomicAdd(&r.counts[2 + p], 1)] = ((uint32_t)pos << 5) | (uint32_t)(k + 1);
+            const int p = picks[k] >> 10;  // list 1 + p of P = 2 + p
+            const int i = p == 0 ? at[0]++ : p == 1 ? at[1]++ : at[2]++;
+            r.pb_list[(size_t)(1 + p) * r.pb_stride + i] = ((uint32_t)pos << 5) | (uint32_t)(k + 1);
         }
     }
     // block-mode masks: the kbm best modes of each needed head; lane l holds modes l + 32u.
@@ -537,45 +640,11 @@ __global__ void __launch_bounds__(128) k_select(const __grid_constant__ KernelAr
         }
         return;
     }
+#pragma unroll 1
     for (int p = 0; p < 4; p++) {
         if (!((heads >> p) & 1)) continue;
         const float* h = z + S.head_base + p * S.nbm_pad;
-        float hv[2 * kMaskWords];
-        uint32_t picked = 0;
-#pragma unroll
-        for (int u = 0; u < 2 * kMaskWords; u++) {
-            const int c = lane + 32 * u;
-            hv[u] = c < S.nbm ? h[c] : 0.0f;
-            if (c >= S.nbm) picked |= 1u << u;  // absent: never offered
-        }
-        // The kbm best modes by (value descending, index ascending), one pick per round.  When
-        // kbm is above half the modes, the rounds pick the others instead, worst first (value
-        // ascending, index descending): the same set in fewer rounds.
-        const int kk = sel.kbm < S.nbm ? sel.kbm : S.nbm;
-        const bool worst = 2 * kk > S.nbm;
-        const int rounds = worst ? S.nbm - kk : kk;
-        for (int k = 0; k < rounds; k++) {
-            uint32_t key = 0;
-            int mine = -1;
-            float mv = 0.0f;
-#pragma unroll
-            for (int u = 0; u < 2 * kMaskWords; u++)
-                if (!((picked >> u) & 1) && (mine < 0 || (worst ? hv[u] <= mv : hv[u] > mv))) { mine = u; mv = hv[u]; }
-            if (mine >= 0) key = worst ? ~okey(mv) : okey(mv);
-            const uint32_t best = __reduce_max_sync(kFull, key);
-            if (best == 0u) break;
-            const uint32_t idx = (uint32_t)(lane + 32 * mine);
-            const uint32_t ci = worst ? __reduce_max_sync(kFull, key == best ? idx : 0u)
-                                      : __reduce_min_sync(kFull, key == best ? idx : 0xFFFFFFFFu);
-            if (mine >= 0 && idx == ci) picked |= 1u << mine;
-        }
-        uint64_t word = 0;
-#pragma unroll
-        for (int u = 0; u < 2 * kMaskWords; u++) {
-            const bool valid = lane + 32 * u < S.nbm;
-            const uint32_t chosen = __ballot_sync(kFull, valid && (((picked >> u) & 1) != 0) != worst);
-            if (lane == (u >> 1)) word |= (uint64_t)chosen << (32 * (u & 1));
-        }
+        const uint64_t word = S.nbm <= 64 ? mode_mask<2>(h, S.nbm, sel.kbm, lane) : mode_mask<2 * kMaskWords>(h, S.nbm, sel.kbm, lane);
         if (lane < kMaskWords) mk[p * kMaskWords + lane] = word;
     }
 }
@@ -594,10 +663,9 @@ cudaError_t launch_mlp_logits(const KernelArgs& a, const Net& net, float* logits
 
 cudaError_t launch_select(const KernelArgs& a, const Net& net, const float* logits, const Select& sel, const Routes& r,
                           cudaStream_t s) {
-    const int grid = (a.nblocks + 3) / 4;
-    if (sel.kmax <= 4) k_select<4><<<grid, 128, 0, s>>>(a, net.s, logits, sel, r);
-    else if (sel.kmax <= 8) k_select<8><<<grid, 128, 0, s>>>(a, net.s, logits, sel, r);
-    else k_select<16><<<grid, 128, 0, s>>>(a, net.s, logits, sel, r);
+    const int grid = (a.nblocks + kSelectWarps - 1) / kSelectWarps;
+    constexpr int threads = kSelectWarps * 32;
+    k_select<<<grid, threads, 0, s>>>(a, net.s, logits, sel, r);
     return cudaGetLastError();
 }
 

@@ -173,3 +173,27 @@ def test_extensions_with_and_without_kept_sums(bx, by):
     assert np.array_equal(sym, ref_sym)
     assert np.array_equal(out, ref_out)
     assert np.any(sym[:, 6] > 0) and np.any(sym[:, 7] > 0)
+
+
+@pytest.mark.parametrize("bx,by", [(4, 4), (6, 6)])
+@pytest.mark.parametrize("kmax,kbm", [(1, 1), (16, 5), (16, 50), (3, 64)])
+def test_selection_among_equal_logits(bx, by, kmax, kbm):
+    """Every partitioning and block mode with the same logit: more candidates than a warp collects,
+    taken in class order."""
+    from astc_implementation_b200 import proposal
+    lay = proposal.Layout(bx, by)
+    net = {"w1": np.zeros((256, lay.inputs)), "b1": np.zeros(256), "w2": np.zeros((256, 256)), "b2": np.zeros(256),
+           "w3": np.zeros((lay.outputs, 256)), "b3": np.full(lay.outputs, 0.25)}
+    enc = ab.ASTCEncoder(device=0, fixed=True)
+    enc.set_proposal_net(net, bx, by)
+    enc.set_pruning(True, max_partitionings=kmax, block_modes=kbm, coverage=1.0, threshold=0.0)
+    w, h = 12 * bx, 9 * by - 1
+    enc.secondaryInit(w, h, bx, by)
+    route, picks, masks = enc.proposal_selection(synth.make_texture(w, h, 3))
+    enc.close()
+    assert np.all(route == 0) and np.all(picks[:, 0] == kmax)
+    assert np.all(picks[:, 2:2 + kmax] == lay.pick_of(np.arange(kmax)))
+    first = (1 << min(kbm, lay.nbm)) - 1
+    for p in (0, 1):  # the single partition, and two partitions (the first classes)
+        got = sum(masks[:, 4 * p + i].astype(object) << (64 * i) for i in range(4))
+        assert np.all(got == first)
