@@ -250,7 +250,8 @@ int astcb200_encode_batch_device(astcb200_ctx* ctx, const astcb200_texture* text
     int rc = make_plan(ctx, textures, n, true, p);
     if (rc) return rc;
     cudaStream_t s = cuda_stream ? (cudaStream_t)cuda_stream : ctx->stream;
-    return launch_plan(ctx, p, s, default_tuning(ctx, p), !(ctx->cfg.flags & ASTCB200_FLAG_NO_GRAPH), nullptr);
+    rc = launch_plan(ctx, p, s, default_tuning(ctx, p), !(ctx->cfg.flags & ASTCB200_FLAG_NO_GRAPH), nullptr);
+    return rc || cuda_stream ? rc : order_default_stream(ctx);
 }
 
 int astcb200_encode_batch(astcb200_ctx* ctx, const astcb200_texture* textures, uint32_t n, astcb200_stats* stats) {

@@ -41,6 +41,18 @@ int wait_stream(astcb200_ctx* ctx, cudaStream_t s) {
     }
 }
 
+int order_default_stream(astcb200_ctx* ctx) {
+    cudaStreamCaptureStatus st;
+    if (cudaStreamIsCapturing(cudaStreamLegacy, &st) != cudaSuccess) {  // a capture forbids its use: no ordering then
+        cudaGetLastError();
+        return ASTCB200_OK;
+    }
+    if (!ctx->ev_order) CK(cudaEventCreateWithFlags(&ctx->ev_order, cudaEventDisableTiming), "cudaEventCreate");
+    CK(cudaEventRecord(ctx->ev_order, ctx->stream), "order event");
+    CK(cudaStreamWaitEvent(cudaStreamLegacy, ctx->ev_order, 0), "order wait");
+    return ASTCB200_OK;
+}
+
 int HostResults::reserve(astcb200_ctx* ctx) {
     size_t need = 0;
     for (Item& it : items) {
@@ -200,6 +212,7 @@ int astcb200_destroy(astcb200_ctx* ctx) {
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+    if (ctx->ev_order) cudaEventDestroy(ctx->ev_order);
     for (cudaEvent_t e : ctx->stage_ev) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -241,7 +254,8 @@ int astcb200_encode_device(astcb200_ctx* ctx, const uint8_t* d_rgba8, uint8_t* d
     if (((uintptr_t)d_rgba8 & 3) || ((uintptr_t)d_out & 15)) return ASTCB200_BAD_ARG;
     ASTCB200_DEVICE_SCOPE(ctx);
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    return run_search(ctx, d_rgba8, d_out, nullptr, s, nullptr);
+    const int rc = run_search(ctx, d_rgba8, d_out, nullptr, s, nullptr);
+    return rc || stream ? rc : order_default_stream(ctx);
 }
 
 static int encode_host(astcb200_ctx* ctx, const uint8_t* rgba8, uint8_t* out_blocks, uint32_t* symbolic, astcb200_stats* stats) {

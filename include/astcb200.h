@@ -112,7 +112,8 @@ int astcb200_encode(astcb200_ctx* ctx, const uint8_t* rgba8, uint8_t* out_blocks
                     astcb200_stats* stats);
 
 /* Same search with both buffers already in device memory of the context's GPU; work is
- * queued on cuda_stream (a cudaStream_t, or NULL for the context's stream) and the call
+ * queued on cuda_stream (a cudaStream_t, or NULL for the context's stream, which later work on
+ * the legacy default stream then waits for) and the call
  * returns without waiting.  d_rgba8 must be 4-byte aligned, d_out_blocks 16-byte aligned. */
 int astcb200_encode_device(astcb200_ctx* ctx, const uint8_t* d_rgba8, uint8_t* d_out_blocks, void* cuda_stream);
 
@@ -158,7 +159,7 @@ int astcb200_encode_batch(astcb200_ctx* ctx, const astcb200_texture* textures, u
 
 /* Same with rgba8 and out_blocks in device memory of the context's GPU (rgba8 4-byte
  * aligned, out_blocks 16-byte aligned); queued on cuda_stream (NULL = the context's
- * stream), no wait.  The textures array itself is host memory and is consumed before the
+ * stream, which later work on the legacy default stream then waits for), no wait.  The textures array itself is host memory and is consumed before the
  * call returns. */
 int astcb200_encode_batch_device(astcb200_ctx* ctx, const astcb200_texture* textures, uint32_t n, void* cuda_stream);
 
