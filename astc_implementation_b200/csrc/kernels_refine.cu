@@ -294,6 +294,7 @@ __device__ __forceinline__ void unpack_endpoints(uint32_t fmt, uint32_t lo, uint
 // ------------------------------------------------------------ k_refine
 constexpr int kRefineThreads = 128;
 constexpr int kRefineCtas = 5;
+constexpr int kOneWaveGroups = 148 * kRefineCtas;
 
 // Candidate threads per partitioned block (the refinement top-N rounded up to a power of
 // two) and partitioned blocks per CTA: 16 x 8 for the full search; more, narrower ones when
@@ -303,6 +304,19 @@ __host__ __device__ inline int refine_pbs(int T, int topn) {
     const int by_threads = kRefineThreads / refine_cpb(topn);
     const int by_smem = 40960 / (T * (T > 16 ? 4 : 16));
     return by_threads < by_smem ? by_threads : (by_smem > 16 ? by_smem : 16);
+}
+
+// Candidates a warp runs at a time in a launch of npb partitioned blocks.  A launch of one wave is as long as
+// its slowest warp, and a warp of 32 different candidates runs the union of their paths and
+// the longest of their loops: with 8 or 16 a warp it is shorter, while the waves still hold every
+// group.  Measured (B200, full search of 64x64 at 4x4, 3,328 partitioned
+// blocks): 519 us with 32, 504 with 16; fallback pass of 200x120 at 4x4 188 us with 32, 167 with 8.
+__host__ __device__ inline int refine_spread(int npb) {
+    return npb <= kOneWaveGroups * 4 ? 8 : npb <= kOneWaveGroups * 8 ? 16 : 32;
+}
+__host__ __device__ inline int refine_group(int T, int cpb, int spread) {  // partitioned blocks per CTA
+    const int pbs = refine_pbs(T, cpb), n = kRefineThreads / 32 * spread / cpb;
+    return n < 1 ? 1 : n < pbs ? n : pbs;
 }
 
 // Candidate state in shared memory, one slot per candidate a CTA runs, arrays of [row][slot]:
@@ -750,8 +764,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
     extern __shared__ __align__(16) uint8_t smem[];
     const int T = a.L.T;
     constexpr int cpb = CPB;
-    const int pbs = CPB == 8 ? kRefineThreads / 8 : refine_pbs(T, CPB);
-    const RefineLayout fl = refine_layout(T, a.L.max_w, pbs, U8, false);
+    const RefineLayout fl = refine_layout(T, a.L.max_w, refine_pbs(T, CPB), U8, false);
     using Px = typename std::conditional<U8, uchar4, float4>::type;
     using Pe = typename std::conditional<U8, uint16_t, uint8_t>::type;
     const int px_row = px_row_bytes(T, U8), part_row = part_row_bytes(T, sizeof(Pe));
@@ -766,13 +779,20 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
     // co-resident warps run the same code), or the proposal pass's work list.
     const int nb = list_blocks(a);
     const int npb = a.pb_list ? pb_total(a) : nb * a.slots;
+    const int spread = refine_spread(npb), pbs = refine_group(T, CPB, spread);
     const int ngroups = (npb + pbs - 1) / pbs;
+    // this thread's place among those that run candidates, the first `spread` lanes of each warp
+    const int place = lane < spread ? warp * spread + lane : kRefineThreads;
     const int iters = a.refine_iters > 0 ? a.refine_iters : 6;
     __shared__ unsigned int refined[4];  // candidates refined by this CTA, by P (work counters)
     __shared__ int live_in_warp[kRefineThreads / 32];
     __shared__ int spill_base;
     if (tid < 4) refined[tid] = 0;
-    bool spill = a.tail != nullptr && T <= kTailMaxTexels;  // until the tail is found full
+    // Hand the last candidates to the tail (until it is found full).  A launch of one wave is as long
+    // as its longest chain of iterations, which a second kernel would lengthen: the full search
+    // keeps its candidates then, the proposal pass hands them over for the last iteration only.
+    const bool one_wave = ngroups <= kOneWaveGroups;
+    bool spill = a.tail != nullptr && T <= kTailMaxTexels && !(one_wave && !a.prop);
     // (the first group's barrier below orders these writes before any read)
     for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
         {
@@ -819,7 +839,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
             if (k == 0 && pbl < pbs) staged[pbl] = item;
         }
         __syncthreads();
-        // Thread tid takes the candidate of rank tid in (partition count, endpoint formats,
+        // The thread of place i takes the candidate of rank i in (partition count, endpoint formats,
         // decimation mode) order, so a warp's candidates mostly take the same packing path
         // and share loop bounds and table rows; the rank is also its slot.
         int cand = -1;  // slot of the candidate this thread runs
@@ -835,7 +855,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
             __syncthreads();
             keys[rank] = tid;
             __syncthreads();
-            const int mine = keys[tid];
+            const int mine = place < kRefineThreads ? keys[place] : kRefineThreads * cpb;
             const int pbl = mine / cpb, k = mine % cpb;
             const uint32_t item = pbl < pbs ? staged[pbl] : 0u;
             if (item != 0) {
@@ -843,9 +863,9 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                 const size_t pbi = (size_t)lb * a.slots + slot;
                 a.snaps[pbi * kNumCand + k].err = ERR_DEFAULT;  // inert slot unless refined below
                 if (k < (int)a.pbrec[pbi].ncand) {
-                    cand = tid;
-                    item_of[tid] = (uint32_t)pbi;
-                    pos_of[tid] = (uint8_t)mine;
+                    cand = place;
+                    item_of[place] = (uint32_t)pbi;
+                    pos_of[place] = (uint8_t)mine;
                     if (a.work) atomicAdd(&refined[a.pbrec[pbi].P - 1], 1u);
                 }
             }
@@ -869,7 +889,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
             }
             if (nlive == 0) break;
             const int rank = before + __popc(bal & ((1u << lane) - 1u));
-            if (spill && it > 0 && nlive <= a.spill_live) {
+            if (spill && it > 0 && nlive <= a.spill_live && (!one_wave || it + 1 >= iters)) {
                 // Few candidates left: hand them to the tail pass, which runs them densely, and
                 // take the next group instead of holding the CTA for them.
                 if (tid == 0) {
@@ -889,7 +909,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
             }
             if (live) keys[rank] = cand;
             __syncthreads();
-            cand = tid < nlive ? keys[tid] : -1;
+            cand = place < nlive ? keys[place] : -1;
             if (cand >= 0) {
                 const int pbl = pos_of[cand] / cpb, k = pos_of[cand] % cpb;
                 const size_t pbi = item_of[cand];
@@ -935,6 +955,11 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
     const int total = min(*a.tail_count, a.tail_cap);
     int* claim = a.tail_count + 1;
     const int iters = a.refine_iters > 0 ? a.refine_iters : 6;
+    // Few entries are spread over more warps, as in k_refine: only the first `spread` lanes of a
+    // warp take any.
+    const int warps = (int)gridDim.x * (kRefineThreads / 32);
+    const int spread = total <= warps * 8 ? 8 : total <= warps * 16 ? 16 : 32;
+    const int place = lane < spread ? warp * spread + lane : kRefineThreads;
     int cand = -1;     // the slot whose candidate this thread runs
     bool dry = false;  // CTA-uniform
     for (;;) {
@@ -951,10 +976,10 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
         }
         int nnew = 0, new_before = 0, filled = -1;
         unsigned bnew = 0;
-        if (!dry && nlive <= kTailRefillAt) {
+        if (!dry && nlive * 32 <= kTailRefillAt * spread) {
             // Thread tid stages into slot tid when that slot is free and its warp's claim
             // reached an entry for it.
-            const bool fr = busy[tid] == 0;
+            const bool fr = busy[tid] == 0 && lane < spread;
             const unsigned fb = __ballot_sync(0xFFFFFFFFu, fr);
             const int nfree = __popc(fb);
             int base = 0;
@@ -1013,7 +1038,7 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
         if (live) keys[before + __popc(bal & below)] = cand;
         if (filled >= 0) keys[nlive + new_before + __popc(bnew & below)] = filled;
         __syncthreads();
-        cand = tid < n ? keys[tid] : -1;
+        cand = place < n ? keys[place] : -1;
         if (cand >= 0) {
             const uint32_t pbi = pbi_of[cand];
             const int k = (int)k_of[cand], it = next_it[cand];
@@ -1670,7 +1695,7 @@ cudaError_t configure_kernels(const TableLayout& L) {
 
 cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s) {
     const int cpb = refine_cpb(a.topn);
-    const int npb = a.nblocks * a.slots, pbs = refine_pbs(a.L.T, cpb);
+    const int npb = a.nblocks * a.slots, pbs = refine_group(a.L.T, cpb, refine_spread(npb));
     int grid = (npb + pbs - 1) / pbs;
     if (a.block_list) grid = std::min(grid, kListGridRefine);
     const size_t smem = refine_smem_bytes(a.L, cpb);
@@ -1690,7 +1715,7 @@ cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s) {
 
 cudaError_t launch_refine_tail(const KernelArgs& a, cudaStream_t s) {
     if (!a.tail || a.L.T > kTailMaxTexels) return cudaSuccess;
-    const int grid = std::min((a.tail_cap + kRefineThreads - 1) / kRefineThreads, 148 * kTailCtas);
+    const int grid = std::min((a.tail_cap + kRefineThreads / 4 - 1) / (kRefineThreads / 4), 148 * kTailCtas);
     k_refine_tail<<<std::max(grid, 1), kRefineThreads, refine_tail_smem_bytes(a.L.T, a.L.max_w), s>>>(a);
     return cudaGetLastError();
 }
