@@ -748,7 +748,7 @@ __device__ __forceinline__ uint32_t bm_quant_weight(const Tabs& tb, const BmQuan
 // block from 70 to 51 KB of shared memory and from three to four CTAs.  Measured (B200, 128
 // threads): passes 02-05 of 13,312 partitioned blocks at 10x8 3.04 -> 1.43 ms, at 8x8 3.18 ->
 // 1.61 ms; with 32 threads 83,200 at 4x4 0.44 -> 0.41 ms.
-template <int NT>
+template <int NT, bool DEEP>
 __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int ndm_run, const int16_t* dm_run, const float* iw,
                                           const float* wes, bool is_const, float* dec, uint16_t* trig, float* lov, float* hiv,
                                           float* buf) {
@@ -783,7 +783,7 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int 
         float v = iw[w];
         if (dmi.W != T) {
             float ws = 0.0f, tc = 1e-10f;
-#pragma unroll 1
+#pragma unroll (DEEP ? 2 : 1)
             for (; n4 > 0; n4--, ent += stride) {
                 const uint4 e4 = *ent;
                 const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
@@ -833,7 +833,7 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int 
         if (W != T) {
             const float* im = inf + m * T;
             float e0 = 1e-10f, e1 = 0.0f;
-#pragma unroll 1
+#pragma unroll (DEEP ? 2 : 1)
             for (; n4 > 0; n4--, ent += stride) {
                 const uint4 e4 = *ent;
                 const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
@@ -871,7 +871,7 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int 
         const float* dw = dec + dmi.w_off;
         const uint2* rows = reinterpret_cast<const uint2*>(trig + dmi.w_off);
         float ax = 0.0f, ay = 0.0f;
-#pragma unroll 2
+#pragma unroll (DEEP ? 4 : 2)
         for (int j = 0; j < W; j += 4) {  // four table values in flight, summed in weight order
             const uint2 k = rows[j >> 2];
             const float2 c0 = tb.trig((int)(k.x & 0xFFFF) + i), c1 = tb.trig((int)(k.x >> 16) + i);
@@ -946,7 +946,7 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int 
 // proposal search's path through the front stays compact in the instruction cache (the
 // front stalls on instruction fetch).
 // pass07 over every block mode, one thread per mode.
-template <int kFrontThreads>
+template <int kFrontThreads, bool DEEP>
 __device__ __noinline__ void pass07_all_modes(const Tabs& tb, int T, int P, int nbm, const float* lov, const float* hiv,
                                               float min_cutoff, const float* dec, float* qfs, const float* iw,
                                               const float* wes, bool is_const, float* bm_err) {
@@ -974,7 +974,7 @@ __device__ __noinline__ void pass07_all_modes(const Tabs& tb, int T, int P, int 
                 err = err + (d * d) * wes[t & tmask];
             }
         } else {
-#pragma unroll 2
+#pragma unroll (DEEP ? 4 : 2)
             for (int t = 0; t < T; t++) {
                 const uint4 e = tb.tw4f(bm.dm, t);
                 float v = qw[entry_index(e.x) * kFrontThreads] * entry_factor(e.x);
@@ -991,7 +991,7 @@ __device__ __noinline__ void pass07_all_modes(const Tabs& tb, int T, int P, int 
 
 // P1: the instance for partitioned blocks of one partition only (the proposal pass's P = 1
 // list), with P a constant the compiler folds into every loop bound and branch.
-template <int NT, bool P1>
+template <int NT, bool P1, bool DEEP>
 __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk, int slot_in_block, uint32_t entry, uint8_t* sm) {
     constexpr int kFrontThreads = NT, kFrontWarps = NT / 32;
     const int P = P1 ? 1 : P_arg;
@@ -1320,12 +1320,12 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     }
 
     // ---------------- passes 02-05
-    dm_passes<NT>(tb, T, a.L.max_w, ndm_run, dm_run, iw, wes, is_const, dec, reinterpret_cast<uint16_t*>(sm + fl.trig), lov, hiv, qfs);
+    dm_passes<NT, DEEP>(tb, T, a.L.max_w, ndm_run, dm_run, iw, wes, is_const, dec, reinterpret_cast<uint16_t*>(sm + fl.trig), lov, hiv, qfs);
     __syncthreads();
 
     // ---------------- pass07: weight quantisation error per block mode
     const int nlist = bmm ? M.nlive : nbm;  // block modes evaluated: the list, or all of them
-    if (!bmm) pass07_all_modes<kFrontThreads>(tb, T, P, nbm, lov, hiv, M.min_cutoff, dec, qfs, iw, wes, is_const, bm_err);
+    if (!bmm) pass07_all_modes<kFrontThreads, DEEP>(tb, T, P, nbm, lov, hiv, M.min_cutoff, dec, qfs, iw, wes, is_const, bm_err);
     // ---------------- pass10: best format combination per quant level and integer total
     // One item per (quant level, integer total), beside pass07 (role-indexed): the format
     // combinations with that total, in the order the one-thread loops visit them (i, j, k, l
@@ -1556,8 +1556,16 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
 
 // Resident CTAs of 128 threads the register budget is sized for.
 constexpr int kFrontMinBlocks128 = 8;
-template <int NT, bool P1>
-__global__ void __launch_bounds__(NT, kFrontMinBlocks128 * 128 / NT > 32 ? 32 : kFrontMinBlocks128 * 128 / NT) k_front(const __grid_constant__ KernelArgs a) {
+// DEEP: the instances for blocks of kDeepTexels or more, of which shared memory leaves four CTAs of
+// 128 threads or fewer: they wait for table loads, so the loops around those are unrolled into the
+// registers that are free.  Measured (B200, 2,048 blocks) without / with: 8x6 2.48 / 2.64 ms, 8x8 5.00 /
+// 4.61, 10x8 6.71 / 6.06, 12x12 15.3 / 13.4; 6x6 1.52 / 1.79.
+constexpr int kDeepTexels = 60;
+constexpr int front_min_ctas(int nt, bool deep) {
+    return deep ? (nt >= 256 ? 2 : 5) : kFrontMinBlocks128 * 128 / nt > 32 ? 32 : kFrontMinBlocks128 * 128 / nt;
+}
+template <int NT, bool P1, bool DEEP>
+__global__ void __launch_bounds__(NT, front_min_ctas(NT, DEEP)) k_front(const __grid_constant__ KernelArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     // Items: every slot of every block in slot-major order (co-resident CTAs work on the
     // same partition count), or the proposal pass's work list grouped by partition count.
@@ -1586,7 +1594,7 @@ __global__ void __launch_bounds__(NT, kFrontMinBlocks128 * 128 / NT > 32 ? 32 : 
             if (threadIdx.x == 0) { PBRec& rec = a.pbrec[(size_t)lb * a.slots + k]; rec.P = P; rec.ncand = 0; rec.entry = 0; rec.seed = 0; }
             continue;  // uniform across the CTA
         }
-        front_body<NT, P1>(a, P, lb, blk, k, entry, smem);
+        front_body<NT, P1, DEEP>(a, P, lb, blk, k, entry, smem);
         __syncthreads();  // the next item reuses shared memory
     }
 }
@@ -1622,8 +1630,8 @@ size_t front_smem_bytes(const TableLayout& L) {  // the largest over the launche
 cudaError_t configure_search_kernels(size_t search_bytes, size_t front_bytes) {
     cudaError_t e = cudaFuncSetAttribute(k_partition_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)search_bytes);
     // the largest shared-memory carveout: occupancy of the front is bounded by shared memory
-    for (auto f : {k_front<256, false>, k_front<128, false>, k_front<64, false>, k_front<32, false>, k_front<128, true>,
-                   k_front<64, true>, k_front<32, true>}) {
+    for (auto f : {k_front<256, false, true>, k_front<128, false, true>, k_front<128, false, false>, k_front<64, false, false>,
+                   k_front<32, false, false>, k_front<128, true, false>, k_front<64, true, false>, k_front<32, true, false>}) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)front_bytes);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
@@ -1644,10 +1652,12 @@ cudaError_t launch_front(const KernelArgs& a, cudaStream_t s) {
     if (a.block_list) grid = std::min(grid, kListGridFront * 128 / nt);
     const size_t smem = front_smem_bytes(a.L, nt, a.bm_mask != nullptr);
     auto go = [&](const KernelArgs& k, bool p1) {
-        if (nt == 32) { if (p1) k_front<32, true><<<grid, 32, smem, s>>>(k); else k_front<32, false><<<grid, 32, smem, s>>>(k); }
-        else if (nt == 64) { if (p1) k_front<64, true><<<grid, 64, smem, s>>>(k); else k_front<64, false><<<grid, 64, smem, s>>>(k); }
-        else if (nt == 256) k_front<256, false><<<grid, 256, smem, s>>>(k);
-        else { if (p1) k_front<128, true><<<grid, 128, smem, s>>>(k); else k_front<128, false><<<grid, 128, smem, s>>>(k); }
+        if (nt == 32) { if (p1) k_front<32, true, false><<<grid, 32, smem, s>>>(k); else k_front<32, false, false><<<grid, 32, smem, s>>>(k); }
+        else if (nt == 64) { if (p1) k_front<64, true, false><<<grid, 64, smem, s>>>(k); else k_front<64, false, false><<<grid, 64, smem, s>>>(k); }
+        else if (nt == 256) k_front<256, false, true><<<grid, 256, smem, s>>>(k);
+        else if (p1) k_front<128, true, false><<<grid, 128, smem, s>>>(k);
+        else if (a.L.T >= kDeepTexels) k_front<128, false, true><<<grid, 128, smem, s>>>(k);
+        else k_front<128, false, false><<<grid, 128, smem, s>>>(k);
     };
     if (a.pb_list && a.pb_from == 0 && a.pb_to == 0) {
         // the proposal pass's work lists: P = 1 by its own instance, then P = 2..4
