@@ -1,8 +1,9 @@
 // Learned proposal: network inference on the tcgen05 tensor cores and the
 // selection of partitionings, block modes and routes from its logits.
 //
-// k_mlp_logits: one CTA of 8 warps per 128 blocks (two threads per block row,
-// each taking half of a row's accumulator columns).  The block texels are
+// k_mlp_logits: one CTA per 128 blocks, eight epilogue warps (two threads per block row, each
+// taking half of a row's accumulator columns), one warp that issues the MMAs of layer 3 and one
+// that fetches its weights.  The block texels are
 // staged in shared memory as bf16 in the tensor core's K-major core-matrix
 // layout; each layer is a chain of tcgen05.mma (M=128, K=16 per instruction,
 // A and B from shared memory, FP32 accumulators in tensor memory) issued by
@@ -10,14 +11,16 @@
 // mbarrier) already laid out on the host in the same core-matrix order.  The
 // two hidden layers' epilogues (bias, ReLU, bf16) read the accumulators with
 // tcgen05.ld and write the next layer's A operand in place; layer 3 runs in
-// 64-column chunks with double-buffered weights and accumulators, so the
-// epilogue of chunk j overlaps the MMAs of chunk j+1 and the copy of chunk
-// j+2.  The layer-3 epilogue adds the bias, stages each row's 64 FP32 logits
-// in shared memory and writes the row with one 256-byte bulk copy to global
-// memory (instead of 64 strided stores per thread); CTAs start the chunk
-// sequence at different chunks so that they do not all fetch the same weights
-// from L2 at once.  Every wait on an mbarrier is bounded (error_flag[1] polls, 0 = 2^24);
-// a CTA that gives up sets error_flag[0], waits (bounded by 2^24 polls) for its own copies
+// 64-column chunks through four weight buffers and eight accumulator buffers (all 512
+// tensor-memory columns): the fetching thread, the issuing thread and the epilogue warps only
+// meet at mbarriers (weights landed; weights consumed; accumulator full; accumulator read).
+// The layer-3 epilogue adds the bias and stores its 32 logits as four 32-byte sectors; CTAs start the
+// chunk sequence at different chunks so that they do not all fetch the same weights
+// from L2 at once.  Two CTA barriers a chunk and a 256-byte bulk copy per row and chunk out of
+// a staging buffer, which this replaces, kept the tensor pipe at 12 % and took 885 us for
+// 262,144 blocks at 4x4 (231 GFLOP, 1.48 GB of logits: 225 us to write); this takes 568 us.
+// Every wait on an mbarrier is bounded (error_flag[1] polls, 0 = 2^24); a thread that gives up
+// makes its CTA give up: it sets error_flag[0], waits (bounded by 2^24 polls) for its own copies
 // and MMAs in flight, frees its tensor memory and returns.
 //
 // k_select: one warp per block turns the logits into the proposal search's
@@ -34,13 +37,12 @@ namespace mlp {
 namespace {
 
 constexpr uint32_t kOffA = 0;                 // 64 KB: X, then H1, then H2 (128 rows x up to 256 bf16)
-constexpr uint32_t kOffW = 65536;             // 128 KB: W1 | W2 | two W3 chunks of 32 KB
+constexpr uint32_t kOffW = 65536;             // 128 KB: W1, W2, then the W3 chunks of 32 KB
 constexpr uint32_t kW3Buf = kChunkN * 256 * 2;               // one W3 chunk (bf16)
-constexpr uint32_t kStageStride = kChunkN + 4;                // floats per staged logit row (padded)
-constexpr uint32_t kStageBuf = kTileRows * kStageStride * 4;  // one staged chunk of logits
-constexpr uint32_t kOffStage = kOffW + 2 * kW3Buf;            // two staging buffers (free after layer 2)
-constexpr uint32_t kOffBar = kOffStage + 2 * kStageBuf;       // mbarriers and flags
-static_assert(kOffBar == 200704 && kOffBar + 1024 + 1024 <= (uint32_t)kMlpSmemBytes, "shared memory plan");
+constexpr int kWBufs = 4;                     // weight buffers of layer 3
+constexpr int kAccBufs = 8;                   // its accumulator buffers, kChunkN tensor-memory columns each
+constexpr uint32_t kOffBar = kOffW + kWBufs * kW3Buf;         // mbarriers and flags
+static_assert(kOffBar == 196608 && kOffBar + 1024 + 1024 == (uint32_t)kMlpSmemBytes, "shared memory plan");
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kWaitLimit = 1u << 24;     // polls of an mbarrier before a CTA gives up
 constexpr uint32_t kCopyPiece = 32768;        // bytes per bulk copy instruction
@@ -116,6 +118,7 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
 __host__ __device__ constexpr uint32_t instr_desc(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
+static_assert(kAccBufs * kChunkN == (int)kTmemCols, "layer 3 uses every column");
 static_assert(instr_desc(128, 256) == 0x08400490u, "instruction descriptor layout");
 
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
@@ -164,15 +167,29 @@ __device__ void hidden_epilogue(uint32_t tmem_row, uint32_t col0, int c0, const 
         tmem_load32(tmem_row + col0 + c, v);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
+            const float4* b4 = reinterpret_cast<const float4*>(bias + c + q * 8);
+            const float4 b0 = __ldg(b4), b1 = __ldg(b4 + 1);
+            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
             float h[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) h[i] = fmaxf(v[q * 8 + i] + __ldg(bias + c + q * 8 + i), 0.0f);
+            for (int i = 0; i < 8; i++) h[i] = fmaxf(v[q * 8 + i] + b[i], 0.0f);
             *reinterpret_cast<uint4*>(sA + core_index(m, c + q * 8, kTileRows) * 2) = pack8(h);
         }
     }
 }
 
-constexpr int kMlpThreads = 2 * kTileRows;  // two threads per row, each taking half of the columns
+constexpr int kEpilogueThreads = 2 * kTileRows;  // two threads per row, each taking half of the columns
+constexpr int kMlpThreads = kEpilogueThreads + 64;  // and the warps of the layer-3 issuer and fetcher
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// Eight consecutive floats, one sector.
+__device__ __forceinline__ void store8(float* p, const float* v) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]),
+                 "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
 
 __global__ void __launch_bounds__(kMlpThreads, 1)
     k_mlp_logits(const __grid_constant__ KernelArgs a, const __grid_constant__ Net net, float* __restrict__ logits, int* error_flag) {
@@ -180,13 +197,19 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sA = sm + kOffA;
     uint8_t* sW = sm + kOffW;
-    uint64_t* bw = reinterpret_cast<uint64_t*>(sm + kOffBar);       // [2] weight buffers
-    uint64_t* bm = bw + 2;                                           // [3] MMA completion: layers 1-2, layer-3 buffers
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bw + 5);
-    int* abort_flag = reinterpret_cast<int*>(bw + 6);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    uint64_t* bw = reinterpret_cast<uint64_t*>(sm + kOffBar);  // weights of layers 1 and 2
+    uint64_t* bm = bw + 1;                                     // their MMAs
+    uint64_t* w_full = bw + 2;                                 // [kWBufs] layer 3: weights landed
+    uint64_t* w_free = w_full + kWBufs;                        // [kWBufs] and consumed
+    uint64_t* acc_full = w_free + kWBufs;                      // [kAccBufs] accumulator complete
+    uint64_t* acc_free = acc_full + kAccBufs;                  // [kAccBufs] and read (by the eight epilogue warps)
+    constexpr int kBars = 2 + 2 * kWBufs + 2 * kAccBufs;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bw + kBars);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bw + kBars + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // this thread's row (block) in the tile and tensor-memory lane; warps w and w + 4 share
     // the lanes of quarter w and split the columns (half)
+    const bool epilogue = tid < kEpilogueThreads;
     const int m = tid % kTileRows, half = tid / kTileRows;
     const int lb = blockIdx.x * kTileRows + m;
     const Shape& S = net.s;
@@ -203,7 +226,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int i = 0; i < 5; i++) mbar_init(&bw[i], 1);
+        for (int i = 0; i < kBars - kAccBufs; i++) mbar_init(&bw[i], 1);
+        for (int i = 0; i < kAccBufs; i++) mbar_init(&acc_free[i], kEpilogueThreads / 32);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -213,16 +237,16 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
     const uint32_t tmem = *tmem_slot;
     const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
 
-    // thread 0's bookkeeping of weight copies and MMA commits in flight: a phase counts as
-    // done only once a wait saw it complete, so the drain after a give-up waits for the rest
-    uint32_t w_issued[2] = {0, 0}, w_done[2] = {0, 0};
-    uint32_t m_issued[3] = {0, 0, 0}, m_done[3] = {0, 0, 0};  // only the waits of all threads advance m_done
-    bool ok = true, failed = false;  // failed: the same in every thread (set only at uniform exits)
+    // thread 0's bookkeeping of layers 1 and 2: a phase counts as done only once a wait saw it
+    // complete, so the drain after a give-up waits for the rest
+    uint32_t w_issued = 0, w_done = 0, m_issued = 0, m_done = 0;  // only the waits of all threads advance m_done
+    int fetched = 0, issued = 0;  // layer-3 chunks the fetching and the issuing thread have started
+    bool ok = true;
 
-    if (tid == 0) { load_weights(sW, net.w1, 256u * S.k0p * 2, &bw[0]); w_issued[0]++; }
+    if (tid == 0) { load_weights(sW, net.w1, 256u * S.k0p * 2, bw); w_issued++; }
 
     // stage the block's texels (RGBA8 / 255 -> bf16), zero rows past the chunk
-    {
+    if (epilogue) {
         const int blk = lb < a.nblocks ? chunk_block(a, lb) : -1;
         const int T = a.L.T;
         BlockSrc src{};
@@ -246,154 +270,127 @@ __global__ void __launch_bounds__(kMlpThreads, 1)
 
     const uint32_t a_base = smem_u32(sA), w_base = smem_u32(sW);
     constexpr uint32_t kLboA = (kTileRows / 8) * 128, kLboW256 = (256 / 8) * 128, kLboW3 = (kChunkN / 8) * 128;
-    auto issue_chunk = [&](int jj) -> bool {  // thread 0: chunk jj's MMAs once its weights have landed
-        const int bb = jj & 1;
-        if (!mbar_wait(&bw[bb], w_done[bb] & 1, wl)) return false;
-        w_done[bb]++;
-        for (int kk = 0; kk < 16; kk++)
-            mma_bf16(tmem + bb * kChunkN, smem_desc(a_base + kk * 2 * kLboA, kLboA, 128),
-                     smem_desc(w_base + bb * kW3Buf + kk * 2 * kLboW3, kLboW3, 128), instr_desc(128, kChunkN), kk > 0);
-        mma_commit(&bm[1 + bb]);
-        m_issued[1 + bb]++;
+    // one of layers 1 and 2: thread 0 issues its MMAs once its weights have landed, all threads wait
+    auto dense = [&](uint32_t d_tmem, int ksteps) -> bool {
+        if (tid == 0) {
+            tc_after();
+            if (!mbar_wait(bw, w_done & 1, wl)) *abort_flag = 1;
+            else {
+                w_done++;
+                for (int kk = 0; kk < ksteps; kk++)
+                    mma_bf16(d_tmem, smem_desc(a_base + kk * 2 * kLboA, kLboA, 128), smem_desc(w_base + kk * 2 * kLboW256, kLboW256, 128),
+                             instr_desc(128, 256), kk > 0);
+                mma_commit(bm);
+                m_issued++;
+            }
+        }
+        __syncthreads();
+        if (*abort_flag) return false;
+        ok = mbar_wait(bm, m_done & 1, wl);
+        if (ok) m_done++;
+        if (__syncthreads_or(!ok)) { *abort_flag = 1; return false; }
+        tc_after();
         return true;
     };
 
     // ---- layer 1: X (128 x k0p) . W1^T -> tensor memory columns [0, 256)
-    if (tid == 0) {
-        tc_after();
-        if (!mbar_wait(&bw[0], w_done[0] & 1, wl)) *abort_flag = 1;
-        else {
-            w_done[0]++;
-            for (int kk = 0; kk < S.k0p / 16; kk++)
-                mma_bf16(tmem, smem_desc(a_base + kk * 2 * kLboA, kLboA, 128), smem_desc(w_base + kk * 2 * kLboW256, kLboW256, 128),
-                         instr_desc(128, 256), kk > 0);
-            mma_commit(&bm[0]);
-            m_issued[0]++;
-        }
-    }
-    __syncthreads();
-    if (*abort_flag) { failed = true; goto cleanup; }
-    ok = mbar_wait(&bm[0], m_done[0] & 1, wl);
-    if (ok) m_done[0]++;
-    if (__syncthreads_or(!ok)) { failed = true; goto cleanup; }
-    tc_after();
-    if (tid == 0) { load_weights(sW, net.w2, 256u * 256u * 2, &bw[0]); w_issued[0]++; }
-    hidden_epilogue(tmem_row, 0, half * 128, net.b1, sA, m);
+    if (!dense(tmem, S.k0p / 16)) goto cleanup;
+    if (tid == 0) { load_weights(sW, net.w2, 256u * 256u * 2, bw); w_issued++; }
+    if (epilogue) hidden_epilogue(tmem_row, 0, half * 128, net.b1, sA, m);
     async_proxy_fence();
     tc_before();
     __syncthreads();
 
     // ---- layer 2: H1 (128 x 256) . W2^T -> columns [256, 512)
-    if (tid == 0) {
-        tc_after();
-        if (!mbar_wait(&bw[0], w_done[0] & 1, wl)) *abort_flag = 1;
-        else {
-            w_done[0]++;
-            for (int kk = 0; kk < 16; kk++)
-                mma_bf16(tmem + 256, smem_desc(a_base + kk * 2 * kLboA, kLboA, 128),
-                         smem_desc(w_base + kk * 2 * kLboW256, kLboW256, 128), instr_desc(128, 256), kk > 0);
-            mma_commit(&bm[0]);
-            m_issued[0]++;
-        }
+    if (!dense(tmem + 256, 16)) goto cleanup;
+    if (tid == kEpilogueThreads + 32) {  // the fetcher: W2 is consumed
+        for (; fetched < kWBufs && fetched < nchunks; fetched++)
+            load_weights(sW + fetched * kW3Buf, net.w3 + (size_t)chunk_of(fetched) * kChunkN * 256, kW3Buf, &w_full[fetched]);
     }
-    __syncthreads();
-    if (*abort_flag) { failed = true; goto cleanup; }
-    ok = mbar_wait(&bm[0], m_done[0] & 1, wl);
-    if (ok) m_done[0]++;
-    if (__syncthreads_or(!ok)) { failed = true; goto cleanup; }
-    tc_after();
-    if (tid == 0) {
-        for (int j = 0; j < 2 && j < nchunks; j++) {
-            load_weights(sW + j * kW3Buf, net.w3 + (size_t)chunk_of(j) * kChunkN * 256, kW3Buf, &bw[j]);
-            w_issued[j]++;
-        }
-    }
-    hidden_epilogue(tmem_row, 256, half * 128, net.b2, sA, m);
+    if (epilogue) hidden_epilogue(tmem_row, 256, half * 128, net.b2, sA, m);
     async_proxy_fence();
     tc_before();
     __syncthreads();
 
-    // ---- layer 3: H2 (128 x 256) . W3^T in chunks of 64 columns, accumulators alternating
-    // between tensor-memory columns [0, 64) and [64, 128).  Chunk 0's MMAs are issued here;
-    // chunk j + 1's right after chunk j's have completed, into the accumulator buffer chunk
-    // j - 1's epilogue read before the previous staging barrier, so that they run while chunk
-    // j's epilogue reads its own.  Two barriers per chunk.
-    if (tid == 0) {
-        tc_after();
-        if (!issue_chunk(0)) *abort_flag = 1;
-    }
-    __syncthreads();
-    if (*abort_flag) { failed = true; goto cleanup; }
-    for (int j = 0; j < nchunks; j++) {
-        const int b = j & 1;
-        // this thread's 32 biases of the chunk, loaded before the wait so that it hides them
-        float bv[32];
-        {
-            const float4* bias4 = reinterpret_cast<const float4*>(net.b3 + chunk_of(j) * kChunkN + half * 32);
+    // ---- layer 3: H2 (128 x 256) . W3^T in chunks of 64 columns.  Use u of a buffer waits for phase
+    // u of its full barrier and phase u - 1 of its free one.
+    {
+        auto wait = [&](uint64_t* bar, int phase) -> bool {  // false: this thread or another gave up
+            for (uint32_t i = 0; i < wl; i++) {
+                if (wl < (1u << 16) ? mbar_test_wait(bar, (uint32_t)phase & 1u) : mbar_try_wait(bar, (uint32_t)phase & 1u)) return true;
+                if (*abort_flag) return false;
+            }
+            *abort_flag = 1;
+            return false;
+        };
+        if (epilogue) {
+            const bool store = lb < a.nblocks;
+            float* out_row = logits + (size_t)lb * S.nout + half * 32;
+            for (int j = 0; j < nchunks; j++) {
+                const int b = j % kAccBufs, c0 = chunk_of(j) * kChunkN;
+                // this thread's 32 biases of the chunk, loaded before the wait so that it hides them
+                float bv[32], v[32];
+                const float4* bias4 = reinterpret_cast<const float4*>(net.b3 + c0 + half * 32);
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const float4 t = __ldg(bias4 + q);
-                bv[4 * q] = t.x; bv[4 * q + 1] = t.y; bv[4 * q + 2] = t.z; bv[4 * q + 3] = t.w;
-            }
-        }
-        ok = mbar_wait(&bm[1 + b], m_done[1 + b] & 1, wl);  // chunk j was issued before this iteration
-        if (ok) m_done[1 + b]++;
-        if (__syncthreads_or(!ok)) { failed = true; goto cleanup; }
-        tc_after();
-        if (tid == 0) {
-            if (j + 2 < nchunks) {  // chunk j's MMAs are done with its weight buffer
-                load_weights(sW + b * kW3Buf, net.w3 + (size_t)chunk_of(j + 2) * kChunkN * 256, kW3Buf, &bw[b]);
-                w_issued[b]++;
-            }
-            if (j + 1 < nchunks && !issue_chunk(j + 1)) *abort_flag = 1;  // seen after the staging barrier
-        }
-        // the row's 64 logits go to padded shared memory (32 from each of its two threads),
-        // then to global memory as one contiguous 256-byte bulk copy issued by the row's first
-        // thread (a warp's direct stores would touch 32 rows)
-        const bool store = lb < a.nblocks;
-        float* st = reinterpret_cast<float*>(sm + kOffStage + b * kStageBuf) + m * kStageStride;
-        {
-            const int c = half * 32;
-            float v[32];
-            tmem_load32(tmem_row + b * kChunkN + c, v);
+                for (int q = 0; q < 8; q++) {
+                    const float4 t = __ldg(bias4 + q);
+                    bv[4 * q] = t.x; bv[4 * q + 1] = t.y; bv[4 * q + 2] = t.z; bv[4 * q + 3] = t.w;
+                }
+                if (!__all_sync(0xFFFFFFFFu, wait(&acc_full[b], j / kAccBufs))) break;  // the tensor-memory load takes whole warps
+                tc_after();
+                tmem_load32(tmem_row + b * kChunkN + half * 32, v);
+                tc_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_free[b]);
+                if (store) {
 #pragma unroll
-            for (int q = 0; q < 8; q++)
-                reinterpret_cast<float4*>(st + c)[q] = make_float4(v[4 * q] + bv[4 * q], v[4 * q + 1] + bv[4 * q + 1],
-                                                                   v[4 * q + 2] + bv[4 * q + 2], v[4 * q + 3] + bv[4 * q + 3]);
-        }
-        async_proxy_fence();
-        tc_before();
-        __syncthreads();  // the row is staged; every read of this accumulator buffer is done
-        if (*abort_flag) { failed = true; goto cleanup; }
-        if (half == 0) {
-            if (store) {
-                float* out = logits + (size_t)lb * S.nout + chunk_of(j) * kChunkN;
-                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out), "r"(smem_u32(st)),
-                             "r"(kChunkN * 4)
-                             : "memory");
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    for (int i = 0; i < 32; i++) v[i] = v[i] + bv[i];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) store8(out_row + c0 + 8 * q, v + 8 * q);
+                }
             }
-            // the other buffer, written next, must have been read by its copy (chunk j - 1);
-            // the barriers of the next iteration order this before those writes
-            asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        } else if (tid == kEpilogueThreads) {  // the issuer
+            tc_after();
+            for (int j = 0; j < nchunks; j++) {
+                const int wb = j % kWBufs, b = j % kAccBufs;
+                if (!wait(&w_full[wb], j / kWBufs)) break;
+                if (j >= kAccBufs) {
+                    if (!wait(&acc_free[b], j / kAccBufs - 1)) break;
+                    tc_after();
+                }
+                for (int kk = 0; kk < 16; kk++)
+                    mma_bf16(tmem + b * kChunkN, smem_desc(a_base + kk * 2 * kLboA, kLboA, 128),
+                             smem_desc(w_base + wb * kW3Buf + kk * 2 * kLboW3, kLboW3, 128), instr_desc(128, kChunkN), kk > 0);
+                mma_commit(&w_free[wb]);
+                mma_commit(&acc_full[b]);
+                issued = j + 1;
+            }
+        } else if (tid == kEpilogueThreads + 32) {  // the fetcher
+            for (int j = fetched; j < nchunks; j++) {
+                const int wb = j % kWBufs;
+                if (!wait(&w_free[wb], j / kWBufs - 1)) break;
+                load_weights(sW + wb * kW3Buf, net.w3 + (size_t)chunk_of(j) * kChunkN * 256, kW3Buf, &w_full[wb]);
+                fetched = j + 1;
+            }
         }
     }
 
 cleanup:
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // this thread's logit rows are written
     __syncthreads();
-    if (failed) {
+    if (*abort_flag) {
         // give up: record it, then let our own copies and MMAs drain (bounded) before the
         // shared and tensor memory are released
         if (tid == 0) {
             atomicExch(error_flag, 1);  // error_flag[0]
-            for (int b = 0; b < 2; b++)
-                while (w_done[b] < w_issued[b]) { mbar_wait(&bw[b], w_done[b] & 1); w_done[b]++; }
-            for (int b = 0; b < 3; b++)
-                for (uint32_t i = m_done[b]; i < m_issued[b]; i++) mbar_wait(&bm[b], i & 1);
+            while (w_done < w_issued) { mbar_wait(bw, w_done & 1); w_done++; }
+            for (uint32_t i = m_done; i < m_issued; i++) mbar_wait(bm, i & 1);
         }
-        __syncthreads();
+        // the last copy into each buffer, and the last chunk's MMAs (commits complete in order)
+        for (int j = fetched > kWBufs ? fetched - kWBufs : 0; j < fetched; j++) mbar_wait(&w_full[j % kWBufs], (uint32_t)(j / kWBufs) & 1u);
+        if (issued) mbar_wait(&acc_full[(issued - 1) % kAccBufs], (uint32_t)((issued - 1) / kAccBufs) & 1u);
     }
+    tc_before();
+    __syncthreads();
     tc_after();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }

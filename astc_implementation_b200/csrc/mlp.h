@@ -109,7 +109,7 @@ constexpr int kRouteCounters = 8;  // ints per chunk: routes, partitioned-block 
 // from, and searching them fully costs next to nothing.
 constexpr int kMinProposalTexels = 1024;
 
-constexpr int kMlpSmemBytes = 200704 + 1024 + 1024;  // operands and staging, barriers, alignment slack
+constexpr int kMlpSmemBytes = 196608 + 1024 + 1024;  // operands, barriers, alignment slack
 
 cudaError_t configure_mlp();
 // logits[lb * nout + c] for the chunk's blocks lb < a.nblocks (addressing as for the search kernels)
