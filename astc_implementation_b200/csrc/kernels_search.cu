@@ -59,8 +59,8 @@ struct Tabs {
     __device__ float2 trig(int i) const { return reinterpret_cast<const float2*>(b + L->off_trig)[i]; }
     __device__ uint4 tw4f(int m, int t) const { return reinterpret_cast<const uint4*>(b + L->off_tw4f)[m * L->T + t]; }
     __device__ uint32_t wt_info(int m, int w) const { return reinterpret_cast<const uint32_t*>(b + L->off_wt_info)[m * 64 + w]; }
-    __device__ int witem(int i) const { return reinterpret_cast<const uint16_t*>(b + L->off_witem)[i]; }
-    __device__ int sitem(int i) const { return reinterpret_cast<const uint16_t*>(b + L->off_sitem)[i]; }
+    __device__ const uint16_t* witems() const { return reinterpret_cast<const uint16_t*>(b + L->off_witem); }
+    __device__ const uint16_t* sitems() const { return reinterpret_cast<const uint16_t*>(b + L->off_sitem); }
     __device__ const uint4* w2tf(int i) const { return reinterpret_cast<const uint4*>(b + L->off_w2tf) + i; }
     __device__ uint32_t wgroup(int i) const { return reinterpret_cast<const uint32_t*>(b + L->off_wgroup)[i]; }
     __device__ const uint4* wgent(int i) const { return reinterpret_cast<const uint4*>(b + L->off_wgent) + 32 * i; }
@@ -639,10 +639,16 @@ __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtas) k_partition_se
 // depend on it.
 
 struct FrontLayout {
-    int px, w, wes, tp, dec, lo, hi, bm_err, ints, trig, qf, misc, dml, bml, total;
+    int px, w, wes, tp, dec, lo, hi, bm_err, ints, trig, qf, misc, dml, bml, witem, sitem, setup, total;
 };
 
+constexpr int kColourLevels = 17;  // colour quant levels 4..20; the tables below count from level 4
+// (the one-partition instance keeps one partition's colour errors and no format combinations: 5.9
+// instead of 9.3 KB at 4x4 with the item lists, so 32 of its warps fit on an SM instead of 22; k_front of
+// the 262,144 blocks of 2048x2048 2.27 -> 2.02 ms)
+template <bool P1>
 struct FrontMisc {
+    static constexpr int kParts = P1 ? 1 : 4, kCombos = P1 ? 1 : kColourLevels;
     float4 avg[4], dir[4], ep0[4], ep1[4];
     float mn[4], mx[4], lsq[4];
     float min_cutoff;
@@ -652,10 +658,10 @@ struct FrontMisc {
     float sxyz[4][3][4];  // pass08: per partition, sums of the deviations along r, g, b (w = 0)
     float acc[4][5];      // pass08: per partition, the five encoding-choice error sums
     float4 axes[4][4];    // pass08: per partition, ub, ua, sb, la
-    float cerr[4][21][4];
-    uint8_t cfmt[4][21][4];
-    float combo_err[21][13];
-    __align__(4) uint8_t combo_fmt[21][13][4];
+    float cerr[kParts][kColourLevels][4];
+    uint8_t cfmt[kParts][kColourLevels][4];
+    float combo_err[kCombos][13];
+    __align__(4) uint8_t combo_fmt[kCombos][13][4];
     int top[kNumCand];
     int ncand;
     int nlive;  // block modes in the proposal search's list
@@ -676,7 +682,7 @@ __host__ __device__ inline int front_layout_qf_floats(int T, int max_w, int nt, 
     return f;
 }
 __host__ __device__ inline int take16(int& o, int bytes) { const int r = o; o = (o + bytes + 15) & ~15; return r; }
-__host__ __device__ inline FrontLayout front_layout(const TableLayout& L, int nt, bool list) {
+__host__ __device__ inline FrontLayout front_layout(const TableLayout& L, int nt, bool list, bool p1) {
     const int T = L.T, ndm = L.ndm, nbm = L.nbm, max_w = L.max_w;
     FrontLayout f;
     int o = 0;
@@ -695,9 +701,12 @@ __host__ __device__ inline FrontLayout front_layout(const TableLayout& L, int nt
     const int rows = early + L.nw_total * 2, qf = front_layout_qf_floats(T, max_w, nt, list) * 4;
     f.qf = take16(o, rows > qf ? rows : qf);
     f.trig = f.qf + early;
-    f.misc = take16(o, (int)sizeof(FrontMisc));
+    f.misc = take16(o, p1 ? (int)sizeof(FrontMisc<true>) : (int)sizeof(FrontMisc<false>));
     f.dml = take16(o, 16 + ndm * 2);
     f.bml = take16(o, nbm * 2);  // the proposal search's block modes, ascending
+    f.witem = take16(o, list ? L.nwi * 2 : 0);  // and the weight and step items of its decimation modes
+    f.sitem = take16(o, list ? L.nsi * 2 : 0);
+    f.setup = take16(o, list ? kListGroup * 32 : 0);  // quantisation of a group's modes
     f.total = o;
     return f;
 }
@@ -742,31 +751,29 @@ __device__ __forceinline__ uint32_t bm_quant_weight(const Tabs& tb, const BmQuan
 // from the tables, sorted by their inner loop's length, so that a warp's lanes end together; a
 // half-warp per mode, which this replaces, kept 16 of 32 lanes busy (a mode has 4 to 64 weights,
 // 1 to 36 texels a weight and 2 to 12 steps) and spent three instructions in four on the loops
-// around the sums.  The proposal search's few modes are numbered by shifts instead.  The sums'
+// around the sums.  The proposal search lists the items of its few modes itself.  The sums'
 // entries are stored four to a load and, for the sorted items, 32 items side by side; the
 // weights of all modes are packed, which with the steps kept in pass07's buffer takes a 10x8
 // block from 70 to 51 KB of shared memory and from three to four CTAs.  Measured (B200, 128
 // threads): passes 02-05 of 13,312 partitioned blocks at 10x8 3.04 -> 1.43 ms, at 8x8 3.18 ->
 // 1.61 ms; with 32 threads 83,200 at 4x4 0.44 -> 0.41 ms.
 template <int NT, bool DEEP>
-__device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int ndm_run, const int16_t* dm_run, const float* iw,
+__device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int ndm_run, const int16_t* dm_run, int nw, int ns,
+                                          const uint16_t* witems, const uint16_t* sitems, const float* iw,
                                           const float* wes, bool is_const, float* dec, uint16_t* trig, float* lov, float* hiv,
                                           float* buf) {
     const int tid = threadIdx.x;
     const int tmask = is_const ? 0 : -1;
-    const int wsh = max_w <= 16 ? 4 : max_w <= 32 ? 5 : 6;  // weights per listed mode, rounded up
-    const int nw = dm_run ? ndm_run << wsh : tb.L->nwi;
     // item it's mode and weight, and its texel entries, `stride` fours apart
     const int stride = dm_run ? 1 : 32;
     auto weight_item = [&](int it, int& m, int& w, const uint4*& ent, int& n4) {
         uint32_t info;
+        const int e = witems[it];
+        m = e >> 6; w = e & 63;
         if (dm_run) {
-            m = dm_run[it >> wsh]; w = it & ((1 << wsh) - 1);
             info = tb.wt_info(m, w);
             ent = tb.w2tf(info & 0xFFFF);
         } else {
-            const int e = tb.witem(it);
-            m = e >> 6; w = e & 63;
             info = tb.wgroup(it >> 5);
             ent = tb.wgent(info & 0xFFFF) + (it & 31);
         }
@@ -779,7 +786,6 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int 
         const uint4* ent;
         weight_item(it, m, w, ent, n4);
         const DevDm dmi = tb.dm(m);
-        if (w >= (int)dmi.W) continue;
         float v = iw[w];
         if (dmi.W != T) {
             float ws = 0.0f, tc = 1e-10f;
@@ -828,7 +834,6 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int 
         weight_item(it, m, w, ent, n4);
         const DevDm dmi = tb.dm(m);
         const int W = dmi.W;
-        if (w >= W) continue;
         float v = dec[dmi.w_off + w];
         if (W != T) {
             const float* im = inf + m * T;
@@ -859,15 +864,11 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int 
     const int nstep = tb.L->ndm * kMaxAngularSteps;
     int2* step_span = reinterpret_cast<int2*>(buf + 4 * nstep);  // span, lowest index (float bits)
     float* ang = buf + 6 * nstep;
-    const int ns = dm_run ? ndm_run << 4 : tb.L->nsi;
 #pragma unroll 1
     for (int it = tid; it < ns; it += NT) {
-        int m, i;
-        if (dm_run) { m = dm_run[it >> 4]; i = it & 15; }
-        else { const int e = tb.sitem(it); m = e >> 4; i = e & 15; }
+        const int e = sitems[it], m = e >> 4, i = e & 15;
         const DevDm dmi = tb.dm(m);
         const int W = dmi.W;
-        if (i >= (int)dmi.max_angular_steps) continue;
         const float* dw = dec + dmi.w_off;
         const uint2* rows = reinterpret_cast<const uint2*>(trig + dmi.w_off);
         float ax = 0.0f, ay = 0.0f;
@@ -897,9 +898,9 @@ __device__ __forceinline__ void dm_passes(const Tabs& tb, int T, int max_w, int 
         }
         const int sp = min(max((int)rn_small((maxidx - minidx) + 1.0f), 2), (int)dmi.max_quant_steps + 3);
         const float ss = 1.0f / rcp, esc = ss * ss;
-        const float e = ev * esc, ecl0 = cl * esc, ech0 = ch * esc;
+        const float err = ev * esc, ecl0 = cl * esc, ech0 = ch * esc;
         const int at = m * kMaxAngularSteps + i;
-        step_err[at] = make_float4(e, e + ecl0, e + ech0, (e + ecl0) + ech0);
+        step_err[at] = make_float4(err, err + ecl0, err + ech0, (err + ecl0) + ech0);
         step_span[at] = make_int2(sp, __float_as_int(minidx));
         ang[at] = off;
     }
@@ -998,7 +999,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     const Tabs tb{a.tables, &a.L};
     const int T = a.L.T, ndm = a.L.ndm, nbm = a.L.nbm;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const FrontLayout fl = front_layout(a.L, NT, a.bm_mask != nullptr);
+    const FrontLayout fl = front_layout(a.L, NT, a.bm_mask != nullptr, P1);
     float4* px = reinterpret_cast<float4*>(sm + fl.px);
     float* iw = reinterpret_cast<float*>(sm + fl.w);
     float* wes = reinterpret_cast<float*>(sm + fl.wes);
@@ -1009,7 +1010,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     float* bm_err = reinterpret_cast<float*>(sm + fl.bm_err);
     uint8_t* mode_ints = sm + fl.ints;  // pass11's integer count per block mode
     float* qfs = reinterpret_cast<float*>(sm + fl.qf);
-    FrontMisc& M = *reinterpret_cast<FrontMisc*>(sm + fl.misc);
+    FrontMisc<P1>& M = *reinterpret_cast<FrontMisc<P1>*>(sm + fl.misc);
     const float4 cw = chan_w();
     // Partition bytes of texels t..t+3 (t a multiple of 4 below Tp) and of texel t < T.  With one
     // partition they are known, 0 for the block's texels and 0xFF (no partition) for the
@@ -1211,6 +1212,8 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     const uint64_t* bmm = a.bm_mask ? a.bm_mask + ((size_t)lb * 4 + (P - 1)) * kMaskWords : nullptr;
     uint32_t* flags = reinterpret_cast<uint32_t*>(sm + fl.dml);  // 4 words: one bit per decimation mode
     int16_t* list = reinterpret_cast<int16_t*>(sm + fl.dml + 16);
+    uint16_t* witems = reinterpret_cast<uint16_t*>(sm + fl.witem);
+    uint16_t* sitems = reinterpret_cast<uint16_t*>(sm + fl.sitem);
     if (bmm && tid < 4) flags[tid] = 0;
     __syncthreads();
     int16_t* blist = reinterpret_cast<int16_t*>(sm + fl.bml);
@@ -1269,7 +1272,17 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
                 n += __popc(b);
             }
         __syncwarp();
-        if (lane == 0) flags[0] = n;  // the flags are no longer needed
+        int nw = 0, ns = 0;  // their weights and angular steps as dm_passes' items
+#pragma unroll 1
+        for (int i = 0; i < n; i++) {
+            const int d = list[i];
+            const DevDm dmi = tb.dm(d);
+            for (int w = lane; w < (int)dmi.W; w += 32) witems[nw + w] = (uint16_t)(d << 6 | w);
+            if (lane < (int)dmi.max_angular_steps) sitems[ns + lane] = (uint16_t)(d << 4 | lane);
+            nw += dmi.W;
+            ns += dmi.max_angular_steps;
+        }
+        if (lane == 0) { flags[0] = n; flags[1] = nw; flags[2] = ns; }  // the flags are no longer needed
     }
 #pragma unroll 1
     for (int v = role; v < 5 * P; v += kFrontThreads) {
@@ -1289,38 +1302,33 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     const int ndm_run = bmm ? (int)flags[0] : ndm;
     const int16_t* dm_run = bmm ? list : nullptr;
     // ---------------- pass09: colour error per partition, quant level and integer count
-    // (role 21p + q; runs beside passes 02-05, which do not read it)
+    // (role 17p + level; runs beside passes 02-05, which do not read it)
 #pragma unroll 1
-    for (int c = role; c < P * 21; c += kFrontThreads) {
-        const int p = c / 21, q = c % 21;
-        if (q < 4) {
-            for (int j = 0; j < 4; j++) M.cerr[p][q][j] = ERR_DEFAULT;
-            M.cfmt[p][q][0] = FMT_LUMINANCE; M.cfmt[p][q][1] = FMT_RGB_SCALE; M.cfmt[p][q][2] = FMT_RGB; M.cfmt[p][q][3] = FMT_RGBA;
-            continue;
-        }
-        const int i = q - 4;
+    for (int c = role; c < P * kColourLevels; c += kFrontThreads) {
+        const int p = c / kColourLevels, i = c % kColourLevels;
         const float rre = M.p9[p][0], are = M.p9[p][1], brgb = M.p9[p][2], ba = M.p9[p][3];
         const bool cbc = M.ece_can_bc[p] == 1, coe = M.ece_can_offset[p] == 1;
         const float bcrgba = cbc ? 0.625f : 1.0f, oergba = coe ? 0.5f : 1.0f, bcrgb = cbc ? 0.5f : 1.0f, oergb = coe ? 0.25f : 1.0f;
         const float acc0 = M.acc[p][0], acc1 = M.acc[p][1], acc2 = M.acc[p][2], acc4 = M.acc[p][4];
         const float rgbs_e = (acc2 - acc1) * 0.7f, lum_e = (acc4 - acc1) * 3.0f, ad_e = acc0 * 3.0f;
-        const float orgba = q >= 19 ? 1.0f : oergba, orgb = q >= 19 ? 1.0f : oergb;
+        const float orgba = i >= 15 ? 1.0f : oergba, orgb = i >= 15 ? 1.0f : oergb;
         const float bq = tb.bqe(i);
         const float qrgb = brgb * bq, qrgba = (brgb + ba) * bq;
-        M.cerr[p][q][3] = (((qrgba * bcrgba) * orgba) + rre) + are; M.cfmt[p][q][3] = FMT_RGBA;
+        M.cerr[p][i][3] = (((qrgba * bcrgba) * orgba) + rre) + are; M.cfmt[p][i][3] = FMT_RGBA;
         const float full = (((qrgb * bcrgb) * orgb) + rre) + ad_e;
         const float rgbsa = ((qrgba + rgbs_e) + rre) + are;
-        if (rgbsa < full) { M.cerr[p][q][2] = rgbsa; M.cfmt[p][q][2] = FMT_RGB_SCALE_ALPHA; }
-        else { M.cerr[p][q][2] = full; M.cfmt[p][q][2] = FMT_RGB; }
+        if (rgbsa < full) { M.cerr[p][i][2] = rgbsa; M.cfmt[p][i][2] = FMT_RGB_SCALE_ALPHA; }
+        else { M.cerr[p][i][2] = full; M.cfmt[p][i][2] = FMT_RGB; }
         const float lrgbs = ((qrgb + rre) + ad_e) + rgbs_e;
         const float la_e = ((qrgba + rre) + are) + lum_e;
-        if (lrgbs < la_e) { M.cerr[p][q][1] = lrgbs; M.cfmt[p][q][1] = FMT_RGB_SCALE; }
-        else { M.cerr[p][q][1] = la_e; M.cfmt[p][q][1] = FMT_LUMINANCE_ALPHA; }
-        M.cerr[p][q][0] = ((qrgb + rre) + ad_e) + lum_e; M.cfmt[p][q][0] = FMT_LUMINANCE;
+        if (lrgbs < la_e) { M.cerr[p][i][1] = lrgbs; M.cfmt[p][i][1] = FMT_RGB_SCALE; }
+        else { M.cerr[p][i][1] = la_e; M.cfmt[p][i][1] = FMT_LUMINANCE_ALPHA; }
+        M.cerr[p][i][0] = ((qrgb + rre) + ad_e) + lum_e; M.cfmt[p][i][0] = FMT_LUMINANCE;
     }
 
     // ---------------- passes 02-05
-    dm_passes<NT, DEEP>(tb, T, a.L.max_w, ndm_run, dm_run, iw, wes, is_const, dec, reinterpret_cast<uint16_t*>(sm + fl.trig), lov, hiv, qfs);
+    dm_passes<NT, DEEP>(tb, T, ndm_run, dm_run, bmm ? (int)flags[1] : a.L.nwi, bmm ? (int)flags[2] : a.L.nsi, bmm ? witems : tb.witems(),
+                        bmm ? sitems : tb.sitems(), iw, wes, is_const, dec, reinterpret_cast<uint16_t*>(sm + fl.trig), lov, hiv, qfs);
     __syncthreads();
 
     // ---------------- pass07: weight quantisation error per block mode
@@ -1333,8 +1341,8 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
     if (P > 1) {
         const int NC = P == 2 ? 7 : P == 3 ? 10 : 13;
 #pragma unroll 1
-        for (int it = role; it < 17 * NC; it += kFrontThreads) {
-            const int q = 4 + it / NC, c = it - (it / NC) * NC;
+        for (int it = role; it < kColourLevels * NC; it += kFrontThreads) {
+            const int q = it / NC, c = it - q * NC;
             float be = ERR_DEFAULT;
             uint32_t bf = 0;
 #pragma unroll 1
@@ -1364,30 +1372,42 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         const int G = qf_floats / (mw + Tp);
         float* qw = qfs;           // [G][mw]
         float* et = qfs + G * mw;  // [G][Tp]
+        float4* setup = reinterpret_cast<float4*>(sm + fl.setup);  // [G][2]; last word: weights (0: a mode that cannot be used) |
+                                                                   // first weight << 8 | decimation mode << 24
+        const uint32_t per_w = 0xFFFFFFFFu / (uint32_t)mw + 1u, per_t = 0xFFFFFFFFu / (uint32_t)Tp + 1u;  // n / mw is umulhi(n, per_w)
 #pragma unroll 1
         for (int g0 = 0; g0 < nlist; g0 += G) {
             const int g = min(G, nlist - g0);
 #pragma unroll 1
-            for (int it = tid; it < g * mw; it += kFrontThreads) {
-                const int k = it / mw, w = it - k * mw;
+            for (int k = tid; k < g; k += kFrontThreads) {
                 const DevBm bm = tb.bm(blist[g0 + k]);
-                const int bc = c_free_bits[P - 1] - (int)bm.weight_bits;
+                const bool usable = bm.quant <= 11 && c_free_bits[P - 1] > (int)bm.weight_bits;
+                BmQuant s{};
                 const DevDm dmi = tb.dm(bm.dm);
-                if (bm.quant > 11 || bc <= 0 || w >= (int)dmi.W) continue;
-                const BmQuant s = bm_quant_setup(tb, bm, lov + bm.dm * 8, hiv + bm.dm * 8, M.min_cutoff);
-                float qf;
-                bm_quant_weight(tb, s, dec[dmi.w_off + w], &qf);
-                qw[k * mw + w] = qf;
+                if (usable) s = bm_quant_setup(tb, bm, lov + bm.dm * 8, hiv + bm.dm * 8, M.min_cutoff);
+                setup[2 * k] = make_float4(s.low, s.scale, s.slb, s.rscale);
+                setup[2 * k + 1] = make_float4(s.qlm1, __uint_as_float(s.q2u_start), __uint_as_float(s.top),
+                                               __uint_as_float(usable ? (uint32_t)dmi.W | (uint32_t)dmi.w_off << 8 | (uint32_t)bm.dm << 24 : 0u));
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int it = tid; it < g * mw; it += kFrontThreads) {
+                const int k = (int)__umulhi((uint32_t)it, per_w), w = it - k * mw;
+                const float4 b = setup[2 * k + 1];
+                const uint32_t wd = __float_as_uint(b.w);
+                if (w >= (int)(wd & 0xFF)) continue;
+                const float4 q = setup[2 * k];
+                const BmQuant s{q.x, q.y, q.z, q.w, b.x, __float_as_uint(b.y), __float_as_uint(b.z)};
+                bm_quant_weight(tb, s, dec[((wd >> 8) & 0xFFFF) + w], &qw[k * mw + w]);
             }
             __syncthreads();
 #pragma unroll 1
             for (int it = tid; it < g * Tp; it += kFrontThreads) {
-                const int k = it / Tp, t = it - k * Tp;
-                const DevBm bm = tb.bm(blist[g0 + k]);
-                const int bc = c_free_bits[P - 1] - (int)bm.weight_bits;
+                const int k = (int)__umulhi((uint32_t)it, per_t), t = it - k * Tp;
+                const uint32_t wd = __float_as_uint(setup[2 * k + 1].w);
                 float term = 0.0f;
-                if (t < T && !(bm.quant > 11 || bc <= 0)) {
-                    const uint4 e = tb.tw4f(bm.dm, t);
+                if (t < T && wd != 0) {
+                    const uint4 e = tb.tw4f((int)(wd >> 24), t);
                     const float* qk = qw + k * mw;
                     float v = qk[entry_index(e.x)] * entry_factor(e.x);
                     v = v + qk[entry_index(e.y)] * entry_factor(e.y);
@@ -1399,13 +1419,11 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
                 et[k * Tp + t] = term;
             }
             __syncthreads();
-            // (the next group's first phase writes only qw, which this one does not read)
+            // (the next group's setups follow a barrier, its weights are not read here)
 #pragma unroll 1
             for (int k = tid; k < g; k += kFrontThreads) {
                 const int i = blist[g0 + k];
-                const DevBm bm = tb.bm(i);
-                const int bc = c_free_bits[P - 1] - (int)bm.weight_bits;
-                if (bm.quant > 11 || bc <= 0) { bm_err[i] = 1e38f; continue; }
+                if (__float_as_uint(setup[2 * k + 1].w) == 0) { bm_err[i] = 1e38f; continue; }
                 const float* x = et + k * Tp;
                 float err = 0.0f;
 #pragma unroll 1
@@ -1415,6 +1433,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
                 }
                 bm_err[i] = err;
             }
+            if (g0 + G < nlist) __syncthreads();
         }
     }
     __syncthreads();
@@ -1433,7 +1452,7 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
         for (int ic = lo; ic <= hi; ic++) {
             const int ql = tb.qmt(ic, bits);
             if (ql < 4) { if (P == 1) continue; break; }
-            const float e = P == 1 ? M.cerr[0][ql][ic - 1] : M.combo_err[ql][ic - P];
+            const float e = P == 1 ? M.cerr[0][ql - 4][ic - 1] : M.combo_err[ql - 4][ic - P];
             if (e < best) { best = e; ints = ic; }
         }
         bm_err[i] = best + werr;
@@ -1533,8 +1552,8 @@ __device__ void front_body(const KernelArgs& a, const int P_arg, int lb, int blk
             const int bits = c_free_bits[P - 1] - (int)bm.weight_bits, ints = mode_ints[i];
             const int ql = tb.qmt(ints, bits), qlm = P == 1 ? ql : tb.qmt(ints, bits + (P == 2 ? 2 : P == 3 ? 5 : 8));
             uint32_t fmt = 0;
-            if (P == 1) fmt = ql >= 4 ? M.cfmt[0][ql][ints - 1] : (uint32_t)FMT_LUMINANCE;
-            else if (ql >= 4) fmt = *reinterpret_cast<const uint32_t*>(M.combo_fmt[ql][ints - P]);
+            if (P == 1) fmt = ql >= 4 ? M.cfmt[0][ql - 4][ints - 1] : (uint32_t)FMT_LUMINANCE;
+            else if (ql >= 4) fmt = *reinterpret_cast<const uint32_t*>(M.combo_fmt[ql - 4][ints - P]);
             // bm, ql, qlm and the four formats: 8-byte aligned in PBRec
             *reinterpret_cast<uint2*>(&c) = make_uint2((uint32_t)i | (uint32_t)(ql & 0xFF) << 16 | (uint32_t)(qlm & 0xFF) << 24, fmt);
         }
@@ -1622,9 +1641,9 @@ static int front_nt(const KernelArgs& a) {
 }
 
 size_t search_smem_bytes(const TableLayout& L) { return (size_t)kSearchWarps * search_layout(L.T).total; }
-size_t front_smem_bytes(const TableLayout& L, int nt, bool list) { return (size_t)front_layout(L, nt, list).total; }
+static size_t front_smem_bytes(const TableLayout& L, int nt, bool list, bool p1) { return (size_t)front_layout(L, nt, list, p1).total; }
 size_t front_smem_bytes(const TableLayout& L) {  // the largest over the launches of this footprint
-    return std::max(front_smem_bytes(L, 128, false), front_smem_bytes(L, front_nt(L.T, false, 1 << 30), false));
+    return std::max(front_smem_bytes(L, 128, false, false), front_smem_bytes(L, front_nt(L.T, false, 1 << 30), false, false));
 }
 
 cudaError_t configure_search_kernels(size_t search_bytes, size_t front_bytes) {
@@ -1650,8 +1669,8 @@ cudaError_t launch_front(const KernelArgs& a, cudaStream_t s) {
     const int nt = front_nt(a);
     int grid = a.nblocks * a.slots;
     if (a.block_list) grid = std::min(grid, kListGridFront * 128 / nt);
-    const size_t smem = front_smem_bytes(a.L, nt, a.bm_mask != nullptr);
     auto go = [&](const KernelArgs& k, bool p1) {
+        const size_t smem = front_smem_bytes(a.L, nt, a.bm_mask != nullptr, p1);
         if (nt == 32) { if (p1) k_front<32, true, false><<<grid, 32, smem, s>>>(k); else k_front<32, false, false><<<grid, 32, smem, s>>>(k); }
         else if (nt == 64) { if (p1) k_front<64, true, false><<<grid, 64, smem, s>>>(k); else k_front<64, false, false><<<grid, 64, smem, s>>>(k); }
         else if (nt == 256) k_front<256, false, true><<<grid, 256, smem, s>>>(k);
