@@ -324,10 +324,10 @@ __host__ __device__ inline int refine_group(int T, int cpb, int spread) {  // pa
 // candidate's rank in its group's initial order, so the first iteration's lanes are on
 // consecutive slots and the gathered ones of later iterations on increasing ones.
 //   ep   [8]      least-squares endpoints (float4): ep0 and ep1 of partition q in rows 2q, 2q + 1
-//   u    [4]      unpacked endpoints of partition q, 0..255 x 257, eight u16: ep0 xyzw, ep1 xyzw
+//   u    [4]      unpacked endpoints of partition q, eight bytes: ep0 xyzw, ep1 xyzw (used times 257)
 //   s    [T]      infilled weight of each texel times 16, 0..1024, exact in half precision
 //   qw   [max_w]  grid weights 0..64
-//   err           best error so far
+// The best error so far is in the candidate's snapshot.
 // The infilled weights are kept as sums of grid weight x (contribution x 16), small integers
 // that pass16 updates when it moves a weight; every use of one (pass13's weight s / 1024,
 // pass16's s / 16, pass17's rounded s / 16) is the exact value the passes' own sums of
@@ -337,9 +337,12 @@ __host__ __device__ inline int refine_group(int T, int cpb, int spread) {  // pa
 // Measured with pass13's walk in partition order (B200): full search of 1024x1024 at 4x4 50.2 -> 47.5 ms,
 // of 64x64 1.08 -> 0.90 ms; proposal search of 2047x2050 at 6x6 8.98 -> 8.13 ms.
 constexpr int kSlotRow16 = kRefineThreads * 16;  // bytes of a row of 16-byte elements
+constexpr int kSlotRow8 = kRefineThreads * 8;    // of 8-byte elements
 constexpr int kSlotRow4 = kRefineThreads * 4;    // of two s or four qw
 struct RefineLayout {
-    int ep, u, s, qw, err, item, pos, px, part, sdir, keys, aux, total;
+    int ep, u, s, qw, pos, map, px, part, staged, total;  // both kernels
+    int item, next_it;                                    // k_refine_tail
+    int keys;                                             // k_refine: over u, which only an iteration holds
 };
 // Texel rows of the staged partitioned blocks, an odd number of banks (or 16-byte bank groups)
 // apart: a warp's candidates, sorted by path, belong to different partitioned blocks.
@@ -351,34 +354,35 @@ __host__ __device__ inline RefineLayout refine_layout(int T, int max_w, int rows
     int o = 0;
     auto take = [&](int bytes) { const int r = o; o += (bytes + 15) & ~15; return r; };
     f.ep = take(8 * kSlotRow16);
-    f.u = take(4 * kSlotRow16);
+    f.keys = f.u = take(4 * kSlotRow8);
     f.s = take((T + 1) / 2 * kSlotRow4);
     f.qw = take((max_w + 3) / 4 * kSlotRow4);
-    f.err = take(kRefineThreads * 4);
-    f.item = take(kRefineThreads * 4);
     f.pos = take(kRefineThreads);
+    f.map = take(kRefineThreads);
     f.px = take(rows * px_row_bytes(T, u8));
     f.part = take(rows * part_row_bytes(T, u8 && !tail ? 2 : 1));
-    f.sdir = take(tail ? 0 : rows * 64);
-    f.keys = take(kRefineThreads * 4);
-    f.aux = take(tail ? kRefineThreads * 4 : rows * 4);
+    f.staged = take(tail ? 0 : rows * 4);
+    f.item = take(tail ? kRefineThreads * 4 : 0);
+    f.next_it = take(tail ? kRefineThreads : 0);
     f.total = o;
     return f;
 }
 struct Cand {  // one slot of the arrays above
     uint8_t *epb, *ub, *sb, *qb;
-    float* err;
     __device__ Cand(uint8_t* sm, const RefineLayout& f, int slot)
-        : epb(sm + f.ep + slot * 16), ub(sm + f.u + slot * 16), sb(sm + f.s + slot * 4), qb(sm + f.qw + slot * 4),
-          err(reinterpret_cast<float*>(sm + f.err) + slot) {}
+        : epb(sm + f.ep + slot * 16), ub(sm + f.u + slot * 8), sb(sm + f.s + slot * 4), qb(sm + f.qw + slot * 4) {}
     __device__ __forceinline__ float4& ep(int i) const { return *reinterpret_cast<float4*>(epb + i * kSlotRow16); }
-    __device__ __forceinline__ uint4& u(int q) const { return *reinterpret_cast<uint4*>(ub + q * kSlotRow16); }
+    __device__ __forceinline__ uint2& u(int q) const { return *reinterpret_cast<uint2*>(ub + q * kSlotRow8); }
     __device__ __forceinline__ __half& s(int t) const { return *reinterpret_cast<__half*>(sb + (t >> 1) * kSlotRow4 + (t & 1) * 2); }
     __device__ __forceinline__ uint8_t& qw(int w) const { return qb[(w >> 2) * kSlotRow4 + (w & 3)]; }
     __device__ __forceinline__ uint32_t& qw4(int i) const { return *reinterpret_cast<uint32_t*>(qb + i * kSlotRow4); }
 };
-// The u16 in the low (hi = false) or high half of v as a float: 2^23 + v has v as its low bits.
-__device__ __forceinline__ float u16f(uint32_t v, bool hi) { return __uint_as_float(__byte_perm(v, 0x4B000000u, hi ? 0x7632 : 0x7610)) - 8388608.0f; }
+// The four bytes of v times 257, as floats: 2^23 + n has n as its low bits, and a byte times 257 is the
+// byte twice.
+__device__ __forceinline__ float4 x257(uint32_t v) {
+    return make_float4(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7600)) - 8388608.0f, __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7611)) - 8388608.0f,
+                       __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7622)) - 8388608.0f, __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7633)) - 8388608.0f);
+}
 // Round to the nearest integer, ties to even, for 0 <= v < 2^22 (rintf on the FP32 adders).
 __device__ __forceinline__ float rn_small(float v) { return (v + 8388608.0f) - 8388608.0f; }
 
@@ -468,8 +472,8 @@ __device__ __forceinline__ float4 scale_dir(float4 avg, float ps) {
 // degenerate keep the previous values, which are these), so packing, unpacking, realignment
 // and the final error repeat exactly and can never lower the error: stopping there gives
 // the result of running the remaining iterations.
-template <class Row, class Part, class SDir>
-__device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, int k, const Row px, const Part pt, const SDir sdir_of,
+template <class Row, class Part>
+__device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, int k, const Row px, const Part pt,
                             const Cand cs, Snap* snap, const int it) {
     const RTabs tb{a.tables, &a.L};
     const int T = a.L.T;
@@ -489,7 +493,6 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         const uint32_t* src = reinterpret_cast<const uint32_t*>(ci.qw);  // 8-byte aligned in PBRec
 #pragma unroll 1
         for (int w = 0; w < (W + 3) / 4; w++) cs.qw4(w) = src[w];
-        *cs.err = ERR_DEFAULT;
         infill(tb, cs, bm.dm, T, direct);
     }
     uint32_t ffmt[4] = {0, 0, 0, 0}, matched = 0, final_q = ci.ql;
@@ -506,9 +509,9 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         for (int t = 0; t < T; t++) {
             const int p = pt.part(t);
             if (p != pc) {
-                const uint4 u = cs.u(p);
-                base = make_float4(u16f(u.x, false), u16f(u.x, true), u16f(u.y, false), u16f(u.y, true));
-                offs = (make_float4(u16f(u.z, false), u16f(u.z, true), u16f(u.w, false), u16f(u.w, true)) - base) * (1.0f / 64.0f);
+                const uint2 u = cs.u(p);
+                base = x257(u.x);
+                offs = (x257(u.y) - base) * (1.0f / 64.0f);
                 base = base + mk(1.0f / 128.0f);
                 pc = p;
             }
@@ -521,8 +524,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
             d.w = x.w - rn_small(base.w + offs.w * w1);
             total = total + dot4(d * d, cw);
         }
-        if (total < *cs.err) {  // the best so far (ERR_DEFAULT at first)
-            *cs.err = total;
+        if (total < snap->err) {  // the best so far (ERR_DEFAULT at first)
             uint4* d = reinterpret_cast<uint4*>(snap);  // 16-byte aligned: 112-byte records
             d[0] = make_uint4(__float_as_uint(total), (uint32_t)ci.bm | final_q << 16 | matched << 24,
                               ffmt[0] | ffmt[1] << 8 | ffmt[2] << 16 | ffmt[3] << 24, 0u);
@@ -549,7 +551,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         const float ps = (float)n;
         // the scale direction and its sums are only read by the formats with a scale
         const bool scale = ci.fmt[q] == FMT_RGB_SCALE || ci.fmt[q] == FMT_RGB_SCALE_ALPHA;
-        const float4 sdir = scale ? sdir_of(q, ps) : mk(0.0f);
+        const float4 sdir = scale ? scale_dir(rec.avg[q], ps) : mk(0.0f);
         float wmin = 1.0f, wmax = 0.0f, ls = 0.0f, ms = 0.0f, rs = 0.0f, smin = 1e10f, smax = 0.0f, sv0 = 0.0f, sv1 = 0.0f;
         float4 cx = mk(0.0f), cy = mk(0.0f);
 #pragma unroll 1
@@ -658,8 +660,8 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     for (int q = 0; q < P; q++) {
         I4 o0, o1;
         unpack_endpoints(q == 0 ? ffmt[0] : q == 1 ? ffmt[1] : q == 2 ? ffmt[2] : ffmt[3], packed[q].x, packed[q].y, o0, o1);
-        cs.u(q) = make_uint4((uint32_t)(o0.x * 257) | (uint32_t)(o0.y * 257) << 16, (uint32_t)(o0.z * 257) | (uint32_t)(o0.w * 257) << 16,
-                             (uint32_t)(o1.x * 257) | (uint32_t)(o1.y * 257) << 16, (uint32_t)(o1.z * 257) | (uint32_t)(o1.w * 257) << 16);
+        cs.u(q) = make_uint2((uint32_t)o0.x | (uint32_t)o0.y << 8 | (uint32_t)o0.z << 16 | (uint32_t)o0.w << 24,
+                             (uint32_t)o1.x | (uint32_t)o1.y << 8 | (uint32_t)o1.z << 16 | (uint32_t)o1.w << 24);
     }
     // ---------------- pass16: move each weight one quant step if that lowers the error
     bool moved = false;
@@ -670,9 +672,9 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     int pc = -1;
     auto endpoints = [&](int p) {  // of texel partition p, read again when it changes
         if (p == pc) return;
-        const uint4 u = cs.u(p);
-        base = make_float4(u16f(u.x, false), u16f(u.x, true), u16f(u.y, false), u16f(u.y, true));
-        offs = (make_float4(u16f(u.z, false), u16f(u.z, true), u16f(u.w, false), u16f(u.w, true)) - base) * (1.0f / 64.0f);
+        const uint2 u = cs.u(p);
+        base = x257(u.x);
+        offs = (x257(u.y) - base) * (1.0f / 64.0f);
         pc = p;
     };
     if (direct) {
@@ -742,11 +744,11 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
 }
 
 // A refinement-tail entry: the partitioned block (lb * slots + slot), the candidate and the
-// next iteration, the best error so far, then the state an iteration carries over (endpoints,
-// weights; the best result so far is in the candidate's snapshot already).
+// next iteration, then the state an iteration carries over (endpoints, weights; the best
+// result so far is in the candidate's snapshot already).
 __device__ __forceinline__ void write_tail(const KernelArgs& a, const Cand& c, uint32_t pbi, int k, int it, int pos) {
     uint4* e = a.tail + (size_t)pos * kTailWords;
-    e[0] = make_uint4(pbi, (uint32_t)k | (uint32_t)it << 8, __float_as_uint(*c.err), 0u);
+    e[0] = make_uint4(pbi, (uint32_t)k | (uint32_t)it << 8, 0u, 0u);
     float4* ep = reinterpret_cast<float4*>(e + 1);
 #pragma unroll
     for (int i = 0; i < 8; i++) ep[i] = c.ep(i);
@@ -768,10 +770,9 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
     using Px = typename std::conditional<U8, uchar4, float4>::type;
     using Pe = typename std::conditional<U8, uint16_t, uint8_t>::type;
     const int px_row = px_row_bytes(T, U8), part_row = part_row_bytes(T, sizeof(Pe));
-    uint32_t* item_of = reinterpret_cast<uint32_t*>(smem + fl.item);  // by slot: lb * slots + slot
-    uint8_t* pos_of = smem + fl.pos;                                  // by slot: staging position
-    uint32_t* staged = reinterpret_cast<uint32_t*>(smem + fl.aux);    // by staged partitioned block: lb + 1 | slot << 27, 0 if none
-    float4* sdirs = reinterpret_cast<float4*>(smem + fl.sdir);
+    uint8_t* pos_of = smem + fl.pos;                                   // by slot: staging position
+    uint8_t* map = smem + fl.map;                                      // by rank: the candidate's slot
+    uint32_t* staged = reinterpret_cast<uint32_t*>(smem + fl.staged);  // by staged partitioned block: lb + 1 | slot << 27, 0 if none
     int* keys = reinterpret_cast<int*>(smem + fl.keys);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // Items: every slot of every block in slot-major order (consecutive CTAs hold
@@ -831,8 +832,6 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                         else row[t] = src_texel(src, a.L.bx, t);
                     }
                     if (k == 0) PartRow<Pe>{reinterpret_cast<Pe*>(smem + fl.part + pbl * part_row)}.set(prow, counts, T);
-#pragma unroll 1
-                    for (int q = k; q < P; q += cpb) sdirs[pbl * 4 + q] = scale_dir(r.avg[q], (float)(P == 1 ? T : (int)counts[q]));
                 }
             }
             keys[tid] = key * kRefineThreads + tid;  // unique keys: P, formats, decimation mode, then position
@@ -852,10 +851,9 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                 const int4 o = k4[j];
                 rank += (o.x < kk) + (o.y < kk) + (o.z < kk) + (o.w < kk);
             }
-            __syncthreads();
-            keys[rank] = tid;
-            __syncthreads();
-            const int mine = place < kRefineThreads ? keys[place] : kRefineThreads * cpb;
+            map[rank] = (uint8_t)tid;
+            __syncthreads();  // also: every thread has read the keys, which the first iteration overwrites
+            const int mine = place < kRefineThreads ? map[place] : kRefineThreads * cpb;
             const int pbl = mine / cpb, k = mine % cpb;
             const uint32_t item = pbl < pbs ? staged[pbl] : 0u;
             if (item != 0) {
@@ -864,7 +862,6 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                 a.snaps[pbi * kNumCand + k].err = ERR_DEFAULT;  // inert slot unless refined below
                 if (k < (int)a.pbrec[pbi].ncand) {
                     cand = place;
-                    item_of[place] = (uint32_t)pbi;
                     pos_of[place] = (uint8_t)mine;
                     if (a.work) atomicAdd(&refined[a.pbrec[pbi].P - 1], 1u);
                 }
@@ -879,7 +876,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
             const bool live = cand >= 0;
             const unsigned bal = __ballot_sync(0xFFFFFFFFu, live);
             if (lane == 0) live_in_warp[warp] = __popc(bal);
-            __syncthreads();  // also: every thread has read keys[] before it is rewritten
+            __syncthreads();  // also: every thread has read map[] before it is rewritten
             int nlive = 0, before = 0;
 #pragma unroll
             for (int w = 0; w < kRefineThreads / 32; w++) {
@@ -901,24 +898,29 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                 if (sb + nlive <= a.tail_cap) {
                     // (the next group's staging writes no slot state: it is first written after
                     // its staging barriers)
-                    if (live) write_tail(a, Cand(smem, fl, cand), item_of[cand], pos_of[cand] % cpb, it, pos);
+                    if (live) {
+                        const uint32_t item = staged[pos_of[cand] / cpb];
+                        const uint32_t pbi = ((item & 0x07FFFFFFu) - 1) * (uint32_t)a.slots + (item >> 27);
+                        write_tail(a, Cand(smem, fl, cand), pbi, pos_of[cand] % cpb, it, pos);
+                    }
+                    __syncthreads();  // staged[] is rewritten next
                     break;
                 }
                 if (live && pos < a.tail_cap) a.tail[(size_t)pos * kTailWords].x = 0xFFFFFFFFu;  // reserved, left empty
                 spill = false;  // the tail is full: finish here
             }
-            if (live) keys[rank] = cand;
+            if (live) map[rank] = (uint8_t)cand;
             __syncthreads();
-            cand = place < nlive ? keys[place] : -1;
+            cand = place < nlive ? map[place] : -1;
             if (cand >= 0) {
                 const int pbl = pos_of[cand] / cpb, k = pos_of[cand] % cpb;
-                const size_t pbi = item_of[cand];
+                const uint32_t item = staged[pbl];
+                const size_t pbi = (size_t)((item & 0x07FFFFFFu) - 1) * a.slots + (item >> 27);
                 const PBRec& rec = a.pbrec[pbi];
                 Snap* snap = &a.snaps[pbi * kNumCand + k];
                 const TexelRow<U8> row{reinterpret_cast<const Px*>(smem + fl.px + pbl * px_row)};
                 const PartRow<Pe> part{reinterpret_cast<Pe*>(smem + fl.part + pbl * part_row)};
-                const float4* sd = sdirs + pbl * 4;
-                const bool moved = refine_step(a, rec, (int)rec.P, k, row, part, [&](int q, float) { return sd[q]; }, Cand(smem, fl, cand), snap, it);
+                const bool moved = refine_step(a, rec, (int)rec.P, k, row, part, Cand(smem, fl, cand), snap, it);
                 if (!moved || it + 1 >= iters) cand = -1;
             }
             // (the next pass's first barrier orders this iteration's state writes before
@@ -941,8 +943,8 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
     const int T = a.L.T;
     const RefineLayout fl = refine_layout(T, a.L.max_w, kRefineThreads, true, true);
     const int px_row = px_row_bytes(T, true), part_row = part_row_bytes(T, 1);
-    int* keys = reinterpret_cast<int*>(smem + fl.keys);
-    int* next_it = reinterpret_cast<int*>(smem + fl.aux);             // by slot
+    uint8_t* map = smem + fl.map;                                     // by rank: the candidate's slot
+    uint8_t* next_it = smem + fl.next_it;                             // by slot
     uint32_t* pbi_of = reinterpret_cast<uint32_t*>(smem + fl.item);   // by slot
     uint8_t* k_of = smem + fl.pos;                                    // by slot: the candidate
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1008,12 +1010,11 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
                     const uint32_t* w = reinterpret_cast<const uint32_t*>(e + 9);
 #pragma unroll 1
                     for (int i = 0; i < n4; i++) c.qw4(i) = w[i];
-                    *c.err = __uint_as_float(h.z);
                     const RTabs tb{a.tables, &a.L};
                     const int dm = tb.bm(r.c[k].bm).dm;
                     infill(tb, c, dm, T, tb.dm(dm).W == T);
                     k_of[tid] = (uint8_t)k;
-                    next_it[tid] = (int)((h.y >> 8) & 0xFF);
+                    next_it[tid] = (uint8_t)(h.y >> 8);
                     pbi_of[tid] = h.x;
                     busy[tid] = 1;
                     filled = tid;
@@ -1035,10 +1036,10 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
             if (dry) break;
             continue;  // every claimed entry was a reservation left empty: claim again
         }
-        if (live) keys[before + __popc(bal & below)] = cand;
-        if (filled >= 0) keys[nlive + new_before + __popc(bnew & below)] = filled;
+        if (live) map[before + __popc(bal & below)] = (uint8_t)cand;
+        if (filled >= 0) map[nlive + new_before + __popc(bnew & below)] = (uint8_t)filled;
         __syncthreads();
-        cand = place < n ? keys[place] : -1;
+        cand = place < n ? map[place] : -1;
         if (cand >= 0) {
             const uint32_t pbi = pbi_of[cand];
             const int k = (int)k_of[cand], it = next_it[cand];
@@ -1046,9 +1047,8 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
             Snap* snap = &a.snaps[(size_t)pbi * kNumCand + k];
             const TexelRow<true> row{reinterpret_cast<const uchar4*>(smem + fl.px + cand * px_row)};
             const PartRow<uint8_t> part{smem + fl.part + cand * part_row};
-            const bool moved = refine_step(a, rec, (int)rec.P, k, row, part, [&](int q, float ps) { return scale_dir(rec.avg[q], ps); },
-                                           Cand(smem, fl, cand), snap, it);
-            next_it[cand] = it + 1;
+            const bool moved = refine_step(a, rec, (int)rec.P, k, row, part, Cand(smem, fl, cand), snap, it);
+            next_it[cand] = (uint8_t)(it + 1);
             if (!moved || it + 1 >= iters) {
                 busy[cand] = 0;  // released: read by the next refill, after the next barrier
                 cand = -1;
