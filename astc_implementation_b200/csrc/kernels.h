@@ -99,14 +99,13 @@ struct KernelArgs {
     int front_threads;        // threads per front CTA: 128, 64 or 32; 0: by footprint and launch size
     int refine_iters;         // refinement iterations (0 selects the reference's 6)
     int fixed;                // 1: FIXED semantics (ASTCB200_FLAG_FIXED_SEMANTICS), 0: the reference's
-    // Refinement tail (null: off): once a refinement CTA has at most spill_live candidates
+    // Refinement tail (null: off): once a refinement CTA has few candidates
     // left, it writes their state here (kTailWords uint4 each, up to tail_cap entries,
     // tail_count[0] reserved so far) and takes its next group; k_refine_tail finishes them,
     // claiming entries from tail_count[1] (zero at its launch).
     uint4* tail;
     int* tail_count;
     int tail_cap;
-    int spill_live;
 };
 constexpr int kTailWords = 13;        // uint4 words of one refinement-tail entry
 constexpr int kTailMaxTexels = 36;    // blocks of more texels are never handed to the tail

@@ -314,6 +314,17 @@ __host__ __device__ inline int refine_pbs(int T, int topn) {
 __host__ __device__ inline int refine_spread(int npb) {
     return npb <= kOneWaveGroups * 4 ? 8 : npb <= kOneWaveGroups * 8 ? 16 : 32;
 }
+// Live candidates at or below which a CTA hands them to the tail (T > 16: u8).  At 4x4, where the sorted
+// warps of a full group are the denser ones, late: proposal search of 900x700 1.90 ms at 64, 2.05 at
+// 96; full search of 436x292 4.14 ms at 32, 4.23 at 64.  Above 16 texels the proposal pass hands over
+// most after the first iteration, which the tail's refilled slots run as densely without holding
+// the groups that wait: 3000x2000 at 6x6 8.54 ms at 64, 7.92 at 96; 1024x1024 mip chain 6.68, 5.83.
+// So does a full search of few waves, whose last one is partly empty: 228x156 at 6x6 (2.7 waves)
+// 2.07 ms at 32, 1.83 at 128; 546x366 (6 waves) 7.53 and 7.50; 654x438 (8.8) 10.3 and 10.9.
+__device__ inline int refine_spill_live(bool u8, bool prop, int ngroups) {
+    if (!u8) return prop ? 64 : 32;
+    return prop ? 96 : ngroups <= 5 * kOneWaveGroups ? kRefineThreads : 32;
+}
 __host__ __device__ inline int refine_group(int T, int cpb, int spread) {  // partitioned blocks per CTA
     const int pbs = refine_pbs(T, cpb), n = kRefineThreads / 32 * spread / cpb;
     return n < 1 ? 1 : n < pbs ? n : pbs;
@@ -328,6 +339,9 @@ __host__ __device__ inline int refine_group(int T, int cpb, int spread) {  // pa
 //   s    [T]      infilled weight of each texel times 16, 0..1024, exact in half precision
 //   qw   [max_w]  grid weights 0..64
 // The best error so far is in the candidate's snapshot.
+// 328 bytes a candidate at 80 texels, with its share of the staged ones 447, so that four CTAs fit on an
+// SM instead of three: k_refine of 1021x765 at 10x8 15.3 -> 13.2 ms.  (Six CTAs of 80 registers
+// instead of five at 4x4: 10.2 and 10.3 ms for 1024x1024.)
 // The infilled weights are kept as sums of grid weight x (contribution x 16), small integers
 // that pass16 updates when it moves a weight; every use of one (pass13's weight s / 1024,
 // pass16's s / 16, pass17's rounded s / 16) is the exact value the passes' own sums of
@@ -794,6 +808,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
     // keeps its candidates then, the proposal pass hands them over for the last iteration only.
     const bool one_wave = ngroups <= kOneWaveGroups;
     bool spill = a.tail != nullptr && T <= kTailMaxTexels && !(one_wave && !a.prop);
+    const int spill_live = refine_spill_live(U8, a.prop != nullptr, ngroups);
     // (the first group's barrier below orders these writes before any read)
     for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
         {
@@ -886,7 +901,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
             }
             if (nlive == 0) break;
             const int rank = before + __popc(bal & ((1u << lane) - 1u));
-            if (spill && it > 0 && nlive <= a.spill_live && (!one_wave || it + 1 >= iters)) {
+            if (spill && it > 0 && nlive <= spill_live && (!one_wave || it + 1 >= iters)) {
                 // Few candidates left: hand them to the tail pass, which runs them densely, and
                 // take the next group instead of holding the CTA for them.
                 if (tid == 0) {

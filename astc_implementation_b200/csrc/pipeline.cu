@@ -109,7 +109,6 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
             CK(cudaMemsetAsync(counts, 0, mlp::kRouteCounters * sizeof(int), s), "reset tail counter");
             a.tail = sc.tail;
             a.tail_cap = (int)std::min<size_t>(sc.cap_tail / (kTailWords * sizeof(uint4)), (size_t)1 << 30);
-            a.spill_live = kSpillLive;
             a.tail_count = counts + 6;  // and its claim counter, counts[7]
             nl = 2;
         }
@@ -174,7 +173,6 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
         // kernel would only lengthen.
         ap.tail = sc.tail;
         ap.tail_cap = (int)std::min<size_t>(sc.cap_tail / (kTailWords * sizeof(uint4)), (size_t)1 << 30);
-        ap.spill_live = kSpillLiveProposal;
         ap.tail_count = counts + 6;  // two free route counters: reservations, claims
     }
     int tails = 0;  // tail launches (timed with their pass's refinement)

@@ -197,3 +197,22 @@ def test_selection_among_equal_logits(bx, by, kmax, kbm):
     for p in (0, 1):  # the single partition, and two partitions (the first classes)
         got = sum(masks[:, 4 * p + i].astype(object) << (64 * i) for i in range(4))
         assert np.all(got == first)
+
+
+@pytest.mark.parametrize("bx,by", [(5, 5), (6, 6)])
+def test_refinement_hands_over_by_launch_size(bx, by):
+    """A launch of one wave keeps its candidates, one of a few waves hands most of them to the
+    tail after the first iteration, a larger one the last of each group: the same blocks."""
+    w, h = 100 * bx - 1, 46 * by - 2  # 4,600 blocks
+    img = synth.make_texture(w, h, 71 + bx)
+    outs, tails = [], []
+    for chunk in (900, 1000, 0):
+        enc = ab.ASTCEncoder(device=0, fixed=True, chunk_blocks=chunk, stage_timing=True)
+        enc.secondaryInit(w, h, bx, by)
+        outs.append(enc.encode(img).reshape(-1, 16))
+        tails.append(int(enc.work_counters()[13]))
+        enc.close()
+    ref, _ = oracle_encode(img[:10 * by], bx, by, True)
+    assert np.array_equal(outs[0][:1000], ref)
+    assert np.array_equal(outs[1], outs[0]) and np.array_equal(outs[2], outs[0])
+    assert tails[0] == 0 and tails[1] > tails[2] > 0
