@@ -309,8 +309,11 @@ __host__ __device__ inline int refine_pbs(int T, int topn) {
 // Candidates a warp runs at a time in a launch of npb partitioned blocks.  A launch of one wave is as long as
 // its slowest warp, and a warp of 32 different candidates runs the union of their paths and
 // the longest of their loops: with 8 or 16 a warp it is shorter, while the waves still hold every
-// group.  Measured (B200, full search of 64x64 at 4x4, 3,328 partitioned
-// blocks): 519 us with 32, 504 with 16; fallback pass of 200x120 at 4x4 188 us with 32, 167 with 8.
+// group, and a candidate's 4 or 2 lanes (8 or 16 apart) share its partitions in passes 13 to 15,
+// of which packing is most of an iteration.  Measured (B200), k_refine of a full search of 64x64 at 4x4 (3,328
+// partitioned blocks) 519 us with 32, 494 with 16, 394 to 421 with 16 and their second lanes; both
+// launches of the proposal search of 200x120 at 4x4 454 us with 8, 365 with 8 and their other lanes.
+// With twice the limits: full search of 256 blocks at 4x4 0.42 -> 0.53 ms, of 1,400 1.12 -> 1.21.
 __host__ __device__ inline int refine_spread(int npb) {
     return npb <= kOneWaveGroups * 4 ? 8 : npb <= kOneWaveGroups * 8 ? 16 : 32;
 }
@@ -486,9 +489,11 @@ __device__ __forceinline__ float4 scale_dir(float4 avg, float ps) {
 // degenerate keep the previous values, which are these), so packing, unpacking, realignment
 // and the final error repeat exactly and can never lower the error: stopping there gives
 // the result of running the remaining iterations.
-template <class Row, class Part>
+// HELP: `lanes` candidates a warp (refine_spread), each run by the 32 / lanes lanes that hold its
+// slot, which must enter together; the first has the result.
+template <bool HELP, class Row, class Part>
 __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, int k, const Row px, const Part pt,
-                            const Cand cs, Snap* snap, const int it) {
+                            const Cand cs, Snap* snap, const int it, const int lanes) {
     const RTabs tb{a.tables, &a.L};
     const int T = a.L.T;
     const CandInit& ci = rec.c[k];
@@ -501,7 +506,10 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     const uint8_t* cu2u = a.tables + a.L.off_cu2u;
     float4 rgbs[4];
     uint2 packed[4], packed_mod[4];
-    if (it == 0) {
+    // this lane's partitions: every qstep-th from q0
+    const int spread = HELP ? lanes : 32, q0 = HELP ? (threadIdx.x & 31) / spread : 0, qstep = 32 / spread, first = threadIdx.x & (spread - 1);
+    const unsigned group = (spread == 32 ? 1u : spread == 16 ? 0x10001u : 0x1010101u) << first;
+    if (it == 0 && q0 == 0) {
 #pragma unroll
         for (int q = 0; q < 4; q++) { cs.ep(2 * q) = rec.ep0[q]; cs.ep(2 * q + 1) = rec.ep1[q]; }
         const uint32_t* src = reinterpret_cast<const uint32_t*>(ci.qw);  // 8-byte aligned in PBRec
@@ -509,7 +517,8 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         for (int w = 0; w < (W + 3) / 4; w++) cs.qw4(w) = src[w];
         infill(tb, cs, bm.dm, T, direct);
     }
-    uint32_t ffmt[4] = {0, 0, 0, 0}, matched = 0, final_q = ci.ql;
+    if (qstep > 1) __syncwarp(group);
+    uint32_t formats = 0, matched = 0, final_q = ci.ql;  // formats: a byte per partition
 
     // The texel's partition endpoints change only with the partition, so they are read again
     // only when it does (never, for one partition).  A decoded channel is floor(v + 1/2) of
@@ -541,7 +550,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
         if (total < snap->err) {  // the best so far (ERR_DEFAULT at first)
             uint4* d = reinterpret_cast<uint4*>(snap);  // 16-byte aligned: 112-byte records
             d[0] = make_uint4(__float_as_uint(total), (uint32_t)ci.bm | final_q << 16 | matched << 24,
-                              ffmt[0] | ffmt[1] << 8 | ffmt[2] << 16 | ffmt[3] << 24, 0u);
+                              formats, 0u);
             d[1] = make_uint4(packed[0].x, packed[0].y, packed[1].x, packed[1].y);
             d[2] = make_uint4(packed[2].x, packed[2].y, packed[3].x, packed[3].y);
             const int nw = (W + 3) / 4;
@@ -558,9 +567,12 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     };
 
     // ---------------- pass13: least-squares endpoints from the current weights
-    int i0 = 0;  // the partition's first texel in partition order
+    int i0 = 0, counted = 0;  // the partition's first texel in partition order
 #pragma unroll 1
-    for (int q = 0; q < P; q++) {
+    for (int q = q0; q < P; q += qstep) {
+        if (HELP)
+#pragma unroll 1
+            for (; counted < q; counted++) i0 += tb.part_count(P, rec.entry, counted);
         const int n = P == 1 ? T : tb.part_count(P, rec.entry, q);
         const float ps = (float)n;
         // the scale direction and its sums are only read by the formats with a scale
@@ -589,6 +601,7 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
             }
         }
         i0 += n;
+        counted = q + 1;
         const float4 colx = cx * cw, coly = cy * cw;
         const float4 lv = mk(ls) * cw, mv = mk(ms) * cw, rv = mk(rs) * cw;
         float4 rg = mk(0.0f);
@@ -632,50 +645,56 @@ __device__ bool refine_step(const KernelArgs& a, const PBRec& rec, const int P, 
     }
     // ---------------- pass14: pack at the trial quant level, then the "mod" level
     {
-        bool all_same = ci.ql != ci.qlm;
-        uint32_t fn[4] = {0, 0, 0, 0};
+        const uint32_t used = 0xFFFFFFFFu >> (8 * (4 - P));
+        auto joined = [&](uint32_t f) {  // of the candidate's lanes
+            for (int o = spread; o < 32; o <<= 1) f |= __shfl_xor_sync(group, f, o);
+            return f;
+        };
 #pragma unroll
         for (int q = 0; q < 4; q++) packed[q] = make_uint2(0u, 0u);
 #pragma unroll 1
-        for (int q = 0; q < P; q++) {
+        for (int q = q0; q < P; q += qstep) {
             const uint4 v = Packer::pack(cu2u, cs.ep(2 * q), cs.ep(2 * q + 1), rgbs[q], ci.fmt[q], ci.ql);
-            const uint32_t f = v.x;
-            fn[0] = q == 0 ? f : fn[0]; fn[1] = q == 1 ? f : fn[1]; fn[2] = q == 2 ? f : fn[2]; fn[3] = q == 3 ? f : fn[3];
+            formats |= v.x << (8 * q);
             packed[q] = make_uint2(v.y, v.z);
-            if (q > 0) all_same = all_same && f == fn[0];
         }
-        bool m = false;
-        if (P >= 2 && all_same) {
-            uint32_t fm[4] = {0, 0, 0, 0};
-            bool same_mod = true;
+        formats = joined(formats);
+        if (P >= 2 && ci.ql != ci.qlm && formats == ((formats & 0xFF) * 0x01010101u & used)) {
+            uint32_t fm = 0;
 #pragma unroll 1
-            for (int q = 0; q < P; q++) {
+            for (int q = q0; q < P; q += qstep) {
                 const uint4 v = Packer::pack(cu2u, cs.ep(2 * q), cs.ep(2 * q + 1), rgbs[q], ci.fmt[q], ci.qlm);
-                const uint32_t f = v.x;
-                fm[0] = q == 0 ? f : fm[0]; fm[1] = q == 1 ? f : fm[1]; fm[2] = q == 2 ? f : fm[2]; fm[3] = q == 3 ? f : fm[3];
+                fm |= v.x << (8 * q);
                 packed_mod[q] = make_uint2(v.y, v.z);
-                if (q > 0 && f != fm[0]) { same_mod = false; break; }
+                if (qstep == 1 && v.x != (fm & 0xFF)) break;
             }
-            if (same_mod) {
-                m = true;
-#pragma unroll
-                for (int q = 0; q < 4; q++) fn[q] = fm[q];
+            fm = joined(fm);
+            if (fm == ((fm & 0xFF) * 0x01010101u & used)) {
+                matched = 1;
+                final_q = ci.qlm;
+                formats = fm;
 #pragma unroll 1
-                for (int q = 0; q < P; q++) packed[q] = packed_mod[q];
+                for (int q = q0; q < P; q += qstep) packed[q] = packed_mod[q];
             }
         }
-        matched = m ? 1 : 0;
-        final_q = m ? ci.qlm : ci.ql;
-#pragma unroll
-        for (int q = 0; q < 4; q++) ffmt[q] = fn[q];
     }
     // ---------------- pass15
 #pragma unroll 1
-    for (int q = 0; q < P; q++) {
+    for (int q = q0; q < P; q += qstep) {
         I4 o0, o1;
-        unpack_endpoints(q == 0 ? ffmt[0] : q == 1 ? ffmt[1] : q == 2 ? ffmt[2] : ffmt[3], packed[q].x, packed[q].y, o0, o1);
+        unpack_endpoints(formats >> (8 * q) & 0xFF, packed[q].x, packed[q].y, o0, o1);
         cs.u(q) = make_uint2((uint32_t)o0.x | (uint32_t)o0.y << 8 | (uint32_t)o0.z << 16 | (uint32_t)o0.w << 24,
                              (uint32_t)o1.x | (uint32_t)o1.y << 8 | (uint32_t)o1.z << 16 | (uint32_t)o1.w << 24);
+    }
+    if (qstep > 1) {  // the rest is the first lane's
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int lane = first + (q & (qstep - 1)) * spread;
+            packed[q].x = __shfl_sync(group, packed[q].x, lane);
+            packed[q].y = __shfl_sync(group, packed[q].y, lane);
+        }
+        __syncwarp(group);
+        if (q0 != 0) return false;
     }
     // ---------------- pass16: move each weight one quant step if that lowers the error
     bool moved = false;
@@ -774,8 +793,9 @@ __device__ __forceinline__ void write_tail(const KernelArgs& a, const Cand& c, u
 
 // CPB: candidate threads per partitioned block (refine_cpb of the launch's top-N), a
 // template parameter so that the full search's instance (8) keeps constant indexing.
-// U8: texels staged as RGBA8 (refine_u8).
-template <int CPB, bool U8>
+// U8: texels staged as RGBA8 (refine_u8).  HELP: launches of few candidates (refine_spread below
+// 32), an instance of its own: with both in one, 1024x1024 at 4x4 took 10.5 ms instead of 10.0.
+template <int CPB, bool U8, bool HELP>
 __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __grid_constant__ KernelArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int T = a.L.T;
@@ -794,7 +814,8 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
     // co-resident warps run the same code), or the proposal pass's work list.
     const int nb = list_blocks(a);
     const int npb = a.pb_list ? pb_total(a) : nb * a.slots;
-    const int spread = refine_spread(npb), pbs = refine_group(T, CPB, spread);
+    if ((refine_spread(npb) < 32) != HELP) return;  // the other instance's launch
+    const int spread = HELP ? refine_spread(npb) : 32, pbs = refine_group(T, CPB, spread);
     const int ngroups = (npb + pbs - 1) / pbs;
     // this thread's place among those that run candidates, the first `spread` lanes of each warp
     const int place = lane < spread ? warp * spread + lane : kRefineThreads;
@@ -927,15 +948,16 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
             if (live) map[rank] = (uint8_t)cand;
             __syncthreads();
             cand = place < nlive ? map[place] : -1;
-            if (cand >= 0) {
-                const int pbl = pos_of[cand] / cpb, k = pos_of[cand] % cpb;
+            const int shared_cand = HELP ? __shfl_sync(0xFFFFFFFFu, cand, lane & (spread - 1)) : cand;
+            if (shared_cand >= 0) {
+                const int pbl = pos_of[shared_cand] / cpb, k = pos_of[shared_cand] % cpb;
                 const uint32_t item = staged[pbl];
                 const size_t pbi = (size_t)((item & 0x07FFFFFFu) - 1) * a.slots + (item >> 27);
                 const PBRec& rec = a.pbrec[pbi];
                 Snap* snap = &a.snaps[pbi * kNumCand + k];
                 const TexelRow<U8> row{reinterpret_cast<const Px*>(smem + fl.px + pbl * px_row)};
                 const PartRow<Pe> part{reinterpret_cast<Pe*>(smem + fl.part + pbl * part_row)};
-                const bool moved = refine_step(a, rec, (int)rec.P, k, row, part, Cand(smem, fl, cand), snap, it);
+                const bool moved = refine_step<HELP>(a, rec, (int)rec.P, k, row, part, Cand(smem, fl, shared_cand), snap, it, spread);
                 if (!moved || it + 1 >= iters) cand = -1;
             }
             // (the next pass's first barrier orders this iteration's state writes before
@@ -1055,16 +1077,18 @@ __global__ void __launch_bounds__(kRefineThreads, kTailCtas) k_refine_tail(const
         if (filled >= 0) map[nlive + new_before + __popc(bnew & below)] = (uint8_t)filled;
         __syncthreads();
         cand = place < n ? map[place] : -1;
-        if (cand >= 0) {
-            const uint32_t pbi = pbi_of[cand];
-            const int k = (int)k_of[cand], it = next_it[cand];
+        const int shared_cand = __shfl_sync(0xFFFFFFFFu, cand, lane & (spread - 1));
+        if (shared_cand >= 0) {
+            const uint32_t pbi = pbi_of[shared_cand];
+            const int k = (int)k_of[shared_cand], it = next_it[shared_cand];
             const PBRec& rec = a.pbrec[pbi];
             Snap* snap = &a.snaps[(size_t)pbi * kNumCand + k];
-            const TexelRow<true> row{reinterpret_cast<const uchar4*>(smem + fl.px + cand * px_row)};
-            const PartRow<uint8_t> part{smem + fl.part + cand * part_row};
-            const bool moved = refine_step(a, rec, (int)rec.P, k, row, part, Cand(smem, fl, cand), snap, it);
-            next_it[cand] = (uint8_t)(it + 1);
-            if (!moved || it + 1 >= iters) {
+            const TexelRow<true> row{reinterpret_cast<const uchar4*>(smem + fl.px + shared_cand * px_row)};
+            const PartRow<uint8_t> part{smem + fl.part + shared_cand * part_row};
+            const bool moved = spread == 32 ? refine_step<false>(a, rec, (int)rec.P, k, row, part, Cand(smem, fl, shared_cand), snap, it, 32)
+                                                : refine_step<true>(a, rec, (int)rec.P, k, row, part, Cand(smem, fl, shared_cand), snap, it, spread);
+            if (cand >= 0) next_it[cand] = (uint8_t)(it + 1);
+            if (cand >= 0 && (!moved || it + 1 >= iters)) {
                 busy[cand] = 0;  // released: read by the next refill, after the next barrier
                 cand = -1;
             }
@@ -1675,6 +1699,15 @@ size_t refine_smem_bytes(const TableLayout& L, int topn) {
     return (size_t)refine_layout(L.T, L.max_w, refine_pbs(L.T, topn), refine_u8(L.T), false).total;
 }
 
+template <bool U8, bool HELP>
+static auto refine_kernel(int cpb) {
+    return cpb == 1 ? k_refine<1, U8, HELP> : cpb == 2 ? k_refine<2, U8, HELP> : cpb == 4 ? k_refine<4, U8, HELP> : k_refine<8, U8, HELP>;
+}
+static auto refine_kernel(int cpb, bool u8, bool help) {
+    return u8 ? help ? refine_kernel<true, true>(cpb) : refine_kernel<true, false>(cpb)
+              : help ? refine_kernel<false, true>(cpb) : refine_kernel<false, false>(cpb);
+}
+
 size_t refine_smem_bytes(const TableLayout& L) {  // the largest over the refinement top-N
     size_t m = 0;
     for (int topn : {1, 2, 4, 8}) m = std::max(m, refine_smem_bytes(L, topn));
@@ -1701,29 +1734,28 @@ cudaError_t configure_kernels(const TableLayout& L) {
     for (int i = 0; i < 4; i++) m[i] = std::max(m[i], need[i]);
     e = configure_search_kernels(m[0], m[1]);
     if (e != cudaSuccess) return e;
-    for (auto f : {k_refine<1, false>, k_refine<2, false>, k_refine<4, false>, k_refine<8, false>, k_refine<1, true>,
-                   k_refine<2, true>, k_refine<4, true>, k_refine<8, true>})
+    using Kernel = void (*)(KernelArgs);
+    Kernel refine[16];
+    for (int i = 0; i < 16; i++) refine[i] = refine_kernel(1 << (i & 3), i & 4, i & 8);
+    for (Kernel f : refine)
         if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m[2])) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(k_extend, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m[3])) != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_refine_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)refine_tail_smem_bytes(kTailMaxTexels, kTailMaxTexels));
 }
 
+// A launch over a list, whose length the device knows, queues both instances where it may be either's;
+// the one it isn't returns at once (2 us).
 cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s) {
     const int cpb = refine_cpb(a.topn);
-    const int npb = a.nblocks * a.slots, pbs = refine_group(a.L.T, cpb, refine_spread(npb));
-    int grid = (npb + pbs - 1) / pbs;
-    if (a.block_list) grid = std::min(grid, kListGridRefine);
+    const int npb = a.nblocks * a.slots;  // of a list: at most
     const size_t smem = refine_smem_bytes(a.L, cpb);
-    if (refine_u8(a.L.T)) {
-        if (cpb == 1) k_refine<1, true><<<grid, kRefineThreads, smem, s>>>(a);
-        else if (cpb == 2) k_refine<2, true><<<grid, kRefineThreads, smem, s>>>(a);
-        else if (cpb == 4) k_refine<4, true><<<grid, kRefineThreads, smem, s>>>(a);
-        else k_refine<8, true><<<grid, kRefineThreads, smem, s>>>(a);
-    } else {
-        if (cpb == 1) k_refine<1, false><<<grid, kRefineThreads, smem, s>>>(a);
-        else if (cpb == 2) k_refine<2, false><<<grid, kRefineThreads, smem, s>>>(a);
-        else if (cpb == 4) k_refine<4, false><<<grid, kRefineThreads, smem, s>>>(a);
-        else k_refine<8, false><<<grid, kRefineThreads, smem, s>>>(a);
+    const bool list = a.block_list || a.pb_list;
+    for (int help = 0; help < 2; help++) {
+        if ((refine_spread(npb) < 32) != (help != 0) && !(list && help)) continue;
+        const int spread = help ? std::min(refine_spread(npb), 16) : 32, pbs = refine_group(a.L.T, cpb, spread);
+        int grid = (npb + pbs - 1) / pbs;
+        if (list) grid = std::min(grid, help ? kOneWaveGroups : kListGridRefine);
+        refine_kernel(cpb, refine_u8(a.L.T), help != 0)<<<grid, kRefineThreads, smem, s>>>(a);
     }
     return cudaGetLastError();
 }
