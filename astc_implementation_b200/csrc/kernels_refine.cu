@@ -4,8 +4,8 @@
 //                  driven by compression_pipeline.cpp:473-484: least-squares
 //                  endpoints, colour endpoint packing (every LDR encoding the
 //                  reference tries), unpacking, weight realignment, final
-//                  error with a best-so-far snapshot.  One thread owns one
-//                  candidate for all six iterations; the 8 candidates of a
+//                  error with a best-so-far snapshot.  One thread runs one
+//                  candidate's iteration; the 8 candidates of a
 //                  partitioned block share a CTA and its staged texels.
 //   k_select_pack  pass18 plus the host argmin over candidates and partition
 //                  counts (compression_pipeline.cpp:500-519), then the ASTC

@@ -199,6 +199,17 @@ def test_selection_among_equal_logits(bx, by, kmax, kbm):
         assert np.all(got == first)
 
 
+@pytest.mark.parametrize("fixed", [False, True])
+@pytest.mark.parametrize("bx,by", [(4, 4), (8, 6)])
+@pytest.mark.parametrize("blocks_x,blocks_y", [(227, 1),   # 2,951 partitioned blocks: 8 candidates a warp, four lanes each
+                                               (12, 19),   # 2,964: 16, two lanes each
+                                               (35, 13),   # 5,915: 16
+                                               (24, 19)])  # 5,928: 32
+def test_refinement_lanes_by_launch_size(bx, by, blocks_x, blocks_y, fixed):
+    img = synth.make_texture(bx * blocks_x, by * blocks_y - 1, 83 + blocks_x)
+    check_full_search(img, bx, by, fixed)
+
+
 @pytest.mark.parametrize("bx,by", [(5, 5), (6, 6)])
 def test_refinement_hands_over_by_launch_size(bx, by):
     """A launch of one wave keeps its candidates, one of a few waves hands most of them to the
