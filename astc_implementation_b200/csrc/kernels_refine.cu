@@ -37,8 +37,6 @@ enum {
 
 struct I4 { int32_t x, y, z, w; };
 __device__ __forceinline__ int32_t ic(const I4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
-__device__ __forceinline__ I4 ivec(float4 v) { return {f2i(v.x), f2i(v.y), f2i(v.z), f2i(v.w)}; }
-__device__ __forceinline__ float4 rnev(float4 v) { return make_float4(rintf(v.x), rintf(v.y), rintf(v.z), rintf(v.w)); }
 __device__ __forceinline__ int32_t shl1(int32_t v) { return (int32_t)((uint32_t)v << 1); }
 
 // x / 257 for an endpoint clamped to [0, 65535], rounded to nearest: the product with the
