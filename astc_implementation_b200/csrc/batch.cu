@@ -137,12 +137,8 @@ int prepare(astcb200_ctx* ctx, const Plan& p, uint32_t chunk, uint32_t streams, 
 // Device buffers a launch sequence with `streams` streams bakes in.
 std::vector<const void*> baked_buffers(const astcb200_ctx* ctx, uint32_t streams) {
     std::vector<const void*> v{ctx->d_segs, ctx->d_counts, ctx->d_mlp_error};
-    for (uint32_t i = 0; i < streams; i++) {
-        const Scratch& sc = ctx->bscratch[i];
-        for (const void* q : {(const void*)sc.picks, (const void*)sc.pbrec, (const void*)sc.snaps, (const void*)sc.logits,
-                              (const void*)sc.lists, (const void*)sc.prop, (const void*)sc.masks, (const void*)sc.pbl, (const void*)sc.full_err})
-            v.push_back(q);
-    }
+    for (uint32_t i = 0; i < streams; i++)
+        for (const void* q : ctx->bscratch[i].buffers()) v.push_back(q);
     return v;
 }
 

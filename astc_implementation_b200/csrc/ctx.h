@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <map>
 #include <string>
 #include <vector>
@@ -38,7 +39,13 @@ struct Scratch {
     uint32_t* pbl = nullptr;       // [4][blocks * kMaxProposals] partitioned-block work lists
     uint4* tail = nullptr;         // refinement-tail entries (kTailWords words each)
     size_t cap_logits = 0, cap_lists = 0, cap_prop = 0, cap_masks = 0, cap_pbl = 0, cap_ferr = 0, cap_tail = 0;
+
+    // Every buffer above: what is freed with the scratch, and what a captured launch sequence
+    // bakes in (any of them may move when a later call needs more).
+    static constexpr size_t kBuffers = 10;
+    std::array<void*, kBuffers> buffers() const { return {picks, pbrec, snaps, logits, lists, full_err, prop, masks, pbl, tail}; }
 };
+static_assert(sizeof(Scratch) == Scratch::kBuffers * (sizeof(void*) + sizeof(size_t)), "Scratch::buffers lists every buffer");
 // Refinement-tail entries per block of a chunk (a CTA that finds the tail full finishes its
 // candidates itself).
 constexpr size_t kTailPerBlock = 4;       // proposal search (about 2.5 spilled per 4x4 block)

@@ -183,3 +183,18 @@ def test_batch_argument_errors(enc):
     with pytest.raises(ab.ASTCError) as e:
         enc.encode_batch([])
     assert e.value.status == ab.BAD_ARG
+
+
+def test_batch_graphs_after_one_buffer_moved():
+    """A large 8x8 batch sizes every shared buffer but the refinement tail, which only 4x4 batches use: the
+    medium 4x4 batch then moves the tail alone, and the small one's graph must not be replayed with
+    the old one."""
+    enc = ab.ASTCEncoder(device=0, fixed=True)
+    large = [(synth.make_texture(480, 400, 21), 8, 8)]   # 3,000 blocks
+    small = [(synth.make_texture(160, 120, 22), 4, 4)]   # 1,200 blocks: more than one wave, so its tail is used
+    medium = [(synth.make_texture(240, 160, 23), 4, 4)]  # 2,400 blocks
+    got = [enc.encode_batch(t) for t in (large, small, medium, small)]
+    for tex, outs in zip((large, small, medium, small), got):
+        for (img, bx, by), o in zip(tex, outs):
+            assert np.array_equal(o, single(enc, img, bx, by))
+    enc.close()
