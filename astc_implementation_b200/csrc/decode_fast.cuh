@@ -17,7 +17,7 @@ namespace {
 // colours by value, bits | trits << 4 | quints << 5 of the quantisation methods, bits of n
 // weights, and the finest colour method of n values in b bits (0: none an LDR block may use),
 // all from the decoder's own functions at compile time.
-struct ValueTables {
+struct alignas(16) ValueTables {  // k_decode copies them as words
     uint16_t trits[256], quints[128];
     uint8_t weight[12][32];
 };

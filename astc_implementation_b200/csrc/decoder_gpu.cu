@@ -19,6 +19,8 @@
 // this replaces, took 463 us a call there; this takes 90 us.
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
 #include "astcb200.h"
 #include "decode_fast.cuh"
 #include "tables.h"
@@ -38,11 +40,13 @@ __global__ void __launch_bounds__(kDecodeThreads) k_decode(const uint8_t* __rest
                                                             int nbx, int nby, int cols, int groups_x, uchar4* __restrict__ out,
                                                             const uchar4* __restrict__ ref, unsigned long long* __restrict__ sse) {
     __shared__ __align__(16) Stage<kDecodeBlocks> s;
-    __shared__ __align__(4) ValueTables tables;
+    __shared__ ValueTables tables;
     const int tid = threadIdx.x;
     const int rows = kDecodeBlocks / cols;
     const int gx = (int)(blockIdx.x % (unsigned)groups_x) * cols, gy = (int)(blockIdx.x / (unsigned)groups_x) * rows;
     {
+        static_assert(alignof(DecodeTables) % 4 == 0 && offsetof(DecodeTables, values) % 4 == 0 && sizeof(ValueTables) % 4 == 0,
+                      "the tables are copied as words");
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&g_tables.values);
         uint32_t* dst = reinterpret_cast<uint32_t*>(&tables);
         for (int i = tid; i < (int)sizeof(ValueTables) / 4; i += kDecodeThreads) dst[i] = src[i];
