@@ -245,7 +245,9 @@ class ASTCEncoder:
         return picks, recs, snaps
 
     def encode_device(self, d_rgba8, d_out_blocks, stream=0):
-        """Queues the search on device buffers (integer device addresses); does not wait."""
+        """Queues the search on device buffers (integer device addresses) on `stream`; does not
+        wait.  0 is the context's own stream, ordered with the default stream only through
+        astc_containers_device, decode_device and decode_error_device without a stream."""
         lib = load_library()
         _check(lib.astcb200_encode_device(self._ctx, ctypes.c_void_p(d_rgba8), ctypes.c_void_p(d_out_blocks),
                                           ctypes.c_void_p(stream or None)), self._ctx)
@@ -277,7 +279,7 @@ class ASTCEncoder:
 
     def encode_batch_device(self, textures, stream=0):
         """Queues a batch of device textures [(d_rgba8, w, h, bx, by, d_out, out_len), ...]
-        (integer device addresses) on `stream`; does not wait."""
+        (integer device addresses) on `stream` (0 as for encode_device); does not wait."""
         arr = self._device_textures(textures)
         _check(load_library().astcb200_encode_batch_device(self._ctx, arr, len(textures), ctypes.c_void_p(stream or None)),
                self._ctx)

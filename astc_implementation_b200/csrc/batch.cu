@@ -247,7 +247,10 @@ int astcb200_encode_batch_device(astcb200_ctx* ctx, const astcb200_texture* text
     if (rc) return rc;
     cudaStream_t s = cuda_stream ? (cudaStream_t)cuda_stream : ctx->stream;
     rc = launch_plan(ctx, p, s, default_tuning(ctx, p), !(ctx->cfg.flags & ASTCB200_FLAG_NO_GRAPH), nullptr);
-    return rc || cuda_stream ? rc : order_default_stream(ctx);
+    if (rc || cuda_stream) return rc;
+    for (uint32_t i = 0; i < n; i++) add_streamless(ctx->streamless, textures[i].out_blocks, blocks_of(textures[i]) * 16);
+    CK(record_streamless(ctx->streamless, s), "encode event");
+    return ASTCB200_OK;
 }
 
 int astcb200_encode_batch(astcb200_ctx* ctx, const astcb200_texture* textures, uint32_t n, astcb200_stats* stats) {

@@ -28,29 +28,21 @@ int cuda_fail(astcb200_ctx* c, cudaError_t e, const char* what) {
 int wait_stream(astcb200_ctx* ctx, cudaStream_t s) {
     if (ctx->cfg.timeout_ms == 0) {
         CK(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        if (s == ctx->stream) clear_streamless(ctx->streamless);
         return ASTCB200_OK;
     }
     const auto t0 = std::chrono::steady_clock::now();
     for (;;) {
         cudaError_t e = cudaStreamQuery(s);
-        if (e == cudaSuccess) return ASTCB200_OK;
+        if (e == cudaSuccess) {
+            if (s == ctx->stream) clear_streamless(ctx->streamless);
+            return ASTCB200_OK;
+        }
         if (e != cudaErrorNotReady) return cuda_fail(ctx, e, "cudaStreamQuery");
         const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         if (ms > ctx->cfg.timeout_ms) { ctx->err = "device work did not finish within timeout_ms"; return ASTCB200_TIMEOUT; }
         std::this_thread::sleep_for(std::chrono::microseconds(200));
     }
-}
-
-int order_default_stream(astcb200_ctx* ctx) {
-    cudaStreamCaptureStatus st;
-    if (cudaStreamIsCapturing(cudaStreamLegacy, &st) != cudaSuccess) {  // a capture forbids its use: no ordering then
-        cudaGetLastError();
-        return ASTCB200_OK;
-    }
-    if (!ctx->ev_order) CK(cudaEventCreateWithFlags(&ctx->ev_order, cudaEventDisableTiming), "cudaEventCreate");
-    CK(cudaEventRecord(ctx->ev_order, ctx->stream), "order event");
-    CK(cudaStreamWaitEvent(cudaStreamLegacy, ctx->ev_order, 0), "order wait");
-    return ASTCB200_OK;
 }
 
 int HostResults::reserve(astcb200_ctx* ctx) {
@@ -193,6 +185,7 @@ int astcb200_create(astcb200_ctx** out, int device_ordinal, const astcb200_confi
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
+    if (e == cudaSuccess) e = register_streamless(ctx->streamless);
     if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "create"); astcb200_destroy(ctx); return rc; }
     *out = ctx;
     return ASTCB200_OK;
@@ -211,7 +204,7 @@ int astcb200_destroy(astcb200_ctx* ctx) {
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
-    if (ctx->ev_order) cudaEventDestroy(ctx->ev_order);
+    release_streamless(ctx->streamless);
     for (cudaEvent_t e : ctx->stage_ev) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -254,7 +247,10 @@ int astcb200_encode_device(astcb200_ctx* ctx, const uint8_t* d_rgba8, uint8_t* d
     ASTCB200_DEVICE_SCOPE(ctx);
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     const int rc = run_search(ctx, d_rgba8, d_out, nullptr, s, nullptr);
-    return rc || stream ? rc : order_default_stream(ctx);
+    if (rc || stream) return rc;
+    add_streamless(ctx->streamless, d_out, (size_t)ctx->nblocks * 16);
+    CK(record_streamless(ctx->streamless, s), "encode event");
+    return ASTCB200_OK;
 }
 
 static int encode_host(astcb200_ctx* ctx, const uint8_t* rgba8, uint8_t* out_blocks, uint32_t* symbolic, astcb200_stats* stats) {
@@ -425,6 +421,7 @@ int astcb200_astc_containers_device(const astcb200_astc_image* images, uint32_t 
         const astcb200_astc_image& m = images[i];
         const size_t blocks = (size_t)((m.width + m.block_x - 1) / m.block_x) * ((m.height + m.block_y - 1) / m.block_y);
         astc_header(m.block_x, m.block_y, m.width, m.height, m.host_out);
+        if (await_streamless(m.d_blocks, blocks * 16, s) != cudaSuccess) return ASTCB200_CUDA_ERROR;
         if (cudaMemcpyAsync(m.host_out + 16, m.d_blocks, blocks * 16, cudaMemcpyDeviceToHost, s) != cudaSuccess)
             return ASTCB200_CUDA_ERROR;
     }

@@ -12,6 +12,7 @@
 #include "device_guard.h"
 #include "kernels.h"
 #include "mlp.h"
+#include "streamless.h"
 #include "tables.h"
 
 namespace astcb200 {
@@ -125,7 +126,7 @@ struct astcb200_ctx {
     uint32_t* d_sym = nullptr;
     size_t sym_cap = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t ev_order = nullptr;                 // device encodes on `stream`, for the default stream
+    astcb200::StreamlessOutputs streamless;         // device encodes on `stream`
     std::vector<cudaEvent_t> stage_ev;  // kStageIntervals + 1 per chunk
     std::vector<int8_t> stage_kind;     // kStageIntervals per chunk
     int stage_chunks = 0;               // chunks recorded by the last encode
@@ -161,9 +162,6 @@ namespace astcb200 {
 
 int cuda_fail(astcb200_ctx* c, cudaError_t e, const char* what);
 int wait_stream(astcb200_ctx* ctx, cudaStream_t s);
-// After a device encode was queued on the context's own stream (the caller gave none): later work
-// on the legacy default stream, where a caller without a stream goes on, waits for it.
-int order_default_stream(astcb200_ctx* ctx);
 int get_tables(astcb200_ctx* ctx, int bx, int by, const FootTables** out);
 int ensure_scratch(astcb200_ctx* ctx, Scratch& sc, size_t blocks, int slots);
 // Scratch for `blocks` blocks per chunk of footprint ft (proposal buffers when it is pruned).

@@ -23,6 +23,7 @@
 
 #include "astcb200.h"
 #include "decode_fast.cuh"
+#include "streamless.h"
 #include "tables.h"
 
 namespace astcb200 {
@@ -140,6 +141,7 @@ int launch_decode(uint32_t bx, uint32_t by, uint32_t dx, uint32_t dy, const uint
     const int nbx = (int)((dx + bx - 1) / bx), nby = (int)((dy + by - 1) / by);
     const int cols = nbx < kDecodeBlocks ? nbx : kDecodeBlocks, rows = kDecodeBlocks / cols;
     const int groups_x = (nbx + cols - 1) / cols, groups_y = (nby + rows - 1) / rows;
+    if (await_streamless(blocks, (size_t)nbx * nby * 16, s) != cudaSuccess) return ASTCB200_CUDA_ERROR;
     k_decode<kError><<<(unsigned)groups_x * (unsigned)groups_y, kDecodeThreads, 0, s>>>(
         blocks, (int)bx, (int)by, (int)dx, (int)dy, nbx, nby, cols, groups_x,
         reinterpret_cast<uchar4*>(out), reinterpret_cast<const uchar4*>(ref), sse);

@@ -112,9 +112,13 @@ int astcb200_encode(astcb200_ctx* ctx, const uint8_t* rgba8, uint8_t* out_blocks
                     astcb200_stats* stats);
 
 /* Same search with both buffers already in device memory of the context's GPU; work is
- * queued on cuda_stream (a cudaStream_t, or NULL for the context's stream, which later work on
- * the legacy default stream then waits for) and the call
- * returns without waiting.  d_rgba8 must be 4-byte aligned, d_out_blocks 16-byte aligned. */
+ * queued on cuda_stream (a cudaStream_t, or NULL for the context's stream) and the call
+ * returns without waiting.  d_rgba8 must be 4-byte aligned, d_out_blocks 16-byte aligned.
+ * The context's stream is not ordered with the legacy default stream: with NULL, the image must
+ * be complete before the call, and of the later work only this library's readers of the blocks
+ * on the default stream (astcb200_astc_containers_device, astcb200_decode_device and
+ * astcb200_decode_error_device with a NULL stream) wait for the encode; before any other use
+ * synchronise the device, or pass a stream. */
 int astcb200_encode_device(astcb200_ctx* ctx, const uint8_t* d_rgba8, uint8_t* d_out_blocks, void* cuda_stream);
 
 /* Encode without allocating (no counterpart in the reference).  For callers that cannot
@@ -159,8 +163,8 @@ int astcb200_encode_batch(astcb200_ctx* ctx, const astcb200_texture* textures, u
 
 /* Same with rgba8 and out_blocks in device memory of the context's GPU (rgba8 4-byte
  * aligned, out_blocks 16-byte aligned); queued on cuda_stream (NULL = the context's
- * stream, which later work on the legacy default stream then waits for), no wait.  The textures array itself is host memory and is consumed before the
- * call returns. */
+ * stream, ordered as for astcb200_encode_device), no wait.  The textures array itself is host
+ * memory and is consumed before the call returns. */
 int astcb200_encode_batch_device(astcb200_ctx* ctx, const astcb200_texture* textures, uint32_t n, void* cuda_stream);
 
 /* Launch configuration of a batch shape, chosen by astcb200_autotune_batch. */
