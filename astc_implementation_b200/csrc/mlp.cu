@@ -497,15 +497,16 @@ __global__ void __launch_bounds__(kSelectWarps * 32, 3) k_select(const __grid_co
     int used = 0;
     uint16_t picks[kMaxProposals];
     if (live) {
-        // the softmax maximum and each lane's best partitioning logit
+        // the softmax maximum and each lane's best partitioning logit (absent classes: -infinity, which
+        // adds 0 to the sum whatever the maximum is)
         float v[kHeld], mx = -3.0e38f, lm = -3.0e38f;
 #pragma unroll
-        for (int i = 0; i < kHeld; i++) { const int c = lane + 32 * i; v[i] = c <= S.p1 ? z[c] : -3.0e38f; }
+        for (int i = 0; i < kHeld; i++) { const int c = lane + 32 * i; v[i] = c <= S.p1 ? z[c] : -INFINITY; }
 #pragma unroll
         for (int i = 0; i < kHeld; i++) { mx = fmaxf(mx, v[i]); if (lane + 32 * i != S.p1) lm = fmaxf(lm, v[i]); }
         for (int c = lane + 32 * kHeld; c <= S.p1; c += 32) { const float x = z[c]; mx = fmaxf(mx, x); if (c < S.p1) lm = fmaxf(lm, x); }
         mx = warp_max(mx);
-        float se = 0.0f;  // (absent classes add 0)
+        float se = 0.0f;
 #pragma unroll
         for (int i = 0; i < kHeld; i++) se += __expf(v[i] - mx);
         for (int c = lane + 32 * kHeld; c <= S.p1; c += 32) se += __expf(z[c] - mx);

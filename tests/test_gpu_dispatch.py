@@ -227,3 +227,23 @@ def test_refinement_hands_over_by_launch_size(bx, by):
     assert np.array_equal(outs[0][:1000], ref)
     assert np.array_equal(outs[1], outs[0]) and np.array_equal(outs[2], outs[0])
     assert tails[0] == 0 and tails[1] > tails[2] > 0
+
+
+@pytest.mark.parametrize("bx,by", [(4, 4), (6, 6)])
+@pytest.mark.parametrize("logit,route", [(-3.2e38, 1), (-2.0e38, 0)])
+def test_selection_with_logits_near_the_lowest_value(bx, by, logit, route):
+    """Below -3e38 no class counts, the softmax is 0 / 0 and the block takes the full search even at
+    threshold 0; the places a lane holds beyond the last class must not stand in for one."""
+    from astc_implementation_b200 import proposal
+    lay = proposal.Layout(bx, by)
+    net = {"w1": np.zeros((256, lay.inputs)), "b1": np.zeros(256), "w2": np.zeros((256, 256)), "b2": np.zeros(256),
+           "w3": np.zeros((lay.outputs, 256)), "b3": np.full(lay.outputs, logit)}
+    enc = ab.ASTCEncoder(device=0, fixed=True)
+    enc.set_proposal_net(net, bx, by)
+    enc.set_pruning(True, max_partitionings=2, block_modes=5, coverage=1.0, threshold=0.0)
+    w, h = 12 * bx, 9 * by - 1
+    enc.secondaryInit(w, h, bx, by)
+    got, picks, _ = enc.proposal_selection(synth.make_texture(w, h, 3))
+    enc.close()
+    assert np.all(got == route)
+    assert np.all(picks[:, 0] == (0 if route else 2))
