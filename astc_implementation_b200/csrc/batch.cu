@@ -121,10 +121,9 @@ int prepare(astcb200_ctx* ctx, const Plan& p, uint32_t chunk, uint32_t streams, 
         ctx->join_ev.push_back(e2);
     }
     if (ctx->bscratch.size() < streams) ctx->bscratch.resize(streams);
-    const size_t need = std::min<size_t>(chunk, p.max_group_blocks);
     for (uint32_t i = 0; i < streams; i++)
-        for (const Group& g : p.groups) {  // sized for the largest need over the footprints
-            int rc = ensure_chunk_scratch(ctx, ctx->bscratch[i], need, g.ft);
+        for (const Group& g : p.groups) {  // sized for the largest need over the queues
+            int rc = ensure_chunk_scratch(ctx, ctx->bscratch[i], std::min<size_t>(chunk, g.full_only ? g.nblocks : p.max_group_blocks), g.ft, g.full_only);
             if (rc) return rc;
         }
     size_t units = 0;

@@ -118,7 +118,8 @@ int run_search(astcb200_ctx* ctx, const uint8_t* d_img, uint8_t* d_out, uint32_t
     a.out_blocks = d_out; a.symbolic = d_sym;
     const bool timing = (ctx->cfg.flags & ASTCB200_FLAG_STAGE_TIMING) != 0;
     const int nchunks = (int)((ctx->nblocks + ctx->chunk - 1) / ctx->chunk);
-    int rc = ensure_chunk_scratch(ctx, ctx->scratch, std::min<size_t>(ctx->chunk, ctx->nblocks), ctx->cur);
+    const bool full_only = (uint64_t)ctx->width * ctx->height < (uint64_t)mlp::kMinProposalTexels;
+    int rc = ensure_chunk_scratch(ctx, ctx->scratch, std::min<size_t>(ctx->chunk, ctx->nblocks), ctx->cur, full_only);
     if (rc) return rc;
     if ((rc = begin_routes(ctx, nchunks, s))) return rc;
     constexpr int E = kStageIntervals + 1;
@@ -140,8 +141,7 @@ int run_search(astcb200_ctx* ctx, const uint8_t* d_img, uint8_t* d_out, uint32_t
         a.block_first = (int)first;
         a.nblocks = (int)std::min<uint32_t>(ctx->chunk, ctx->nblocks - first);
         if ((rc = enqueue_chunk(ctx, a, ctx->cur, ctx->scratch, s, timing ? &ctx->stage_ev[(size_t)E * c] : nullptr,
-                                timing ? &ctx->stage_kind[(size_t)kStageIntervals * c] : nullptr, &n,
-                                (uint64_t)ctx->width * ctx->height < (uint64_t)mlp::kMinProposalTexels)))
+                                timing ? &ctx->stage_kind[(size_t)kStageIntervals * c] : nullptr, &n, full_only)))
             return rc;
     }
     if (launches) *launches = n;

@@ -47,10 +47,6 @@ struct Scratch {
     std::array<void*, kBuffers> buffers() const { return {picks, pbrec, snaps, logits, lists, full_err, prop, masks, pbl, tail}; }
 };
 static_assert(sizeof(Scratch) == Scratch::kBuffers * (sizeof(void*) + sizeof(size_t)), "Scratch::buffers lists every buffer");
-// Refinement-tail entries per block of a chunk (a CTA that finds the tail full finishes its
-// candidates itself).
-constexpr size_t kTailPerBlock = 4;       // proposal search (about 2.5 spilled per 4x4 block)
-constexpr size_t kTailPerBlockFull = 16;  // full search (104 candidates per block)
 
 // A footprint's proposal network on the device.
 struct NetDev {
@@ -164,8 +160,9 @@ int cuda_fail(astcb200_ctx* c, cudaError_t e, const char* what);
 int wait_stream(astcb200_ctx* ctx, cudaStream_t s);
 int get_tables(astcb200_ctx* ctx, int bx, int by, const FootTables** out);
 int ensure_scratch(astcb200_ctx* ctx, Scratch& sc, size_t blocks, int slots);
-// Scratch for `blocks` blocks per chunk of footprint ft (proposal buffers when it is pruned).
-int ensure_chunk_scratch(astcb200_ctx* ctx, Scratch& sc, size_t blocks, const FootTables* ft);
+// Scratch for `blocks` blocks per chunk of footprint ft (proposal buffers when it is pruned and the
+// textures are not full_only, as for enqueue_chunk).
+int ensure_chunk_scratch(astcb200_ctx* ctx, Scratch& sc, size_t blocks, const FootTables* ft, bool full_only);
 const NetDev* net_for(const astcb200_ctx* ctx, const FootTables* ft);  // null: full search
 // Room for `chunks` route counters; resets the per-call counter index and (on stream s)
 // the inference kernel's give-up flag.

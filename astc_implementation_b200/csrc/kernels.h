@@ -94,7 +94,7 @@ struct KernelArgs {
     // Work counters (null: not counted): [0..3] partitioned blocks searched by the front,
     // by P; [4] decimation modes and [5] block modes it evaluated; [6..9] candidates
     // refined, by P; [10..12] partition searches, P = 2..4; [13] candidates the refinement
-    // handed to its tail pass.
+    // offered to its tail pass, [14] those of them the tail had room for.
     unsigned long long* work;
     int front_threads;        // threads per front CTA: 128, 64 or 32; 0: by footprint and launch size
     int refine_iters;         // refinement iterations (0 selects the reference's 6)
@@ -108,6 +108,11 @@ struct KernelArgs {
     int tail_cap;
 };
 constexpr int kTailWords = 13;        // uint4 words of one refinement-tail entry
+// Refinement-tail entries per block of a chunk (a CTA that finds the tail full finishes its
+// candidates, and those of its later groups, itself).  Offered on measured textures: proposal search 1.7 to
+// 3.2 a block at 4x4, 0.6 to 1.6 at 6x6; full search 9 to 18; a full search that offers every candidate
+// after its first iteration (refine_few_waves) 40 to 48 of 104.
+constexpr size_t kTailPerBlock = 4, kTailPerBlockFull = 16, kTailPerBlockAll = kSlotsPerBlock * kNumCand;
 constexpr int kTailMaxTexels = 36;    // blocks of more texels are never handed to the tail
 constexpr int kWorkCounters = 16;
 
@@ -206,6 +211,10 @@ __device__ __forceinline__ uint4* block_dst(const KernelArgs& a, int blk) {
 // Shared-memory sizes the launches need for one footprint.
 size_t front_smem_bytes(const TableLayout& L);
 size_t refine_smem_bytes(const TableLayout& L);
+
+// Tail entries of a full search's launch over nblocks blocks, and of any of up to nblocks.
+size_t refine_tail_entries(const TableLayout& L, int nblocks);
+size_t refine_tail_entries_up_to(const TableLayout& L, int nblocks);
 size_t search_smem_bytes(const TableLayout& L);
 
 cudaError_t configure_kernels(const TableLayout& L);

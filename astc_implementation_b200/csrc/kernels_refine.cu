@@ -320,16 +320,20 @@ __host__ __device__ inline int refine_spread(int npb) {
 // 96; full search of 436x292 4.14 ms at 32, 4.23 at 64.  Above 16 texels the proposal pass hands over
 // most after the first iteration, which the tail's refilled slots run as densely without holding
 // the groups that wait: 3000x2000 at 6x6 8.54 ms at 64, 7.92 at 96; 1024x1024 mip chain 6.68, 5.83.
-// So does a full search of few waves, whose last one is partly empty: 228x156 at 6x6 (2.7 waves)
-// 2.07 ms at 32, 1.83 at 128; 546x366 (6 waves) 7.53 and 7.50; 654x438 (8.8) 10.3 and 10.9.
+// So does a full search of few waves, whose last one is partly empty, with room in the tail for every
+// candidate: at 6x6 228x156 (1.1 waves) 2.06 ms at 32, 1.81 at 128; 300x180 (1.6) 2.69 and 2.43; 420x240
+// (3.1) 4.17 and 4.01; 540x300 (4.9) 6.23 and 6.15; 600x360 (6.6) 7.97 and 7.97; 660x480 (9.7) 11.27 and
+// 11.41.  (With room for 16 a block, which most CTAs find full, 2.09, 2.74, 4.34 and 6.48 for the first four.)
+__host__ __device__ inline bool refine_few_waves(bool u8, int ngroups) { return u8 && ngroups <= 5 * kOneWaveGroups; }
 __device__ inline int refine_spill_live(bool u8, bool prop, int ngroups) {
     if (!u8) return prop ? 64 : 32;
-    return prop ? 96 : ngroups <= 5 * kOneWaveGroups ? kRefineThreads : 32;
+    return prop ? 96 : refine_few_waves(u8, ngroups) ? kRefineThreads : 32;
 }
 __host__ __device__ inline int refine_group(int T, int cpb, int spread) {  // partitioned blocks per CTA
     const int pbs = refine_pbs(T, cpb), n = kRefineThreads / 32 * spread / cpb;
     return n < 1 ? 1 : n < pbs ? n : pbs;
 }
+__host__ __device__ inline int refine_groups(int npb, int pbs) { return (npb + pbs - 1) / pbs; }
 
 // Candidate state in shared memory, one slot per candidate a CTA runs, arrays of [row][slot]:
 // lanes on consecutive slots hit consecutive banks whatever rows they read.  A slot is the
@@ -814,7 +818,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
     const int npb = a.pb_list ? pb_total(a) : nb * a.slots;
     if ((refine_spread(npb) < 32) != HELP) return;  // the other instance's launch
     const int spread = HELP ? refine_spread(npb) : 32, pbs = refine_group(T, CPB, spread);
-    const int ngroups = (npb + pbs - 1) / pbs;
+    const int ngroups = refine_groups(npb, pbs);
     // this thread's place among those that run candidates, the first `spread` lanes of each warp
     const int place = lane < spread ? warp * spread + lane : kRefineThreads;
     const int iters = a.refine_iters > 0 ? a.refine_iters : 6;
@@ -937,6 +941,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
                         const uint32_t pbi = ((item & 0x07FFFFFFu) - 1) * (uint32_t)a.slots + (item >> 27);
                         write_tail(a, Cand(smem, fl, cand), pbi, pos_of[cand] % cpb, it, pos);
                     }
+                    if (a.work && tid == 0) atomicAdd(a.work + 14, (unsigned long long)nlive);
                     __syncthreads();  // staged[] is rewritten next
                     break;
                 }
@@ -1751,11 +1756,21 @@ cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s) {
     for (int help = 0; help < 2; help++) {
         if ((refine_spread(npb) < 32) != (help != 0) && !(list && help)) continue;
         const int spread = help ? std::min(refine_spread(npb), 16) : 32, pbs = refine_group(a.L.T, cpb, spread);
-        int grid = (npb + pbs - 1) / pbs;
+        int grid = refine_groups(npb, pbs);
         if (list) grid = std::min(grid, help ? kOneWaveGroups : kListGridRefine);
         refine_kernel(cpb, refine_u8(a.L.T), help != 0)<<<grid, kRefineThreads, smem, s>>>(a);
     }
     return cudaGetLastError();
+}
+
+size_t refine_tail_entries(const TableLayout& L, int nblocks) {
+    const int npb = nblocks * kSlotsPerBlock;
+    const bool few = refine_few_waves(refine_u8(L.T), refine_groups(npb, refine_group(L.T, refine_cpb(kNumCand), refine_spread(npb))));
+    return (size_t)nblocks * (few ? kTailPerBlockAll : kTailPerBlockFull);
+}
+size_t refine_tail_entries_up_to(const TableLayout& L, int nblocks) {  // the most blocks of few waves, or all of them
+    const int few = 5 * kOneWaveGroups * refine_group(L.T, refine_cpb(kNumCand), 32) / kSlotsPerBlock;
+    return std::max(refine_tail_entries(L, nblocks), refine_tail_entries(L, std::min(nblocks, few)));
 }
 
 cudaError_t launch_refine_tail(const KernelArgs& a, cudaStream_t s) {

@@ -13,6 +13,7 @@
 //      ended without any candidate, which the first select-pack appends)
 // The two passes use separate record and snapshot regions.  Kernels past a
 // list's device-side count return at once.
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -33,12 +34,18 @@ const NetDev* net_for(const astcb200_ctx* ctx, const FootTables* ft) {
     return nullptr;
 }
 
-int ensure_chunk_scratch(astcb200_ctx* ctx, Scratch& sc, size_t blocks, const FootTables* ft) {
-    const NetDev* nd = net_for(ctx, ft);
+// Tail entries a chunk may fill: as many as its own blocks call for, whatever an earlier call made the
+// buffer hold.
+static int tail_cap(const Scratch& sc, size_t entries) {
+    return (int)std::min({sc.cap_tail / (kTailWords * sizeof(uint4)), entries, (size_t)1 << 30});
+}
+
+int ensure_chunk_scratch(astcb200_ctx* ctx, Scratch& sc, size_t blocks, const FootTables* ft, bool full_only) {
+    const NetDev* nd = full_only ? nullptr : net_for(ctx, ft);
     if (!nd) {
         const int rc = ensure_scratch(ctx, sc, blocks, kSlotsPerBlock);
         if (rc || ft->L.T > kTailMaxTexels) return rc;
-        return ensure_buf(ctx, sc.tail, sc.cap_tail, blocks * kTailPerBlockFull * kTailWords * sizeof(uint4), "cudaMalloc refinement tail");
+        return ensure_buf(ctx, sc.tail, sc.cap_tail, refine_tail_entries_up_to(ft->L, (int)blocks) * kTailWords * sizeof(uint4), "cudaMalloc refinement tail");
     }
     int rc;
     if ((rc = ensure_scratch(ctx, sc, blocks, kSlotsPerBlock + kMaxSlots))) return rc;
@@ -108,7 +115,7 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
             int* counts = ctx->d_counts + mlp::kRouteCounters * ctx->counts_used++;
             CK(cudaMemsetAsync(counts, 0, mlp::kRouteCounters * sizeof(int), s), "reset tail counter");
             a.tail = sc.tail;
-            a.tail_cap = (int)std::min<size_t>(sc.cap_tail / (kTailWords * sizeof(uint4)), (size_t)1 << 30);
+            a.tail_cap = tail_cap(sc, refine_tail_entries(ft->L, a.nblocks));
             a.tail_count = counts + 6;  // and its claim counter, counts[7]
             nl = 2;
         }
@@ -172,7 +179,7 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
         // it holds few blocks, so its duration is one CTA's chain, which a second, serial
         // kernel would only lengthen.
         ap.tail = sc.tail;
-        ap.tail_cap = (int)std::min<size_t>(sc.cap_tail / (kTailWords * sizeof(uint4)), (size_t)1 << 30);
+        ap.tail_cap = tail_cap(sc, (size_t)ap.nblocks * kTailPerBlock);
         ap.tail_count = counts + 6;  // two free route counters: reservations, claims
     }
     int tails = 0;  // tail launches (timed with their pass's refinement)

@@ -247,3 +247,33 @@ def test_selection_with_logits_near_the_lowest_value(bx, by, logit, route):
     enc.close()
     assert np.all(got == route)
     assert np.all(picks[:, 0] == (0 if route else 2))
+
+
+@pytest.mark.parametrize("bx,by,blocks_x,blocks_y", [(6, 6, 46, 22),   # 1,012 blocks: 823 groups, little over one wave
+                                                     (5, 5, 64, 71),   # 4,544: 3,692, little below five
+                                                     (6, 6, 64, 72)])  # 4,608: 3,744, above: the last of each group only
+def test_refinement_tail_takes_what_the_rule_offers(bx, by, blocks_x, blocks_y):
+    """A launch of few waves offers the tail all of its candidates, which must have room for them; how many it
+    takes does not depend on what the encoder encoded before."""
+    img = synth.make_texture(bx * blocks_x - 1, by * blocks_y, 91)
+    big = synth.make_texture(bx * 100, by * 100, 92)
+    few = blocks_x * blocks_y <= 4553
+    taken, outs = [], []
+    for warm in (False, True):
+        enc = ab.ASTCEncoder(device=0, fixed=True, stage_timing=True)
+        if warm:
+            enc.secondaryInit(big.shape[1], big.shape[0], bx, by)
+            enc.encode(big)
+        enc.secondaryInit(img.shape[1], img.shape[0], bx, by)
+        outs.append(enc.encode(img))
+        c = enc.work_counters()
+        offered, accepted = int(c[13]), int(c[14])
+        if few:
+            assert accepted == offered > 30 * enc.numBlocks
+        else:
+            assert 0 < accepted <= min(offered, 16 * enc.numBlocks)
+        taken.append(accepted)
+        enc.close()
+    assert np.array_equal(outs[0], outs[1])
+    if few:
+        assert taken[0] == taken[1]
