@@ -219,8 +219,9 @@ size_t search_smem_bytes(const TableLayout& L);
 
 cudaError_t configure_kernels(const TableLayout& L);
 cudaError_t launch_partition_search(const KernelArgs& a, cudaStream_t s);
-cudaError_t launch_front(const KernelArgs& a, cudaStream_t s);
-cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s);
+// launched: the kernels queued are added to it
+cudaError_t launch_front(const KernelArgs& a, cudaStream_t s, int* launched = nullptr);
+cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s, int* launched = nullptr);
 // Finishes the candidates k_refine handed to the tail (a.tail, a.tail_count).
 cudaError_t launch_refine_tail(const KernelArgs& a, cudaStream_t s);
 cudaError_t launch_select_pack(const KernelArgs& a, cudaStream_t s);

@@ -1748,13 +1748,14 @@ cudaError_t configure_kernels(const TableLayout& L) {
 
 // A launch over a list, whose length the device knows, queues both instances where it may be either's;
 // the one it isn't returns at once (2 us).
-cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s) {
+cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s, int* launched) {
     const int cpb = refine_cpb(a.topn);
     const int npb = a.nblocks * a.slots;  // of a list: at most
     const size_t smem = refine_smem_bytes(a.L, cpb);
     const bool list = a.block_list || a.pb_list;
     for (int help = 0; help < 2; help++) {
         if ((refine_spread(npb) < 32) != (help != 0) && !(list && help)) continue;
+        if (launched) ++*launched;
         const int spread = help ? std::min(refine_spread(npb), 16) : 32, pbs = refine_group(a.L.T, cpb, spread);
         int grid = refine_groups(npb, pbs);
         if (list) grid = std::min(grid, help ? kOneWaveGroups : kListGridRefine);

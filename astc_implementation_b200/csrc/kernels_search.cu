@@ -1665,11 +1665,12 @@ cudaError_t launch_partition_search(const KernelArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_front(const KernelArgs& a, cudaStream_t s) {
+cudaError_t launch_front(const KernelArgs& a, cudaStream_t s, int* launched) {
     const int nt = front_nt(a);
     int grid = a.nblocks * a.slots;
     if (a.block_list) grid = std::min(grid, kListGridFront * 128 / nt);
     auto go = [&](const KernelArgs& k, bool p1) {
+        if (launched) ++*launched;
         const size_t smem = front_smem_bytes(a.L, nt, a.bm_mask != nullptr, p1);
         if (nt == 32) { if (p1) k_front<32, true, false><<<grid, 32, smem, s>>>(k); else k_front<32, false, false><<<grid, 32, smem, s>>>(k); }
         else if (nt == 64) { if (p1) k_front<64, true, false><<<grid, 64, smem, s>>>(k); else k_front<64, false, false><<<grid, 64, smem, s>>>(k); }

@@ -89,7 +89,8 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
     a.picks = sc.picks;
     a.pbrec = sc.pbrec;
     a.snaps = sc.snaps;
-    int ni = 0;  // launches queued so far; ev[ni] precedes launch ni
+    int ni = 0;      // intervals queued so far; ev[ni] precedes interval ni
+    int queued = 0;  // and their kernels
     if (ev) {
         for (int i = 0; i < kStageIntervals; i++) kinds[i] = -1;
         CK(cudaEventRecord(ev[0], s), "stage event");
@@ -101,14 +102,25 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
             CK(cudaEventRecord(ev[ni + 1], s), "stage event");
         }
         ni++;
+        queued += nl;
         return ASTCB200_OK;
+    };
+    auto front = [&](const KernelArgs& k) -> int {
+        int nl = 0;
+        const cudaError_t e = launch_front(k, s, &nl);
+        return done(e, "k_front", 1, nl);
+    };
+    auto refine = [&](const KernelArgs& k) -> int {  // with its tail
+        int nl = 0;
+        cudaError_t e = launch_refine(k, s, &nl);
+        if (e == cudaSuccess && k.tail) { e = launch_refine_tail(k, s); nl++; }
+        return done(e, "k_refine", 2, nl);
     };
     int rc;
     const NetDev* nd = full_only ? nullptr : net_for(ctx, ft);
     if (!nd) {
         a.slots = kSlotsPerBlock;
         a.topn = kNumCand;
-        int nl = 1;  // launches of the refinement interval
         if (sc.tail && ft->L.T <= kTailMaxTexels &&
             (ctx->counts_used + 1) * mlp::kRouteCounters <= ctx->counts_cap / sizeof(int)) {
             // the refinement hands its last candidates to the tail, as in the proposal pass
@@ -117,18 +129,13 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
             a.tail = sc.tail;
             a.tail_cap = tail_cap(sc, refine_tail_entries(ft->L, a.nblocks));
             a.tail_count = counts + 6;  // and its claim counter, counts[7]
-            nl = 2;
         }
         if ((rc = done(launch_partition_search(a, s), "k_partition_search", 0))) return rc;
-        if ((rc = done(launch_front(a, s), "k_front", 1))) return rc;
-        {
-            cudaError_t e = launch_refine(a, s);
-            if (e == cudaSuccess && a.tail) e = launch_refine_tail(a, s);
-            if ((rc = done(e, "k_refine", 2, nl))) return rc;
-        }
+        if ((rc = front(a))) return rc;
+        if ((rc = refine(a))) return rc;
         if ((rc = done(launch_select_pack(a, s), "k_select_pack", 3))) return rc;
-        if (ext) { CK(launch_extend(a, ext, s), "k_extend"); ni++; }
-        if (launches) *launches += ni + (nl - 1);
+        if (ext) { CK(launch_extend(a, ext, s), "k_extend"); queued++; }
+        if (launches) *launches += queued;
         return ASTCB200_OK;
     }
     const Pruning pr = resolve_pruning(ctx->pruning, ft->L.T);
@@ -182,26 +189,19 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
         ap.tail_cap = tail_cap(sc, (size_t)ap.nblocks * kTailPerBlock);
         ap.tail_count = counts + 6;  // two free route counters: reservations, claims
     }
-    int tails = 0;  // tail launches (timed with their pass's refinement)
-    auto refine = [&](const KernelArgs& k, const char* what) -> int {
-        cudaError_t e = launch_refine(k, s);
-        const int nl = k.tail ? 2 : 1;
-        if (e == cudaSuccess && k.tail) { e = launch_refine_tail(k, s); tails++; }
-        return done(e, what, 2, nl);
-    };
 
     CK(cudaMemsetAsync(counts, 0, mlp::kRouteCounters * sizeof(int), s), "reset route counters");
     if ((rc = done(mlp::launch_mlp_logits(a, nd->net, sc.logits, ctx->d_mlp_error, s), "k_mlp_logits", 0))) return rc;
     if ((rc = done(mlp::launch_select(a, nd->net, sc.logits, sel, r, s), "k_select", 0))) return rc;
-    if ((rc = done(launch_front(ap, s), "k_front", 1, 2))) return rc;  // the P = 1 list, then the others
-    if ((rc = refine(ap, "k_refine"))) return rc;
+    if ((rc = front(ap))) return rc;  // the P = 1 list, then the others
+    if ((rc = refine(ap))) return rc;
     if ((rc = done(launch_select_pack(ap, s), "k_select_pack", 3))) return rc;
     if ((rc = done(launch_partition_search(af, s), "k_partition_search", 0))) return rc;
-    if ((rc = done(launch_front(af, s), "k_front", 1))) return rc;
-    if ((rc = refine(af, "k_refine"))) return rc;
+    if ((rc = front(af))) return rc;
+    if ((rc = refine(af))) return rc;
     if ((rc = done(launch_select_pack(af, s), "k_select_pack", 3))) return rc;
-    if (ext) { CK(launch_extend(a, ext, s), "k_extend"); ni++; }  // every block of the chunk, after both passes
-    if (launches) *launches += ni + tails;
+    if (ext) { CK(launch_extend(a, ext, s), "k_extend"); queued++; }  // every block of the chunk, after both passes
+    if (launches) *launches += queued;
     return ASTCB200_OK;
 }
 

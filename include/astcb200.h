@@ -354,11 +354,12 @@ int astcb200_search_stages(astcb200_ctx* ctx, const uint8_t* rgba8, void* picks,
 /* Device milliseconds spent in each of the four kernels (partition search, front,
  * refine, select/pack) by the last encode call, summed over chunks; needs
  * ASTCB200_FLAG_STAGE_TIMING.  launches[4] receives the launch counts (optional).  The
- * proposal pass's refinement includes its tail pass, a second launch. */
+ * refinement includes its tail pass, and over a list, whose length only the device knows, the
+ * instance for small launches beside the plain one; the proposal pass's front is two launches. */
 int astcb200_stage_times(astcb200_ctx* ctx, float* ms4, uint32_t* launches4);
 
-/* Per-launch device milliseconds of the last encode, summed over chunks by the launch's
- * position in its chunk's sequence (full search: 4 launches; proposal search: network,
+/* Device milliseconds of the last encode by stage launch, summed over chunks by its
+ * position in its chunk's sequence (full search: 4 positions; proposal search: network,
  * selection, front, refine, select-pack of the proposal pass, then partition search, front,
  * refine, select-pack of the full-search pass); stage9 receives each position's stage
  * (0-3 as for astcb200_stage_times, -1 unused).  Needs ASTCB200_FLAG_STAGE_TIMING. */
