@@ -212,7 +212,8 @@ __device__ __forceinline__ uint4* block_dst(const KernelArgs& a, int blk) {
 size_t front_smem_bytes(const TableLayout& L);
 size_t refine_smem_bytes(const TableLayout& L);
 
-// Tail entries of a full search's launch over nblocks blocks, and of any of up to nblocks.
+// Tail entries of a full search's launch over nblocks blocks (0: it hands nothing over), and the most of
+// any launch of up to nblocks.
 size_t refine_tail_entries(const TableLayout& L, int nblocks);
 size_t refine_tail_entries_up_to(const TableLayout& L, int nblocks);
 size_t search_smem_bytes(const TableLayout& L);

@@ -334,6 +334,7 @@ __host__ __device__ inline int refine_group(int T, int cpb, int spread) {  // pa
     return n < 1 ? 1 : n < pbs ? n : pbs;
 }
 __host__ __device__ inline int refine_groups(int npb, int pbs) { return (npb + pbs - 1) / pbs; }
+__host__ __device__ inline bool refine_one_wave(int ngroups) { return ngroups <= kOneWaveGroups; }
 
 // Candidate state in shared memory, one slot per candidate a CTA runs, arrays of [row][slot]:
 // lanes on consecutive slots hit consecutive banks whatever rows they read.  A slot is the
@@ -829,7 +830,7 @@ __global__ void __launch_bounds__(kRefineThreads, kRefineCtas) k_refine(const __
     // Hand the last candidates to the tail (until it is found full).  A launch of one wave is as long
     // as its longest chain of iterations, which a second kernel would lengthen: the full search
     // keeps its candidates then, the proposal pass hands them over for the last iteration only.
-    const bool one_wave = ngroups <= kOneWaveGroups;
+    const bool one_wave = refine_one_wave(ngroups);
     bool spill = a.tail != nullptr && T <= kTailMaxTexels && !(one_wave && !a.prop);
     const int spill_live = refine_spill_live(U8, a.prop != nullptr, ngroups);
     // (the first group's barrier below orders these writes before any read)
@@ -1765,9 +1766,9 @@ cudaError_t launch_refine(const KernelArgs& a, cudaStream_t s, int* launched) {
 }
 
 size_t refine_tail_entries(const TableLayout& L, int nblocks) {
-    const int npb = nblocks * kSlotsPerBlock;
-    const bool few = refine_few_waves(refine_u8(L.T), refine_groups(npb, refine_group(L.T, refine_cpb(kNumCand), refine_spread(npb))));
-    return (size_t)nblocks * (few ? kTailPerBlockAll : kTailPerBlockFull);
+    const int npb = nblocks * kSlotsPerBlock, ngroups = refine_groups(npb, refine_group(L.T, refine_cpb(kNumCand), refine_spread(npb)));
+    if (L.T > kTailMaxTexels || refine_one_wave(ngroups)) return 0;
+    return (size_t)nblocks * (refine_few_waves(refine_u8(L.T), ngroups) ? kTailPerBlockAll : kTailPerBlockFull);
 }
 size_t refine_tail_entries_up_to(const TableLayout& L, int nblocks) {  // the most blocks of few waves, or all of them
     const int few = 5 * kOneWaveGroups * refine_group(L.T, refine_cpb(kNumCand), 32) / kSlotsPerBlock;

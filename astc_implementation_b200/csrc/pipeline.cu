@@ -44,8 +44,9 @@ int ensure_chunk_scratch(astcb200_ctx* ctx, Scratch& sc, size_t blocks, const Fo
     const NetDev* nd = full_only ? nullptr : net_for(ctx, ft);
     if (!nd) {
         const int rc = ensure_scratch(ctx, sc, blocks, kSlotsPerBlock);
-        if (rc || ft->L.T > kTailMaxTexels) return rc;
-        return ensure_buf(ctx, sc.tail, sc.cap_tail, refine_tail_entries_up_to(ft->L, (int)blocks) * kTailWords * sizeof(uint4), "cudaMalloc refinement tail");
+        const size_t entries = refine_tail_entries_up_to(ft->L, (int)blocks);
+        if (rc || entries == 0) return rc;
+        return ensure_buf(ctx, sc.tail, sc.cap_tail, entries * kTailWords * sizeof(uint4), "cudaMalloc refinement tail");
     }
     int rc;
     if ((rc = ensure_scratch(ctx, sc, blocks, kSlotsPerBlock + kMaxSlots))) return rc;
@@ -121,13 +122,14 @@ int enqueue_chunk(astcb200_ctx* ctx, const KernelArgs& base, const FootTables* f
     if (!nd) {
         a.slots = kSlotsPerBlock;
         a.topn = kNumCand;
-        if (sc.tail && ft->L.T <= kTailMaxTexels &&
+        const size_t entries = refine_tail_entries(ft->L, a.nblocks);
+        if (sc.tail && entries > 0 &&
             (ctx->counts_used + 1) * mlp::kRouteCounters <= ctx->counts_cap / sizeof(int)) {
             // the refinement hands its last candidates to the tail, as in the proposal pass
             int* counts = ctx->d_counts + mlp::kRouteCounters * ctx->counts_used++;
             CK(cudaMemsetAsync(counts, 0, mlp::kRouteCounters * sizeof(int), s), "reset tail counter");
             a.tail = sc.tail;
-            a.tail_cap = tail_cap(sc, refine_tail_entries(ft->L, a.nblocks));
+            a.tail_cap = tail_cap(sc, entries);
             a.tail_count = counts + 6;  // and its claim counter, counts[7]
         }
         if ((rc = done(launch_partition_search(a, s), "k_partition_search", 0))) return rc;

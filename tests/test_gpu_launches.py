@@ -40,7 +40,10 @@ def test_launch_counts(w, h, bx, by, extend, chunk, stages):
     assert total == sum(stages) + (1 if extend else 0)
 
 
-@pytest.mark.parametrize("w,h,refine", [(400, 300, 2)])  # 7,500 blocks: more than one wave, with a tail
+@pytest.mark.parametrize("w,h,refine", [(400, 300, 2),        # 7,500 blocks: more than one wave, with a tail
+                                        (4 * 911, 4, 2),      # 741 groups of 16 partitioned blocks: as few as have one
+                                        (4 * 910, 4, 1),      # 740: one wave hands nothing over and has none
+                                        (64, 64, 1)])
 def test_launch_counts_of_a_full_search(w, h, refine):
     total, got = launches(w, h, 4, 4, False)
     assert got == [1, 1, refine, 1] and total == 3 + refine
