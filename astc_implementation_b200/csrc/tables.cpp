@@ -448,12 +448,44 @@ std::unique_ptr<HostTables> make_host_tables(int bx, int by) {
     return hp;
 }
 
+// Room for n zeros at the end of the blob, valid until it grows again; off: where.
+template <class T = uint32_t>
+T* room(std::vector<uint8_t>& blob, size_t n, uint32_t& off) {
+    off = (uint32_t)((blob.size() + 15) & ~size_t(15));
+    blob.resize(off + n * sizeof(T));
+    return reinterpret_cast<T*>(blob.data() + off);
+}
 template <class T>
 uint32_t put(std::vector<uint8_t>& blob, const T* data, size_t n) {
-    size_t off = (blob.size() + 15) & ~size_t(15);
-    blob.resize(off + n * sizeof(T));
-    if (n) std::memcpy(blob.data() + off, data, n * sizeof(T));
-    return (uint32_t)off;
+    uint32_t off;
+    T* to = room<T>(blob, n, off);
+    if (n) std::memcpy(to, data, n * sizeof(T));
+    return off;
+}
+
+// Sorts by a key of a byte, equal keys in their order.
+template <class Key>
+void stable_by(std::vector<uint16_t>& v, Key key) {
+    uint32_t at[257] = {};
+    for (uint16_t x : v) at[(uint8_t)key(x) + 1]++;
+    for (int i = 0; i < 256; i++) at[i + 1] += at[i];
+    std::vector<uint16_t> out(v.size());
+    for (uint16_t x : v) out[at[(uint8_t)key(x)]++] = x;
+    v.swap(out);
+}
+
+// Sixteen bytes of 0..3 as a word, two bits each, the first lowest.
+uint32_t pack2(const uint8_t* b) {
+    uint32_t out = 0;
+    for (int half = 0; half < 2; half++) {
+        uint64_t v;
+        std::memcpy(&v, b + 8 * half, 8);  // (little-endian)
+        v = (v | v >> 6) & 0x000F000F000F000Full;
+        v = (v | v >> 12) & 0x000000FF000000FFull;
+        v = (v | v >> 24) & 0xFFFFull;
+        out |= (uint32_t)v << (16 * half);
+    }
+    return out;
 }
 
 }  // namespace
@@ -492,24 +524,27 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     for (int i = 0; i < 4; i++) L.count_selected[i] = h.sel[i];
     std::memcpy(L.kmeans, h.kmeans, sizeof(L.kmeans));
     const int T = h.T, ndm = L.ndm;
+    blob.reserve(size_t(1200) << 10);  // 12x12's: 1.1 MB
     std::vector<DevDm> dms(ndm);
-    std::vector<uint8_t> twc((size_t)ndm * T, 0), wtc((size_t)ndm * 64, 0);
-    std::vector<int> tw_base(ndm);
-    std::vector<uint16_t> tws((size_t)ndm * T, 0), wts((size_t)ndm * 64, 0), t2w, w2t;
+    std::vector<uint8_t> wtc((size_t)ndm * 64, 0);
+    std::vector<uint16_t> wts((size_t)ndm * 64, 0), w2t;
+    std::vector<uint64_t> tw4((size_t)ndm * T, 0);
+    w2t.reserve(h.w2t_t.size());
     for (int m = 0; m < ndm; m++) {
         const HostTables::Dm& d = h.dms[h.valid_dms[m]];
+        if (d.steps > (uint32_t)kMaxAngularSteps) return false;
         DevDm& o = dms[m];
         o.W = (uint8_t)d.W; o.wx = (uint8_t)d.wx; o.wy = (uint8_t)d.wy; o.max_quant_level = (uint8_t)d.maxq;
         o.max_angular_steps = (uint8_t)d.steps; o.max_quant_steps = (uint8_t)d.qsteps; o.w_off = (uint16_t)L.nw_total;
         L.nw_total += (int)((d.W + 3) & ~3u);
-        tw_base[m] = (int)t2w.size(); o.pad = 0; o.wt_base = (uint16_t)w2t.size();
+        o.pad = 0; o.wt_base = (uint16_t)w2t.size();
         for (int t = 0; t < T; t++) {
-            twc[(size_t)m * T + t] = (uint8_t)d.tw_count[t];
-            tws[(size_t)m * T + t] = (uint16_t)(t2w.size() - tw_base[m]);
+            uint64_t v = 0;
             for (uint32_t j = 0; j < d.tw_count[t]; j++) {
                 const uint32_t e = d.tw_off[t] + j;
-                t2w.push_back((uint16_t)(h.t2w_w[e] | (h.t2w_k[e] << 8)));
+                v |= (uint64_t)(uint16_t)(h.t2w_w[e] | (h.t2w_k[e] << 8)) << (16 * j);
             }
+            tw4[(size_t)m * T + t] = v;
         }
         for (uint32_t w = 0; w < d.W; w++) {
             wtc[(size_t)m * 64 + w] = (uint8_t)d.wt_count[w];
@@ -520,14 +555,6 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
             }
         }
     }
-    std::vector<uint64_t> tw4((size_t)ndm * T, 0);
-    for (int m = 0; m < ndm; m++)
-        for (int t = 0; t < T; t++) {
-            uint64_t v = 0;
-            const int n = twc[(size_t)m * T + t], base = tw_base[m] + tws[(size_t)m * T + t];
-            for (int j = 0; j < n; j++) v |= (uint64_t)t2w[base + j] << (16 * j);
-            tw4[(size_t)m * T + t] = v;
-        }
     L.max_w = 0;
     for (int m = 0; m < ndm; m++) L.max_w = std::max<int>(L.max_w, dms[m].W);
     std::vector<DevBm> bms(L.nbm);
@@ -535,26 +562,12 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
         const HostTables::Bm& b = h.bms[h.valid_bms[i].first];
         bms[i] = DevBm{(uint16_t)b.mode, (uint8_t)h.valid_bms[i].second, (uint8_t)b.quant, (uint8_t)b.bits, 0, 0, 0};
     }
-    std::vector<uint8_t> pcnt((size_t)3 * 1024 * 4);
-    const int part2_words = (T + 15) / 16;
-    std::vector<uint32_t> pinfo(3 * 1024), part2((size_t)3 * 1024 * part2_words, 0);
-    std::vector<uint64_t> cov((size_t)3 * 1024 * 4, 0);
-    for (int pc = 2; pc <= 4; pc++)
-        for (int e = 0; e < 1024; e++) {
-            const HostTables::Part& p = h.parts[(pc - 2) * 1024 + e];
-            const size_t k = (size_t)(pc - 2) * 1024 + e;
-            for (int t = 0; t < T; t++) part2[k * part2_words + t / 16] |= (uint32_t)p.of[t] << (2 * (t & 15));
-            for (int q = 0; q < 4; q++) pcnt[k * 4 + q] = (uint8_t)p.tcount[q];
-            pinfo[k] = p.seed;
-            for (int q = 0; q < pc; q++) cov[k * 4 + q] = h.cov[pc][(size_t)e * pc + q];
-        }
     std::vector<DevBm> dual;  // dual-plane block modes whose grid is a trial decimation mode
     {
         std::vector<uint32_t> lookup(h.dms.size(), 0xFFFF);
         for (uint32_t d = 0; d < h.valid_dms.size(); d++) lookup[h.valid_dms[d]] = d;
         for (const HostTables::Bm& b : h.bms)
-            if (b.dual && lookup[b.dm] != 0xFFFF)
-{
+            if (b.dual && lookup[b.dm] != 0xFFFF) {
                 DevBm d{(uint16_t)b.mode, (uint8_t)lookup[b.dm], (uint8_t)b.quant, (uint8_t)b.bits, 0, 0, 0};
                 for (int q = 4; q <= 20; q++) {
                     if (dec::ise_bits(6, q) <= 109 - (int)b.bits) d.colour6 = (uint8_t)q;
@@ -573,7 +586,7 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     L.ndual_w = (int)dual_w.size();
     std::vector<uint16_t> order(L.nbm);
     for (int i = 0; i < L.nbm; i++) order[i] = (uint16_t)i;
-    std::stable_sort(order.begin(), order.end(), [&](uint16_t x, uint16_t y) { return bms[x].dm < bms[y].dm; });
+    stable_by(order, [&](uint16_t x) { return bms[x].dm; });
     L.off_dm = put(blob, dms.data(), dms.size());
     L.off_bm = put(blob, bms.data(), bms.size());
     L.off_wt_count = put(blob, wtc.data(), wtc.size());
@@ -584,27 +597,37 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
     L.off_dual = put(blob, dual.data(), dual.size());
     L.off_dual_w = put(blob, dual_w.data(), dual_w.size());
     L.off_dual_first = put(blob, dual_first.data(), dual_first.size());
-    L.off_part2 = put(blob, part2.data(), part2.size());
-    L.off_part_info = put(blob, pinfo.data(), pinfo.size());
-    L.off_part_counts = put(blob, pcnt.data(), pcnt.size());
-    L.off_cov = put(blob, cov.data(), cov.size());
-    std::vector<float> trig(2 * (h.cos_t.size() + 16), 0.0f);
-    for (size_t i = 0; i < h.cos_t.size(); i++) { trig[2 * i] = h.cos_t[i]; trig[2 * i + 1] = h.sin_t[i]; }
-    L.off_trig = put(blob, trig.data(), trig.size());
+    {
+        const int words = (T + 15) / 16;
+        uint32_t* part2 = room(blob, (size_t)3 * 1024 * words, L.off_part2);
+        for (size_t k = 0; k < 3 * 1024; k++) {
+            const HostTables::Part& p = h.parts[k];
+            for (int w = 0; w < words; w++) *part2++ = pack2(p.of + 16 * w);  // (0 past the last texel)
+        }
+        uint32_t* pinfo = room(blob, 3 * 1024, L.off_part_info);
+        for (size_t k = 0; k < 3 * 1024; k++) pinfo[k] = h.parts[k].seed;
+        uint8_t* pcnt = room<uint8_t>(blob, 3 * 1024 * 4, L.off_part_counts);
+        for (size_t k = 0; k < 3 * 1024; k++)
+            for (int q = 0; q < 4; q++) pcnt[k * 4 + q] = (uint8_t)h.parts[k].tcount[q];
+        uint64_t* cov = room<uint64_t>(blob, 3 * 1024 * 4, L.off_cov);
+        for (int pc = 2; pc <= 4; pc++)
+            for (size_t e = 0; e < 1024; e++)
+                for (int q = 0; q < pc; q++) cov[((size_t)(pc - 2) * 1024 + e) * 4 + q] = h.cov[pc][e * pc + q];
+        float* trig = room<float>(blob, 2 * (h.cos_t.size() + 16), L.off_trig);
+        for (size_t i = 0; i < h.cos_t.size(); i++) { trig[2 * i] = h.cos_t[i]; trig[2 * i + 1] = h.sin_t[i]; }
+    }
     // entries with the contribution k / 16 (k <= 16, exact in bf16) ready to use as the high half of a float
-    auto ready = [](uint32_t e) {
-        const float c = (float)(e >> 8) * (1.0f / 16.0f);
-        uint32_t u;
-        std::memcpy(&u, &c, 4);
-        return (u & 0xFFFF0000u) | (e & 0xFF);
-    };
-    std::vector<uint32_t> tw4f((size_t)ndm * T * 4), w2tf;
-    for (size_t i = 0; i < tw4.size(); i++)
-        for (int j = 0; j < 4; j++) tw4f[4 * i + j] = ready((uint32_t)(tw4[i] >> (16 * j)) & 0xFFFF);
-    std::vector<uint32_t> wt_info((size_t)ndm * 64, 0);
+    uint32_t factor[17];
+    for (int k = 0; k <= 16; k++) {
+        const float c = (float)k * (1.0f / 16.0f);
+        std::memcpy(&factor[k], &c, 4);
+    }
+    auto ready = [&](uint32_t e) { return factor[e >> 8] | (e & 0xFF); };
+    std::vector<uint32_t> w2tf, wt_info((size_t)ndm * 64, 0);
     std::vector<uint16_t> witem, sitem;
+    w2tf.reserve(w2t.size() + 3 * (size_t)L.nw_total);
+    witem.reserve(L.nw_total);
     for (int m = 0; m < ndm; m++) {
-        if (dms[m].max_angular_steps > kMaxAngularSteps) return false;
         for (int w = 0; w < dms[m].W; w++) {
             const int first = dms[m].wt_base + wts[(size_t)m * 64 + w], n = wtc[(size_t)m * 64 + w];
             wt_info[(size_t)m * 64 + w] = (uint32_t)(w2tf.size() / 4) | (uint32_t)((n + 3) / 4) << 16;
@@ -614,28 +637,30 @@ bool build_tables(int bx, int by, TableLayout& L, std::vector<uint8_t>& blob) {
         for (int i = 0; i < dms[m].max_angular_steps; i++) sitem.push_back((uint16_t)(m << 4 | i));
     }
     auto texels_of = [&](uint16_t e) -> uint32_t { return dms[e >> 6].W == T ? 0 : wt_info[e] >> 16; };  // in fours
-    std::stable_sort(witem.begin(), witem.end(), [&](uint16_t x, uint16_t y) { return texels_of(x) > texels_of(y); });
-    std::stable_sort(sitem.begin(), sitem.end(), [&](uint16_t x, uint16_t y) { return dms[x >> 4].W > dms[y >> 4].W; });
+    stable_by(witem, [&](uint16_t x) { return (uint8_t)(255 - texels_of(x)); });
+    stable_by(sitem, [&](uint16_t x) { return (uint8_t)(255 - dms[x >> 4].W); });
     L.nwi = (int)witem.size(); L.nsi = (int)sitem.size();
-    std::vector<uint32_t> wgroup, wgent;  // items of a mode of one weight a texel have no entries
+    std::vector<uint32_t> wgroup;  // items of a mode of one weight a texel have no entries
+    uint32_t fours = 0;
     for (size_t g = 0; g < witem.size(); g += 32) {
-        uint32_t n4 = 0;
-        for (size_t i = g; i < std::min(g + 32, witem.size()); i++) n4 = std::max(n4, (texels_of(witem[i]) + 0u));
-        wgroup.push_back((uint32_t)(wgent.size() / 128) | n4 << 16);
-        for (uint32_t j = 0; j < n4; j++)
-            for (size_t i = g; i < g + 32; i++)
-                for (int k = 0; k < 4; k++) {
-                    const bool has = i < witem.size() && j < texels_of(witem[i]);
-                    wgent.push_back(has ? w2tf[((wt_info[witem[i]] & 0xFFFF) + j) * 4 + k] : 0u);
-                }
+        const uint32_t n4 = texels_of(witem[g]);  // the group's largest
+        wgroup.push_back(fours | n4 << 16);
+        fours += n4;
     }
-    if (w2tf.size() / 4 > 0xFFFF || wgent.size() / 128 > 0xFFFF) return false;
+    if (w2tf.size() / 4 > 0xFFFF || fours > 0xFFFF) return false;
     L.off_wgroup = put(blob, wgroup.data(), wgroup.size());
-    L.off_wgent = put(blob, wgent.data(), wgent.size());
+    uint32_t* wgent = room(blob, (size_t)fours * 128, L.off_wgent);
+    for (size_t i = 0; i < witem.size(); i++) {
+        uint32_t* to = wgent + ((size_t)(wgroup[i / 32] & 0xFFFF) * 32 + i % 32) * 4;
+        const uint32_t* from = w2tf.data() + (size_t)(wt_info[witem[i]] & 0xFFFF) * 4;
+        for (uint32_t j = 0; j < texels_of(witem[i]); j++) std::memcpy(to + j * 128, from + j * 4, 16);
+    }
     L.off_wt_info = put(blob, wt_info.data(), wt_info.size());
     L.off_witem = put(blob, witem.data(), witem.size());
     L.off_sitem = put(blob, sitem.data(), sitem.size());
-    L.off_tw4f = put(blob, tw4f.data(), tw4f.size());
+    uint32_t* tw4f = room(blob, tw4.size() * 4, L.off_tw4f);
+    for (size_t i = 0; i < tw4.size(); i++)
+        for (int j = 0; j < 4; j++) tw4f[4 * i + j] = ready((uint32_t)(tw4[i] >> (16 * j)) & 0xFFFF);
     L.off_w2tf = put(blob, w2tf.data(), w2tf.size());
     L.off_q2u = put(blob, c.q2u, 142);
     L.off_q2u_start = put(blob, c.q2u_start, 12);

@@ -152,3 +152,30 @@ def test_nudge_loop_bisection_matches_stepwise():
         if i % 5 == 2:
             c0 = [f32(np.floor(v) + 0.5) for v in c0]
         assert _nudge_bisect(tab, c0, c1) == _nudge_stepwise(tab, c0, c1), i
+
+
+def test_device_tables_are_built_quickly():
+    """A footprint's device tables are built once per context, in its first secondaryInit.  Building
+    12x12's word by word took 7.4 times as long as astcb200_tables_partitions takes to write out the
+    partition tables; 2 times now."""
+    import time
+    bx = by = 12
+    lib = ab.load_library()
+    out = [np.zeros((3073, 150), np.uint32), np.zeros((1024, 2), np.uint64), np.zeros((1024, 3), np.uint64),
+           np.zeros((1024, 4), np.uint64), np.zeros(64, np.uint32), np.zeros((3, 1024), np.uint16)]
+
+    def best(call):
+        t = []
+        for _ in range(20):
+            t0 = time.perf_counter()
+            call()
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    ratios = []
+    for _ in range(5):  # (a loaded machine)
+        dump = best(lambda: lib.astcb200_tables_partitions(bx, by, *[_libs.ptr(o) for o in out]))
+        ratios.append(best(lambda: lib.astcb200_proposal_layout(bx, by, *[None] * 7)) / dump)
+        if ratios[-1] < 4.5:
+            return
+    raise AssertionError(ratios)
