@@ -349,3 +349,24 @@ def test_pruning_settings_are_checked_and_applied():
     n = sym.shape[0]
     assert stats[0] == n
     assert (sym[:, 2] > 1).sum() >= n - stats[1]
+
+
+@pytest.mark.parametrize("bx,by,sizes", [(4, 4, [(32, 32), (131, 90)]),    # 64 blocks, below 592 partitioned blocks; 759
+                                         (6, 6, [(65, 58), (200, 151)])])  # 110; 884
+def test_front_threads_do_not_change_the_blocks(bx, by, sizes):
+    """The one-partition and the general list instances of the front at every thread count, against
+    the default's choice by footprint and launch size."""
+    enc = ab.ASTCEncoder(device=0, fixed=True)
+    enc.set_proposal_net(proposal.load_weights(bx, by))
+    for w, h in sizes:
+        img = synth.make_texture(w, h, 40 + bx)
+        enc.secondaryInit(w, h, bx, by)
+        ref = None
+        for threads in (0, 32, 64, 128):
+            enc.set_pruning(True, front_threads=threads)
+            got = enc.encode_symbolic(img), enc.encode(img)
+            assert enc.pruning_stats()[0] > 0
+            if ref is None:
+                ref = got
+            assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+    enc.close()
