@@ -1,7 +1,7 @@
-// ASTC LDR block decoding, written from the ASTC specification, shared by the host
-// decoder (decoder.cpp) and the device decoder (decoder_gpu.cu) so that both produce
-// the same texels.  A block is parsed once (parse_block: block mode, partitioning,
-// endpoint formats, integer-sequence-encoded colour values and weights, unquantised)
+// ASTC LDR block decoding, written from the ASTC specification: the host decoder (decoder.cpp), and the
+// functions the device's (decode_fast.cuh) builds its tables from at compile time or runs itself.  A
+// block is parsed once (parse_block: block mode, partitioning, endpoint formats,
+// integer-sequence-encoded colour values and weights, unquantised)
 // and then any texel of it can be evaluated (texel16: weight infill, endpoint
 // interpolation, 16-bit result; to_unorm8 gives the 8-bit texel).  Blocks that are
 // not valid LDR blocks (reserved modes, HDR endpoints, too many colour values) decode
@@ -9,16 +9,11 @@
 #pragma once
 #include <stdint.h>
 
+// Run on the device too; the others are the host's, or the compiler's for its tables.
 #ifdef __CUDACC__
 #define ASTC_HD __host__ __device__ __forceinline__ constexpr
-// The unquantisation functions stay out of line in device code: inlined into
-// parse_block, the optimised device build decoded some weights wrongly (found by the
-// device-against-host decoder tests; the debug build and the out-of-line build agree
-// with the host on every block).
-#define ASTC_HD_CALL static __host__ __device__ __noinline__ constexpr
 #else
 #define ASTC_HD inline constexpr
-#define ASTC_HD_CALL inline constexpr
 #endif
 
 namespace astcb200 {
@@ -26,35 +21,35 @@ namespace dec {
 
 struct Bits {
     const uint8_t* p;
-    ASTC_HD uint32_t get(int off, int n) const {
+    constexpr uint32_t get(int off, int n) const {
         uint32_t v = 0;
         for (int i = 0; i < n; i++) v |= (uint32_t)((p[(off + i) >> 3] >> ((off + i) & 7)) & 1) << i;
         return v;
     }
 };
 
-ASTC_HD int level_count(int q) {
+inline constexpr int level_count(int q) {
     const int L[21] = {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64, 80, 96, 128, 160, 192, 256};
     return L[q];
 }
 // bits, trits, quints of quantisation method q
-ASTC_HD void btq(int q, int& bits, int& trits, int& quints) {
+inline constexpr void btq(int q, int& bits, int& trits, int& quints) {
     int L = level_count(q);
     trits = quints = 0;
     if (L % 3 == 0) { trits = 1; L /= 3; } else if (L % 5 == 0) { quints = 1; L /= 5; }
     bits = 0;
     while ((1 << bits) < L) bits++;
 }
-ASTC_HD int ise_bits(int n, int q) {
+inline constexpr int ise_bits(int n, int q) {
     int b = 0, t = 0, qu = 0;
     btq(q, b, t, qu);
     if (t) return (n * (8 + 5 * b) + 4) / 5;
     if (qu) return (n * (7 + 3 * b) + 2) / 3;
     return n * b;
 }
-ASTC_HD int bit_of(int x, int i) { return (x >> i) & 1; }
+inline constexpr int bit_of(int x, int i) { return (x >> i) & 1; }
 // the five trits packed in the 8-bit value T
-ASTC_HD void trit_digits(int T, int t[5]) {
+inline constexpr void trit_digits(int T, int t[5]) {
     int C = 0;
     if (((T >> 2) & 7) == 7) { C = (((T >> 5) & 7) << 2) | (T & 3); t[4] = 2; t[3] = 2; }
     else {
@@ -66,7 +61,7 @@ ASTC_HD void trit_digits(int T, int t[5]) {
     else { t[2] = bit_of(C, 4); t[1] = (C >> 2) & 3; t[0] = (bit_of(C, 1) << 1) | (bit_of(C, 0) & ~bit_of(C, 1) & 1); }
 }
 // the three quints packed in the 7-bit value Q
-ASTC_HD void quint_digits(int Q, int q[3]) {
+inline constexpr void quint_digits(int Q, int q[3]) {
     if (((Q >> 1) & 3) == 3 && ((Q >> 5) & 3) == 0) {
         const int b0 = bit_of(Q, 0);
         q[2] = (b0 << 2) | ((bit_of(Q, 4) & (1 - b0)) << 1) | (bit_of(Q, 3) & (1 - b0));
@@ -79,7 +74,7 @@ ASTC_HD void quint_digits(int Q, int q[3]) {
     if ((C & 7) == 5) { q[1] = 4; q[0] = (C >> 3) & 3; } else { q[1] = (C >> 3) & 3; q[0] = C & 7; }
 }
 // Integer-sequence decode of n values of method q starting at bit `off`.
-ASTC_HD void decode_ise(const Bits& b, int off, int n, int q, int* out) {
+inline constexpr void decode_ise(const Bits& b, int off, int n, int q, int* out) {
     int bits = 0, trits = 0, quints = 0;
     btq(q, bits, trits, quints);
     if (trits) {
@@ -113,13 +108,13 @@ ASTC_HD void decode_ise(const Bits& b, int off, int n, int q, int* out) {
 // v (bits bits, 1..8) repeated from the top until width bits are filled.  The loop has a
 // fixed bound: an unbounded one (endless for bits = 0, which never occurs) lets a compiler
 // draw conclusions about callers that miscompile the weight and colour unquantisation.
-ASTC_HD int replicate(int v, int bits, int width) {
+inline constexpr int replicate(int v, int bits, int width) {
     if (bits <= 0) return 0;
     int out = 0, have = 0;
     for (int i = 0; i < 8 && have < width; i++) { out = (out << bits) | v; have += bits; }
     return out >> (have - width);
 }
-ASTC_HD_CALL int unq_color(int q, int v) {
+inline constexpr int unq_color(int q, int v) {
     int bits = 0, trits = 0, quints = 0;
     btq(q, bits, trits, quints);
     if (!trits && !quints) return replicate(v, bits, 8);
@@ -142,7 +137,7 @@ ASTC_HD_CALL int unq_color(int q, int v) {
     }
     return (A & 0x80) | (((D * C + B) ^ A) >> 2);
 }
-ASTC_HD_CALL int unq_weight(int q, int v) {
+inline constexpr int unq_weight(int q, int v) {
     int bits = 0, trits = 0, quints = 0;
     btq(q, bits, trits, quints);
     int r = 0;
@@ -198,7 +193,7 @@ ASTC_HD bool decode_grid(int m, Mode& o) {
     return true;
 }
 // The same, false also for grids whose weights do not fit the spec's limits.
-ASTC_HD bool decode_mode(int m, Mode& o) {
+inline constexpr bool decode_mode(int m, Mode& o) {
     if (!decode_grid(m, o)) return false;
     const int n = o.xw * o.yw * (o.dual ? 2 : 1);
     return n <= 64 && ise_bits(n, o.q) >= 24 && ise_bits(n, o.q) <= 96;
@@ -209,7 +204,7 @@ ASTC_HD uint32_t hash52(uint32_t v) {
     return v;
 }
 // Partition of texel (x, y) for partitioning `seed` of pc partitions.
-ASTC_HD int select_partition(int seed, int x, int y, int pc, bool small) {
+inline constexpr int select_partition(int seed, int x, int y, int pc, bool small) {
     if (small) { x <<= 1; y <<= 1; }
     seed += (pc - 1) * 1024;
     const uint32_t r = hash52((uint32_t)seed);
@@ -283,9 +278,8 @@ struct Block {
     uint16_t vc[4];
 };
 
-ASTC_HD void parse_block(const uint8_t* blk, int bx, int by, Block& o) {
+inline constexpr void parse_block(const uint8_t* blk, int bx, int by, Block& o) {
     const Bits b{blk};
-    const int T = bx * by;
     o.kind = 0;
     const int mode = (int)b.get(0, 11);
     if ((mode & 0x1FF) == 0x1FC) {  // void extent
@@ -343,11 +337,10 @@ ASTC_HD void parse_block(const uint8_t* blk, int bx, int by, Block& o) {
     }
     o.xw = m.xw; o.yw = m.yw; o.dual = m.dual ? 1 : 0; o.ccs = ccs; o.pc = pc; o.seed = seed;
     o.kind = 2;
-    (void)T;
 }
 
 // The 16-bit texel (x, y) of a parsed block of footprint bx x by.
-ASTC_HD void texel16(const Block& k, int bx, int by, int x, int y, uint16_t* out) {
+inline constexpr void texel16(const Block& k, int bx, int by, int x, int y, uint16_t* out) {
     if (k.kind == 0) { out[0] = 0xFFFF; out[1] = 0; out[2] = 0xFFFF; out[3] = 0xFFFF; return; }
     if (k.kind == 1) { for (int c = 0; c < 4; c++) out[c] = k.vc[c]; return; }
     const int ds = (1024 + bx / 2) / (bx - 1), dt = (1024 + by / 2) / (by - 1);
@@ -371,7 +364,7 @@ ASTC_HD void texel16(const Block& k, int bx, int by, int x, int y, uint16_t* out
 }
 
 // 16-bit channel to 8-bit UNORM, rounded to nearest.
-ASTC_HD uint8_t to_unorm8(uint32_t v) { return (uint8_t)((v * 255u + 32767u) / 65535u); }
+inline constexpr uint8_t to_unorm8(uint32_t v) { return (uint8_t)((v * 255u + 32767u) / 65535u); }
 
 }  // namespace dec
 }  // namespace astcb200

@@ -1,7 +1,6 @@
 // ASTC LDR block decoder (host), written from the ASTC specification.
 // The reference has no decoder; this one measures quality (PSNR) and checks
-// that every block the encoder emits decodes as the encoder intended.  The block
-// decoding itself (decode_block.cuh) is shared with the device decoder.
+// that every block the encoder emits decodes as the encoder intended.
 #include <cstdint>
 #include <cstring>
 

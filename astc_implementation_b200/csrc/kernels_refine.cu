@@ -5,8 +5,10 @@
 //                  endpoints, colour endpoint packing (every LDR encoding the
 //                  reference tries), unpacking, weight realignment, final
 //                  error with a best-so-far snapshot.  One thread runs one
-//                  candidate's iteration; the 8 candidates of a
-//                  partitioned block share a CTA and its staged texels.
+//                  candidate's iteration (in launches of one wave with the
+//                  help of two or four lanes in passes 13-15); the 8
+//                  candidates of a partitioned block share a CTA and its
+//                  staged texels.
 //   k_select_pack  pass18 plus the host argmin over candidates and partition
 //                  counts (compression_pipeline.cpp:500-519), then the ASTC
 //                  physical block layout (code/physical_compression.cpp:843)
@@ -54,8 +56,8 @@ __device__ __forceinline__ float4 over257(float4 c) { return make_float4(over257
 // ------------------------------------------------------------ pass14 colour endpoint packing
 // The endpoints it packs are clamped to 0..255, so every value converted to an integer here is
 // finite and small.  The refinement kernels stalled on instruction fetch first (4.7 of 13 warps
-// per issue at 7,500 instructions), so this code and the iteration are written for size: one
-// copy of each encoding's body and of the final error, loops left rolled; 4,200 instructions.
+// per issue), so this code and the iteration are written for size: one
+// copy of each encoding's body and of the final error, loops left rolled.
 // Measured with f2i / f2u as one conversion: full search of 1024x1024 at 4x4 47.5 -> 39.3 ms, of
 // 1021x765 at 10x8 72.5 -> 69.6 ms; proposal search of 2048x2048 at 4x4 10.2 -> 8.8 ms.
 __device__ __forceinline__ int32_t rni(float v) { return __float2int_rn(v); }
@@ -352,7 +354,7 @@ __host__ __device__ inline bool refine_one_wave(int ngroups) { return ngroups <=
 // that pass16 updates when it moves a weight; every use of one (pass13's weight s / 1024,
 // pass16's s / 16, pass17's rounded s / 16) is the exact value the passes' own sums of
 // products give, since those sums are exact too.  Before, each texel's four table entries
-// and weights were read again at every use (about 45 instructions, two to three uses per
+// and weights were read again at every use (two to three uses per
 // texel and iteration in pass13 and pass17 and one per texel of each weight in pass16).
 // Measured with pass13's walk in partition order (B200): full search of 1024x1024 at 4x4 50.2 -> 47.5 ms,
 // of 64x64 1.08 -> 0.90 ms; proposal search of 2047x2050 at 6x6 8.98 -> 8.13 ms.

@@ -88,9 +88,9 @@ __device__ __forceinline__ float dist_sq(float4 a, float4 b) {
 
 // ============================================================ passes 001-007
 // A warp searches one partition count of a block (small launches: a CTA of four warps, each
-// taking one of the four rounds of 32 candidates).  The kernel issues about a thousand
-// instructions per candidate and waits on instruction fetch, branches and the conversion pipe,
-// not on memory, so: loops are left rolled (18,400 -> 13,400 instructions for the three counts),
+// taking one of the four rounds of 32 candidates).  The kernel waited on
+// instruction fetch, branches and the conversion pipe,
+// not on memory, so: loops are left rolled,
 // sort keys are 32 bits with the reference's partial network on registers and shuffles, the
 // mismatch is one matching over popcounts of the overlaps, texel partitions come two bits a
 // texel, and sums of truncated texels reuse the truncations.  Measured (B200): 11.6 -> 5.4 ms for
@@ -750,8 +750,7 @@ __device__ __forceinline__ uint32_t bm_quant_weight(const Tabs& tb, const BmQuan
 // and 04, (mode, quant level) for pass05.  The full search takes the first and the step items
 // from the tables, sorted by their inner loop's length, so that a warp's lanes end together; a
 // half-warp per mode, which this replaces, kept 16 of 32 lanes busy (a mode has 4 to 64 weights,
-// 1 to 36 texels a weight and 2 to 12 steps) and spent three instructions in four on the loops
-// around the sums.  The proposal search lists the items of its few modes itself.  The sums'
+// 1 to 36 texels a weight and 2 to 12 steps).  The proposal search lists the items of its few modes itself.  The sums'
 // entries are stored four to a load and, for the sorted items, 32 items side by side; the
 // weights of all modes are packed, which with the steps kept in pass07's buffer takes a 10x8
 // block from 70 to 51 KB of shared memory and from three to four CTAs.  Measured (B200, 128
@@ -1628,7 +1627,9 @@ __global__ void __launch_bounds__(NT, front_min_ctas(NT, DEEP)) k_front(const __
 // 411 / 465 / 567 / 995, 5x4 584 / 651 / 680 / 1110, 5x5 928 / 895 / 893 / 1304, 6x6 2198 / 1616 /
 // 1542 / 1836, 10x8 15259 / 8785 / 6768 / 8017, 12x10 40427 / 21252 / 12438 / 11803, 12x12 74917 /
 // 40147 / 23795 / 15542.  Proposal search's lists of 1024x1024: 4x4 861 / 1060 / 1377, 6x6 712 / 669
-// / 720.  A launch that leaves SMs without a warp is as long as one item: 128 threads then.
+// / 720.  A launch that leaves SMs without a warp is as long as one item: 128 threads then.  (Full searches
+// of 1 to 45 blocks with 256 there instead: 12x12 5 to 8 % less; 12x10 4 to 8 % less, but 4 % more for 32
+// blocks; 10x10 5 % less up to 16 blocks, 4 % more from 32.)
 static int front_nt(int T, bool list, int items) {
     if (items < 148 * 4) return 128;
     if (T <= 20) return 32;

@@ -72,7 +72,7 @@ __host__ __device__ inline uint32_t core_index(uint32_t n, uint32_t k, uint32_t 
 struct Net {
     const uint16_t* w1;   // [256 x k0p]
     const uint16_t* w2;   // [256 x 256]
-    const uint16_t* w3;   // [nout/128][128 x 256]
+    const uint16_t* w3;   // [nout/kChunkN][kChunkN x 256]
     const float* b1;      // [256]
     const float* b2;      // [256]
     const float* b3;      // [nout]
