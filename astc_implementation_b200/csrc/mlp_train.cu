@@ -34,7 +34,8 @@ constexpr int kRowA = kBM + 4, kRowB = kBN + 4;  // floats of a K row in shared 
 constexpr int kStageFloats = kBK * (kRowA + kRowB);
 
 // Loads a `rows` x kBK slice (rows along the stride s_r, K along s_k) of a matrix of n_r x n_k, zeros
-// outside, into registers: kind 0 four floats along K, 1 four along the rows, 2 single floats.
+// outside, into registers: kind 0 four floats along K, 1 four along the rows, 2 and 3 single floats,
+// consecutive threads on consecutive rows or on consecutive fours of a row.
 template <int ROWS>
 struct Slice {
     static constexpr int kVec = ROWS * kBK / 4 / kGemmThreads;
@@ -44,10 +45,10 @@ struct Slice {
         for (int j = 0; j < kVec; j++) {
             const int e = threadIdx.x + j * kGemmThreads;
             // along K: consecutive threads on consecutive fours of a row; else on consecutive rows
-            const int r = r0 + (kind == 1 ? (e % (ROWS / 4)) * 4 : kind == 0 ? e / (kBK / 4) : e % ROWS);
-            const int k = k0 + (kind == 1 ? e / (ROWS / 4) : kind == 0 ? (e % (kBK / 4)) * 4 : (e / ROWS) * 4);
+            const int r = r0 + (kind == 1 ? (e % (ROWS / 4)) * 4 : kind != 2 ? e / (kBK / 4) : e % ROWS);
+            const int k = k0 + (kind == 1 ? e / (ROWS / 4) : kind != 2 ? (e % (kBK / 4)) * 4 : (e / ROWS) * 4);
             float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (kind == 2) {
+            if (kind >= 2) {
                 if (r < n_r) {
                     if (k < n_k) x.x = p[r * s_r + k * s_k];
                     if (k + 1 < n_k) x.y = p[r * s_r + (k + 1) * s_k];
@@ -67,7 +68,7 @@ struct Slice {
             if (kind == 1) {
                 *reinterpret_cast<float4*>(sm + (e / (ROWS / 4)) * row_floats + (e % (ROWS / 4)) * 4) = v[j];
             } else {
-                const int r = kind == 0 ? e / (kBK / 4) : e % ROWS, k = kind == 0 ? (e % (kBK / 4)) * 4 : (e / ROWS) * 4;
+                const int r = kind != 2 ? e / (kBK / 4) : e % ROWS, k = kind != 2 ? (e % (kBK / 4)) * 4 : (e / ROWS) * 4;
                 sm[k * row_floats + r] = v[j].x;
                 sm[(k + 1) * row_floats + r] = v[j].y;
                 sm[(k + 2) * row_floats + r] = v[j].z;
@@ -275,10 +276,10 @@ int astcb200_train_gemm(const float* A, const float* B, float* C, int M, int N, 
     if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return ASTCB200_BAD_ARG;
     // four floats at a time along a stride of 1, when every row starts on 16 bytes and the extent is a multiple of four
     auto kind = [](const float* p, int n_r, int n_k, int64_t s_r, int64_t s_k) {
-        if ((uintptr_t)p & 15) return 2;
-        if (s_k == 1 && s_r % 4 == 0 && n_k % 4 == 0) return 0;
-        if (s_r == 1 && s_k % 4 == 0 && n_r % 4 == 0) return 1;
-        return 2;
+        const bool aligned = ((uintptr_t)p & 15) == 0;
+        if (aligned && s_k == 1 && s_r % 4 == 0 && n_k % 4 == 0) return 0;
+        if (aligned && s_r == 1 && s_k % 4 == 0 && n_r % 4 == 0) return 1;
+        return s_k == 1 ? 3 : 2;
     };
     const int kind_a = kind(A, M, K, sa_i, sa_l), kind_b = kind(B, N, K, sb_j, sb_l);
     const long long tiles = (long long)((N + kBN - 1) / kBN) * ((M + kBM - 1) / kBM);
@@ -294,7 +295,7 @@ int astcb200_train_gemm(const float* A, const float* B, float* C, int M, int N, 
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = (unsigned)split; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = split > 1 ? 1 : 0;
     if (cudaLaunchKernelEx(&cfg, k_gemm, A, B, C, M, N, K, (long long)sa_i, (long long)sa_l, (long long)sb_l, (long long)sb_j, kind_a, kind_b,
                            bias, relu, accumulate) != cudaSuccess) {
         cudaGetLastError();
