@@ -3,7 +3,8 @@
 //
 //   k_gemm      C = A . B (+ bias) (ReLU), A and B addressed by arbitrary row and
 //               column strides, so forward (X W^T), input gradient (dY W) and
-//               weight gradient (dY^T X) are the same kernel.
+//               weight gradient (dY^T X) are the same kernel; k_gemm_short for
+//               products of few terms.
 //   k_xent      softmax cross-entropy of the partition head (all valid
 //               partitionings and the single-partition class) plus that of the
 //               block-mode head of the label's partition count; writes dZ
@@ -29,7 +30,7 @@ namespace cg = cooperative_groups;
 // depends on the shape only.  Measured (B200, one step at 4x4, 2,048 rows): one 64x64 tile a CTA
 // without a split and 4x4 outputs a thread 743 us, this with k_colsum below 189 us.
 constexpr int kBM = 128, kBN = 64, kBK = 16, kGemmThreads = 128;
-constexpr int kMaxSplit = 8;
+constexpr int kMaxSplit = 8, kSplitK = 2 * 4 * kBK;  // terms from which a sum is split
 constexpr int kRowA = kBM + 4, kRowB = kBN + 4;  // floats of a K row in shared memory
 constexpr int kStageFloats = kBK * (kRowA + kRowB);
 
@@ -167,6 +168,61 @@ __global__ void __launch_bounds__(kGemmThreads, 3) k_gemm(const float* __restric
     cl.sync();  // the others may still be reading this CTA's tile
 }
 
+// Products of few terms (short_product), whose sums k_gemm would not split, in the same order: 64x64 tiles of 4x4 outputs a
+// thread, four times as many threads on an output as k_gemm's, and little code.  They are bound by the call's latency
+// or, with one slice of terms, by writing C.  Measured (B200, k_gemm / this, along-K operands): 16x16x16 11.4 / 8.3 us,
+// 33x4097x7 12.2 / 8.3, 8192x4096x16 76 / 67; 256x256x64 15.6 / 12.5, 2048x256x64 15.7 / 14.2, 20000x8x64 (313 tiles) 18.0 /
+// 16.5, 2048x700x127 (352) 34 / 28; 2048x1408x32 (704) 18.1 / 18.8, x64 23.8 / 28.5.
+constexpr int kShortTile = 64, kShortTiles = 3 * 148;
+__host__ inline long long short_tiles(int M, int N) {
+    return (long long)((N + kShortTile - 1) / kShortTile) * ((M + kShortTile - 1) / kShortTile);
+}
+__host__ inline bool short_product(int M, int N, int K) { return K <= kBK || (K < kSplitK && short_tiles(M, N) <= kShortTiles); }
+__global__ void __launch_bounds__(256) k_gemm_short(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
+                                                    int M, int N, int K, long long sa_i, long long sa_l, long long sb_l, long long sb_j,
+                                                    const float* __restrict__ bias, int relu, int accumulate) {
+    __shared__ __align__(16) float as[kBK][kShortTile + 4], bs[kBK][kShortTile + 4];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int tiles_n = (N + kShortTile - 1) / kShortTile;
+    const int i0 = (int)(blockIdx.x / (unsigned)tiles_n) * kShortTile, j0 = (int)(blockIdx.x % (unsigned)tiles_n) * kShortTile;
+    const bool a_k = sa_l == 1, b_k = sb_l == 1;  // consecutive threads along K, or along the rows
+    float acc[4][4] = {};
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += kBK) {
+        if (k0 > 0) __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kBK * kShortTile / 256; j++) {
+            const int e = tid + 256 * j, l0 = e / kShortTile, r0 = e % kShortTile, l1 = e % kBK, r1 = e / kBK;
+            const int la = a_k ? l1 : l0, ra = a_k ? r1 : r0, lb = b_k ? l1 : l0, rb = b_k ? r1 : r0;
+            as[la][ra] = k0 + la < K && i0 + ra < M ? A[(i0 + ra) * sa_i + (k0 + la) * sa_l] : 0.0f;
+            bs[lb][rb] = k0 + lb < K && j0 + rb < N ? B[(k0 + lb) * sb_l + (j0 + rb) * sb_j] : 0.0f;
+        }
+        __syncthreads();
+        const int ln = min(kBK, K - k0);
+#pragma unroll 2
+        for (int l = 0; l < ln; l++) {
+            const float4 a4 = *reinterpret_cast<const float4*>(&as[l][4 * ty]), b4 = *reinterpret_cast<const float4*>(&bs[l][4 * tx]);
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int gi = i0 + 4 * ty + r, gj = j0 + 4 * tx + c;
+            if (gi >= M || gj >= N) continue;
+            float v = acc[r][c];
+            if (accumulate) v += C[(size_t)gi * N + gj];
+            if (bias) v += bias[gj];
+            if (relu) v = fmaxf(v, 0.0f);
+            C[(size_t)gi * N + gj] = v;
+        }
+}
+
 struct XentShape {
     int nout, nbm, head_stride, batch;
     mlp::Shape cls;  // class plan (p1, part_base, head_base)
@@ -274,6 +330,12 @@ extern "C" {
 int astcb200_train_gemm(const float* A, const float* B, float* C, int M, int N, int K, int64_t sa_i, int64_t sa_l, int64_t sb_l,
                         int64_t sb_j, const float* bias, int relu, int accumulate, void* stream) {
     if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return ASTCB200_BAD_ARG;
+    if (short_product(M, N, K)) {
+        const long long tiles = short_tiles(M, N);
+        if (tiles > 0x7FFFFFFFll) return ASTCB200_CUDA_ERROR;
+        k_gemm_short<<<(unsigned)tiles, 256, 0, (cudaStream_t)stream>>>(A, B, C, M, N, K, sa_i, sa_l, sb_l, sb_j, bias, relu, accumulate);
+        return launch_status();
+    }
     // four floats at a time along a stride of 1, when every row starts on 16 bytes and the extent is a multiple of four
     auto kind = [](const float* p, int n_r, int n_k, int64_t s_r, int64_t s_k) {
         const bool aligned = ((uintptr_t)p & 15) == 0;

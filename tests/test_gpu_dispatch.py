@@ -277,3 +277,12 @@ def test_refinement_tail_takes_what_the_rule_offers(bx, by, blocks_x, blocks_y):
     assert np.array_equal(outs[0], outs[1])
     if few:
         assert taken[0] == taken[1]
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn", "odd stride", "unaligned"])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 16), (65, 63, 15), (2000, 900, 16),          # one slice, any number of tiles
+                                   (33, 70, 17), (64, 64, 127), (2368, 768, 48),       # up to 444 tiles of 64x64
+                                   (2369, 768, 48), (64, 64, 128), (200, 130, 1)])    # 456 tiles; split sums
+def test_training_gemm_of_few_terms(M, N, K, layout):
+    """Both sides of the small tiles' range, read along K and along the rows."""
+    test_training_gemm_tiles_splits_and_layouts(M, N, K, layout)
