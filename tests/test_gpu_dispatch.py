@@ -286,3 +286,20 @@ def test_refinement_tail_takes_what_the_rule_offers(bx, by, blocks_x, blocks_y):
 def test_training_gemm_of_few_terms(M, N, K, layout):
     """Both sides of the small tiles' range, read along K and along the rows."""
     test_training_gemm_tiles_splits_and_layouts(M, N, K, layout)
+
+
+@pytest.mark.parametrize("rows,cols", [(32, 4095), (32, 4096), (33, 4096), (1, 5000), (33, 32768), (128, 32769), (129, 32768)])
+def test_training_column_sums_of_many_columns(rows, cols):
+    """One thread a column or 32: the same partial sums, added in the same order."""
+    import ctypes
+    import torch
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(rows))
+    lib, s = ab.load_library(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    d, out, part = x.cuda(), torch.zeros(cols, device="cuda"), torch.zeros(64, device="cuda")
+    ab._check(lib.astcb200_train_colsum(ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(out.data_ptr()), rows, cols, s))
+    few = d[:, -64:].contiguous()  # 64 columns: 32 threads each
+    ab._check(lib.astcb200_train_colsum(ctypes.c_void_p(few.data_ptr()), ctypes.c_void_p(part.data_ptr()), rows, 64, s))
+    torch.cuda.synchronize()
+    assert bool((out[-64:] == part).all())
+    bound = rows * 2.0 ** -24 * x.abs().double().sum(0) + 1e-30
+    assert bool(((out.cpu().double() - x.double().sum(0)).abs() <= bound).all())
